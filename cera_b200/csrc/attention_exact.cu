@@ -10,17 +10,21 @@
 // position order.  The last step is a serial chain per output element that an online-softmax
 // (flash-decode) kernel cannot reproduce, so the work is split differently here:
 //
-//   scores kernel : one half-warp per (position, query head): its sixteen lanes are the sixteen chains, and
-//                   four shuffle steps add them in the reference's order.  Scores go to a workspace
-//                   [n_heads][ld].
-//   values kernel : one CTA per (KV head, 32 output dims).  Its warps first turn the scores of the
-//                   group's heads into probabilities (maximum, ggml_expf, f64 sum by a fixed tree,
-//                   scaling; the heads side by side), while all threads stage the V slice through
-//                   shared memory with asynchronous copies, in tiles of 256 positions, two tiles
-//                   ahead (a context of up to 768 positions is requested whole before the softmax
-//                   starts); then one warp per head - a lane per output dim - walks the positions
-//                   in order with one FMA per position, and finally emits the f32 outputs and their
-//                   Q8_0 form (a 32-dim slice of a head is one Q8_0 block: one warp).
+//   scores  : sixteen positions per warp, two lanes per position: lane bit 0 picks the accumulator (a), a lane holds its
+//             eight chains, so a K row arrives in 128-bit loads and is read once for all heads of the group; five shuffles
+//             add the chains in the reference's order.
+//   up to 1024 positions, ONE launch (attn_fused_exact_kernel): the hd / 32 CTAs of a KV head are a cluster, each scores a
+//             share of the positions into the tables of all, then runs the softmax and the value chains of its 32 dims.
+//   beyond  : attn_scores_exact_kernel writes scores and the maximum of every sixteen; attn_exp_exact_kernel turns them into
+//             exponentials in place and leaves one f64 sum per 1024 positions; attn_chain_exact_kernel multiplies by
+//             1 / sum and walks the chains, one warp per (head, 32 dims), fed by copying warps through a ring.
+//
+// The chain of an output element is one dependent FMA per position, 4 cycles: 2.1 ns per position at 1.96 GHz bounds a long
+// context (34 us at 16384).  What a chain warp adds to that is the issue of its loads, which do not overlap the FMAs they stand
+// between, and the wait for them when other warps keep the load / store unit busy: V therefore arrives by TMA, probabilities
+// are multiplied by 1 / sum beforehand and fetched four at a time, and operands are loaded 32 positions ahead of their FMAs.  Alone
+// on an SM: 6.5 cycles per position (f32; f16 6.7); eight positions ahead it is 10.8 cycles in either form, and V transposed
+// to [dim][position] by copying warps - 5.1 alone - costs 9 to 13 beside those warps.
 //
 // The f64 sum of the exponentials is a tree, the reference's a left-to-right loop: the two can differ
 // in the last bits of the f64 sum, which survive the narrowing to f32 only in about one softmax in
@@ -33,6 +37,8 @@
 
 #include "act.cuh"
 #include "ops.h"
+#include "tensor_map.h"
+#include "tma.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -40,259 +46,251 @@ namespace cera {
 
 namespace {
 
-constexpr int AX_VTHREADS = 512;   // threads of the values and fused kernels
+constexpr int AX_VTHREADS = 512;   // threads of the fused kernel
 
-// One HALF-WARP per (position, query head): its sixteen lanes are the reference's sixteen FMA chains (accumulator a,
-// lane L) - lane c = 8a + L multiplies elements 16j + c of the head for j = 0, 1, ... - and four xor-shuffle steps add
-// them in the reference's order (the two accumulators, then hsum256: lanes L and L+4, then (0,2) and (1,3), then the
-// two).  The two half-warps of a warp take two heads of the same position, so they read the same K row; the heads of
-// a group iterate over the warp pairs.  blockDim.x = 256 (eight warps = eight positions per pass); dynamic shared
-// memory: G * hd floats of q.
-constexpr int AX_SWARPS = 8;
-template <int HD>  // head size known at compile time (0: read it from the argument)
-__global__ void __launch_bounds__(AX_SWARPS * 32)
-attn_scores_exact_kernel(const float *__restrict__ q, const void *__restrict__ kc, int kv_f16, uint32_t seq_len,
-                         const uint32_t *__restrict__ seq_dev, uint32_t n_kv, uint32_t G, uint32_t hd_arg, float scale,
-                         float *__restrict__ ws, uint32_t ld) {
-    extern __shared__ __align__(16) float ax_q[];
-    const uint32_t hd = HD ? (uint32_t)HD : hd_arg;
-    pdl_trigger();
-    pdl_wait();
-    const uint32_t seq = seq_dev ? *seq_dev : seq_len;
-    const uint32_t kvh = blockIdx.y;
-    for (uint32_t i = threadIdx.x; i < G * hd; i += blockDim.x) ax_q[i] = q[(size_t)kvh * G * hd + i];
-    __syncthreads();
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = lane & 15, hsel = lane >> 4;
-    const size_t kv_dim = (size_t)n_kv * hd;
-    const uint32_t nv = hd / 8, a = c >> 3, steps = (nv + 1) / 2;
-    for (uint32_t t = blockIdx.x * AX_SWARPS + warp; t < seq; t += gridDim.x * AX_SWARPS) {
-        const size_t row = (size_t)t * kv_dim + (size_t)kvh * hd;
-        // this lane's elements of the K row: 16j + c while chunk 2j + a exists (at most 16 of them: hd <= 256)
-        float kv[16];
+__device__ unsigned int g_ax_status = 0;  // bit 0: a chain warp's wait ran out, bit 1: a copying warp's
+
+// This lane's half (accumulator a) of one K row: chunks 2j + a of eight elements, j = 0 .. HD/16 - 1.  `vec`: the cache starts
+// on a 16-byte boundary (every row and chunk then does).
+template <int HD, bool F16>
+__device__ __forceinline__ void ax_load_k(float (&k)[HD / 16][8], const void *__restrict__ kc, size_t row, uint32_t a, bool vec) {
+    const size_t e0 = row + 8 * a;
+    if (vec) {
+        if constexpr (F16) {
+            uint4 raw[HD / 16];
 #pragma unroll
-        for (uint32_t j = 0; j < 16; ++j) {
-            kv[j] = 0.0f;
-            if (j < steps && 2 * j + a < nv) {
-                const size_t e = row + 16 * j + c;
-                kv[j] = kv_f16 ? __half2float(__ldg(reinterpret_cast<const __half *>(kc) + e)) : __ldg(reinterpret_cast<const float *>(kc) + e);
+            for (int j = 0; j < HD / 16; ++j) raw[j] = __ldg(reinterpret_cast<const uint4 *>(reinterpret_cast<const __half *>(kc) + e0 + 16 * j));
+#pragma unroll
+            for (int j = 0; j < HD / 16; ++j) {
+                const uint32_t w[4] = {raw[j].x, raw[j].y, raw[j].z, raw[j].w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    k[j][2 * i] = h2f((uint16_t)(w[i] & 0xFFFF));
+                    k[j][2 * i + 1] = h2f((uint16_t)(w[i] >> 16));
+                }
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < HD / 16; ++j) {
+                const float4 *src = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(kc) + e0 + 16 * j);
+                const float4 lo = __ldg(src), hi = __ldg(src + 1);
+                k[j][0] = lo.x, k[j][1] = lo.y, k[j][2] = lo.z, k[j][3] = lo.w;
+                k[j][4] = hi.x, k[j][5] = hi.y, k[j][6] = hi.z, k[j][7] = hi.w;
             }
         }
-        for (uint32_t h0 = 0; h0 < G; h0 += 2) {
-            const uint32_t h = h0 + hsel;
-            const bool live = h < G;
-            const float *qh = ax_q + (live ? h : 0) * hd;
-            float acc = 0.0f;
+        return;
+    }
 #pragma unroll
-            for (uint32_t j = 0; j < 16; ++j)
-                if (j < steps && 2 * j + a < nv) acc = fmaf(qh[16 * j + c], kv[j], acc);
-            // accumulators 0 and 1 of the same lane L, then hsum256
-            acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 8));
-            acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 4));
-            acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 2));
-            acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 1));
-            if (live && c == 0) ws[(size_t)(kvh * G + h) * ld + t] = __fmul_rn(acc, scale);
+    for (int j = 0; j < HD / 16; ++j)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            k[j][i] = F16 ? __half2float(__ldg(reinterpret_cast<const __half *>(kc) + e0 + 16 * j + i)) : __ldg(reinterpret_cast<const float *>(kc) + e0 + 16 * j + i);
+}
+
+// Scaled score of one head (qh: its query in shared memory) against the row whose halves this lane and lane ^ X hold; both
+// lanes return it.  Chain (a, i) multiplies elements 16j + 8a + i in the order of j; then the two accumulators are added lane by
+// lane and reduced as hsum256 does: i and i + 4, then (0,2) and (1,3), then the two.
+template <int HD, int X>
+__device__ __forceinline__ float ax_score(const float *qh, const float (&k)[HD / 16][8], uint32_t a, float scale) {
+    float acc[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = 0.0f;
+#pragma unroll
+    for (int j = 0; j < HD / 16; ++j) {
+        const float4 lo = *reinterpret_cast<const float4 *>(qh + 16 * j + 8 * a), hi = *reinterpret_cast<const float4 *>(qh + 16 * j + 8 * a + 4);
+        acc[0] = fmaf(lo.x, k[j][0], acc[0]);
+        acc[1] = fmaf(lo.y, k[j][1], acc[1]);
+        acc[2] = fmaf(lo.z, k[j][2], acc[2]);
+        acc[3] = fmaf(lo.w, k[j][3], acc[3]);
+        acc[4] = fmaf(hi.x, k[j][4], acc[4]);
+        acc[5] = fmaf(hi.y, k[j][5], acc[5]);
+        acc[6] = fmaf(hi.z, k[j][6], acc[6]);
+        acc[7] = fmaf(hi.w, k[j][7], acc[7]);
+    }
+    float r[4];  // both accumulators' lanes a, a + 2, a + 4, a + 6
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        const float keep = a ? acc[2 * m + 1] : acc[2 * m], send = a ? acc[2 * m] : acc[2 * m + 1];
+        r[m] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, X));
+    }
+    const float u = __fadd_rn(__fadd_rn(r[0], r[2]), __fadd_rn(r[1], r[3]));
+    return __fmul_rn(__fadd_rn(u, __shfl_xor_sync(0xffffffffu, u, X)), scale);
+}
+
+// Scores of all heads of one KV head, and the maximum of every sixteen positions.  grid (any, n_kv), AX_SWARPS warps;
+// dynamic shared memory: G * HD floats of q.  ws: scores [n_heads][ld]; aux: [n_heads][ld], its first ld / 16 entries per head
+// receive the maxima.  16384 f16 positions, 32 heads of 128 in groups of 4: 33.5 MB of keys in 15.7 us (36 us with a half-warp
+// per position and head, whose 2-byte loads left 8 KB in flight per SM).
+constexpr int AX_SWARPS = 8;
+template <int HD, bool F16>
+__global__ void __launch_bounds__(AX_SWARPS * 32)
+attn_scores_exact_kernel(const float *__restrict__ q, const void *__restrict__ kc, int vec, uint32_t seq_len,
+                         const uint32_t *__restrict__ seq_dev, uint32_t n_kv, uint32_t G, float scale, float *__restrict__ ws,
+                         float *__restrict__ aux, uint32_t ld) {
+    extern __shared__ __align__(16) float ax_q[];
+    pdl_trigger();
+    pdl_wait();
+    const uint32_t seq = seq_dev ? min(*seq_dev, ld) : seq_len;
+    const uint32_t kvh = blockIdx.y;
+    for (uint32_t i = threadIdx.x; i < G * HD; i += blockDim.x) ax_q[i] = q[(size_t)kvh * G * HD + i];
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, a = lane & 1;
+    const size_t kv_dim = (size_t)n_kv * HD;
+    const uint32_t tiles = (seq + 15) / 16;
+    for (uint32_t tile = blockIdx.x * AX_SWARPS + warp; tile < tiles; tile += gridDim.x * AX_SWARPS) {
+        const uint32_t t = tile * 16 + (lane >> 1);
+        float k[HD / 16][8];
+        ax_load_k<HD, F16>(k, kc, (size_t)min(t, seq - 1) * kv_dim + (size_t)kvh * HD, a, vec);
+        for (uint32_t h = 0; h < G; ++h) {
+            const float s = ax_score<HD, 1>(ax_q + h * HD, k, a, scale);
+            const size_t row = (size_t)(kvh * G + h) * ld;
+            if (a == 0 && t < seq) ws[row + t] = s;
+            float mx = t < seq ? fmaxf(-INFINITY, s) : -INFINITY;  // f32::max fold: NaN scores are ignored
+#pragma unroll
+            for (int o = 16; o > 1; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            if (lane == 0) aux[row + tile] = mx;
         }
     }
 }
 
+// Exponentials of one head's scores, in place, and their f64 sum per AX_EPOS positions (thread-strided partials, xor shuffles,
+// warps in index order) behind the maxima in aux.  grid (any, n_heads), AX_ETHREADS threads.
+constexpr uint32_t AX_EPOS = 1024, AX_ETHREADS = 256;
+__device__ __host__ __forceinline__ uint32_t ax_sums_at(uint32_t ld) { return ld / 16; }  // 2 * ceil(ld / 1024) words follow: within ld, a multiple of 64
+__global__ void __launch_bounds__(AX_ETHREADS)
+attn_exp_exact_kernel(float *__restrict__ ws, float *__restrict__ aux, uint32_t ld, uint32_t seq_len, const uint32_t *__restrict__ seq_dev) {
+    __shared__ float red_f[AX_ETHREADS / 32];
+    __shared__ double red_d[AX_ETHREADS / 32];
+    pdl_trigger();
+    pdl_wait();
+    const uint32_t seq = seq_dev ? min(*seq_dev, ld) : seq_len;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (blockIdx.x * AX_EPOS >= seq) return;
+    float *row = ws + (size_t)blockIdx.y * ld;
+    float *maxima = aux + (size_t)blockIdx.y * ld;
+    float mx = -INFINITY;
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < (seq + 15) / 16; i += AX_ETHREADS) mx = fmaxf(mx, maxima[i]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) red_f[warp] = mx;
+    __syncthreads();
+    mx = red_f[0];
+#pragma unroll
+    for (uint32_t w = 1; w < AX_ETHREADS / 32; ++w) mx = fmaxf(mx, red_f[w]);
+    for (uint32_t part = blockIdx.x; part * AX_EPOS < seq; part += gridDim.x) {
+        double sum = 0.0;
+#pragma unroll
+        for (uint32_t i = 0; i < AX_EPOS / AX_ETHREADS; ++i) {
+            const uint32_t t = part * AX_EPOS + i * AX_ETHREADS + threadIdx.x;
+            if (t < seq) {
+                const float e = ggml_expf(__fsub_rn(row[t], mx));
+                row[t] = e;
+                sum += (double)e;
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) red_d[warp] = sum;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (uint32_t w = 1; w < AX_ETHREADS / 32; ++w) sum += red_d[w];
+            // two words: the workspace is only known to be aligned to floats
+            float *dst = maxima + ax_sums_at(ld) + 2 * part;
+            dst[0] = __int_as_float(__double2hiint(sum));
+            dst[1] = __int_as_float(__double2loint(sum));
+        }
+        __syncthreads();
+    }
+}
+
 __device__ __forceinline__ void ax_cp16(void *smem, const void *gmem) {
-    const uint32_t a = (uint32_t)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(gmem) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tma::smem_u32(smem)), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void ax_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void ax_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-constexpr int AX_VT = 256;     // positions per staged V tile
-constexpr int AX_VSTAGES = 3;  // tiles in the ring (two in flight while one is walked)
-constexpr int AX_VTHREADS_C = AX_VTHREADS;
-
-// AX_VT positions (or fewer) of one lane's chain: out = fma(p[t], V[t][d], out) in position order.  `base`: the tile,
-// one row of 32 dims per position; pp: the head's probabilities from this tile's first position on, 16-byte aligned.
+// cnt positions of one lane's chain: out = fma(p, V, out) in position order.  va: the lane's element of the first of cnt rows of 32
+// dims; pa: the head's probabilities, 16-byte aligned (shared-memory addresses).  The loads are volatile so that the compiler
+// leaves them 32 positions ahead of their FMAs.
 template <bool F16>
-__device__ __forceinline__ float ax_chain_tile(const char *base, const float *__restrict__ pp, uint32_t cnt, uint32_t d, float inv, float acc) {
-    auto v_at = [&](uint32_t i) -> float {
-        if (F16) return __half2float(*reinterpret_cast<const __half *>(base + (size_t)i * 64 + d * 2));
-        return *reinterpret_cast<const float *>(base + (size_t)i * 128 + d * 4);
+__device__ __forceinline__ float ax_chain(uint32_t va, uint32_t pa, uint32_t cnt, float acc) {
+    constexpr int R = 8, ROW = F16 ? 64 : 128;  // quads of positions in registers
+    auto ld_v = [](uint32_t &r, uint32_t a) {
+        if constexpr (F16) asm volatile("ld.shared.u16 %0, [%1];" : "=r"(r) : "r"(a) : "memory");
+        else asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(a) : "memory");
     };
-    uint32_t i = 0;
-    // eight positions per step (two 128-bit loads of probabilities, eight values), fetched one step ahead of their FMAs:
-    // the chain is a dependent FMA per position, the loads must never be what it waits for
-    if (cnt >= 8) {
-        float4 pa = *reinterpret_cast<const float4 *>(pp), pb = *reinterpret_cast<const float4 *>(pp + 4);
-        float v[8];
+    auto ld_p = [](float4 &r, uint32_t a) {
+        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "r"(a) : "memory");
+    };
+    auto val = [](uint32_t r) -> float {
+        if constexpr (F16) return h2f((uint16_t)r);
+        else return __uint_as_float(r);
+    };
+    const uint32_t full = cnt / (4 * R);
+    if (full) {
+        uint32_t v[R][4];
+        float4 p[R];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = v_at(j);
-        for (; i + 16 <= cnt; i += 8) {
-            const float4 na = *reinterpret_cast<const float4 *>(pp + i + 8), nb = *reinterpret_cast<const float4 *>(pp + i + 12);
-            float nv[8];
+        for (int i = 0; i < R; ++i) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) nv[j] = v_at(i + 8 + j);
-            acc = fmaf(__fmul_rn(pa.x, inv), v[0], acc);
-            acc = fmaf(__fmul_rn(pa.y, inv), v[1], acc);
-            acc = fmaf(__fmul_rn(pa.z, inv), v[2], acc);
-            acc = fmaf(__fmul_rn(pa.w, inv), v[3], acc);
-            acc = fmaf(__fmul_rn(pb.x, inv), v[4], acc);
-            acc = fmaf(__fmul_rn(pb.y, inv), v[5], acc);
-            acc = fmaf(__fmul_rn(pb.z, inv), v[6], acc);
-            acc = fmaf(__fmul_rn(pb.w, inv), v[7], acc);
-            pa = na;
-            pb = nb;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = nv[j];
+            for (int j = 0; j < 4; ++j) ld_v(v[i][j], va + (4 * i + j) * ROW);
+            ld_p(p[i], pa + 16 * i);
         }
-        acc = fmaf(__fmul_rn(pa.x, inv), v[0], acc);
-        acc = fmaf(__fmul_rn(pa.y, inv), v[1], acc);
-        acc = fmaf(__fmul_rn(pa.z, inv), v[2], acc);
-        acc = fmaf(__fmul_rn(pa.w, inv), v[3], acc);
-        acc = fmaf(__fmul_rn(pb.x, inv), v[4], acc);
-        acc = fmaf(__fmul_rn(pb.y, inv), v[5], acc);
-        acc = fmaf(__fmul_rn(pb.z, inv), v[6], acc);
-        acc = fmaf(__fmul_rn(pb.w, inv), v[7], acc);
-        i += 8;
+#pragma unroll 1
+        for (uint32_t b = 1; b < full; ++b) {
+            va += 4 * R * ROW;
+            pa += 16 * R;
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                acc = fmaf(p[i].x, val(v[i][0]), acc);
+                ld_v(v[i][0], va + (4 * i) * ROW);
+                acc = fmaf(p[i].y, val(v[i][1]), acc);
+                ld_v(v[i][1], va + (4 * i + 1) * ROW);
+                acc = fmaf(p[i].z, val(v[i][2]), acc);
+                ld_v(v[i][2], va + (4 * i + 2) * ROW);
+                acc = fmaf(p[i].w, val(v[i][3]), acc);
+                ld_v(v[i][3], va + (4 * i + 3) * ROW);
+                ld_p(p[i], pa + 16 * i);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            acc = fmaf(p[i].x, val(v[i][0]), acc);
+            acc = fmaf(p[i].y, val(v[i][1]), acc);
+            acc = fmaf(p[i].z, val(v[i][2]), acc);
+            acc = fmaf(p[i].w, val(v[i][3]), acc);
+        }
+        va += 4 * R * ROW;
+        pa += 16 * R;
     }
-    for (; i < cnt; ++i) acc = fmaf(__fmul_rn(pp[i], inv), v_at(i), acc);
+    const uint32_t rest = cnt % (4 * R);
+#pragma unroll 1
+    for (uint32_t i = 0; i < rest / 4; ++i) {
+        uint32_t v[4];
+        float4 p;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ld_v(v[j], va + (4 * i + j) * ROW);
+        ld_p(p, pa + 16 * i);
+        acc = fmaf(p.x, val(v[0]), acc);
+        acc = fmaf(p.y, val(v[1]), acc);
+        acc = fmaf(p.z, val(v[2]), acc);
+        acc = fmaf(p.w, val(v[3]), acc);
+    }
+#pragma unroll 1
+    for (uint32_t i = rest & ~3u; i < rest; ++i) {
+        uint32_t v, p;
+        ld_v(v, va + i * ROW);
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(p) : "r"(pa + 4 * i) : "memory");
+        acc = fmaf(__uint_as_float(p), val(v), acc);
+    }
     return acc;
 }
 
-// Requests V tile `tile` (AX_VT positions x 32 dims of one KV head) into its ring slot; every thread commits one group
-// per call, empty or not, so the wait counts stay uniform.
-__device__ __forceinline__ void ax_stage_tile(uint32_t tile, uint32_t n_tiles, uint32_t seq, uint32_t per_pos, float *vt, const void *vc,
-                                              size_t kv_dim, size_t col0, int kv_f16, int tid) {
-    if (tile < n_tiles) {
-        char *dst = reinterpret_cast<char *>(vt + (size_t)(tile % AX_VSTAGES) * AX_VT * 32);
-        const uint32_t t0 = tile * AX_VT, cnt = min((uint32_t)AX_VT, seq - t0) * per_pos;
-        const uint32_t sh = kv_f16 ? 2 : 3;  // per_pos = 4 or 8 pieces of 16 bytes
-        const char *src0 = reinterpret_cast<const char *>(vc) + ((size_t)t0 * kv_dim + col0) * (kv_f16 ? 2 : 4);
-        const size_t row_bytes = kv_dim * (kv_f16 ? 2 : 4);
-        for (uint32_t i = tid; i < cnt; i += AX_VTHREADS_C) {
-            const uint32_t pl = i >> sh, pc = i & (per_pos - 1);
-            ax_cp16(dst + (size_t)i * 16, src0 + (size_t)pl * row_bytes + pc * 16);
-        }
-    }
-    ax_commit();
-}
-
-// grid (hd / 32, n_kv), AX_VTHREADS threads.  ws: scores [n_heads][ld]; pw: probabilities [n_heads][ld] in global
-// memory, used when the positions do not fit shared memory (every CTA of a KV head writes the same values there).
-// Dynamic shared memory: AX_VSTAGES V tiles of AX_VT x 32 floats, then smem_pos * G floats of probabilities.
-// Softmax of the group's heads, the position-ordered value chains of one 32-dim slice, and the outputs (f32 + Q8_0).
-// The first V tiles have been requested by the caller.  scores_in_smem: ax_p already holds the scores (the fused
-// kernel); otherwise they are read from ws.
-__device__ __forceinline__ void ax_softmax_chain_emit(const float *__restrict__ ws, float *__restrict__ pw, uint32_t ld, const void *__restrict__ vc,
-                                                      int kv_f16, uint32_t seq, uint32_t n_kv, uint32_t G, uint32_t hd, uint32_t smem_pos,
-                                                      uint32_t kvh, uint32_t d0, float *vt, float *ax_p, double *red_d, float *red_f, float *inv_h,
-                                                      bool scores_in_smem, float *__restrict__ out, float *scales, int8_t *quants,
-                                                      int16_t *sums, const TpHook &tp) {
-    const uint32_t pstride = smem_pos + 4;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const size_t kv_dim = (size_t)n_kv * hd;
-    const bool in_smem = seq <= smem_pos;
-    const uint32_t n_tiles = (seq + AX_VT - 1) / AX_VT;
-    const uint32_t per_pos = kv_f16 ? 4 : 8;  // 16-byte pieces per position
-
-    // ---- probabilities of the group's heads.  Head h is handled by warps [h * nwh, (h + 1) * nwh).
-    const uint32_t nwh = (AX_VTHREADS / 32) / G, h_mine = warp / nwh, wl = warp % nwh;  // warps past G * nwh idle here
-    const bool has_head = h_mine < G;
-    const uint32_t hth = nwh * 32, hti = wl * 32 + lane;  // threads of my head, my index among them
-    const float *s_row = ws + (size_t)(kvh * G + (has_head ? h_mine : 0)) * ld;
-    float *p_row = pw + (size_t)(kvh * G + (has_head ? h_mine : 0)) * ld;
-    float mx = -INFINITY;
-    if (has_head) {
-#pragma unroll 4
-        for (uint32_t t = hti; t < seq; t += hth) {  // (unrolled: the loads of four steps are in flight together)
-            const float v = scores_in_smem ? ax_p[(size_t)h_mine * pstride + t] : s_row[t];
-            if (in_smem && !scores_in_smem) ax_p[(size_t)h_mine * pstride + t] = v;
-            mx = fmaxf(mx, v);  // f32::max fold: NaN scores are ignored
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) red_f[warp] = mx;
-    __syncthreads();
-    if (has_head) {
-        mx = red_f[h_mine * nwh];
-        for (uint32_t w = 1; w < nwh; ++w) mx = fmaxf(mx, red_f[h_mine * nwh + w]);
-    }
-    // exponentials and their f64 sum (fixed tree: thread-strided partials, xor shuffles, the head's warps in index order)
-    double sum = 0.0;
-    if (has_head) {
-#pragma unroll 4
-        for (uint32_t t = hti; t < seq; t += hth) {
-            const float e = ggml_expf(__fsub_rn(in_smem ? ax_p[(size_t)h_mine * pstride + t] : s_row[t], mx));
-            if (in_smem) ax_p[(size_t)h_mine * pstride + t] = e;
-            else p_row[t] = e;  // every CTA of the KV head stores the same value; the chain multiplies by 1 / sum
-            sum += (double)e;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane == 0) red_d[warp] = sum;
-    __syncthreads();
-    if (has_head) {
-        double tot = red_d[h_mine * nwh];
-        for (uint32_t w = 1; w < nwh; ++w) tot += red_d[h_mine * nwh + w];
-        const float inv = (float)(1.0 / tot);
-        if (wl == 0 && lane == 0) inv_h[h_mine] = inv;
-        if (in_smem) {
-#pragma unroll 4
-            for (uint32_t t = hti; t < seq; t += hth) ax_p[(size_t)h_mine * pstride + t] = __fmul_rn(ax_p[(size_t)h_mine * pstride + t], inv);
-        }
-    }
-    // (the first barrier of the tile loop below also publishes the probabilities)
-    // Probabilities that went through global memory come back tile by tile, by asynchronous copies into a ring beside
-    // the V tiles (a chain that read them with global loads spent its time on their latency): tiles 0-2 as groups of
-    // their own here, later ones in the group of the V tile they belong to.
-    float *pt = ax_p;  // [AX_VSTAGES][G][AX_VT], in place of the (unused) probability table
-    auto stage_p = [&](uint32_t tile) {
-        if (tile < n_tiles) {
-            const uint32_t t0 = tile * AX_VT, pieces = (min((uint32_t)AX_VT, seq - t0) + 3) / 4;
-            float *dst = pt + (size_t)(tile % AX_VSTAGES) * G * AX_VT;
-            for (uint32_t i = tid; i < G * (AX_VT / 4); i += AX_VTHREADS_C) {
-                const uint32_t hh = i / (AX_VT / 4), pc = i % (AX_VT / 4);
-                if (pc < pieces) ax_cp16(dst + (size_t)hh * AX_VT + pc * 4, pw + (size_t)(kvh * G + hh) * ld + t0 + pc * 4);
-            }
-        }
-    };
-    if (!in_smem) {
-        __syncthreads();  // every thread's probabilities are written
-#pragma unroll
-        for (int i = 0; i < AX_VSTAGES; ++i) {
-            stage_p(i);
-            ax_commit();
-        }
-    }
-
-    // ---- out[d] = fma(p[t], V[t][d], out[d]) in position order: warp h walks head h, a lane per output dim
-    const bool chain = (uint32_t)warp < G;
-    const uint32_t h = warp, d = lane;
-    float acc = 0.0f;
-    for (uint32_t tile = 0; tile < n_tiles; ++tile) {
-        // this thread's copies of tile `tile` have landed: tiles 0-2 were committed up front, tile j + 2 in iteration j,
-        // so at most two younger groups (iteration 0) or one (later) may still be in flight
-        if (tile == 0) ax_wait<2>();
-        else ax_wait<1>();
-        __syncthreads();  // everyone's have; and every chain warp is done with the slot restaged below
-        if (tile > 0) {
-            if (!in_smem) stage_p(tile - 1 + AX_VSTAGES);  // joins the commit group of the V tile below
-            ax_stage_tile(tile - 1 + AX_VSTAGES, n_tiles, seq, per_pos, vt, vc, kv_dim, (size_t)kvh * hd + d0, kv_f16, tid);
-        }
-        if (chain) {
-            const uint32_t t0 = tile * AX_VT, cnt = min((uint32_t)AX_VT, seq - t0);
-            const char *base = reinterpret_cast<const char *>(vt + (size_t)(tile % AX_VSTAGES) * AX_VT * 32);
-            // separate instantiations so that shared-memory probabilities are read with shared loads, not generic ones
-            if (in_smem) acc = kv_f16 ? ax_chain_tile<true>(base, ax_p + (size_t)h * pstride + t0, cnt, d, 1.0f, acc)
-                                      : ax_chain_tile<false>(base, ax_p + (size_t)h * pstride + t0, cnt, d, 1.0f, acc);
-            else {
-                const float *pp = pt + (size_t)(tile % AX_VSTAGES) * G * AX_VT + (size_t)h * AX_VT;
-                const float inv = inv_h[h];  // the staged values are the exponentials: p = e * (1 / sum), rounded, as the reference stores it
-                acc = kv_f16 ? ax_chain_tile<true>(base, pp, cnt, d, inv, acc) : ax_chain_tile<false>(base, pp, cnt, d, inv, acc);
-            }
-        }
-    }
-    ax_wait<0>();
-    if (!chain) return;
-    const size_t o = (size_t)(kvh * G + h) * hd + d0 + d;
+// One warp writes the 32 outputs of a head's block: f32 (o: this lane's index) and, if asked for, Q8_0.
+__device__ __forceinline__ void ax_emit(float acc, size_t o, uint32_t d, float *__restrict__ out, float *scales, int8_t *quants, int16_t *sums,
+                                        const TpHook &tp) {
     out[o] = acc;
     if (quants) {
         // Q8_0 of the 32-dim block this warp holds (cera/src/backend/cpu.rs:942-958)
@@ -325,131 +323,294 @@ __device__ __forceinline__ void ax_softmax_chain_emit(const float *__restrict__ 
     }
 }
 
-// grid (hd / 32, n_kv), AX_VTHREADS threads.  ws: scores [n_heads][ld]; pw: probabilities [n_heads][ld] in global
-// memory, used when the positions do not fit shared memory (every CTA of a KV head writes the same values there).
-// Dynamic shared memory: AX_VSTAGES V tiles of AX_VT x 32 floats, then smem_pos * G floats of probabilities.
-__global__ void __launch_bounds__(AX_VTHREADS)
-attn_values_exact_kernel(const float *__restrict__ ws, float *__restrict__ pw, uint32_t ld, const void *__restrict__ vc, int kv_f16,
-                         uint32_t seq_len, const uint32_t *__restrict__ seq_dev, uint32_t n_kv, uint32_t G, uint32_t hd,
-                         uint32_t smem_pos, float *__restrict__ out, float *scales, int8_t *quants, int16_t *sums, const TpHook tp) {
-    extern __shared__ __align__(16) float ax_dyn[];
-    float *vt = ax_dyn;                                  // [AX_VSTAGES][AX_VT][32] (f16 caches use half of each tile)
-    float *ax_p = ax_dyn + AX_VSTAGES * AX_VT * 32;      // [G][smem_pos + 4]: a head's probabilities are contiguous, heads four banks apart
-    __shared__ double red_d[AX_VTHREADS / 32];
-    __shared__ float red_f[AX_VTHREADS / 32];
-    __shared__ float inv_h[8];  // 1 / sum of every head of the group
+// The value chains of a long context.  grid (hd / 32, n_kv, ceil(G / AXC_HEADS)); a CTA has one warp per head of its share, one
+// thread that requests V tiles (AXC_T positions x 32 dims, two TMA boxes) and three warps that prepare the heads' probabilities
+// of every third tile.  Slots of the ring are handed over through mbarriers, every wait bounded.  The positions of a last,
+// incomplete box are copied by the probability warp: a box may not reach past the cache.  Two heads per CTA: one would read
+// every V slice from L2 once per head, four would share one load / store unit among four chains.
+// 16384 f16 positions, 32 heads of 128 in groups of 4: 66 us, and 86 us with the two kernels ahead (218 and 254 us before; f32 61 and 87).
+constexpr int AXC_HEADS = 2, AXC_PWARPS = 3, AXC_T = 512, AXC_BOX = 256;
+constexpr uint32_t AXC_THREADS = (AXC_HEADS + AXC_PWARPS + 1) * 32;
+template <bool F16>
+struct AxChain {
+    static constexpr int STAGES = F16 ? 4 : 3;
+    // a probability warp waits for the slot of its next tile by parity: the phase before that one must be over, which the tile it
+    // filled last shows only while it skips no more tiles than there are slots
+    static_assert(AXC_PWARPS <= STAGES, "a parity wait may not run two phases ahead");
+    static constexpr uint32_t ROW = 32 * (F16 ? 2 : 4), V_BYTES = AXC_T * ROW, STAGE = V_BYTES + AXC_HEADS * AXC_T * 4, SMEM = STAGES * STAGE + 128;
+};
+template <bool F16>
+__global__ void __launch_bounds__(AXC_THREADS)
+attn_chain_exact_kernel(const __grid_constant__ CUtensorMap v_map, const float *__restrict__ ws, const float *__restrict__ aux, uint32_t ld,
+                        const void *__restrict__ vc, uint32_t seq_len, const uint32_t *__restrict__ seq_dev, uint32_t n_kv, uint32_t G, uint32_t hd,
+                        float *__restrict__ out, float *scales, int8_t *quants, int16_t *sums, const TpHook tp) {
+    using C = AxChain<F16>;
+    extern __shared__ __align__(128) char axc_dyn[];
+    __shared__ uint64_t full[C::STAGES], empty[C::STAGES];
+    __shared__ uint32_t gave_up;
+    char *ring = axc_dyn + ((128 - (tma::smem_u32(axc_dyn) & 127)) & 127);
+    const uint32_t kvh = blockIdx.y, d0 = blockIdx.x * 32, h0 = blockIdx.z * AXC_HEADS, nh = min((uint32_t)AXC_HEADS, G - h0);
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        gave_up = 0;
+        for (int i = 0; i < C::STAGES; ++i) {
+            tma::mbar_init(full + i, 2);    // the V request's expect_tx, the probability warp
+            tma::mbar_init(empty + i, nh);  // the chain warps
+        }
+        tma::mbar_init_fence();
+    }
+    __syncthreads();
     pdl_trigger();
-    const uint32_t kvh = blockIdx.y, d0 = blockIdx.x * 32;
     pdl_wait();
-    uint32_t seq = seq_dev ? *seq_dev : seq_len;
-    // a launch planned with a probability table serves lengths up to the table (the host checks this for lengths it knows
-    // and plans captured launches from the length they will meet); never index past it
-    if (smem_pos && seq > smem_pos) seq = smem_pos;
-    const uint32_t n_tiles = (seq + AX_VT - 1) / AX_VT;
-    // V tiles: a position's 32-dim slice is 128 contiguous bytes (64 for an f16 cache): 16-byte asynchronous copies,
-    // the first tiles are requested before the softmax so that they land while it runs
+    const uint32_t seq = seq_dev ? min(*seq_dev, ld) : seq_len;
+    const uint32_t n_tiles = (seq + AXC_T - 1) / AXC_T;
+    if (warp == AXC_HEADS + AXC_PWARPS) {
+        if (lane) return;
+        uint32_t tile = 0;
+        for (; tile < n_tiles; ++tile) {
+            const uint32_t slot = tile % C::STAGES;
+            if (tile >= C::STAGES && !tma::mbar_wait_blocking(empty + slot, (tile / C::STAGES - 1) & 1, &gave_up, &g_ax_status, 2u)) break;
+            const uint32_t boxes = min((uint32_t)AXC_T, seq - tile * AXC_T) / AXC_BOX;
+            if (!boxes) {
+                tma::mbar_arrive(full + slot);
+                continue;
+            }
+            tma::mbar_expect_tx(full + slot, boxes * AXC_BOX * C::ROW);
+            for (uint32_t i = 0; i < boxes; ++i)
+                tma::tensor_g2s_2d(ring + slot * C::STAGE + i * AXC_BOX * C::ROW, &v_map, (int)(kvh * hd + d0), (int)(tile * AXC_T + i * AXC_BOX), full + slot);
+        }
+        // no copy may be in flight into this CTA's memory once it is gone
+        for (uint32_t t = tile > C::STAGES ? tile - C::STAGES : 0; t < tile; ++t)
+            for (uint32_t i = 0; i < (tma::SPIN_LIMIT >> 4) && !tma::mbar_try(full + t % C::STAGES, (t / C::STAGES) & 1) && !*(volatile uint32_t *)&gave_up; ++i) {}
+        return;
+    }
+    if (warp >= AXC_HEADS) {
+        // 1 / sum of the CTA's heads: lane-strided partials of the sums per AX_EPOS positions, then xor shuffles
+        float inv[AXC_HEADS];
 #pragma unroll
-    for (int i = 0; i < AX_VSTAGES; ++i)
-        ax_stage_tile(i, n_tiles, seq, kv_f16 ? 4 : 8, vt, vc, (size_t)n_kv * hd, (size_t)kvh * hd + d0, kv_f16, threadIdx.x);
-    ax_softmax_chain_emit(ws, pw, ld, vc, kv_f16, seq, n_kv, G, hd, smem_pos, kvh, d0, vt, ax_p, red_d, red_f, inv_h, false, out, scales, quants,
-                          sums, tp);
+        for (int hh = 0; hh < AXC_HEADS; ++hh) {
+            const float *parts = aux + (size_t)(kvh * G + h0 + min((uint32_t)hh, nh - 1)) * ld + ax_sums_at(ld);
+            double tot = 0.0;
+            for (uint32_t i = lane; i < (seq + AX_EPOS - 1) / AX_EPOS; i += 32)
+                tot += __hiloint2double(__float_as_int(parts[2 * i]), __float_as_int(parts[2 * i + 1]));
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+            inv[hh] = (float)(1.0 / tot);
+        }
+        for (uint32_t tile = warp - AXC_HEADS; tile < n_tiles; tile += AXC_PWARPS) {
+            const uint32_t slot = tile % C::STAGES, t0 = tile * AXC_T, cnt = min((uint32_t)AXC_T, seq - t0);
+            float e[AXC_HEADS][AXC_T / 32];
+#pragma unroll
+            for (uint32_t hh = 0; hh < AXC_HEADS; ++hh)
+#pragma unroll
+                for (uint32_t i = 0; i < AXC_T / 32; ++i)
+                    e[hh][i] = hh < nh && 32 * i + lane < cnt ? ws[(size_t)(kvh * G + h0 + hh) * ld + t0 + 32 * i + lane] : 0.0f;
+            if (tile >= C::STAGES && !tma::mbar_wait_blocking(empty + slot, (tile / C::STAGES - 1) & 1, &gave_up, &g_ax_status, 2u)) return;
+            char *dst = ring + slot * C::STAGE;
+            float *pd = reinterpret_cast<float *>(dst + C::V_BYTES);
+#pragma unroll
+            for (uint32_t hh = 0; hh < AXC_HEADS; ++hh)  // p = e * (1 / sum), rounded, as the reference stores it
+#pragma unroll
+                for (uint32_t i = 0; i < AXC_T / 32; ++i) pd[hh * AXC_T + 32 * i + lane] = __fmul_rn(e[hh][i], inv[hh]);
+            const size_t row_bytes = (size_t)n_kv * hd * (F16 ? 2 : 4);
+            const char *src = reinterpret_cast<const char *>(vc) + ((size_t)kvh * hd + d0) * (F16 ? 2 : 4) + (size_t)t0 * row_bytes;
+            constexpr uint32_t PIECES = C::ROW / 16;
+            for (uint32_t i = cnt / AXC_BOX * AXC_BOX * PIECES + lane; i < cnt * PIECES; i += 32) ax_cp16(dst + (size_t)i * 16, src + i / PIECES * row_bytes + i % PIECES * 16);
+            ax_commit();
+            ax_wait<0>();
+            __syncwarp();
+            if (lane == 0) tma::mbar_arrive(full + slot);
+        }
+        return;
+    }
+    if (warp >= nh) return;
+    float acc = 0.0f;
+    for (uint32_t tile = 0; tile < n_tiles; ++tile) {
+        const uint32_t slot = tile % C::STAGES;
+        if (!tma::mbar_wait_blocking(full + slot, (tile / C::STAGES) & 1, &gave_up, &g_ax_status, 1u)) return;
+        const uint32_t base = tma::smem_u32(ring + slot * C::STAGE);
+        acc = ax_chain<F16>(base + lane * (F16 ? 2 : 4), base + C::V_BYTES + warp * AXC_T * 4, min((uint32_t)AXC_T, seq - tile * AXC_T), acc);
+        __syncwarp();
+        if (lane == 0) tma::mbar_arrive(empty + slot);
+    }
+    ax_emit(acc, (size_t)(kvh * G + h0 + warp) * hd + d0 + lane, lane, out, scales, quants, sums, tp);
 }
 
-// ONE launch for contexts whose scores fit shared memory: the hd / 32 CTAs of a KV head are a thread-block cluster.
-// CTA r computes the scores of the r-th share of the positions (a half-warp per (position, head) as above, four
-// positions in flight per warp) and stores each into the score table of EVERY CTA of the cluster (distributed shared
-// memory); after one cluster barrier each CTA runs the softmax on its own copy and the value chains of its 32 dims.
-// grid = n_kv * CL CTAs (CL = hd / 32), AX_VTHREADS threads; dynamic shared memory: V tiles, score table, G * hd floats of q.
-template <int HD>
+// ONE launch for contexts of up to 1024 positions: a thread-block cluster per KV head, (hd / 32) x HS CTAs; a CTA walks the chains of
+// 32 dims of HC = ceil(G / HS) heads.  Every CTA computes the scores of its share of the positions for all heads and stores
+// them into the tables of the CTAs that walk those heads (distributed shared memory); after one cluster barrier each CTA runs
+// the softmax on its own table and then the chains.  All of V's slice is requested at the start (cp.async) and lands meanwhile;
+// the share's K rows come the same way, in whole lines, padded by 16 bytes so that eight rows are read without bank conflicts.
+// 32 heads of 128 in groups of 4, f32, 512 / 1024 positions: 9.5 / 12.9 us alone (12.4 / 18 with four heads per CTA, K rows read
+// in 32-byte pieces and chains that waited for their loads).
+// grid = n_kv * cluster size CTAs, AX_VTHREADS threads; dynamic shared memory: AxFused.
+template <int HD, bool F16>
+struct AxFused {
+    static constexpr uint32_t ES = F16 ? 2 : 4, KROWS = 128 * 128 / HD, KSTRIDE = HD * ES + 16;  // K rows staged at a time
+    static constexpr uint32_t K_BYTES = KROWS * KSTRIDE;
+    static size_t smem(uint32_t pos, uint32_t G, uint32_t HC) { return (size_t)pos * 32 * ES + K_BYTES + ((size_t)(pos + 4) * HC + (size_t)G * HD) * 4; }
+};
+template <int HD, bool F16>
 __global__ void __launch_bounds__(AX_VTHREADS)
-attn_fused_exact_kernel(const float *__restrict__ q, const void *__restrict__ kc, const void *__restrict__ vc, int kv_f16, uint32_t seq_len,
-                        const uint32_t *__restrict__ seq_dev, uint32_t n_kv, uint32_t G, float scale, uint32_t smem_pos,
+attn_fused_exact_kernel(const float *__restrict__ q, const void *__restrict__ kc, const void *__restrict__ vc, int vec, uint32_t seq_len,
+                        const uint32_t *__restrict__ seq_dev, uint32_t n_kv, uint32_t G, uint32_t HC, float scale, uint32_t smem_pos,
                         float *__restrict__ out, float *scales, int8_t *quants, int16_t *sums, const TpHook tp) {
-    extern __shared__ __align__(16) float ax_dyn[];
-    constexpr uint32_t CL = HD / 32, NK = HD / 16;       // cluster size; K elements per lane of a half-warp
-    float *vt = ax_dyn;
-    float *ax_p = ax_dyn + AX_VSTAGES * AX_VT * 32;      // [G][smem_pos + 4]
+    using F = AxFused<HD, F16>;
+    extern __shared__ __align__(16) char axf_dyn[];
+    constexpr uint32_t SL = HD / 32, WARPS = AX_VTHREADS / 32, ES = F::ES;  // SL: slices of a head
+    char *vt = axf_dyn;                                  // [smem_pos][32]
+    char *kt = vt + (size_t)smem_pos * 32 * ES;          // [KROWS][KSTRIDE]
+    float *ax_p = reinterpret_cast<float *>(kt + F::K_BYTES);  // [HC][smem_pos + 4]
     const uint32_t pstride = smem_pos + 4;
-    float *ax_q = ax_p + (size_t)G * pstride;            // [G][HD]
-    __shared__ double red_d[AX_VTHREADS / 32];
-    __shared__ float red_f[AX_VTHREADS / 32];
-    __shared__ float inv_h[8];  // 1 / sum of every head of the group
+    float *ax_q = ax_p + (size_t)HC * pstride;           // [G][HD]
+    __shared__ double red_d[WARPS];
+    __shared__ float red_f[WARPS];
     cg::cluster_group cluster = cg::this_cluster();
-    const uint32_t r = cluster.block_rank(), kvh = blockIdx.x / CL, d0 = r * 32;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t CL = cluster.num_blocks(), r = cluster.block_rank(), kvh = blockIdx.x / CL, d0 = r % SL * 32, h0 = r / SL * HC, nh = min(HC, G - h0);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // a CTA's shared memory may be written by its peers only once it runs: every CTA arrives here, and waits for the
     // others just before its first remote store
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     pdl_trigger();
     pdl_wait();
     uint32_t seq = seq_dev ? *seq_dev : seq_len;
-    if (seq > smem_pos) seq = smem_pos;  // the score tables hold smem_pos positions (see the values kernel)
-    const uint32_t n_tiles = (seq + AX_VT - 1) / AX_VT;
-#pragma unroll
-    for (int i = 0; i < AX_VSTAGES; ++i)
-        ax_stage_tile(i, n_tiles, seq, kv_f16 ? 4 : 8, vt, vc, (size_t)n_kv * HD, (size_t)kvh * HD + d0, kv_f16, tid);
-    for (uint32_t i = tid; i < G * HD; i += AX_VTHREADS) ax_q[i] = q[(size_t)kvh * G * HD + i];
-    __syncthreads();
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    // ---- scores of this CTA's share of the positions, into every CTA's table
-    {
-        const uint32_t share = (seq + CL - 1) / CL, t_begin = r * share, t_end = min(seq, t_begin + share);
-        const uint32_t c16 = lane & 15, hsel = lane >> 4;
-        float *peer_p = cluster.map_shared_rank(ax_p, c16 < CL ? c16 : 0);  // lane c of a half-warp stores into CTA c's table
-        const size_t kv_dim = (size_t)n_kv * HD;
-        constexpr uint32_t UN = 4;  // positions in flight per warp
-        for (uint32_t t0 = t_begin + warp * UN; t0 < t_end; t0 += (AX_VTHREADS / 32) * UN) {
-            // lane c16 = 8a + L holds elements 16j + c16 of each K row (chunk 2j + a of the reference's alternating accumulators)
-            float kv[UN][NK];
-#pragma unroll
-            for (uint32_t u = 0; u < UN; ++u) {
-                const uint32_t t = min(t0 + u, t_end - 1);
-                const size_t row = (size_t)t * kv_dim + (size_t)kvh * HD;
-#pragma unroll
-                for (uint32_t j = 0; j < NK; ++j) {
-                    const size_t e = row + 16 * j + c16;
-                    kv[u][j] = kv_f16 ? __half2float(__ldg(reinterpret_cast<const __half *>(kc) + e)) : __ldg(reinterpret_cast<const float *>(kc) + e);
-                }
+    if (seq > smem_pos) seq = smem_pos;  // the score tables hold smem_pos positions; the host plans launches for the lengths they meet
+    const size_t row_bytes = (size_t)n_kv * HD * ES;
+    const uint32_t share = (seq + CL - 1) / CL, t_begin = min(seq, r * share), t_end = min(seq, t_begin + share);
+    auto stage_k = [&](uint32_t t0) {
+        const uint32_t rows = min(F::KROWS, t_end - t0);
+        const char *src = reinterpret_cast<const char *>(kc) + (size_t)t0 * row_bytes + (size_t)kvh * HD * ES;
+        constexpr uint32_t PIECES = HD * ES / 16;
+        if (vec) {
+            for (uint32_t i = tid; i < rows * PIECES; i += AX_VTHREADS) ax_cp16(kt + i / PIECES * F::KSTRIDE + i % PIECES * 16, src + i / PIECES * row_bytes + i % PIECES * 16);
+        } else {  // a cache that does not start on a 16-byte boundary
+            for (uint32_t i = tid; i < rows * HD; i += AX_VTHREADS) {
+                char *d = kt + i / HD * F::KSTRIDE + i % HD * ES;
+                const char *g = src + i / HD * row_bytes + i % HD * ES;
+                if (F16) *reinterpret_cast<uint16_t *>(d) = __ldg(reinterpret_cast<const uint16_t *>(g));
+                else *reinterpret_cast<uint32_t *>(d) = __ldg(reinterpret_cast<const uint32_t *>(g));
             }
-            for (uint32_t h0 = 0; h0 < G; h0 += 2) {
-                const uint32_t h = h0 + hsel;
-                const bool live = h < G;
-                const float *qh = ax_q + (live ? h : 0) * HD;
-                float qv[NK];
+        }
+        ax_commit();
+    };
+    if (t_begin < t_end) stage_k(t_begin);
+    else ax_commit();
+    {
+        const char *src = reinterpret_cast<const char *>(vc) + ((size_t)kvh * HD + d0) * ES;
+        constexpr uint32_t PIECES = 32 * ES / 16;
+        for (uint32_t i = tid; i < seq * PIECES; i += AX_VTHREADS) ax_cp16(vt + (size_t)i * 16, src + i / PIECES * row_bytes + i % PIECES * 16);
+        ax_commit();
+    }
+    for (uint32_t i = tid; i < G * HD; i += AX_VTHREADS) ax_q[i] = q[(size_t)kvh * G * HD + i];
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    // ---- scores of this CTA's share of the positions: sixteen positions per warp, lanes p and p + 16 take position p
+    for (uint32_t tk = t_begin; tk < t_end; tk += F::KROWS) {
+        if (tk > t_begin) {
+            __syncthreads();  // everyone is done with the rows staged before
+            stage_k(tk);
+            ax_wait<0>();
+        } else {
+            ax_wait<1>();
+        }
+        __syncthreads();
+        const uint32_t a = lane >> 4, rows = min(F::KROWS, t_end - tk), tiles = (rows + 15) / 16;
+        // where the tiles leave warps idle, the heads are dealt out too
+        const uint32_t hs = min(max(WARPS / tiles, 1u), G);
+        for (uint32_t item = warp; item < tiles * hs; item += WARPS) {
+            const uint32_t row = item / hs * 16 + (lane & 15);
+            const char *kr = kt + min(row, rows - 1) * F::KSTRIDE + 8 * a * ES;
+            float k[HD / 16][8];
+            auto load = [&] {
 #pragma unroll
-                for (uint32_t j = 0; j < NK; ++j) qv[j] = qh[16 * j + c16];
+                for (int j = 0; j < HD / 16; ++j) {
+                    if constexpr (F16) {
+                        const uint4 w = *reinterpret_cast<const uint4 *>(kr + 32 * j);
+                        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-                for (uint32_t u = 0; u < UN; ++u) {
-                    float acc = 0.0f;
-#pragma unroll
-                    for (uint32_t j = 0; j < NK; ++j) acc = fmaf(qv[j], kv[u][j], acc);
-                    // accumulators 0 and 1 of the same lane L, then hsum256
-                    acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 8));
-                    acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 4));
-                    acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 2));
-                    acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 1));
-                    const float sc = __fmul_rn(acc, scale);
-                    if (live && c16 < CL && t0 + u < t_end) peer_p[(size_t)h * pstride + t0 + u] = sc;
+                        for (int i = 0; i < 8; ++i) k[j][i] = h2f((uint16_t)(ww[i / 2] >> (16 * (i & 1))));
+                    } else {
+                        const float4 lo = *reinterpret_cast<const float4 *>(kr + 64 * j), hi = *reinterpret_cast<const float4 *>(kr + 64 * j + 16);
+                        k[j][0] = lo.x, k[j][1] = lo.y, k[j][2] = lo.z, k[j][3] = lo.w;
+                        k[j][4] = hi.x, k[j][5] = hi.y, k[j][6] = hi.z, k[j][7] = hi.w;
+                    }
                 }
+            };
+            if (HD <= 128) load();
+#pragma unroll 1
+            for (uint32_t h = item % hs; h < G; h += hs) {
+                if (HD > 128) load();  // 128 values do not stay in registers
+                const float sc = ax_score<HD, 16>(ax_q + h * HD, k, a, scale);
+                const uint32_t first = h / HC * SL;  // the CTAs of this head
+#pragma unroll
+                for (uint32_t c = 0; c < SL; c += 2)
+                    if (row < rows && c + a < SL) cluster.map_shared_rank(ax_p, first + c + a)[(size_t)(h % HC) * pstride + tk + row] = sc;
             }
         }
     }
     cluster.sync();  // every CTA's table is complete; nothing remote is touched after this point
-    ax_softmax_chain_emit(nullptr, nullptr, 0, vc, kv_f16, seq, n_kv, G, HD, smem_pos, kvh, d0, vt, ax_p, red_d, red_f, inv_h, true, out, scales,
-                          quants, sums, tp);
+
+    // ---- probabilities of the CTA's heads.  Head h is handled by warps [h * nwh, (h + 1) * nwh).
+    const uint32_t nwh = WARPS / HC, h_mine = warp / nwh, wl = warp % nwh;  // warps past nh * nwh idle here
+    const bool has_head = h_mine < nh;
+    const uint32_t hth = nwh * 32, hti = wl * 32 + lane;  // threads of my head, my index among them
+    float *p_row = ax_p + (size_t)(has_head ? h_mine : 0) * pstride;
+    float mx = -INFINITY;
+    if (has_head) {
+#pragma unroll 4
+        for (uint32_t t = hti; t < seq; t += hth) mx = fmaxf(mx, p_row[t]);  // f32::max fold: NaN scores are ignored
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) red_f[warp] = mx;
+    __syncthreads();
+    if (has_head) {
+        mx = red_f[h_mine * nwh];
+        for (uint32_t w = 1; w < nwh; ++w) mx = fmaxf(mx, red_f[h_mine * nwh + w]);
+    }
+    // exponentials and their f64 sum (fixed tree: thread-strided partials, xor shuffles, the head's warps in index order)
+    double sum = 0.0;
+    if (has_head) {
+#pragma unroll 4
+        for (uint32_t t = hti; t < seq; t += hth) {
+            const float e = ggml_expf(__fsub_rn(p_row[t], mx));
+            p_row[t] = e;
+            sum += (double)e;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) red_d[warp] = sum;
+    __syncthreads();
+    if (has_head) {
+        double tot = red_d[h_mine * nwh];
+        for (uint32_t w = 1; w < nwh; ++w) tot += red_d[h_mine * nwh + w];
+        const float inv = (float)(1.0 / tot);
+#pragma unroll 4
+        for (uint32_t t = hti; t < seq; t += hth) p_row[t] = __fmul_rn(p_row[t], inv);
+    }
+    ax_wait<0>();  // this thread's part of V has landed
+    __syncthreads();
+
+    // ---- out[d] = fma(p[t], V[t][d], out[d]) in position order: warp h walks head h, a lane per output dim
+    if (warp >= nh) return;
+    const float acc = ax_chain<F16>(tma::smem_u32(vt) + lane * ES, tma::smem_u32(ax_p + (size_t)warp * pstride), seq, 0.0f);
+    ax_emit(acc, (size_t)(kvh * G + h0 + warp) * HD + d0 + lane, lane, out, scales, quants, sums, tp);
 }
 
 constexpr size_t AX_SMEM_MAX = 226 * 1024;  // dynamic shared memory the values / fused kernels may ask for
 
-template <int HD>
-int32_t launch_fused(uint32_t cl, size_t smem, cudaStream_t st, const float *q, const void *kc, const void *vc, int kv_f16, uint32_t seq_len,
-                     const uint32_t *seq_dev, uint32_t nkv, uint32_t G, float scale, uint32_t fpos, float *out, float *scales,
-                     int8_t *quants, int16_t *sums, const TpHook &tp) {
-    static thread_local int raised_dev = -1;  // per head size: opt in to more than 48 KB once per device
+bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+template <int HD, bool F16>
+int32_t launch_fused(size_t smem, cudaStream_t st, const float *q, const void *kc, const void *vc, uint32_t seq_len, const uint32_t *seq_dev,
+                     uint32_t nkv, uint32_t G, uint32_t HC, float scale, uint32_t fpos, float *out, float *scales, int8_t *quants, int16_t *sums,
+                     const TpHook &tp) {
+    const uint32_t cl = HD / 32 * ((G + HC - 1) / HC);
+    static thread_local int raised_dev = -1;  // per instantiation: opt in to more than 48 KB once per device
     int dev = 0;
     cudaGetDevice(&dev);
     if (raised_dev != dev) {
-        CERA_CUDA_TRY(cudaFuncSetAttribute(attn_fused_exact_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AX_SMEM_MAX));
+        CERA_CUDA_TRY(cudaFuncSetAttribute(attn_fused_exact_kernel<HD, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AX_SMEM_MAX));
         raised_dev = dev;
     }
     cudaLaunchConfig_t cfg = {};
@@ -467,9 +628,52 @@ int32_t launch_fused(uint32_t cl, size_t smem, cudaStream_t st, const float *q, 
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
     count_launch();
-    return check_cuda(cudaLaunchKernelEx(&cfg, attn_fused_exact_kernel<HD>, q, kc, vc, kv_f16, seq_len, seq_dev, nkv, G, scale, fpos, out, scales,
-                                         quants, sums, tp),
+    return check_cuda(cudaLaunchKernelEx(&cfg, attn_fused_exact_kernel<HD, F16>, q, kc, vc, (int)aligned16(kc), seq_len, seq_dev, nkv, G, HC, scale, fpos, out,
+                                         scales, quants, sums, tp),
                       "attention (fused) launch");
+}
+
+template <int HD, bool F16>
+int32_t launch_scores(dim3 grid, cudaStream_t st, const float *q, const void *kc, uint32_t seq_len, const uint32_t *seq_dev, uint32_t nkv, uint32_t G,
+                      float scale, float *ws, float *aux, uint32_t ld) {
+    return check_cuda(launch_k(attn_scores_exact_kernel<HD, F16>, grid, dim3(AX_SWARPS * 32), (size_t)G * HD * sizeof(float), st, q, kc, (int)aligned16(kc),
+                               seq_len, seq_dev, nkv, G, scale, ws, aux, ld),
+                      "attention (scores) launch");
+}
+
+template <bool F16>
+int32_t launch_scores_hd(uint32_t hd, dim3 grid, cudaStream_t st, const float *q, const void *kc, uint32_t seq_len, const uint32_t *seq_dev, uint32_t nkv,
+                         uint32_t G, float scale, float *ws, float *aux, uint32_t ld) {
+    switch (hd) {
+        case 32: return launch_scores<32, F16>(grid, st, q, kc, seq_len, seq_dev, nkv, G, scale, ws, aux, ld);
+        case 64: return launch_scores<64, F16>(grid, st, q, kc, seq_len, seq_dev, nkv, G, scale, ws, aux, ld);
+        case 96: return launch_scores<96, F16>(grid, st, q, kc, seq_len, seq_dev, nkv, G, scale, ws, aux, ld);
+        case 128: return launch_scores<128, F16>(grid, st, q, kc, seq_len, seq_dev, nkv, G, scale, ws, aux, ld);
+        case 160: return launch_scores<160, F16>(grid, st, q, kc, seq_len, seq_dev, nkv, G, scale, ws, aux, ld);
+        case 192: return launch_scores<192, F16>(grid, st, q, kc, seq_len, seq_dev, nkv, G, scale, ws, aux, ld);
+        case 224: return launch_scores<224, F16>(grid, st, q, kc, seq_len, seq_dev, nkv, G, scale, ws, aux, ld);
+        case 256: return launch_scores<256, F16>(grid, st, q, kc, seq_len, seq_dev, nkv, G, scale, ws, aux, ld);
+        default: return fail(CERA_CUDA_ERR_UNSUPPORTED, "decode_attention: head_dim %u", hd);
+    }
+}
+
+template <bool F16>
+int32_t launch_chain(cudaStream_t st, const float *ws, const float *aux, uint32_t ld, uint32_t reach, const void *vc, uint32_t seq_len,
+                     const uint32_t *seq_dev, uint32_t nkv, uint32_t G, uint32_t hd, float *out, float *scales, int8_t *quants, int16_t *sums, const TpHook &tp) {
+    constexpr size_t smem = AxChain<F16>::SMEM;
+    static thread_local int raised_dev = -1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (raised_dev != dev) {
+        CERA_CUDA_TRY(cudaFuncSetAttribute(attn_chain_exact_kernel<F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        raised_dev = dev;
+    }
+    CUtensorMap v_map;
+    CERA_TRY(tensor_map_2d(&v_map, F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, F16 ? 2 : 4, vc, reach, (uint64_t)nkv * hd, 32,
+                           AXC_BOX, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE));
+    return check_cuda(launch_k(attn_chain_exact_kernel<F16>, dim3(hd / 32, nkv, (G + AXC_HEADS - 1) / AXC_HEADS), dim3(AXC_THREADS), smem, st,
+                               v_map, ws, aux, ld, vc, seq_len, seq_dev, nkv, G, hd, out, scales, quants, sums, tp),
+                      "attention (values) launch");
 }
 
 // CERA_CUDA_ATTN=flash (or any of the split-kernel selectors) keeps decode attention on the online-softmax kernels.
@@ -489,8 +693,8 @@ bool attn_exact_supports(size_t n_heads, size_t n_kv_heads, size_t head_dim) {
     return G >= 1 && G <= 8 && head_dim % 32 == 0 && head_dim >= 32 && head_dim <= 256;
 }
 
-// Plan word of the reference-order kernels: ATT_EXACT_FLAG | b, b = 1..4: probabilities of up to b * 1024 positions
-// stay in shared memory; b = 5: they go through global memory.
+// Plan word of the reference-order kernels: ATT_EXACT_FLAG | b, b = 1..4: launches that serve up to b * 1024 positions (b = 1: in
+// one launch); b = 5: as many as the workspace holds.
 constexpr uint32_t ATT_EXACT_FLAG = 0x200;
 
 uint32_t attn_exact_plan(size_t seq_len_hint) {
@@ -519,53 +723,52 @@ int32_t launch_decode_attention_exact(const float *q, const void *kc, const void
     size_t reach = b >= 5 ? cap : (size_t)b * 1024;  // longest length this launch may meet
     if (reach > cap) reach = cap;
     if (seq_len > reach) return fail(CERA_CUDA_ERR_BAD_ARG, "decode_attention: plan 0x%x does not cover %zu positions", plan, seq_len);
-    float *ws = (float *)workspace, *pw = ws + n_heads * (size_t)ld;
+    float *ws = (float *)workspace, *aux = ws + n_heads * (size_t)ld;
     // ---- one launch when the scores fit shared memory (CERA_CUDA_ATTN_EXACT=split keeps the two-kernel form)
     static const bool no_fused = [] { const char *e = getenv("CERA_CUDA_ATTN_EXACT"); return e && strcmp(e, "split") == 0; }();
-    if (!no_fused && b == 1 && (hd == 64 || hd == 128 || hd == 256)) {  // up to 1024 positions (measured: 12.7 against 14.3 us at 512, slower than the pair at 4096)
-        const uint32_t fpos = (uint32_t)reach;
-        const size_t fsmem = ((size_t)AX_VSTAGES * AX_VT * 32 + ((size_t)fpos + 4) * G + (size_t)G * hd) * sizeof(float);
-        if (fsmem <= AX_SMEM_MAX) {
-            const uint32_t cl = hd / 32;
-            const TpHook hook = tp ? *tp : TpHook{};
-            if (hd == 64)
-                return launch_fused<64>(cl, fsmem, st, q, kc, vc, kv_f16, (uint32_t)seq_len, seq_len_dev, nkv, G, scale, fpos, out, scales, quants, sums, hook);
-            if (hd == 128)
-                return launch_fused<128>(cl, fsmem, st, q, kc, vc, kv_f16, (uint32_t)seq_len, seq_len_dev, nkv, G, scale, fpos, out, scales, quants, sums, hook);
-            return launch_fused<256>(cl, fsmem, st, q, kc, vc, kv_f16, (uint32_t)seq_len, seq_len_dev, nkv, G, scale, fpos, out, scales, quants, sums, hook);
-        }
+    if (!no_fused && b == 1 && (hd == 64 || hd == 128 || hd == 256)) {  // up to 1024 positions
+        const uint32_t fpos = (uint32_t)reach, sl = (uint32_t)seq_len;
+        const TpHook hook = tp ? *tp : TpHook{};
+        uint32_t hs = 1;  // CTAs that share a slice's heads: two heads each if the cluster (at most 8) allows
+        while (2 * hs * (hd / 32) <= 8 && 2 * hs <= (G + 1) / 2) hs *= 2;
+        const uint32_t hc = (G + hs - 1) / hs;
+#define CERA_AX_FUSED(HD, F16)                                                                                                        \
+    if (hd == HD && (kv_f16 != 0) == F16 && AxFused<HD, F16>::smem(fpos, G, hc) <= AX_SMEM_MAX)                                          \
+    return launch_fused<HD, F16>(AxFused<HD, F16>::smem(fpos, G, hc), st, q, kc, vc, sl, seq_len_dev, nkv, G, hc, scale, fpos, out, scales, \
+                                 quants, sums, hook)
+        CERA_AX_FUSED(64, true);
+        CERA_AX_FUSED(64, false);
+        CERA_AX_FUSED(128, true);
+        CERA_AX_FUSED(128, false);
+        CERA_AX_FUSED(256, true);
+        CERA_AX_FUSED(256, false);
+#undef CERA_AX_FUSED
     }
     // scores: a fixed number of CTAs per KV head walks the position tiles, so one captured launch serves every length
-    const uint32_t tiles = (uint32_t)((reach + AX_SWARPS - 1) / AX_SWARPS);
-    uint32_t per_head = (uint32_t)(4 * sm_count() / (int)nkv);
+    const uint32_t tiles = (uint32_t)((reach + 16 * AX_SWARPS - 1) / (16 * AX_SWARPS)), sl = (uint32_t)seq_len;
+    uint32_t per_head = (uint32_t)(2 * sm_count() / (int)nkv);
     if (per_head < 1) per_head = 1;
     if (per_head > tiles) per_head = tiles;
-    count_launch();
-    const dim3 sgrid(per_head, nkv), sblock(AX_SWARPS * 32);
-    const size_t sq = (size_t)G * hd * sizeof(float);
-    const uint32_t sl32 = (uint32_t)seq_len;
-    if (hd == 128) CERA_CUDA_TRY(launch_k(attn_scores_exact_kernel<128>, sgrid, sblock, sq, st, q, kc, kv_f16, sl32, seq_len_dev, nkv, G, hd, scale, ws, ld));
-    else if (hd == 64) CERA_CUDA_TRY(launch_k(attn_scores_exact_kernel<64>, sgrid, sblock, sq, st, q, kc, kv_f16, sl32, seq_len_dev, nkv, G, hd, scale, ws, ld));
-    else CERA_CUDA_TRY(launch_k(attn_scores_exact_kernel<0>, sgrid, sblock, sq, st, q, kc, kv_f16, sl32, seq_len_dev, nkv, G, hd, scale, ws, ld));
-    uint32_t smem_pos = b >= 5 ? 0u : (uint32_t)reach;
-    if (((size_t)AX_VSTAGES * AX_VT * 32 + ((size_t)smem_pos + 4) * G) * sizeof(float) > AX_SMEM_MAX) smem_pos = 0;  // probabilities through global memory
-    // probability table [G][smem_pos + 4], or - probabilities through global memory - a ring of probability tiles [stages][G][AX_VT]
-    const size_t smem = ((size_t)AX_VSTAGES * AX_VT * 32 + (smem_pos ? ((size_t)smem_pos + 4) * G : (size_t)AX_VSTAGES * G * AX_VT)) * sizeof(float);
-    {
-        // static + dynamic shared memory can pass the 48 KB default even at the shortest contexts: opt in once per device
-        static thread_local int raised_dev = -1;
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (raised_dev != dev) {
-            CERA_CUDA_TRY(cudaFuncSetAttribute(attn_values_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AX_SMEM_MAX));
-            raised_dev = dev;
-        }
-    }
-    count_launch();
-    return check_cuda(launch_k(attn_values_exact_kernel, dim3(hd / 32, nkv), dim3(AX_VTHREADS), smem, st, (const float *)ws, pw, ld, vc,
-                               kv_f16, (uint32_t)seq_len, seq_len_dev, nkv, G, hd, smem_pos, out, scales, quants, sums,
-                               tp ? *tp : TpHook{}),
-                      "attention (values) launch");
+    const TpHook hook = tp ? *tp : TpHook{};
+    count_launch(3);
+    const dim3 sgrid(per_head, nkv);
+    CERA_TRY(kv_f16 ? launch_scores_hd<true>(hd, sgrid, st, q, kc, sl, seq_len_dev, nkv, G, scale, ws, aux, ld)
+                    : launch_scores_hd<false>(hd, sgrid, st, q, kc, sl, seq_len_dev, nkv, G, scale, ws, aux, ld));
+    // exponentials: likewise, about four CTAs per SM
+    uint32_t parts = (uint32_t)((reach + AX_EPOS - 1) / AX_EPOS);
+    const uint32_t part_ctas = (uint32_t)(4 * sm_count() / (int)n_heads);
+    if (parts > part_ctas) parts = part_ctas ? part_ctas : 1;
+    CERA_TRY(check_cuda(launch_k(attn_exp_exact_kernel, dim3(parts, (unsigned)n_heads), dim3(AX_ETHREADS), 0, st, ws, aux,
+                                 ld, sl, seq_len_dev),
+                        "attention (exponentials) launch"));
+    return kv_f16 ? launch_chain<true>(st, ws, aux, ld, (uint32_t)reach, vc, sl, seq_len_dev, nkv, G, hd, out, scales, quants, sums, hook)
+                  : launch_chain<false>(st, ws, aux, ld, (uint32_t)reach, vc, sl, seq_len_dev, nkv, G, hd, out, scales, quants, sums, hook);
 }
+
+static const bool g_ax_status_registered = register_kernel_status([] {
+    unsigned int v = 0;
+    cudaMemcpyFromSymbol(&v, g_ax_status, sizeof(v));
+    return (uint32_t)v << 23;  // bits 23, 24
+});
 
 }  // namespace cera

@@ -7,8 +7,6 @@
 // Grouped by expert the tiles come from a device-built work list.  With NA = 2 a stage holds two weight tiles (an expert's
 // gate rows and the same up rows; without groups, the matrix's first and second half) against one activation tile, and the
 // epilogue forms the gated unit from the two accumulators.  Every wait is bounded (tma.cuh); a wait that runs out empties the CTA and raises a status bit.
-#include <cudaTypedefs.h>
-
 #include "dense.cuh"
 #include "tc.cuh"
 #include "tensor_map.h"
@@ -23,23 +21,6 @@ static const bool g_dense_tc_registered = register_kernel_status([] {
     cudaMemcpyFromSymbol(&v, g_dense_tc_status, sizeof(v));
     return (uint32_t)v << 17;
 });
-
-int32_t tensor_map_bf16(CUtensorMap *map, const void *base, uint64_t rows, uint64_t ld, uint32_t box_cols, uint32_t box_rows) {
-    static PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return (PFN_cuTensorMapEncodeTiled_v12000)p;
-    }();
-    if (!encode) return fail(CERA_CUDA_ERR_CUDA, "the driver offers no cuTensorMapEncodeTiled");
-    const cuuint64_t dims[2] = {ld, rows}, strides[1] = {ld * 2};
-    const cuuint32_t box[2] = {box_cols, box_rows}, es[2] = {1, 1};
-    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(CERA_CUDA_ERR_CUDA, "cuTensorMapEncodeTiled: error %d for [%llu x %llu]", (int)r, (unsigned long long)rows, (unsigned long long)ld);
-    return CERA_CUDA_OK;
-}
 
 namespace {
 

@@ -5,7 +5,10 @@
 #include <cstdio>
 #include <cstdlib>
 
+#include <cudaTypedefs.h>
+
 #include "common.cuh"
+#include "tensor_map.h"
 
 namespace cera {
 
@@ -57,6 +60,24 @@ int sm_count() {
         cached_dev = dev;
     }
     return cached;
+}
+
+int32_t tensor_map_2d(CUtensorMap *map, CUtensorMapDataType type, uint32_t elem_bytes, const void *base, uint64_t rows, uint64_t ld, uint32_t box_cols,
+                      uint32_t box_rows, CUtensorMapSwizzle swizzle, CUtensorMapL2promotion promotion) {
+    static PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return (PFN_cuTensorMapEncodeTiled_v12000)p;
+    }();
+    if (!encode) return fail(CERA_CUDA_ERR_CUDA, "the driver offers no cuTensorMapEncodeTiled");
+    const cuuint64_t dims[2] = {ld, rows}, strides[1] = {ld * elem_bytes};
+    const cuuint32_t box[2] = {box_cols, box_rows}, es[2] = {1, 1};
+    const CUresult r = encode(map, type, 2, const_cast<void *>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              swizzle, promotion, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(CERA_CUDA_ERR_CUDA, "cuTensorMapEncodeTiled: error %d for [%llu x %llu]", (int)r, (unsigned long long)rows, (unsigned long long)ld);
+    return CERA_CUDA_OK;
 }
 
 }  // namespace cera

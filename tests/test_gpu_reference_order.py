@@ -85,6 +85,32 @@ def test_decode_attention_bits(nh, nkv, hd, seq, kv_f16):
     assert_bits(got, want, f"attention {nh}/{nkv} x {hd}, {seq} positions, f16={kv_f16}")
 
 
+# edges of the score tiles (16 positions), value tiles (256), sums (1024) and of the one-launch form (1024); every head size
+# that has a score kernel; groups that leave a chain CTA half empty; a key cache that starts off a 16-byte boundary
+@pytest.mark.parametrize("kv_f16", [0, 1])
+@pytest.mark.parametrize("nh,nkv,hd,seq,off", [
+    (4, 1, 128, 15, 0), (4, 1, 128, 17, 0), (8, 2, 64, 255, 0), (8, 2, 64, 257, 0), (4, 1, 256, 272, 0), (32, 8, 128, 1023, 0),
+    (32, 8, 128, 1024, 0), (32, 8, 128, 1025, 0), (6, 2, 128, 1041, 0), (8, 1, 64, 2048, 0), (8, 1, 128, 2049, 0), (3, 1, 256, 1300, 0),
+    (5, 1, 32, 40, 0), (2, 2, 160, 1291, 0), (4, 2, 192, 513, 0), (4, 1, 224, 16, 0), (24, 3, 128, 4200, 0), (64, 8, 128, 3075, 0),
+    (4, 1, 128, 300, 2), (4, 1, 64, 1500, 1), (2, 1, 96, 100, 3)])
+def test_decode_attention_bits_at_tile_edges(nh, nkv, hd, seq, off, kv_f16):
+    torch = need_gpu()
+    import cera_b200 as cb
+    n = seq * nkv * hd
+    kc = cb.synth_normal(n + off, seed=seq, sigma=1.0)
+    vc = cb.synth_normal(n, seed=seq + 1, sigma=1.0).reshape(seq, nkv * hd)
+    q = cb.synth_normal(nh * hd, seed=seq + 2, sigma=1.0)
+    if kv_f16:
+        kc, vc = kc.half(), vc.half()
+    kc = kc[off:].reshape(seq, nkv * hd)
+    scale = 1.0 / math.sqrt(hd)
+    got = cb.decode_attention(q, kc, vc, nh, nkv, hd, seq, scale).cpu().numpy()
+    kh = kc.cpu().numpy().view(np.uint16) if kv_f16 else kc.cpu().numpy()
+    vh = vc.cpu().numpy().view(np.uint16) if kv_f16 else vc.cpu().numpy()
+    want = O.decode_attention(q.cpu().numpy(), kh, vh, nh, nkv, hd, seq, scale)
+    assert_bits(got, want, f"attention {nh}/{nkv} x {hd}, {seq} positions, f16={kv_f16}")
+
+
 @pytest.mark.parametrize("kv_f16", [0, 1])
 def test_model_logits_bit_identical_to_the_oracle(kv_f16):
     """A llama-architecture model whose matrices are K-quants with row lengths that are multiples of 512 runs every
