@@ -1199,6 +1199,22 @@ static const bool g_tc_status_registered = register_kernel_status([] {
     return (uint32_t)v << 8;
 });
 
+// By default a stream-ordered pool hands everything back to the driver at every synchronise, and the next prompt's first
+// allocations pay for mapping it again; up to 1 GB of scratch stays cached.  Once per device and thread.
+void keep_stream_pool() {
+    static thread_local int pooled_dev = -1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (pooled_dev == dev) return;
+    cudaMemPool_t pool = nullptr;
+    if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
+        uint64_t keep = 1ull << 30;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    cudaGetLastError();
+    pooled_dev = dev;
+}
+
 // One activation matrix against up to three weights (q / k / v, gate / up): the activation operands are converted once
 // and, when every weight has its image, ONE kernel launch covers all of them (the small matrices' CTAs run beside the
 // large one's instead of after them).  *taken = false: not these kernels' case, nothing launched.
@@ -1224,22 +1240,7 @@ int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, s
     const uint32_t nb32 = w.k / 32, n_mit = (nb32 + TCW_MIN_J - 1) / TCW_MIN_J;
     const size_t img_bytes = (size_t)tiles * n_it * (2 * TC_OP_BYTES), min_bytes = (size_t)tiles * n_sb * TC_MINOP_BYTES,
                  xm_bytes = (size_t)tiles * n_mit * (2 * TCW_MINT_BYTES);
-    {
-        // keep the stream-ordered pool's memory across synchronisations (by default a pool hands everything back to the
-        // driver at every synchronise, and the next prompt's first allocations pay for mapping it again); once per device
-        static thread_local int pooled_dev = -1;
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (pooled_dev != dev) {
-            cudaMemPool_t pool = nullptr;
-            if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
-                uint64_t keep = 1ull << 30;  // up to 1 GB of scratch stays cached
-                cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-            }
-            cudaGetLastError();
-            pooled_dev = dev;
-        }
-    }
+    keep_stream_pool();
     uint8_t *scratch = nullptr;
     if (cudaMallocAsync((void **)&scratch, img_bytes + min_bytes + xm_bytes + (size_t)n_pad * 8, st) != cudaSuccess) {
         cudaGetLastError();  // no room for the operand scratch: leave the GEMM to the kernels that need none

@@ -214,6 +214,8 @@ int32_t launch_gemm_ex(const WeightView &w, const ActView &x, size_t n, float *o
         bool taken = false;
         CERA_TRY(launch_gemm_tc(w, x, n, out, ldy, ldc, epilogue, st, &taken));  // tcgen05 / TMEM
         if (taken) return CERA_CUDA_OK;
+        CERA_TRY(launch_gemm_tcq(w, x, n, out, ldy, ldc, epilogue, st, &taken));  // tcgen05 from the quantized bytes
+        if (taken) return CERA_CUDA_OK;
         CERA_TRY(launch_gemm_mma(w, x, n, out, ldy, ldc, epilogue, st, &taken));  // warp-level mma.sync
         if (taken) return CERA_CUDA_OK;
     }

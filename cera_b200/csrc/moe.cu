@@ -261,11 +261,16 @@ bool moe_force_dp4a() {
     return v;
 }
 
-// One grouped projection over the work list: the tensor-core GEMM when the plan was made for it, else the dp4a kernel.
-// cap / max_small: where the list of narrow items starts inside p.tiles and how many it can hold (tensor-core plan only).
-int32_t grouped_projection(bool mma, const MoeGemmParams &p, uint32_t max_tiles, uint32_t cap, uint32_t max_small, bool single,
+// How the projections of a batch run: few tokens per expert on dp4a, otherwise on a tensor-core kernel.
+enum class MoePlan { DP4A, MMA, TCQ };
+
+// One grouped projection over the work list, by the kernel that the plan was made for.  cap / max_small: where the list of narrow
+// items starts inside p.tiles and how many it can hold (MMA only); scratch: the TCQ kernel's.
+int32_t grouped_projection(MoePlan plan, const MoeGemmParams &p, uint32_t max_tiles, uint32_t cap, uint32_t max_small, bool single, void *scratch,
                            cudaStream_t st) {
-    if (mma) {
+    if (plan == MoePlan::TCQ)
+        return launch_gemm_tcq_grouped(p.w, p.y, p.n_segs, p.x, p.tiles, p.n_tiles, max_tiles, p.m, p.ldc, scratch, st);
+    if (plan == MoePlan::MMA) {
         for (int s = 0; s < p.n_segs; ++s) {
             bool taken = false;
             CERA_TRY(launch_gemm_mma_grouped(p.w[s], p.x, p.tiles, p.n_tiles, max_tiles, p.m, p.y[s], p.ldc, MOE_NC_MMA, st, &taken));
@@ -443,6 +448,7 @@ int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softm
     const uint32_t hs = h->hidden, ff = h->ff, ku = h->n_used, E = h->n_expert;
     const size_t entries = n * ku, rmax = h->max_total * ku;
     const bool mma = gemm_mma_supports(h->gate->v.type, hs) && gemm_mma_supports(h->down->v.type, ff) && !moe_force_dp4a();
+    const MoePlan plan = mma ? MoePlan::MMA : MoePlan::DP4A;
     const uint32_t nc = mma ? MOE_NC_MMA : MOE_NC;
     const uint32_t max_tiles = (uint32_t)(rmax / nc + E / h->ep_size);
     uint32_t *counts_mine = (uint32_t *)(h->region + h->lay.counts) + (size_t)h->ep_rank * E;
@@ -478,7 +484,7 @@ int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softm
     p.ldc = ff;
     p.tiles = h->tiles;
     p.n_tiles = h->n_tiles;
-    CERA_TRY(grouped_projection(mma, p, max_tiles, cap, max_small, false, st));
+    CERA_TRY(grouped_projection(plan, p, max_tiles, cap, max_small, false, nullptr, st));
     const size_t worst = rmax * ff;
     moe_silu_q8_kernel<<<(unsigned)((worst + 255) / 256), 256, 0, st>>>(h->g, h->u, ff, n_recv, h->f_scales, h->f_quants, h->f_sums);
     count_launch();
@@ -492,7 +498,7 @@ int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softm
     d.ldc = hs;
     d.tiles = h->tiles;
     d.n_tiles = h->n_tiles;
-    CERA_TRY(grouped_projection(mma, d, max_tiles, cap, max_small, false, st));
+    CERA_TRY(grouped_projection(plan, d, max_tiles, cap, max_small, false, nullptr, st));
     moe_ep_return_kernel<<<(unsigned)rmax, 128, 0, st>>>(h->ep, h->lay, h->expert_out, hs, n_recv);
     count_launch();
     CERA_CUDA_TRY(cudaGetLastError());
@@ -506,6 +512,56 @@ int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softm
         if (ids_out_dev) CERA_CUDA_TRY(cudaMemcpyAsync(ids_out_dev, h->ids, entries * 4, cudaMemcpyDeviceToDevice, st));
         if (weights_out_dev) CERA_CUDA_TRY(cudaMemcpyAsync(weights_out_dev, h->weights, entries * 4, cudaMemcpyDeviceToDevice, st));
     }
+    return CERA_CUDA_OK;
+}
+
+// The layer on one GPU, n >= 1.
+int32_t moe_ffn_planned(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softmax_gate, float *out_dev, uint32_t *ids_out_dev, float *weights_out_dev,
+                        MoePlan plan, void *scratch, cudaStream_t st) {
+    const uint32_t hs = h->hidden, ff = h->ff, ku = h->n_used;
+    const size_t entries = n * ku;
+    const bool single = n == 1;
+    const uint32_t nc = single ? 1 : plan == MoePlan::TCQ ? TCQ_COLUMNS : plan == MoePlan::MMA ? MOE_NC_MMA : MOE_NC;
+    const uint32_t max_tiles = (uint32_t)(entries / nc + (single ? 0 : h->n_expert));
+    CERA_TRY(launch_quantize(x_dev, hs, n, false, h->xs, h->xq, h->xsum, st));
+    CERA_TRY(launch_moe_route(x_dev, hs, n, h->router, h->bias, hs, h->n_expert, ku, softmax_gate, 1, h->ids, h->weights, h->counts, st));
+    const uint32_t cap = (uint32_t)(h->max_total * ku + h->n_expert), max_small = h->n_expert;
+    CERA_TRY(launch_moe_plan(h->counts, h->n_expert, nc, plan == MoePlan::MMA ? nc / 2 : 0, cap, h->cursor, h->tiles, h->n_tiles, st));
+    moe_scatter_kernel<<<(unsigned)entries, 128, 0, st>>>(h->ids, ku, hs, ActView{h->xs, h->xq, h->xsum}, h->cursor, h->entry_of,
+                                                          h->g_scales, h->g_quants, h->g_sums);
+    count_launch();
+    CERA_CUDA_TRY(cudaGetLastError());
+    MoeGemmParams p{};
+    p.w[0] = h->gate->v;
+    p.w[1] = h->up->v;
+    p.y[0] = h->g;
+    p.y[1] = h->u;
+    p.n_segs = 2;
+    p.m = ff;
+    p.k = hs;
+    p.x = ActView{h->g_scales, h->g_quants, h->g_sums};
+    p.ldc = ff;
+    p.tiles = h->tiles;
+    p.n_tiles = h->n_tiles;
+    CERA_TRY(grouped_projection(plan, p, max_tiles, cap, max_small, single, scratch, st));
+    CERA_TRY(launch_silu_mul(h->g, h->u, ff, entries, h->f_scales, h->f_quants, h->f_sums, st));
+    MoeGemmParams d{};
+    d.w[0] = h->down->v;
+    d.y[0] = h->expert_out;
+    d.n_segs = 1;
+    d.m = hs;
+    d.k = ff;
+    d.x = ActView{h->f_scales, h->f_quants, h->f_sums};
+    d.ldc = hs;
+    d.tiles = h->tiles;
+    d.n_tiles = h->n_tiles;
+    CERA_TRY(grouped_projection(plan, d, max_tiles, cap, max_small, single, scratch, st));
+    const size_t total = n * hs;
+    moe_combine_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(h->expert_out, h->entry_of, h->weights, ku, hs, n, out_dev);
+    count_launch();
+    CERA_CUDA_TRY(cudaGetLastError());
+    if (ids_out_dev) CERA_CUDA_TRY(cudaMemcpyAsync(ids_out_dev, h->ids, entries * 4, cudaMemcpyDeviceToDevice, st));
+    if (weights_out_dev) CERA_CUDA_TRY(cudaMemcpyAsync(weights_out_dev, h->weights, entries * 4, cudaMemcpyDeviceToDevice, st));
     return CERA_CUDA_OK;
 }
 
@@ -583,53 +639,27 @@ int32_t cera_cuda_moe_ffn(cera_cuda_moe *h, const float *x_dev, size_t n, int32_
     cudaStream_t st = (cudaStream_t)stream;
     if (h->ep_size > 1) return moe_ffn_ep(h, x_dev, n, softmax_gate, out_dev, ids_out_dev, weights_out_dev, st);  // n == 0 still takes part
     if (n == 0) return CERA_CUDA_OK;
-    const uint32_t hs = h->hidden, ff = h->ff, ku = h->n_used;
-    const size_t entries = n * ku;
-    const bool single = n == 1;
-    // a handful of tokens: dp4a work items of 8 columns (1 for a single token); a batch: tensor-core items of 64
-    const bool mma = n >= 16 && gemm_mma_supports(h->gate->v.type, hs) && gemm_mma_supports(h->down->v.type, ff) && !moe_force_dp4a();
-    const uint32_t nc = single ? 1 : mma ? MOE_NC_MMA : MOE_NC;
-    const uint32_t max_tiles = (uint32_t)(entries / nc + (single ? 0 : h->n_expert));
-    CERA_TRY(launch_quantize(x_dev, hs, n, false, h->xs, h->xq, h->xsum, st));
-    CERA_TRY(launch_moe_route(x_dev, hs, n, h->router, h->bias, hs, h->n_expert, ku, softmax_gate, 1, h->ids, h->weights, h->counts, st));
-    const uint32_t cap = (uint32_t)(h->max_total * ku + h->n_expert), max_small = h->n_expert;
-    CERA_TRY(launch_moe_plan(h->counts, h->n_expert, nc, mma ? nc / 2 : 0, cap, h->cursor, h->tiles, h->n_tiles, st));
-    moe_scatter_kernel<<<(unsigned)entries, 128, 0, st>>>(h->ids, ku, hs, ActView{h->xs, h->xq, h->xsum}, h->cursor, h->entry_of,
-                                                          h->g_scales, h->g_quants, h->g_sums);
-    count_launch();
-    CERA_CUDA_TRY(cudaGetLastError());
-    MoeGemmParams p{};
-    p.w[0] = h->gate->v;
-    p.w[1] = h->up->v;
-    p.y[0] = h->g;
-    p.y[1] = h->u;
-    p.n_segs = 2;
-    p.m = ff;
-    p.k = hs;
-    p.x = ActView{h->g_scales, h->g_quants, h->g_sums};
-    p.ldc = ff;
-    p.tiles = h->tiles;
-    p.n_tiles = h->n_tiles;
-    CERA_TRY(grouped_projection(mma, p, max_tiles, cap, max_small, single, st));
-    CERA_TRY(launch_silu_mul(h->g, h->u, ff, entries, h->f_scales, h->f_quants, h->f_sums, st));
-    MoeGemmParams d{};
-    d.w[0] = h->down->v;
-    d.y[0] = h->expert_out;
-    d.n_segs = 1;
-    d.m = hs;
-    d.k = ff;
-    d.x = ActView{h->f_scales, h->f_quants, h->f_sums};
-    d.ldc = hs;
-    d.tiles = h->tiles;
-    d.n_tiles = h->n_tiles;
-    CERA_TRY(grouped_projection(mma, d, max_tiles, cap, max_small, single, st));
-    const size_t total = n * hs;
-    moe_combine_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(h->expert_out, h->entry_of, h->weights, ku, hs, n, out_dev);
-    count_launch();
-    CERA_CUDA_TRY(cudaGetLastError());
-    if (ids_out_dev) CERA_CUDA_TRY(cudaMemcpyAsync(ids_out_dev, h->ids, entries * 4, cudaMemcpyDeviceToDevice, st));
-    if (weights_out_dev) CERA_CUDA_TRY(cudaMemcpyAsync(weights_out_dev, h->weights, entries * 4, cudaMemcpyDeviceToDevice, st));
-    return CERA_CUDA_OK;
+    const uint32_t hs = h->hidden, ff = h->ff;
+    const size_t entries = n * h->n_used;
+    // a handful of tokens: dp4a work items of 8 columns (1 for a single token); a batch: tensor-core items of 64, or of 128 straight
+    // from the quantized bytes.  The latter converts an expert's weights whatever the number of its tokens; measured (whole layer,
+    // us, it / the other): Q8_0 (else on dp4a) 448 / 426 at 8 entries per expert, 453 / 759 at 16 (32 experts, 4 used, 2048 x 1792);
+    // Q4_0 (else on mma.sync) 361 / 347 at 32, 424 / 540 at 64; 16 experts: 202 / 158 at 16, 221 / 291 at 32.
+    MoePlan plan = MoePlan::DP4A;
+    void *scratch = nullptr;
+    if (n >= 16 && !moe_force_dp4a()) {
+        const bool mma = gemm_mma_supports(h->gate->v.type, hs) && gemm_mma_supports(h->down->v.type, ff);
+        if (entries >= (size_t)h->n_expert * (mma ? 40 : 12) && gemm_tcq_supports(h->gate->v.type, hs) && gemm_tcq_supports(h->down->v.type, ff)) {
+            const uint32_t items = (uint32_t)(entries / TCQ_COLUMNS + h->n_expert);
+            keep_stream_pool();
+            if (cudaMallocAsync(&scratch, gemm_tcq_grouped_scratch(hs > ff ? hs : ff, items), st) == cudaSuccess) plan = MoePlan::TCQ;
+            else cudaGetLastError();
+        }
+        if (plan == MoePlan::DP4A && mma) plan = MoePlan::MMA;
+    }
+    const int32_t rc = moe_ffn_planned(h, x_dev, n, softmax_gate, out_dev, ids_out_dev, weights_out_dev, plan, scratch, st);
+    if (scratch) cudaFreeAsync(scratch, st);  // after the kernels above, in stream order
+    return rc;
 }
 
 size_t cera_cuda_moe_memory_bytes(const cera_cuda_moe *h) {

@@ -92,6 +92,17 @@ int32_t launch_moe_route(const float *x, size_t ld_x, size_t n, const float *rou
                          uint32_t n_used, int softmax_gate, int renorm, uint32_t *ids, float *weights, uint32_t *counts, cudaStream_t st);
 int32_t launch_moe_plan(uint32_t *counts, uint32_t n_expert, uint32_t nc, uint32_t small_nc, uint32_t cap, uint32_t *cursor, MoeTile *tiles,
                         uint32_t *n_tiles, cudaStream_t st);
+// tcgen05 product straight from the quantized bytes (gemm_tcq.cu).  The plain form takes Q4_0, Q4_1, Q8_0 and Q6_K where it is the
+// faster one; *taken = false: not its case, nothing launched.  The grouped form takes every block format (K-quants: k a multiple
+// of 256), up to two matrices (gate, up), work items of up to TCQ_COLUMNS columns and the caller's scratch.
+constexpr uint32_t TCQ_COLUMNS = 128;
+bool gemm_tcq_supports(int type, size_t k);
+int32_t launch_gemm_tcq(const WeightView &w, const ActView &x, size_t n, float *out, size_t ldy, size_t ldc, int epilogue, cudaStream_t st, bool *taken);
+size_t gemm_tcq_grouped_scratch(size_t k, uint32_t max_tiles);  // bytes
+int32_t launch_gemm_tcq_grouped(const WeightView *ws, float *const *outs, int n_segs, const ActView &x, const MoeTile *tiles, const uint32_t *n_tiles,
+                                uint32_t max_tiles, uint32_t rows_per_expert, size_t ldc, void *scratch, cudaStream_t st);
+// Keeps the current device's stream-ordered pool from handing its memory back at every synchronisation (gemm_tc.cu).
+void keep_stream_pool();
 // The tensor-core GEMM over a device-side list of such items (one column tile of up to `bn` = 64 or 32 columns per item):
 // w stacks `rows_per_expert` rows per expert; cell (row i of the expert, column c) goes to out[c * ldc + i].
 // *taken = false: no tensor-core path for this weight type / shape.

@@ -185,6 +185,31 @@ def test_gemm_tensor_core_shapes(t, m, n, k):
         assert_close(cb.gemm_preq(w, acts, out2).cpu().numpy(), want, f"{O.NAMES[t]} {m}x{n}x{k} (weight image)")
 
 
+@pytest.mark.parametrize("t,m,n,k", [
+    # Q8_0 / Q4_1: 16 columns up (48 for small matrices), any k: half a stage, one stage, ragged 128s, a split of k, one row
+    (O.Q8_0, 1, 48, 32), (O.Q8_0, 127, 64, 96), (O.Q8_0, 129, 65, 320), (O.Q8_0, 300, 129, 64), (O.Q8_0, 130, 16, 32800), (O.Q8_0, 2048, 17, 2080),
+    (O.Q8_0, 4100, 33, 1024), (O.Q4_1, 128, 48, 160), (O.Q4_1, 200, 200, 2048), (O.Q4_1, 2100, 31, 2016), (O.Q4_1, 33, 128, 4096),
+    # Q4_0 / Q6_K: 48 columns up, from 2^22 weights on
+    (O.Q4_0, 2050, 48, 2080), (O.Q4_0, 2049, 64, 2048), (O.Q4_0, 131, 65, 32800), (O.Q4_0, 4096, 128, 1056), (O.Q4_0, 4097, 257, 1024),
+    (O.Q6_K, 2049, 48, 2048), (O.Q6_K, 300, 63, 14336), (O.Q6_K, 4223, 130, 1024), (O.Q6_K, 4096, 300, 2816)])
+def test_gemm_from_quantized_bytes(t, m, n, k):
+    """The tcgen05 product that converts the weights itself, at the edges of its rows, columns, stages and of its rule; both cell layouts
+    that its splits of k and its direct stores write."""
+    torch = need_gpu()
+    import cera_b200 as cb
+    raw = cb.quantize_weights(t, cb.synth_normal(m * k, seed=7 * t + m + n, sigma=0.02)).cpu().numpy()
+    X = cb.synth_normal(n * k, seed=n + k, sigma=1.0)
+    acts = cb.quantize_q8_0(X, k=k, n=n)
+    w = cb.QuantWeight(t, m, k, raw)
+    out = torch.full((m, n), float("nan"), device="cuda")
+    got = cb.gemm_preq(w, acts, out).cpu().numpy()
+    want = O.gemm_preq(t, raw, acts.scales.cpu().numpy(), acts.quants.cpu().numpy(), m, n, k, avx2=O.has_avx2(), threads=4)
+    # the block sums are exact; what is left is the order of k / 32 f32 additions: 2e-6 of the result's size (measured 2e-7)
+    err = np.linalg.norm((got - want).astype(np.float64)) / np.linalg.norm(want.astype(np.float64))
+    assert err < 2e-6, f"{O.NAMES[t]} {m}x{n}x{k}: {err}"
+    assert_close(got, want, f"{O.NAMES[t]} {m}x{n}x{k}")
+
+
 def test_gemm_on_reference_fixtures():
     """The reference's own extreme fixtures (-128 weights, +/-127 activations)."""
     torch = need_gpu()

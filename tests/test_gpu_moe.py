@@ -102,6 +102,16 @@ def test_routed_ffn_batches_on_the_tensor_core_path(t_name, n):
     _run(getattr(cb, t_name), n_expert=8, n_used=2, hidden=512, ff=256, n=n, seed=61)
 
 
+@pytest.mark.parametrize("t_name,hidden,ff,n", [("Q8_0", 256, 96, 50), ("Q8_0", 288, 160, 130), ("Q4_1", 256, 128, 60), ("Q4_0", 512, 384, 170), ("Q4_0", 256, 128, 400),
+                                                ("Q4_K", 512, 256, 165), ("Q6_K", 256, 512, 180)])
+def test_routed_ffn_from_quantized_bytes(t_name, hidden, ff, n):
+    """Enough entries per expert for the 128-column work items: two matrices in one launch, widths that fill no row tile or stage, experts
+    with several items."""
+    need_gpu()
+    import cera_b200 as cb
+    _run(getattr(cb, t_name), n_expert=8, n_used=2, hidden=hidden, ff=ff, n=n, seed=71)
+
+
 def test_selection_bias_steers_rank_not_weight():
     """exp_probs_b changes which experts are picked; the combine weights stay the unbiased probabilities."""
     need_gpu()
