@@ -1,16 +1,18 @@
-// Causal attention of a chunk of prompt tokens (prefill), tiled through shared memory.
+// Causal attention of a chunk of prompt tokens (prefill) on the tensor cores, in f32 accuracy.
 //
-// A CTA owns one KV head and PA_BQ consecutive query tokens; warp w owns query w of the block with all G query heads of
-// the group, so every staged K / V row serves PA_BQ * G (query, head) pairs.  Keys go by in tiles of 32, double-buffered
-// with cp.async:
-//   scores : lane = key.  The lane keeps 32 dims of its K row in registers at a time and reads the queries as
-//            shared-memory broadcasts: no shuffle per key, four FMAs per broadcast load.
-//   softmax: one running maximum / sum per (query, head), updated once per tile (two warp reductions and ONE expf per
-//            key, against a reduction and two expf per key in the one-warp-per-row kernel).
-//   P.V    : lane = four output dims.  The tile's probabilities sit in shared memory, V rows are read as float4 and
-//            shared by the G heads.
-// Rows are padded to 132 floats (f16 caches: staged as stored, 272 bytes per row, widened on the way to the registers),
-// so the lane = key reads (stride one row) hit all 32 banks.
+// A CTA owns one KV head and WARPS * 16 rows, a row = (query, head of the group), so every staged K / V row serves all of them.
+// A warp holds its sixteen queries in registers and walks the keys in tiles as flash attention does: scores, running softmax,
+// weighted values.  The products are mma.sync on f16 halves: a float enters as a high and a low f16, 22 bits of it, and the
+// product of two such floats is three MMAs - low x high, high x low, high x high, in this order, so that the sums are truncated
+// at full size by the last third only; an f16 cache is exact as it is and takes two.  Operands are scaled by powers of two
+// (queries by row, an f32 cache's K and V by tile, probabilities by 2^14) so that f16 neither overflows nor becomes subnormal
+// where it matters.  A tile's weighted values start from zero and are added to the running output in f32.
+//
+// What bounds it: the tensor pipe at the rate of mma.sync, 256 to 384 MMAs per 16 rows x 64 keys beside 32 exponentials a lane.  It stays
+// on mma.sync because scores, probabilities and their halves live in registers between the two products.
+// Tiles are staged by cp.async: f16 as stored, two tiles deep; f32 raw, two to three tiles ahead, and split into halves by the whole CTA.
+// 32 heads of 128 in groups of 4: 512 tokens 50 us over an f16 cache, 82 us over f32 (153, 100 with FMAs on the CUDA cores); 2047
+// tokens 345, 576 us (1125, 1366).  Error against 64 bits 3.0e-7 and 3.7e-7 (4.0e-7, 5.7e-7).
 //
 // Arithmetic contract: cera/src/backend/cpu.rs:4028-4241 (scaled dot, causal limit start_pos + j, online softmax);
 // the f32 summation order is this kernel's own.
@@ -20,48 +22,328 @@
 #include <cstring>
 
 #include "act.cuh"
+#include "mma.cuh"
 #include "ops.h"
-#include "tma.cuh"
 
 namespace cera {
 
 namespace {
 
+template <int HD, bool F16>
+struct Pa {
+    static constexpr int TK = F16 ? 64 : 32;          // keys per tile
+    static constexpr int ROW = HD * 2 + 16;           // bytes of a staged f16 row: eight rows of an ldmatrix hit all banks
+    static constexpr int TILE = TK * ROW;
+    static constexpr int RAW = TK * HD * 4;           // an f32 tile as stored
+    static constexpr int STAGES = F16 ? 2 : 3;        // tiles in flight or in use as they come from the cache
+    // f16: [stage][K, V]; f32: [K high, K low, V high, V low], [stage][raw K, raw V]
+    static constexpr size_t SMEM = F16 ? STAGES * 2 * TILE : 4 * TILE + STAGES * 2 * RAW;
+};
+
+// Biased exponent of the power of two that brings values up to mx (its float's bits) below 2^14; 254 - it is the inverse's.
+__device__ __forceinline__ uint32_t pa_up(uint32_t mx_bits) {
+    const uint32_t e = mx_bits >> 23;
+    return min(267u - e, 253u);
+}
+__device__ __forceinline__ float pa_pow2(uint32_t biased) { return __uint_as_float(biased << 23); }
+
+template <int HD, bool F16, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) attn_prefill_mma_kernel(const float *__restrict__ q, const uint8_t *__restrict__ kc,
+                                                                      const uint8_t *__restrict__ vc, uint32_t n_heads, uint32_t n_kv_heads, uint32_t n,
+                                                                      uint32_t start_pos, float scale, float *__restrict__ out) {
+    using S = Pa<HD, F16>;
+    extern __shared__ __align__(16) uint8_t pa_smem[];
+    __shared__ uint32_t tile_max[2][2];  // f32: bits of the largest |k| and |v| of a tile, by parity
+    constexpr int TK = S::TK, NT = TK / 8, KS = HD / 16, KK = TK / 16, ND = HD / 8, THREADS = WARPS * 32, ES = F16 ? 2 : 4;
+    constexpr int PIECES = HD * ES / 16;  // 16-byte pieces of a cache row
+    pdl_trigger();
+    pdl_wait();
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kvh = blockIdx.x, G = n_heads / n_kv_heads;
+    const uint32_t rows = n * G, r_cta = (gridDim.y - 1 - blockIdx.y) * WARPS * 16;  // the longest rows start first
+    const size_t kv_dim = (size_t)n_kv_heads * HD, q_dim = (size_t)n_heads * HD;
+    const uint32_t cta_kv = start_pos + (min(r_cta + WARPS * 16, rows) - 1) / G + 1;  // keys the CTA's last query sees
+    const uint32_t n_tiles = (cta_kv + TK - 1) / TK;
+    const uint8_t *k_src = kc + (size_t)kvh * HD * ES, *v_src = vc + (size_t)kvh * HD * ES;
+
+    auto issue = [&](uint32_t t) {
+        uint8_t *kd = F16 ? pa_smem + (t & 1) * 2 * S::TILE : pa_smem + 4 * S::TILE + t % S::STAGES * 2 * S::RAW, *vd = kd + (F16 ? S::TILE : S::RAW);
+        constexpr int ROW = F16 ? S::ROW : HD * 4;
+        for (uint32_t i = tid; i < TK * PIECES && t < n_tiles; i += THREADS) {
+            const uint32_t r = i / PIECES, pc = i % PIECES;
+            const size_t src = (size_t)min(t * TK + r, cta_kv - 1) * kv_dim * ES + pc * 16;  // rows past the limit are masked; keep the read in range
+            tma::cp_async16(kd + r * ROW + pc * 16, k_src + src);
+            tma::cp_async16(vd + r * ROW + pc * 16, v_src + src);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    issue(0);
+    if constexpr (!F16) {
+        issue(1);
+        issue(2);
+    }
+    if (tid < 4) tile_max[tid >> 1][tid & 1] = 0;
+
+    // ---- queries of the warp's rows, as A fragments: rows g and g + 8, columns 16 ks + 2 c + {0, 1, 8, 9}
+    const uint32_t g = lane >> 2, c = lane & 3, r_warp = r_cta + warp * 16;
+    const bool live = r_warp < rows;
+    uint32_t qh[KS][4], ql[KS][4];
+    float qf[2];      // 2^-u of both rows
+    uint32_t lim[2];  // last key of both rows
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t r = min(r_warp + g + 8 * h, rows - 1);
+        lim[h] = start_pos + r / G;
+        const float *src = q + (size_t)(r / G) * q_dim + ((size_t)kvh * G + r % G) * HD + 2 * c;
+        float2 v[KS][2];
+        float mx = 0.0f;
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                v[ks][j] = *reinterpret_cast<const float2 *>(src + 16 * ks + 8 * j);
+                mx = fmaxf(mx, fmaxf(fabsf(v[ks][j].x), fabsf(v[ks][j].y)));
+            }
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        const uint32_t up = pa_up(__float_as_uint(mx));
+        const float f = pa_pow2(up);
+        qf[h] = pa_pow2(254u - up);
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) split_f16(v[ks][j].x * f, v[ks][j].y * f, qh[ks][2 * j + h], ql[ks][2 * j + h]);
+    }
+
+    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f}, o[ND][4];
+#pragma unroll
+    for (int i = 0; i < ND; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[i][j] = 0.0f;
+    const uint32_t warp_kv = live ? start_pos + (min(r_warp + 16, rows) - 1) / G + 1 : 0;
+
+    for (uint32_t t = 0; t < n_tiles; ++t) {
+        float kf = 1.0f, vf = 1.0f / 16384.0f;  // 2^-u of the tile's K; of its V and of the probabilities
+        const uint8_t *kt, *vt;
+        if constexpr (F16) {
+            if (t + 1 < n_tiles) {
+                issue(t + 1);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
+            __syncthreads();
+            kt = pa_smem + (t & 1) * 2 * S::TILE;
+            vt = kt + S::TILE;
+        } else {
+            asm volatile("cp.async.wait_group 2;" ::: "memory");
+            __syncthreads();  // the raw tile is there, and everyone is done with the halves of the tile before
+            const float4 *raw = reinterpret_cast<const float4 *>(pa_smem + 4 * S::TILE + t % S::STAGES * 2 * S::RAW);
+            constexpr int QUADS = TK * HD / 4;
+            float mx[2] = {0.0f, 0.0f};
+#pragma unroll
+            for (int w = 0; w < 2; ++w) {
+#pragma unroll 4
+                for (uint32_t i = tid; i < QUADS; i += THREADS) {
+                    const float4 x = raw[w * QUADS + i];
+                    mx[w] = fmaxf(mx[w], fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
+                }
+#pragma unroll
+                for (int s = 16; s > 0; s >>= 1) mx[w] = fmaxf(mx[w], __shfl_xor_sync(0xffffffffu, mx[w], s));
+                if (lane == 0) atomicMax(&tile_max[t & 1][w], __float_as_uint(mx[w]));  // magnitudes order like their bits
+            }
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < 2; ++w) {
+                const uint32_t up = pa_up(tile_max[t & 1][w]);
+                const float f = pa_pow2(up);
+                if (w == 0) kf = pa_pow2(254u - up);
+                else vf = pa_pow2(254u - up) * (1.0f / 16384.0f);
+                uint8_t *hi_t = pa_smem + w * 2 * S::TILE, *lo_t = hi_t + S::TILE;
+#pragma unroll 4
+                for (uint32_t i = tid; i < QUADS; i += THREADS) {
+                    const float4 x = raw[w * QUADS + i];
+                    uint2 hi, lo;
+                    split_f16(x.x * f, x.y * f, hi.x, lo.x);
+                    split_f16(x.z * f, x.w * f, hi.y, lo.y);
+                    const uint32_t off = i / (HD / 4) * S::ROW + i % (HD / 4) * 8;
+                    *reinterpret_cast<uint2 *>(hi_t + off) = hi;
+                    *reinterpret_cast<uint2 *>(lo_t + off) = lo;
+                }
+            }
+            __syncthreads();
+            if (tid < 2) tile_max[t & 1][tid] = 0;  // for the tile after the next
+            issue(t + 3);
+            kt = pa_smem;
+            vt = pa_smem + 2 * S::TILE;
+        }
+        if (t * TK < warp_kv) {
+            // ---- scores: keys 8 nt + 2 c + {0, 1} of rows g (0, 1) and g + 8 (2, 3)
+            float s[NT][4];
+            const uint8_t *kl = kt + (lane & 7) * S::ROW + (lane >> 3) * 16;
+            // two key groups side by side, so that an MMA does not wait for the one before it
+#pragma unroll
+            for (int nt = 0; nt < NT; nt += 2) {
+                float u[2][4];  // the second half of the high products on its own: fewer truncations, more chains
+#pragma unroll
+                for (int p = 0; p < 2; ++p)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) s[nt + p][j] = u[p][j] = 0.0f;
+                uint32_t b[2][KS / 2][4];
+                if constexpr (!F16) {
+#pragma unroll
+                    for (int k2 = 0; k2 < KS / 2; ++k2)
+#pragma unroll
+                        for (int p = 0; p < 2; ++p) ldsm4(b[p][k2], kl + S::TILE + (nt + p) * 8 * S::ROW + k2 * 64);
+#pragma unroll
+                    for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+                        for (int p = 0; p < 2; ++p) mma_f16(s[nt + p], qh[ks], b[p][ks / 2][2 * (ks & 1)], b[p][ks / 2][2 * (ks & 1) + 1]);
+                }
+#pragma unroll
+                for (int k2 = 0; k2 < KS / 2; ++k2)
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) ldsm4(b[p][k2], kl + (nt + p) * 8 * S::ROW + k2 * 64);
+#pragma unroll
+                for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) mma_f16(s[nt + p], ql[ks], b[p][ks / 2][2 * (ks & 1)], b[p][ks / 2][2 * (ks & 1) + 1]);
+#pragma unroll
+                for (int ks = 0; ks < KS / 2; ++ks)
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) {
+                        constexpr int H = KS / 2;
+                        mma_f16(s[nt + p], qh[ks], b[p][ks / 2][2 * (ks & 1)], b[p][ks / 2][2 * (ks & 1) + 1]);
+                        mma_f16(u[p], qh[H + ks], b[p][(H + ks) / 2][2 * (ks & 1)], b[p][(H + ks) / 2][2 * (ks & 1) + 1]);
+                    }
+#pragma unroll
+                for (int p = 0; p < 2; ++p)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) s[nt + p][j] += u[p][j];
+            }
+            // ---- running softmax
+            const uint32_t key0 = t * TK + 2 * c;
+            float mx[2] = {-INFINITY, -INFINITY}, corr[2];
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const bool seen = key0 + 8 * nt + (j & 1) <= lim[j >> 1];
+                    s[nt][j] = seen ? __fmul_rn(s[nt][j] * qf[j >> 1] * kf, scale) : -INFINITY;
+                    mx[j >> 1] = fmaxf(mx[j >> 1], s[nt][j]);
+                }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
+                mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
+                const float m_new = fmaxf(m_run[h], mx[h]);  // finite: key 0 is seen by every row
+                corr[h] = m_run[h] == -INFINITY ? 0.0f : ggml_expf(__fsub_rn(m_run[h], m_new));
+                m_run[h] = m_new;
+                l_run[h] *= corr[h];
+            }
+            uint32_t ph[KK][4], pl[KK][4];
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float p[2];
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const bool seen = key0 + 8 * nt + j <= lim[h];
+                        p[j] = seen ? ggml_expf(__fsub_rn(s[nt][2 * h + j], m_run[h])) : 0.0f;
+                        l_run[h] += p[j];
+                    }
+                    split_f16(p[0] * 16384.0f, p[1] * 16384.0f, ph[nt / 2][2 * (nt & 1) + h], pl[nt / 2][2 * (nt & 1) + h]);
+                }
+            // ---- weighted values: dims 8 nd + 2 c + {0, 1}
+            const uint8_t *vl = vt + ((lane >> 3) * 8 + (lane & 7)) * S::ROW;
+            constexpr int W = 4;  // groups of dims side by side
+#pragma unroll
+            for (int nd = 0; nd < ND; nd += W) {
+                float a[W][4];
+#pragma unroll
+                for (int p = 0; p < W; ++p)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) a[p][j] = 0.0f;
+                uint32_t b[W][KK / 2][4];
+                if constexpr (!F16) {
+#pragma unroll
+                    for (int k2 = 0; k2 < KK / 2; ++k2)
+#pragma unroll
+                        for (int p = 0; p < W; ++p) ldsm4_trans(b[p][k2], vl + S::TILE + k2 * 32 * S::ROW + (nd + p) * 16);
+#pragma unroll
+                    for (int kk = 0; kk < KK; ++kk)
+#pragma unroll
+                        for (int p = 0; p < W; ++p) mma_f16(a[p], ph[kk], b[p][kk / 2][2 * (kk & 1)], b[p][kk / 2][2 * (kk & 1) + 1]);
+                }
+#pragma unroll
+                for (int k2 = 0; k2 < KK / 2; ++k2)
+#pragma unroll
+                    for (int p = 0; p < W; ++p) ldsm4_trans(b[p][k2], vl + k2 * 32 * S::ROW + (nd + p) * 16);
+#pragma unroll
+                for (int kk = 0; kk < KK; ++kk)
+#pragma unroll
+                    for (int p = 0; p < W; ++p) mma_f16(a[p], pl[kk], b[p][kk / 2][2 * (kk & 1)], b[p][kk / 2][2 * (kk & 1) + 1]);
+#pragma unroll
+                for (int kk = 0; kk < KK; ++kk)
+#pragma unroll
+                    for (int p = 0; p < W; ++p) mma_f16(a[p], ph[kk], b[p][kk / 2][2 * (kk & 1)], b[p][kk / 2][2 * (kk & 1) + 1]);
+#pragma unroll
+                for (int p = 0; p < W; ++p)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) o[nd + p][j] = fmaf(a[p][j], vf, o[nd + p][j] * corr[j >> 1]);
+            }
+        }
+        if constexpr (F16) __syncthreads();  // the stage is refilled by the copy issued in the next iteration
+    }
+
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 1);
+        l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 2);
+        const uint32_t r = r_warp + g + 8 * h;
+        if (r >= rows) continue;
+        const float inv = 1.0f / l_run[h];
+        float *dst = out + (size_t)(r / G) * q_dim + ((size_t)kvh * G + r % G) * HD + 2 * c;
+#pragma unroll
+        for (int nd = 0; nd < ND; ++nd) *reinterpret_cast<float2 *>(dst + 8 * nd) = make_float2(o[nd][2 * h] * inv, o[nd][2 * h + 1] * inv);
+    }
+}
+
+template <int HD, bool F16, int WARPS>
+int32_t launch_mma(const float *q, const uint8_t *kc, const uint8_t *vc, uint32_t nh, uint32_t nkv, uint32_t n, uint32_t sp, float scale, float *out,
+                   cudaStream_t st) {
+    constexpr size_t smem = Pa<HD, F16>::SMEM;
+    static thread_local int configured_dev = -1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (configured_dev != dev) {
+        CERA_CUDA_TRY(cudaFuncSetAttribute(attn_prefill_mma_kernel<HD, F16, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        configured_dev = dev;
+    }
+    const dim3 grid(nkv, (unsigned)(((size_t)n * (nh / nkv) + WARPS * 16 - 1) / (WARPS * 16)));
+    count_launch();
+    return check_cuda(launch_k(attn_prefill_mma_kernel<HD, F16, WARPS>, grid, dim3(WARPS * 32), smem, st, q, kc, vc, nh, nkv, n, sp, scale, out),
+                      "prefill attention (tensor cores) launch");
+}
+
+// ---- few rows over an f32 cache -----------------------------------------------------------------------------------------
+// With one or two warps' worth of rows the splitting of every tile above costs more than its MMAs save (32 heads in groups of 4, 5
+// queries after 4000 positions: 450 against 420 us; 2 after 3000: 334 against 275).  Here a CTA owns one KV head and PA_BQ
+// consecutive queries; warp w owns query w with all G heads of the group.  Keys go by in tiles of 32, double-buffered with cp.async:
+//   scores : lane = key.  The lane keeps 32 dims of its K row in registers at a time and reads the queries as
+//            shared-memory broadcasts: no shuffle per key, four FMAs per broadcast load.
+//   softmax: one running maximum / sum per (query, head), updated once per tile.
+//   P.V    : lane = four output dims.  The tile's probabilities sit in shared memory, V rows are read as float4 and
+//            shared by the G heads.
+// Rows are padded to 132 floats, so the lane = key reads (stride one row) hit all 32 banks.
 constexpr int PA_WARPS = 8, PA_THREADS = PA_WARPS * 32, PA_BQ = PA_WARPS;
 constexpr int PA_TK = 32;        // keys per tile
 constexpr int PA_HD = 128;       // head dim
-constexpr int PA_ROW_F32 = 528, PA_ROW_F16 = 272;   // bytes per staged row (512 / 256 of data + padding)
+constexpr int PA_ROW = 528;      // bytes per staged row (512 of data + padding)
 
-template <int G, bool F16>
+template <int G>
 constexpr size_t pa_smem_bytes() {
-    return (size_t)2 * 2 * PA_TK * (F16 ? PA_ROW_F16 : PA_ROW_F32) + (size_t)(PA_BQ * G * PA_HD + PA_WARPS * G * PA_TK) * sizeof(float);
-}
-
-// Eight consecutive elements of a staged row as two float4.
-template <bool F16>
-__device__ __forceinline__ void pa_load8(const uint8_t *row, int first, float4 &a, float4 &b) {
-    if (F16) {
-        const uint4 r = *reinterpret_cast<const uint4 *>(row + first * 2);
-        const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&r.x));
-        const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&r.y));
-        const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&r.z));
-        const float2 f3 = __half22float2(*reinterpret_cast<const __half2 *>(&r.w));
-        a = make_float4(f0.x, f0.y, f1.x, f1.y);
-        b = make_float4(f2.x, f2.y, f3.x, f3.y);
-    } else {
-        a = *reinterpret_cast<const float4 *>(row + first * 4);
-        b = *reinterpret_cast<const float4 *>(row + first * 4 + 16);
-    }
-}
-template <bool F16>
-__device__ __forceinline__ float4 pa_load4(const uint8_t *row, int first) {
-    if (F16) {
-        const uint2 r = *reinterpret_cast<const uint2 *>(row + first * 2);
-        const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&r.x));
-        const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&r.y));
-        return make_float4(f0.x, f0.y, f1.x, f1.y);
-    }
-    return *reinterpret_cast<const float4 *>(row + first * 4);
+    return (size_t)2 * 2 * PA_TK * PA_ROW + (size_t)(PA_BQ * G * PA_HD + PA_WARPS * G * PA_TK) * sizeof(float);
 }
 
 __device__ __forceinline__ float pa_warp_max(float v) {
@@ -70,13 +352,13 @@ __device__ __forceinline__ float pa_warp_max(float v) {
     return v;
 }
 
-template <int G, bool F16>
+template <int G>
 __global__ void __launch_bounds__(PA_THREADS) attn_prefill_tiled_kernel(const float *__restrict__ q, const uint8_t *__restrict__ kc,
                                                                         const uint8_t *__restrict__ vc, uint32_t n_heads,
                                                                         uint32_t n_kv_heads, uint32_t n, uint32_t start_pos,
                                                                         float scale, float *__restrict__ out) {
     extern __shared__ __align__(16) uint8_t pa_smem[];
-    constexpr int ROWB = F16 ? PA_ROW_F16 : PA_ROW_F32, ESZ = F16 ? 2 : 4, STAGE = PA_TK * ROWB;
+    constexpr int ROWB = PA_ROW, ESZ = 4, STAGE = PA_TK * ROWB;
     constexpr int PIECES = PA_HD * ESZ / 16;          // 16-byte pieces per cache row
     uint8_t *ks = pa_smem;                            // [2][32][ROWB]
     uint8_t *vs = ks + 2 * STAGE;                     // [2][32][ROWB]
@@ -148,7 +430,7 @@ __global__ void __launch_bounds__(PA_THREADS) attn_prefill_tiled_kernel(const fl
             for (int dc = 0; dc < PA_HD / 32; ++dc) {
                 float4 kr[8];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) pa_load8<F16>(kt, dc * 32 + 8 * i, kr[2 * i], kr[2 * i + 1]);
+                for (int i = 0; i < 8; ++i) kr[i] = *reinterpret_cast<const float4 *>(kt + (dc * 32 + 4 * i) * 4);
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
 #pragma unroll
@@ -178,10 +460,10 @@ __global__ void __launch_bounds__(PA_THREADS) attn_prefill_tiled_kernel(const fl
             __syncwarp();
 #pragma unroll
             for (int k4 = 0; k4 < PA_TK / 4; ++k4) {
-                const float4 v0 = pa_load4<F16>(vt + (4 * k4 + 0) * ROWB, 4 * lane);
-                const float4 v1 = pa_load4<F16>(vt + (4 * k4 + 1) * ROWB, 4 * lane);
-                const float4 v2 = pa_load4<F16>(vt + (4 * k4 + 2) * ROWB, 4 * lane);
-                const float4 v3 = pa_load4<F16>(vt + (4 * k4 + 3) * ROWB, 4 * lane);
+                const float4 v0 = *reinterpret_cast<const float4 *>(vt + (4 * k4 + 0) * ROWB + 16 * lane);
+                const float4 v1 = *reinterpret_cast<const float4 *>(vt + (4 * k4 + 1) * ROWB + 16 * lane);
+                const float4 v2 = *reinterpret_cast<const float4 *>(vt + (4 * k4 + 2) * ROWB + 16 * lane);
+                const float4 v3 = *reinterpret_cast<const float4 *>(vt + (4 * k4 + 3) * ROWB + 16 * lane);
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
                     const float4 pp = *reinterpret_cast<const float4 *>(pw + g * PA_TK + 4 * k4);
@@ -210,27 +492,27 @@ __global__ void __launch_bounds__(PA_THREADS) attn_prefill_tiled_kernel(const fl
     }
 }
 
-template <int G, bool F16>
+template <int G>
 int32_t launch_tiled(const float *q, const uint8_t *kc, const uint8_t *vc, uint32_t nh, uint32_t nkv, uint32_t n, uint32_t sp,
                      float scale, float *out, cudaStream_t st) {
-    constexpr size_t smem = pa_smem_bytes<G, F16>();
+    constexpr size_t smem = pa_smem_bytes<G>();
     static thread_local int configured_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_dev != dev) {
-        CERA_CUDA_TRY(cudaFuncSetAttribute(attn_prefill_tiled_kernel<G, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CERA_CUDA_TRY(cudaFuncSetAttribute(attn_prefill_tiled_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured_dev = dev;
     }
     const dim3 grid(nkv, (n + PA_BQ - 1) / PA_BQ);
     count_launch();
-    return check_cuda(launch_k(attn_prefill_tiled_kernel<G, F16>, grid, dim3(PA_THREADS), smem, st, q, kc, vc, nh, nkv, n, sp, scale, out),
+    return check_cuda(launch_k(attn_prefill_tiled_kernel<G>, grid, dim3(PA_THREADS), smem, st, q, kc, vc, nh, nkv, n, sp, scale, out),
                       "prefill attention (tiled) launch");
 }
 
 }  // namespace
 
-// f32 or f16 cache, head_dim 128, group size 1, 2, 4 or 8, 16-byte aligned operands; anything else: *taken = false and the
-// caller runs the one-warp-per-row kernel.  CERA_CUDA_PREFILL_ATTN=rows turns this kernel off.
+// f32 or f16 cache, head_dim 64 or 128, 16-byte aligned operands; anything else: *taken = false and the caller runs the
+// one-warp-per-row kernel.  CERA_CUDA_PREFILL_ATTN=rows turns this kernel off.
 int32_t launch_prefill_attention_tiled(const float *q, const void *kc, const void *vc, int kv_f16, size_t n_heads,
                                        size_t n_kv_heads, size_t head_dim, size_t n, size_t start_pos, float scale, float *out,
                                        cudaStream_t st, bool *taken) {
@@ -239,24 +521,24 @@ int32_t launch_prefill_attention_tiled(const float *q, const void *kc, const voi
         const char *e = getenv("CERA_CUDA_PREFILL_ATTN");
         return e && strcmp(e, "rows") == 0;
     }();
-    if (off || head_dim != PA_HD || n == 0) return CERA_CUDA_OK;
+    if (off || (head_dim != 64 && head_dim != 128) || n == 0) return CERA_CUDA_OK;
     if (((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc | (uintptr_t)out) % 16) return CERA_CUDA_OK;
-    const size_t g = n_heads / n_kv_heads;
     const uint32_t nh = (uint32_t)n_heads, nkv = (uint32_t)n_kv_heads, nn = (uint32_t)n, sp = (uint32_t)start_pos;
     const uint8_t *kf = (const uint8_t *)kc, *vf = (const uint8_t *)vc;
     *taken = true;
-#define CERA_PA_CASE(GG)                                                                              \
-    case GG:                                                                                          \
-        return kv_f16 ? launch_tiled<GG, true>(q, kf, vf, nh, nkv, nn, sp, scale, out, st)            \
-                      : launch_tiled<GG, false>(q, kf, vf, nh, nkv, nn, sp, scale, out, st)
-    switch (g) {
-        CERA_PA_CASE(1);
-        CERA_PA_CASE(2);
-        CERA_PA_CASE(4);
-        CERA_PA_CASE(8);
-        default: *taken = false; return CERA_CUDA_OK;
+    const size_t G = n_heads / n_kv_heads;
+    if (!kv_f16 && head_dim == PA_HD && n * G <= 32) {
+        switch (G) {
+            case 1: return launch_tiled<1>(q, kf, vf, nh, nkv, nn, sp, scale, out, st);
+            case 2: return launch_tiled<2>(q, kf, vf, nh, nkv, nn, sp, scale, out, st);
+            case 4: return launch_tiled<4>(q, kf, vf, nh, nkv, nn, sp, scale, out, st);
+            case 8: return launch_tiled<8>(q, kf, vf, nh, nkv, nn, sp, scale, out, st);
+        }
     }
-#undef CERA_PA_CASE
+    // f16: 64 rows per CTA, two CTAs on an SM; f32, whose tiles every CTA splits anew: 128
+    if (head_dim == 128)
+        return kv_f16 ? launch_mma<128, true, 4>(q, kf, vf, nh, nkv, nn, sp, scale, out, st) : launch_mma<128, false, 8>(q, kf, vf, nh, nkv, nn, sp, scale, out, st);
+    return kv_f16 ? launch_mma<64, true, 4>(q, kf, vf, nh, nkv, nn, sp, scale, out, st) : launch_mma<64, false, 8>(q, kf, vf, nh, nkv, nn, sp, scale, out, st);
 }
 
 }  // namespace cera

@@ -167,6 +167,36 @@ def test_prefill_attention_tiled_shapes(nh, nkv, n, start, f16):
     assert_close(got, want, f"tiled prefill attention {nh}/{nkv} n={n} start={start} f16={f16}")
 
 
+@pytest.mark.parametrize("nh,nkv,hd,n,start", [
+    (4, 1, 128, 16, 0), (4, 1, 128, 17, 48), (8, 2, 128, 33, 31), (3, 1, 128, 100, 0), (8, 8, 128, 65, 63), (8, 1, 128, 9, 120), (24, 3, 128, 40, 7),
+    (16, 4, 64, 130, 61), (4, 4, 64, 1, 0), (5, 1, 64, 70, 0), (32, 8, 128, 200, 500)])
+@pytest.mark.parametrize("f16,spread", [(False, 0), (True, 0), (False, 1), (False, 2)])
+def test_prefill_attention_products_of_halves(nh, nkv, hd, n, start, f16, spread):
+    """Edges of the 16-row and 32- / 64-key tiles, any group size; f32 caches whose rows lie far apart in size, or far from 1."""
+    torch = need_gpu()
+    import cera_b200 as cb
+    total = start + n
+    kc = cb.synth_normal(total * nkv * hd, seed=11, sigma=1.0).reshape(total, nkv * hd)
+    vc = cb.synth_normal(total * nkv * hd, seed=12, sigma=1.0).reshape(total, nkv * hd)
+    q = cb.synth_normal(n * nh * hd, seed=13, sigma=1.0).reshape(n, nh * hd)
+    scale = 1.0 / math.sqrt(hd)
+    if spread == 1:  # sizes over six orders of magnitude between neighbouring rows
+        size = 10.0 ** (torch.arange(total, device="cuda") % 7 - 6.0)
+        kc, vc = kc * size[:, None], vc * size[:, None]
+    elif spread == 2:  # beyond f16 in every operand
+        q, kc, vc = q * 1e5, kc * 1e-9, vc * 3e6
+    kk, vv = (kc.half(), vc.half()) if f16 else (kc, vc)
+    got = cb.prefill_attention(q, kk, vv, nh, nkv, hd, n, start, scale).double()
+    g = nh // nkv
+    qd, kd, vd = q.double().reshape(n, nh, hd), kk.double().reshape(total, nkv, hd), vv.double().reshape(total, nkv, hd)
+    s = torch.einsum("nhd,thd->hnt", qd, kd.repeat_interleave(g, dim=1)) * scale
+    s = s.masked_fill(torch.arange(total, device="cuda")[None, :] > start + torch.arange(n, device="cuda")[:, None], float("-inf"))
+    want = torch.einsum("hnt,thd->nhd", torch.softmax(s, 2), vd.repeat_interleave(g, dim=1)).reshape(n, nh * hd)
+    # 22 bits of every operand, f32 sums over hd and over the keys: a few 1e-7 of the result's size (measured up to 5e-7)
+    err = ((got - want).norm() / want.norm()).item()
+    assert err < 2e-6, err
+
+
 @pytest.mark.parametrize("f16", [False, True])
 def test_prefill_attention_matches_flash_oracle(f16):
     torch = need_gpu()
