@@ -1219,7 +1219,7 @@ void keep_stream_pool() {
 // and, when every weight has its image, ONE kernel launch covers all of them (the small matrices' CTAs run beside the
 // large one's instead of after them).  *taken = false: not these kernels' case, nothing launched.
 int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, size_t n, size_t ldy, int epilogue, cudaStream_t st,
-                             bool *taken) {
+                             bool *taken, GemmScratch lent) {
     *taken = false;
     static const bool off = [] {
         const char *e = getenv("CERA_CUDA_GEMM");
@@ -1234,17 +1234,21 @@ int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, s
     for (int i = 1; i < count; ++i)  // several weights: the same k, Q4_K / Q5_K, every one with its image
         if (t[i].w.k != w.k || !t[i].w.tc || !w.tc || (t[i].w.type != CERA_TYPE_Q4_K && t[i].w.type != CERA_TYPE_Q5_K)) return CERA_CUDA_OK;
     if ((uintptr_t)x.quants % 16 || (uintptr_t)x.scales % 16 || (uintptr_t)x.sums % 16) return CERA_CUDA_OK;
-    // the activation operands, converted once for all row tiles: a stream-ordered scratch allocation that lives for this
-    // call (token tiles x stages x 32 KB, the min operand's token side, g and 1 / g)
+    // the activation operands, converted once for all row tiles, in lent memory or a stream-ordered allocation that lives for
+    // this call (token tiles x stages x 32 KB, the min operand's token side, g and 1 / g)
     const uint32_t tiles = (uint32_t)((n + TC_BM - 1) / TC_BM), n_pad = tiles * TC_BM, n_it = w.k / TC_KS, n_sb = w.k / 256;
     const uint32_t nb32 = w.k / 32, n_mit = (nb32 + TCW_MIN_J - 1) / TCW_MIN_J;
     const size_t img_bytes = (size_t)tiles * n_it * (2 * TC_OP_BYTES), min_bytes = (size_t)tiles * n_sb * TC_MINOP_BYTES,
                  xm_bytes = (size_t)tiles * n_mit * (2 * TCW_MINT_BYTES);
-    keep_stream_pool();
-    uint8_t *scratch = nullptr;
-    if (cudaMallocAsync((void **)&scratch, img_bytes + min_bytes + xm_bytes + (size_t)n_pad * 8, st) != cudaSuccess) {
-        cudaGetLastError();  // no room for the operand scratch: leave the GEMM to the kernels that need none
-        return CERA_CUDA_OK;
+    const size_t need = img_bytes + min_bytes + xm_bytes + (size_t)n_pad * 8;
+    const bool borrowed = lent.p && lent.bytes >= need;
+    uint8_t *scratch = (uint8_t *)lent.p;
+    if (!borrowed) {
+        keep_stream_pool();
+        if (cudaMallocAsync((void **)&scratch, need, st) != cudaSuccess) {
+            cudaGetLastError();  // no room for the operand scratch: leave the GEMM to the kernels that need none
+            return CERA_CUDA_OK;
+        }
     }
     uint8_t *xm = scratch + img_bytes + min_bytes;
     float *g_tab = reinterpret_cast<float *>(xm + xm_bytes), *ginv_tab = g_tab + n_pad;
@@ -1302,16 +1306,16 @@ int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, s
         else
             rc = w.type == CERA_TYPE_Q4_K ? launch_tc_typed<CERA_TYPE_Q4_K, false>(p, y, st) : launch_tc_typed<CERA_TYPE_Q5_K, false>(p, y, st);
     }
-    cudaFreeAsync(scratch, st);  // after the kernels above, in stream order
+    if (!borrowed) cudaFreeAsync(scratch, st);  // after the kernels above, in stream order
     return rc;
 }
 
 // tcgen05 GEMM for K-quant weights stored with interleaved row groups, k a multiple of 256, n > 32 columns.
 // *taken = false: not this kernel's case, nothing launched.  CERA_CUDA_GEMM=mma keeps the warp-level kernel.
 int32_t launch_gemm_tc(const WeightView &w, const ActView &x, size_t n, float *out, size_t ldy, size_t ldc, int epilogue,
-                       cudaStream_t st, bool *taken) {
+                       cudaStream_t st, bool *taken, GemmScratch lent) {
     const GemmTarget t{w, out, ldc};
-    return launch_gemm_tc_multi(&t, 1, x, n, ldy, epilogue, st, taken);
+    return launch_gemm_tc_multi(&t, 1, x, n, ldy, epilogue, st, taken, lent);
 }
 
 }  // namespace cera

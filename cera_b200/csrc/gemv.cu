@@ -208,11 +208,11 @@ int32_t launch_gemv(const GemvSeg *segs, int n_segs, const ActView &x, size_t n_
 // belong to the tensor-core GEMM.  Cell (row i, column j) goes to out[i*ldy + j*ldc]:
 // (ldy, ldc) = (n, 1) is the reference's row-major [m x n]; (1, m) is token-major.
 int32_t launch_gemm_ex(const WeightView &w, const ActView &x, size_t n, float *out, size_t ldy, size_t ldc, int epilogue,
-                       cudaStream_t st) {
+                       cudaStream_t st, GemmScratch lent) {
     const size_t k = w.k;
     {
         bool taken = false;
-        CERA_TRY(launch_gemm_tc(w, x, n, out, ldy, ldc, epilogue, st, &taken));  // tcgen05 / TMEM
+        CERA_TRY(launch_gemm_tc(w, x, n, out, ldy, ldc, epilogue, st, &taken, lent));  // tcgen05 / TMEM
         if (taken) return CERA_CUDA_OK;
         CERA_TRY(launch_gemm_tcq(w, x, n, out, ldy, ldc, epilogue, st, &taken));  // tcgen05 from the quantized bytes
         if (taken) return CERA_CUDA_OK;

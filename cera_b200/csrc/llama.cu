@@ -20,6 +20,7 @@
 // logits) sit in an exchange region whose slices the ranks push to each other (tp.cu) after the
 // kernel that produced them: four exchanges per layer plus one for the logits or the greedy pick.
 // RMSNorm, the embedding row and the RoPE table are recomputed on every rank.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -58,6 +59,9 @@ struct Layer {
 };
 
 constexpr size_t PREFILL_CHUNK = 512;
+// A prompt that needs only its last logits goes through the layers this many tokens at a time on one GPU.  At 512 the wide tcgen05
+// product of the 8B shape's gate and up matrices has 448 tiles for 148 SMs, 3.03 rounds, and pays for 4; at 2048 12.1, and 13.
+constexpr size_t PROMPT_CHUNK = 2048;
 
 struct LlamaModel : cera_cuda_model {
     explicit LlamaModel(const cera_cuda_config &c) : cera_cuda_model(c.vocab_size, c.hidden_size, c.max_seq_len, c.device), cfg(c) {}
@@ -65,6 +69,7 @@ struct LlamaModel : cera_cuda_model {
     int32_t add_tensor(int32_t role, int32_t layer, int32_t type, size_t rows, size_t cols, const void *bytes, size_t nbytes) override;
     int32_t build() override;
     size_t chunk_tokens() const override { return PREFILL_CHUNK; }
+    size_t prompt_chunk() const override { return pf_chunk; }
     uint32_t plan(size_t n_positions) const override { return attn_plan(l_heads, l_kv_heads, cfg.head_dim, n_positions); }
     int32_t enqueue_step(int kind, uint32_t n_splits) override;
     bool batched(size_t n) const override;
@@ -80,6 +85,7 @@ struct LlamaModel : cera_cuda_model {
     int32_t restore(const void *data, size_t bytes) override;
 
     cera_cuda_config cfg{};
+    size_t pf_chunk = PREFILL_CHUNK;  // tokens that the pf_ buffers hold
     bool tc_prepared = false;  // the prefill GEMM's weight images have been asked for
     cera_cuda_weight *embd = nullptr, *output = nullptr;
     cera_cuda_weight *embd_rows = nullptr;  // tensor parallel: this rank's rows of a tied embedding, as LM head
@@ -95,7 +101,7 @@ struct LlamaModel : cera_cuda_model {
     float theta_scale = 0.0f;
     float *rope_cs = nullptr;  // [head_dim/2][2] cos/sin at the current position
     float *rope_table = nullptr;  // [max_seq_len][head_dim/2][2] cos/sin of every position, computed on the host (null: too large)
-    // batched prefill (chunks of PREFILL_CHUNK tokens, token-major buffers)
+    // batched prefill (chunks of pf_chunk tokens, token-major buffers)
     float *pf_hidden = nullptr, *pf_q = nullptr, *pf_k = nullptr, *pf_v = nullptr, *pf_attn = nullptr, *pf_g = nullptr,
           *pf_u = nullptr;
     float *pf_attn_local = nullptr;  // = pf_attn (every rank computes all heads)
@@ -116,6 +122,10 @@ struct LlamaModel : cera_cuda_model {
     uint32_t l_heads = 0, l_kv_heads = 0;
     size_t l_qd = 0, l_kvd = 0, l_ff = 0, l_hs = 0, l_vocab = 0;
 };
+
+// A chunk-wide f32 buffer of `width` that also holds a product's converted operands over k = width: 4 bytes a value, a sixteenth more
+// for the minimum's operands, whole tiles of 1024 values and 128 tokens.
+size_t pf_lent_bytes(size_t chunk, size_t width) { return (chunk + 127) / 128 * 128 * ((width + 1023) / 1024 * 1024 * 17 / 4 + 64); }
 
 int32_t alloc_act(LlamaModel *m, ActBuf &a, size_t k) {
     CERA_TRY(m->dev_alloc((void **)&a.scales, k / 32 * 4));
@@ -321,7 +331,7 @@ int32_t enqueue_llama_step(LlamaModel *m, int kind, uint32_t n_splits) {
     return CERA_CUDA_OK;
 }
 
-// One chunk (n <= PREFILL_CHUNK) of prompt tokens through every layer with batched kernels: column
+// One chunk (n <= pf_chunk) of prompt tokens through every layer with batched kernels: column
 // RMSNorm + Q8_0, multi-column GEMMs (token-major outputs), batched RoPE + KV append, causal attention,
 // SiLU*mul + Q8_0 (cera/src/model/llama.rs:738-1523).  Leaves the hidden state of the chunk's last token
 // in m->hidden so the ordinary LM-head path can finish.
@@ -364,13 +374,20 @@ int32_t llama_chunk(LlamaModel *m, const uint32_t *tokens, size_t n, size_t star
     };
     // projections that share their activations (q / k / v, gate / up): one tensor-core launch when every weight has its
     // operand image, else one GEMM each
-    auto gemm_group = [&](std::initializer_list<GemmTarget> ts, const ActView &x) -> int32_t {
+    auto gemm_group = [&](std::initializer_list<GemmTarget> ts, const ActView &x, GemmScratch lent) -> int32_t {
         bool taken = false;
-        CERA_TRY(launch_gemm_tc_multi(ts.begin(), (int)ts.size(), x, n, 1, EPI_STORE, st, &taken));
+        CERA_TRY(launch_gemm_tc_multi(ts.begin(), (int)ts.size(), x, n, 1, EPI_STORE, st, &taken, lent));
         if (taken) return CERA_CUDA_OK;
-        for (const GemmTarget &t : ts) CERA_TRY(launch_gemm_ex(t.w, x, n, t.out, 1, t.ldc, EPI_STORE, st));
+        for (const GemmTarget &t : ts) CERA_TRY(launch_gemm_ex(t.w, x, n, t.out, 1, t.ldc, EPI_STORE, st, lent));
         return CERA_CUDA_OK;
     };
+    // Lent to the products for their converted activations: the gate projection's buffer, whose values are used up before the next
+    // layer's, and the queries', used up by the attention.  (Tensor parallel: peers write into the former at any time.)
+    GemmScratch in_g, in_q;
+    if (!tp) {
+        in_g = {m->pf_g, pf_lent_bytes(m->pf_chunk, ff)};
+        in_q = {m->pf_q, pf_lent_bytes(m->pf_chunk, qd)};
+    }
     if (tp) CERA_TRY(launch_tp_tick(m->tp_words, st));
     CERA_CUDA_TRY(cudaMemcpyAsync(m->pf_tokens, tokens, n * 4, cudaMemcpyHostToDevice, st));
     CERA_TRY(launch_embed_batch(m->embd->v, m->pf_tokens, n, m->pf_hidden, st));
@@ -381,21 +398,21 @@ int32_t llama_chunk(LlamaModel *m, const uint32_t *tokens, size_t n, size_t star
         const uint32_t s0 = 4 * li++;
         CERA_TRY(launch_rmsnorm(m->pf_hidden, L.attn_norm, hs, n, c.rms_norm_eps, nullptr, m->pf_act_hs.scales,
                                 m->pf_act_hs.quants, m->pf_act_hs.sums, st));
-        CERA_TRY(gemm_group({{L.wq->v, m->pf_q, l_qd}, {L.wk->v, m->pf_k, l_kvd}, {L.wv->v, m->pf_v, l_kvd}}, m->pf_act_hs.view()));
+        CERA_TRY(gemm_group({{L.wq->v, m->pf_q, l_qd}, {L.wk->v, m->pf_k, l_kvd}, {L.wv->v, m->pf_v, l_kvd}}, m->pf_act_hs.view(), in_g));
         CERA_TRY(launch_rope_batch(m->pf_q, m->pf_k, m->pf_v, start_pos, n, m->l_heads, m->l_kv_heads, c.head_dim,
                                    m->theta_scale, m->rope_freqs, c.rope_type, L.kc, L.vc, c.kv_f16, st, m->rope_table));
         CERA_TRY(launch_prefill_attention(m->pf_q, L.kc, L.vc, c.kv_f16, m->l_heads, m->l_kv_heads, c.head_dim, n, start_pos,
                                           scale, m->pf_attn_local, st));
         CERA_TRY(launch_quantize(m->pf_attn, qd, n, false, m->pf_act_q.scales, m->pf_act_q.quants, m->pf_act_q.sums, st));
         if (res_scale != 1.0f) {  // block output into pf_g (free until the gate projection), then hidden += out * s
-            CERA_TRY(launch_gemm_ex(L.wo->v, m->pf_act_q.view(), n, m->pf_g, 1, hs, EPI_STORE, st));
+            CERA_TRY(launch_gemm_ex(L.wo->v, m->pf_act_q.view(), n, m->pf_g, 1, hs, EPI_STORE, st, in_q));
             CERA_TRY(launch_scaled_add(m->pf_hidden, m->pf_g, n * hs, res_scale, st));
         } else {
-            CERA_TRY(launch_gemm_ex(L.wo->v, m->pf_act_q.view(), n, m->pf_hidden, 1, hs, EPI_ADD, st));  // whole on every rank
+            CERA_TRY(launch_gemm_ex(L.wo->v, m->pf_act_q.view(), n, m->pf_hidden, 1, hs, EPI_ADD, st, in_g));  // whole on every rank
         }
         CERA_TRY(launch_rmsnorm(m->pf_hidden, L.ffn_norm, hs, n, c.rms_norm_eps, nullptr, m->pf_act_hs.scales,
                                 m->pf_act_hs.quants, m->pf_act_hs.sums, st));
-        CERA_TRY(gemm_group({{L.gate->v, m->pf_g + (size_t)r * l_ff, ff}, {L.up->v, m->pf_u + (size_t)r * l_ff, ff}}, m->pf_act_hs.view()));
+        CERA_TRY(gemm_group({{L.gate->v, m->pf_g + (size_t)r * l_ff, ff}, {L.up->v, m->pf_u + (size_t)r * l_ff, ff}}, m->pf_act_hs.view(), in_q));
         if (tp) {
             // (two copies, one signal: the second gather carries the slot)
             const size_t col_off = (size_t)r * l_ff, off = (size_t)((char *)(m->pf_g + col_off) - m->region);
@@ -406,10 +423,10 @@ int32_t llama_chunk(LlamaModel *m, const uint32_t *tokens, size_t n, size_t star
         }
         CERA_TRY(launch_silu_mul(m->pf_g, m->pf_u, ff, n, m->pf_act_ff.scales, m->pf_act_ff.quants, m->pf_act_ff.sums, st));
         if (res_scale != 1.0f) {  // pf_u is free once the SwiGLU product is quantized
-            CERA_TRY(launch_gemm_ex(L.down->v, m->pf_act_ff.view(), n, m->pf_u, 1, hs, EPI_STORE, st));
+            CERA_TRY(launch_gemm_ex(L.down->v, m->pf_act_ff.view(), n, m->pf_u, 1, hs, EPI_STORE, st, in_g));
             CERA_TRY(launch_scaled_add(m->pf_hidden, m->pf_u, n * hs, res_scale, st));
         } else {
-            CERA_TRY(launch_gemm_ex(L.down->v, m->pf_act_ff.view(), n, m->pf_hidden + (size_t)r * l_hs, 1, hs, EPI_ADD, st));
+            CERA_TRY(launch_gemm_ex(L.down->v, m->pf_act_ff.view(), n, m->pf_hidden + (size_t)r * l_hs, 1, hs, EPI_ADD, st, in_g));
             if (tp) CERA_TRY(gather(m->pf_hidden, hs, l_hs, m->pf_hidden + (size_t)r * l_hs, hs, s0 + 3));
         }
     }
@@ -589,15 +606,22 @@ int32_t LlamaModel::build() {
     CERA_TRY(m->dev_alloc((void **)&m->g, m->l_ff * 4));
     CERA_TRY(m->dev_alloc((void **)&m->u, m->l_ff * 4));
     CERA_TRY(alloc_act(m, m->act_hs, hs));
+    if (m->tp_size == 1 && c.max_seq_len > PREFILL_CHUNK) {
+        // (rounded so that the longest prompt fits one chunk; 512 where the device is nearly full)
+        const size_t want = std::min(PROMPT_CHUNK, ((size_t)c.max_seq_len + 127) / 128 * 128), more = (want - PREFILL_CHUNK) * 4 * (3 * hs + 4 * qd + 3 * ff);
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b > more + (4ull << 30)) m->pf_chunk = want;
+        cudaGetLastError();
+    }
     {
-        const size_t C = PREFILL_CHUNK;
-        CERA_TRY(m->dev_alloc((void **)&m->pf_q, C * m->l_qd * 4));
+        const size_t C = m->pf_chunk;
+        CERA_TRY(m->dev_alloc((void **)&m->pf_q, pf_lent_bytes(C, m->l_qd)));
         CERA_TRY(m->dev_alloc((void **)&m->pf_k, C * m->l_kvd * 4));
         CERA_TRY(m->dev_alloc((void **)&m->pf_v, C * m->l_kvd * 4));
         if (m->tp_size == 1) {
             CERA_TRY(m->dev_alloc((void **)&m->pf_hidden, C * hs * 4));
             CERA_TRY(m->dev_alloc((void **)&m->pf_attn, C * qd * 4));
-            CERA_TRY(m->dev_alloc((void **)&m->pf_g, C * ff * 4));
+            CERA_TRY(m->dev_alloc((void **)&m->pf_g, pf_lent_bytes(C, ff)));
             CERA_TRY(m->dev_alloc((void **)&m->pf_u, C * ff * 4));
             m->pf_attn_local = m->pf_attn;
         } else {

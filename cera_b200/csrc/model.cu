@@ -51,7 +51,7 @@ int32_t cera_cuda_model::dev_alloc(void **p, size_t bytes) {
 int32_t cera_cuda_model::alloc_common() {
     if (!logits) CERA_TRY(dev_alloc((void **)&logits, (size_t)vocab_size * 4));
     if (!final_hidden) CERA_TRY(dev_alloc((void **)&final_hidden, (size_t)hidden_size * 4));
-    CERA_TRY(dev_alloc((void **)&pf_tokens, (chunk_tokens() + 1) * 4));
+    CERA_TRY(dev_alloc((void **)&pf_tokens, (prompt_chunk() + 1) * 4));
     CERA_TRY(dev_alloc((void **)&argmax_scratch, argmax_scratch_words() * 4));
     CERA_TRY(dev_alloc((void **)&dyn, 8 * 4));
     CERA_TRY(dev_alloc((void **)&tok_out, 4));
@@ -131,7 +131,7 @@ int32_t cera_cuda_model::run_prompt(const uint32_t *tokens, size_t n, size_t sta
     // Batched kernels, one chunk at a time (the reference's ubatch loop, cera/src/model/mod.rs:303-332).
     size_t cn = 0;
     for (size_t done = 0; done < n; done += cn) {
-        cn = n - done < chunk_tokens() ? n - done : chunk_tokens();
+        cn = n - done < prompt_chunk() ? n - done : prompt_chunk();
         CERA_TRY(prefill_chunk(tokens + done, cn, start_pos + done));
         CERA_CUDA_TRY(cudaStreamSynchronize(stream));  // the host token slice may go away after the call
         seq_len = start_pos + done + cn;

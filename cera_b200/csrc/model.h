@@ -68,10 +68,12 @@ struct cera_cuda_model {
     virtual int32_t add_tensor(int32_t role, int32_t layer, int32_t type, size_t rows, size_t cols, const void *bytes, size_t nbytes) = 0;
     virtual int32_t build() = 0;  // finalize: every tensor is there; allocate state and scratch
     virtual size_t chunk_tokens() const = 0;
+    // ... and at a time when only the last token's logits are wanted (at least chunk_tokens())
+    virtual size_t prompt_chunk() const { return chunk_tokens(); }
     virtual uint32_t plan(size_t n_positions) const = 0;  // launch plan of a decode step over n_positions, part of the graph key
     virtual int32_t enqueue_step(int kind, uint32_t plan) = 0;
     virtual bool batched(size_t n) const = 0;  // does a prompt portion of n tokens take the batched kernels?
-    // one chunk (n <= chunk_tokens()) of prompt tokens, all layers; the hidden states of the chunk stay on the device
+    // one chunk (n <= prompt_chunk()) of prompt tokens, all layers; the hidden states of the chunk stay on the device
     virtual int32_t prefill_chunk(const uint32_t *tokens, size_t n, size_t start_pos) = 0;
     virtual int32_t logits_of_last(size_t n) = 0;  // final norm + head of the chunk's last row, into `logits`
     // logits of chunk rows rows[0..n_rows) (null: of all n rows) to host memory, asynchronous on `stream`

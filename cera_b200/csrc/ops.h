@@ -47,8 +47,14 @@ struct GemvFusion {
 // (EPI_STORE / EPI_ADD, single column) into the peers' regions.
 int32_t launch_gemv(const GemvSeg *segs, int n_segs, const ActView &x, size_t n_cols, size_t ldy, int epilogue,
                     cudaStream_t st, size_t ldc = 1, bool batch_tile = false, const TpHook *tp = nullptr);
+// Device memory a caller lends a product for its converted operands, from launch to launch on one stream (256-byte aligned); too
+// small or none: a stream-ordered allocation for the call.
+struct GemmScratch {
+    void *p = nullptr;
+    size_t bytes = 0;
+};
 int32_t launch_gemm_ex(const WeightView &w, const ActView &x, size_t n, float *out, size_t ldy, size_t ldc, int epilogue,
-                       cudaStream_t st);
+                       cudaStream_t st, GemmScratch lent = {});
 // Register-resident-activation single-column GEMV.  *taken = false: shape outside its rules,
 // nothing was launched and the caller uses the item-wise kernel.
 int32_t launch_gemv_rows(const GemvSeg *segs, int n_segs, const ActView &x, int epilogue, const GemvFusion *fusion,
@@ -72,7 +78,7 @@ int32_t launch_gemm_mma(const WeightView &w, const ActView &x, size_t n, float *
                         cudaStream_t st, bool *taken);
 // The same product on tcgen05 / TMEM (gemm_tc.cu): Q4_K / Q5_K, k a multiple of 256, more than 32 columns.
 int32_t launch_gemm_tc(const WeightView &w, const ActView &x, size_t n, float *out, size_t ldy, size_t ldc, int epilogue,
-                       cudaStream_t st, bool *taken);
+                       cudaStream_t st, bool *taken, GemmScratch lent = {});
 // The same for up to three weights that take the same activations, in one launch when every weight has its image.
 struct GemmTarget {
     WeightView w;
@@ -80,7 +86,7 @@ struct GemmTarget {
     size_t ldc;
 };
 int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, size_t n, size_t ldy, int epilogue, cudaStream_t st,
-                             bool *taken);
+                             bool *taken, GemmScratch lent = {});
 // One work item of an expert-grouped GEMM: `count` consecutive activation columns starting at `first` go through
 // expert `expert`'s rows of a stacked weight matrix (built on the device by the routed-FFN kernels).
 struct MoeTile {
