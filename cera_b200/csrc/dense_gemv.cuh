@@ -1,5 +1,5 @@
 // Building blocks of the one-column products: a row group (R rows that share the activation vector) is walked by WPR warps
-// of a CTA, 16 bytes per lane and row at a time; the first loads are issued before the kernel waits for its predecessor
+// of a CTA (all of them where nothing but the sums follows, dense_gemv.cu), 16 bytes per lane and row at a time; the first loads are issued before the kernel waits for its predecessor
 // (weights never change).
 #pragma once
 
