@@ -264,6 +264,9 @@ bool moe_force_dp4a() {
 // How the projections of a batch run: few tokens per expert on dp4a, otherwise on a tensor-core kernel.
 enum class MoePlan { DP4A, MMA, TCQ };
 
+// Columns of a work item.
+uint32_t moe_columns(MoePlan plan) { return plan == MoePlan::TCQ ? TCQ_COLUMNS : plan == MoePlan::MMA ? MOE_NC_MMA : MOE_NC; }
+
 // One grouped projection over the work list, by the kernel that the plan was made for.  cap / max_small: where the list of narrow
 // items starts inside p.tiles and how many it can hold (MMA only); scratch: the TCQ kernel's.
 int32_t grouped_projection(MoePlan plan, const MoeGemmParams &p, uint32_t max_tiles, uint32_t cap, uint32_t max_small, bool single, void *scratch,
@@ -441,15 +444,34 @@ int32_t moe_create_impl(uint32_t n_expert, uint32_t n_used, uint32_t hidden, uin
     return CERA_CUDA_OK;
 }
 
+// How a call of n tokens with `entries` (token, pick) pairs runs, and the scratch that takes (null or to be freed in stream order); the
+// work list covers `experts` of the layer's experts.  A handful of tokens: dp4a work items of 8 columns (1 for a single token); a
+// batch: tensor-core items of 64, or of 128 straight from the quantized bytes.  The latter converts an expert's weights whatever
+// the number of its tokens; measured (whole layer, us, it / the other): Q8_0 (else on dp4a) 448 / 426 at 8 entries per expert, 453 / 759
+// at 16 (32 experts, 4 used, 2048 x 1792); Q4_0 (else on mma.sync) 361 / 347 at 32, 424 / 540 at 64; 16 experts: 202 / 158 at 16,
+// 221 / 291 at 32.
+MoePlan moe_pick_plan(const cera_cuda_moe *h, size_t n, size_t entries, uint32_t experts, cudaStream_t st, void **scratch) {
+    *scratch = nullptr;
+    if (n < 16 || moe_force_dp4a()) return MoePlan::DP4A;
+    const int gt = h->gate->v.type, dt = h->down->v.type;
+    const bool mma = gemm_mma_supports(gt, h->hidden) && gemm_mma_supports(dt, h->ff);
+    if (entries >= (size_t)h->n_expert * (mma ? 40 : 12) && gemm_tcq_supports(gt, h->hidden) && gemm_tcq_supports(dt, h->ff)) {
+        const uint32_t items = (uint32_t)(entries / TCQ_COLUMNS + experts);
+        keep_stream_pool();
+        if (cudaMallocAsync(scratch, gemm_tcq_grouped_scratch(h->hidden > h->ff ? h->hidden : h->ff, items), st) == cudaSuccess) return MoePlan::TCQ;
+        cudaGetLastError();
+        *scratch = nullptr;
+    }
+    return mma ? MoePlan::MMA : MoePlan::DP4A;
+}
+
 // The expert-parallel call: see the file header.
 int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softmax_gate, float *out_dev, uint32_t *ids_out_dev,
-                   float *weights_out_dev, cudaStream_t st) {
+                   float *weights_out_dev, MoePlan plan, void *scratch, cudaStream_t st) {
     if (!h->connected) return fail(CERA_CUDA_ERR_STATE, "moe_ffn: expert-parallel layer is not connected to its peers");
     const uint32_t hs = h->hidden, ff = h->ff, ku = h->n_used, E = h->n_expert;
     const size_t entries = n * ku, rmax = h->max_total * ku;
-    const bool mma = gemm_mma_supports(h->gate->v.type, hs) && gemm_mma_supports(h->down->v.type, ff) && !moe_force_dp4a();
-    const MoePlan plan = mma ? MoePlan::MMA : MoePlan::DP4A;
-    const uint32_t nc = mma ? MOE_NC_MMA : MOE_NC;
+    const uint32_t nc = moe_columns(plan);
     const uint32_t max_tiles = (uint32_t)(rmax / nc + E / h->ep_size);
     uint32_t *counts_mine = (uint32_t *)(h->region + h->lay.counts) + (size_t)h->ep_rank * E;
     uint32_t *n_recv = h->ep_words + 32;
@@ -463,7 +485,7 @@ int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softm
     CERA_TRY(launch_tp_exchange(h->ep, &cr, 1, 0, st));
     const uint32_t cap = (uint32_t)(rmax + E), max_small = E / h->ep_size;
     uint32_t *skip = h->ep_words + 33;
-    moe_ep_plan_kernel<<<1, 32, 0, st>>>(h->ep, h->lay, E, nc, mma ? nc / 2 : 0, cap, (uint32_t)rmax, h->my_base, h->cursor, h->tiles,
+    moe_ep_plan_kernel<<<1, 32, 0, st>>>(h->ep, h->lay, E, nc, plan == MoePlan::MMA ? nc / 2 : 0, cap, (uint32_t)rmax, h->my_base, h->cursor, h->tiles,
                                          h->n_tiles, n_recv, skip);
     if (n)
         moe_ep_dispatch_kernel<<<(unsigned)entries, 128, 0, st>>>(h->ep, h->lay, h->ids, ku, hs, E, ActView{h->xs, h->xq, h->xsum},
@@ -484,7 +506,7 @@ int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softm
     p.ldc = ff;
     p.tiles = h->tiles;
     p.n_tiles = h->n_tiles;
-    CERA_TRY(grouped_projection(plan, p, max_tiles, cap, max_small, false, nullptr, st));
+    CERA_TRY(grouped_projection(plan, p, max_tiles, cap, max_small, false, scratch, st));
     const size_t worst = rmax * ff;
     moe_silu_q8_kernel<<<(unsigned)((worst + 255) / 256), 256, 0, st>>>(h->g, h->u, ff, n_recv, h->f_scales, h->f_quants, h->f_sums);
     count_launch();
@@ -498,7 +520,7 @@ int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softm
     d.ldc = hs;
     d.tiles = h->tiles;
     d.n_tiles = h->n_tiles;
-    CERA_TRY(grouped_projection(plan, d, max_tiles, cap, max_small, false, nullptr, st));
+    CERA_TRY(grouped_projection(plan, d, max_tiles, cap, max_small, false, scratch, st));
     moe_ep_return_kernel<<<(unsigned)rmax, 128, 0, st>>>(h->ep, h->lay, h->expert_out, hs, n_recv);
     count_launch();
     CERA_CUDA_TRY(cudaGetLastError());
@@ -521,7 +543,7 @@ int32_t moe_ffn_planned(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t 
     const uint32_t hs = h->hidden, ff = h->ff, ku = h->n_used;
     const size_t entries = n * ku;
     const bool single = n == 1;
-    const uint32_t nc = single ? 1 : plan == MoePlan::TCQ ? TCQ_COLUMNS : plan == MoePlan::MMA ? MOE_NC_MMA : MOE_NC;
+    const uint32_t nc = single ? 1 : moe_columns(plan);
     const uint32_t max_tiles = (uint32_t)(entries / nc + (single ? 0 : h->n_expert));
     CERA_TRY(launch_quantize(x_dev, hs, n, false, h->xs, h->xq, h->xsum, st));
     CERA_TRY(launch_moe_route(x_dev, hs, n, h->router, h->bias, hs, h->n_expert, ku, softmax_gate, 1, h->ids, h->weights, h->counts, st));
@@ -637,26 +659,16 @@ int32_t cera_cuda_moe_ffn(cera_cuda_moe *h, const float *x_dev, size_t n, int32_
     if (!h || (n && (!x_dev || !out_dev))) return fail(CERA_CUDA_ERR_BAD_ARG, "moe_ffn: null argument");
     if (n > h->max_tokens) return fail(CERA_CUDA_ERR_BAD_ARG, "moe_ffn: %zu tokens, created for at most %zu", n, h->max_tokens);
     cudaStream_t st = (cudaStream_t)stream;
-    if (h->ep_size > 1) return moe_ffn_ep(h, x_dev, n, softmax_gate, out_dev, ids_out_dev, weights_out_dev, st);  // n == 0 still takes part
-    if (n == 0) return CERA_CUDA_OK;
-    const uint32_t hs = h->hidden, ff = h->ff;
-    const size_t entries = n * h->n_used;
-    // a handful of tokens: dp4a work items of 8 columns (1 for a single token); a batch: tensor-core items of 64, or of 128 straight
-    // from the quantized bytes.  The latter converts an expert's weights whatever the number of its tokens; measured (whole layer,
-    // us, it / the other): Q8_0 (else on dp4a) 448 / 426 at 8 entries per expert, 453 / 759 at 16 (32 experts, 4 used, 2048 x 1792);
-    // Q4_0 (else on mma.sync) 361 / 347 at 32, 424 / 540 at 64; 16 experts: 202 / 158 at 16, 221 / 291 at 32.
-    MoePlan plan = MoePlan::DP4A;
-    void *scratch = nullptr;
-    if (n >= 16 && !moe_force_dp4a()) {
-        const bool mma = gemm_mma_supports(h->gate->v.type, hs) && gemm_mma_supports(h->down->v.type, ff);
-        if (entries >= (size_t)h->n_expert * (mma ? 40 : 12) && gemm_tcq_supports(h->gate->v.type, hs) && gemm_tcq_supports(h->down->v.type, ff)) {
-            const uint32_t items = (uint32_t)(entries / TCQ_COLUMNS + h->n_expert);
-            keep_stream_pool();
-            if (cudaMallocAsync(&scratch, gemm_tcq_grouped_scratch(hs > ff ? hs : ff, items), st) == cudaSuccess) plan = MoePlan::TCQ;
-            else cudaGetLastError();
-        }
-        if (plan == MoePlan::DP4A && mma) plan = MoePlan::MMA;
+    if (h->ep_size > 1) {  // n == 0 still takes part; the plan follows from the tokens of a full call, alike on every rank
+        void *scratch = nullptr;
+        const MoePlan plan = moe_pick_plan(h, 16, h->max_total * h->n_used, h->n_expert / h->ep_size, st, &scratch);
+        const int32_t rc = moe_ffn_ep(h, x_dev, n, softmax_gate, out_dev, ids_out_dev, weights_out_dev, plan, scratch, st);
+        if (scratch) cudaFreeAsync(scratch, st);  // after the kernels above, in stream order
+        return rc;
     }
+    if (n == 0) return CERA_CUDA_OK;
+    void *scratch = nullptr;
+    const MoePlan plan = moe_pick_plan(h, n, n * h->n_used, h->n_expert, st, &scratch);
     const int32_t rc = moe_ffn_planned(h, x_dev, n, softmax_gate, out_dev, ids_out_dev, weights_out_dev, plan, scratch, st);
     if (scratch) cudaFreeAsync(scratch, st);  // after the kernels above, in stream order
     return rc;
