@@ -9,33 +9,32 @@ namespace {
 
 using namespace gv;
 
-// Rows of this CTA's two units: gate, gate, up, up (an odd count's last pair repeats its unit).
-template <class T>
-__device__ __forceinline__ void unit_rows(const T *(&rows)[4], const T *w, uint32_t ff_p, uint32_t ld) {
-#pragma unroll
-    for (uint32_t r = 0; r < 4; ++r) rows[r] = w + (size_t)(min(blockIdx.x * 2 + (r & 1), ff_p - 1) + (r >> 1) * ff_p) * ld;
-}
+// Rows of GV_LONG vectors and more: where a warp has one to itself, four rows a warp, which share its reads of x, two vectors of each in
+// flight, and CTAs of four warps, so that few warps wait for a CTA's last; where warps share it, two rows and four vectors.  Shorter
+// rows: one and eight, from 28 rows an SM on two and four.  us, the last / what is chosen: 32768 x 4096 bf16 41.8 / 40.4 (6.6 TB/s), 18560 x 4096
+// 26.0 / 24.8, 9600 x 4096 17.6 / 15.7, but with four rows a warp 8192 x 2048 7.7 / 8.7; one row and eight vectors / what is chosen: 4096 x 8192
+// 18.1 / 13.5, 4096 x 4096 10.2 / 7.8, but with two rows 3072 x 2048 5.4 / 5.6.
+constexpr int GV_LONG_WARPS = 4;
+constexpr uint32_t GV_LONG = 512;
 
-// A CTA per R rows, each shared by all its warps, two vectors of a row in flight per lane.  What bounds it: HBM.  Many warps that load
-// little each keep it busier than few with long batches, whose later batches wait for the earlier ones' sums: 4096 x 8192 bf16
-// 13.3 us (5.0 TB/s), 4096 x 4096 8.0, 18560 x 4096 24.1 (6.3 TB/s), 2048 x 2048 3.4; one row per two warps and eight vectors per
-// lane: 18.1, 10.2, 25.8, 4.1.  R = 4 where that leaves every SM a CTA, R = 1 for fewer rows (a router's).
-template <class T, int R>
-__global__ void __launch_bounds__(GV_WARPS * 32) gemv_kernel(const T *__restrict__ w, uint32_t rows, uint32_t ld, const T *x, float *y) {
-    __shared__ float red[GV_WARPS][R];
+// W warps a CTA, WPR of them share R rows, U vectors of each in flight per lane.  What bounds it: HBM.  Of R, W and U the results do
+// not depend; WPR fixes the order in which a row is added up, and stays what it is for a shape (see launch_dense_gemv).
+template <class T, int W, int R, int WPR, int U>
+__global__ void __launch_bounds__(W * 32) gemv_kernel(const T *__restrict__ w, uint32_t rows, uint32_t ld, const T *x, float *y) {
+    __shared__ float red[W][R];
     pdl_trigger();
     const int warp = threadIdx.x >> 5;
-    const uint32_t g = blockIdx.x;
-    RowDot<T, R, R == 1 ? 8 : 2> d;
+    const uint32_t g = blockIdx.x * (W / WPR) + warp / WPR;
+    RowDot<T, R, U> d;
 #pragma unroll
     for (int r = 0; r < R; ++r) d.w[r] = w + (size_t)min(g * R + r, rows - 1) * ld;
-    d.start(ld, warp, GV_WARPS);
+    d.start(ld, warp % WPR, WPR);
     d.fetch();
     pdl_wait();
     float acc[R] = {};
     d.run(x, acc);
-    group_sum<R, GV_WARPS>(acc, red);
-    if (threadIdx.x == 0) {
+    group_sum<R, WPR>(acc, red);
+    if (warp % WPR == 0 && (threadIdx.x & 31) == 0) {
 #pragma unroll
         for (int r = 0; r < R; ++r)
             if (g * R + r < rows) y[g * R + r] = acc[r];
@@ -67,22 +66,30 @@ __global__ void __launch_bounds__(GV_WARPS * 32) mingru_step_kernel(const T *__r
     }
 }
 
-// Rows [0, ff_p) gate, [ff_p, 2 ff_p) up of w; out = unit(gate, up).  A CTA per two units.
-template <class T>
-__global__ void __launch_bounds__(GV_WARPS * 32) gated_unit_step_kernel(const T *__restrict__ w, uint32_t ff_p, uint32_t ld, const T *x, ExpertAct a, T *out) {
-    __shared__ float red[GV_WARPS][4];
+// Rows [0, ff_p) gate, [ff_p, 2 ff_p) up of w; out = unit(gate, up).  W warps a CTA, WPR of them share N units (2 N rows).
+template <class T, int W, int N, int WPR, int U>
+__global__ void __launch_bounds__(W * 32) gated_unit_step_kernel(const T *__restrict__ w, uint32_t ff_p, uint32_t ld, const T *x, ExpertAct a, T *out) {
+    __shared__ float red[W][2 * N];
     pdl_trigger();
     const int warp = threadIdx.x >> 5;
-    RowDot<T, 4, 2> d;
-    unit_rows(d.w, w, ff_p, ld);
-    d.start(ld, warp, GV_WARPS);
+    const uint32_t g = (blockIdx.x * (W / WPR) + warp / WPR) * N;
+    RowDot<T, 2 * N, U> d;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        d.w[2 * i] = w + (size_t)min(g + i, ff_p - 1) * ld;
+        d.w[2 * i + 1] = d.w[2 * i] + (size_t)ff_p * ld;
+    }
+    d.start(ld, warp % WPR, WPR);
     d.fetch();
     pdl_wait();
-    float acc[4] = {};
+    float acc[2 * N] = {};
     d.run(x, acc);
-    group_sum<4, GV_WARPS>(acc, red);
-    const uint32_t g = blockIdx.x * 2 + threadIdx.x;
-    if (threadIdx.x < 2 && g < ff_p) out[g] = Elem<T>::from(gated_unit(threadIdx.x ? acc[1] : acc[0], threadIdx.x ? acc[3] : acc[2], a));
+    group_sum<2 * N, WPR>(acc, red);
+    if (warp % WPR == 0 && (threadIdx.x & 31) == 0) {
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (g + i < ff_p) out[g + i] = Elem<T>::from(gated_unit(acc[2 * i], acc[2 * i + 1], a));
+    }
 }
 
 // grid (row groups, picks).  Every CTA repeats the pick from the router logits - few CTAs with long rows therefore (a CTA per two
@@ -123,26 +130,26 @@ __global__ void __launch_bounds__(GV_WARPS * 32) expert_gate_up_kernel(const T *
     }
 }
 
-// A CTA per R rows.  The picks' rows are walked as one row of n_used * ld elements, U vectors of it in flight per lane and row.
-template <class T>
+template <class T, int WPR>
 __global__ void __launch_bounds__(GV_WARPS * 32) expert_down_kernel(const T *__restrict__ w, uint32_t rows, uint32_t ld, const T *act, uint32_t n_used,
                                                                     int weight_input, const uint32_t *ids, const float *weights, float *y) {
-    constexpr int R = 2, U = 4;
-    __shared__ float red[GV_WARPS][R];
+    __shared__ float red[GV_WARPS][1];
     pdl_trigger();
     pdl_wait();
-    const uint32_t g = blockIdx.x * R, g1 = min(g + 1, rows - 1), nv = ld / Elem<T>::N, all = n_used * nv, step = 32u * GV_WARPS;
-    float total[R] = {};
-    for (uint32_t c = threadIdx.x; c < all; c += U * step) {
-        uint4 wb[R][U], xb[U];
+    const int warp = threadIdx.x >> 5;
+    const uint32_t g = blockIdx.x * (GV_WARPS / WPR) + warp / WPR, gi = min(g, rows - 1);
+    // the picks' rows are walked as one row of n_used * ld elements, U vectors of it in flight per lane
+    constexpr int U = 8;
+    const uint32_t nv = ld / Elem<T>::N, all = n_used * nv, step = 32u * WPR;
+    float total[1] = {0.0f};
+    for (uint32_t c = (warp % WPR) * 32u + (threadIdx.x & 31); c < all; c += U * step) {
+        uint4 wb[U], xb[U];
         float sc[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const uint32_t v = c + u * step, s = v / nv;
             if (v < all) {
-                const T *expert = w + (size_t)ids[s] * rows * ld;
-                wb[0][u] = ld_stream(reinterpret_cast<const uint4 *>(expert + (size_t)g * ld) + (v - s * nv));
-                wb[1][u] = ld_stream(reinterpret_cast<const uint4 *>(expert + (size_t)g1 * ld) + (v - s * nv));
+                wb[u] = ld_stream(reinterpret_cast<const uint4 *>(w + ((size_t)ids[s] * rows + gi) * ld) + (v - s * nv));
                 xb[u] = *(reinterpret_cast<const uint4 *>(act) + v);
                 sc[u] = weight_input ? 1.0f : weights[s];
             }
@@ -150,35 +157,44 @@ __global__ void __launch_bounds__(GV_WARPS * 32) expert_down_kernel(const T *__r
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (c + u * step < all) {
-                float xf[Elem<T>::N];
+                float wf[Elem<T>::N], xf[Elem<T>::N], a = 0.0f;
+                Elem<T>::unpack(wb[u], wf);
                 Elem<T>::unpack(xb[u], xf);
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    float wf[Elem<T>::N], a = 0.0f;
-                    Elem<T>::unpack(wb[r][u], wf);
-#pragma unroll
-                    for (int i = 0; i < Elem<T>::N; ++i) a = fmaf(wf[i], xf[i], a);
-                    total[r] = fmaf(sc[u], a, total[r]);
-                }
+                for (int i = 0; i < Elem<T>::N; ++i) a = fmaf(wf[i], xf[i], a);
+                total[0] = fmaf(sc[u], a, total[0]);
             }
     }
-    group_sum<R, GV_WARPS>(total, red);
-    if (threadIdx.x == 0) {
-        y[g] = total[0];
-        if (g + 1 < rows) y[g + 1] = total[1];
-    }
+    group_sum<1, WPR>(total, red);
+    if (warp % WPR == 0 && (threadIdx.x & 31) == 0 && g < rows) y[g] = total[0];
 }
 
 }  // namespace
 
+// The warps that share a row (wpr) are part of the result: they fix the order of its additions, and with it each last bit, which the
+// rounding to bf16 widens and a router with two experts almost level turns into another pick.  A shape keeps its wpr; only the layout
+// around it is free.
 int32_t launch_dense_gemv(const DenseView &w, const void *x, float *y, cudaStream_t st) {
-    const bool four = w.rows >= (uint32_t)sm_count() * 4;
+    const bool pairs = w.rows >= (uint32_t)sm_count() * 28;
+    const int wpr = pick_wpr(pairs ? (w.rows + 1) / 2 : w.rows, (size_t)w.ld * (w.f32 ? 4 : 2), pairs ? 4 : 8);
     count_launch();
     return with_type(w.f32, [&](auto t) {
         using T = decltype(t);
-        return check_cuda(four ? launch_k(gemv_kernel<T, 4>, dim3((w.rows + 3) / 4), dim3(GV_WARPS * 32), 0, st, (const T *)w.w, w.rows, w.ld, (const T *)x, y)
-                               : launch_k(gemv_kernel<T, 1>, dim3(w.rows), dim3(GV_WARPS * 32), 0, st, (const T *)w.w, w.rows, w.ld, (const T *)x, y),
-                          "dense gemv launch");
+        const bool long_rows = w.ld / Elem<T>::N >= GV_LONG;
+        if (wpr == 1 && long_rows)
+            return check_cuda(launch_k(gemv_kernel<T, GV_LONG_WARPS, 4, 1, 2>, gv_grid((w.rows + 3) / 4, 1, 1, GV_LONG_WARPS), dim3(GV_LONG_WARPS * 32), 0, st,
+                                       (const T *)w.w, w.rows, w.ld, (const T *)x, y),
+                              "dense gemv launch");
+        return with_wpr(wpr, [&](auto n) {
+            constexpr int WPR = decltype(n)::value, R = WPR == 8 ? 1 : 2;  // (eight warps share a row where there are few: a CTA each)
+            if (R == 2 && (pairs || long_rows))
+                return check_cuda(launch_k(gemv_kernel<T, GV_WARPS, R, WPR, 8 / R>, gv_grid((w.rows + R - 1) / R, wpr), dim3(GV_WARPS * 32), 0, st,
+                                           (const T *)w.w, w.rows, w.ld, (const T *)x, y),
+                                  "dense gemv launch");
+            return check_cuda(launch_k(gemv_kernel<T, GV_WARPS, 1, WPR, 8>, gv_grid(w.rows, wpr), dim3(GV_WARPS * 32), 0, st, (const T *)w.w, w.rows, w.ld,
+                                       (const T *)x, y),
+                              "dense gemv launch");
+        });
     });
 }
 
@@ -198,11 +214,19 @@ int32_t launch_mingru_step(const DenseView &w, const void *x, const float *z_bia
 
 int32_t launch_gated_unit_step(const DenseView &w, const void *x, const ExpertAct &a, void *out, cudaStream_t st) {
     const uint32_t ff_p = w.rows / 2;
+    const int wpr = pick_wpr(ff_p, (size_t)w.ld * (w.f32 ? 4 : 2), 4);
     count_launch();
     return with_type(w.f32, [&](auto t) {
         using T = decltype(t);
-        return check_cuda(launch_k(gated_unit_step_kernel<T>, dim3((ff_p + 1) / 2), dim3(GV_WARPS * 32), 0, st, (const T *)w.w, ff_p, w.ld, (const T *)x, a, (T *)out),
-                          "gated unit launch");
+        if (wpr == 1 && w.ld / Elem<T>::N >= GV_LONG)
+            return check_cuda(launch_k(gated_unit_step_kernel<T, GV_LONG_WARPS, 2, 1, 2>, gv_grid((ff_p + 1) / 2, 1, 1, GV_LONG_WARPS),
+                                       dim3(GV_LONG_WARPS * 32), 0, st, (const T *)w.w, ff_p, w.ld, (const T *)x, a, (T *)out),
+                              "gated unit launch");
+        return with_wpr(wpr, [&](auto n) {
+            return check_cuda(launch_k(gated_unit_step_kernel<T, GV_WARPS, 1, decltype(n)::value, 4>, gv_grid(ff_p, wpr), dim3(GV_WARPS * 32), 0, st,
+                                       (const T *)w.w, ff_p, w.ld, (const T *)x, a, (T *)out),
+                              "gated unit launch");
+        });
     });
 }
 
@@ -222,12 +246,15 @@ int32_t launch_expert_gate_up_step(const DenseView &w, const void *x, const floa
 
 int32_t launch_expert_down_step(const DenseView &w, uint32_t rows_per_expert, const void *act, const RouterRule &r, const uint32_t *ids,
                                 const float *weights, float *y, cudaStream_t st) {
+    const int wpr = pick_wpr(rows_per_expert, (size_t)w.ld * (w.f32 ? 4 : 2), 2);
     count_launch();
     return with_type(w.f32, [&](auto t) {
         using T = decltype(t);
-        return check_cuda(launch_k(expert_down_kernel<T>, dim3((rows_per_expert + 1) / 2), dim3(GV_WARPS * 32), 0, st, (const T *)w.w, rows_per_expert, w.ld,
-                                   (const T *)act, r.n_used, r.weight_input, ids, weights, y),
-                          "expert down launch");
+        return with_wpr(wpr, [&](auto n) {
+            return check_cuda(launch_k(expert_down_kernel<T, decltype(n)::value>, gv_grid(rows_per_expert, wpr), dim3(GV_WARPS * 32), 0, st,
+                                       (const T *)w.w, rows_per_expert, w.ld, (const T *)act, r.n_used, r.weight_input, ids, weights, y),
+                              "expert down launch");
+        });
     });
 }
 

@@ -1,5 +1,5 @@
 // Building blocks of the one-column products: a row group (R rows that share the activation vector) is walked by WPR warps
-// of a CTA (all of them where nothing but the sums follows, dense_gemv.cu), 16 bytes per lane and row at a time; the first loads are issued before the kernel waits for its predecessor
+// of a CTA, 16 bytes per lane and row at a time; the first loads are issued before the kernel waits for its predecessor
 // (weights never change).
 #pragma once
 
@@ -94,7 +94,7 @@ template <class F>
 int32_t with_type(int f32, F f) {
     return f32 ? f(float{}) : f(bf16{});
 }
-inline dim3 gv_grid(size_t groups, int wpr, uint32_t y = 1) { return dim3((unsigned)((groups * wpr + GV_WARPS - 1) / GV_WARPS), y); }
+inline dim3 gv_grid(size_t groups, int wpr, uint32_t y = 1, int warps = GV_WARPS) { return dim3((unsigned)((groups * wpr + warps - 1) / warps), y); }
 
 }  // namespace gv
 

@@ -64,3 +64,21 @@ def test_cuda_path_against_golden_attention_and_glue():
     assert_bits(cb.silu_mul(g, u).cpu().numpy(), GOLD["glue_silu_mul"], "silu_mul")
     got = cb.rmsnorm(g, torch.from_numpy(GOLD["glue_norm_w"]).cuda(), 1e-5).cpu().numpy()
     assert np.allclose(got, GOLD["glue_rmsnorm"], rtol=2e-7, atol=0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("name", ["goletar", "piditar"])
+def test_layered_decode_keeps_its_bits(name, dtype):
+    import importlib.util
+    import json
+    from gpu_util import need_gpu
+    torch = need_gpu()
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("recorded on 148 SMs, whose number decides how many warps share a row")
+    here = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden")
+    spec = importlib.util.spec_from_file_location("make_layered_decode_bits", os.path.join(here, "make_layered_decode_bits.py"))
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    with open(os.path.join(here, "layered_decode_bits.json")) as f:
+        assert mod.build(name, dtype) == json.load(f)[f"{name}_{dtype}"]
