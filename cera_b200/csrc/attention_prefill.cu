@@ -1,18 +1,22 @@
-// Causal attention of a chunk of prompt tokens (prefill) on the tensor cores, in f32 accuracy.
+// Causal attention of a chunk of prompt tokens (prefill), in f32 accuracy: on the tensor cores over an f16 cache, with FMAs over an
+// f32 cache.
 //
-// A CTA owns one KV head and WARPS * 16 rows, a row = (query, head of the group), so every staged K / V row serves all of them.
-// A warp holds its sixteen queries in registers and walks the keys in tiles as flash attention does: scores, running softmax,
-// weighted values.  The products are mma.sync on f16 halves: a float enters as a high and a low f16, 22 bits of it, and the
-// product of two such floats is three MMAs - low x high, high x low, high x high, in this order, so that the sums are truncated
-// at full size by the last third only; an f16 cache is exact as it is and takes two.  Operands are scaled by powers of two
-// (queries by row, an f32 cache's K and V by tile, probabilities by 2^14) so that f16 neither overflows nor becomes subnormal
-// where it matters.  A tile's weighted values start from zero and are added to the running output in f32.
-//
-// What bounds it: the tensor pipe at the rate of mma.sync, 256 to 384 MMAs per 16 rows x 64 keys beside 32 exponentials a lane.  It stays
+// f16: a CTA owns one KV head and 64 rows, a row = (query, head of the group), so every staged K / V row serves all of them.
+// A warp holds its sixteen queries in registers and walks the keys in tiles of 64 as flash attention does: scores, running softmax,
+// weighted values.  The products are mma.sync on f16: the cache's values as they are; a query and a probability enter as a high and a
+// low f16, 22 bits, so that a product is two MMAs, the low one first, and its sums are truncated at full size by the second half
+// only.  Queries are scaled by a power of two per row, probabilities by 2^14; what f16 then cannot tell from zero is 2^-39 of the row's
+// largest |q| and of 1.  A tile's weighted values start from zero and are added to the running output in f32.
+// What bounds it: the tensor pipe at the rate of mma.sync, 256 MMAs per 16 rows x 64 keys beside 32 exponentials a lane.  It stays
 // on mma.sync because scores, probabilities and their halves live in registers between the two products.
-// Tiles are staged by cp.async: f16 as stored, two tiles deep; f32 raw, two to three tiles ahead, and split into halves by the whole CTA.
-// 32 heads of 128 in groups of 4: 512 tokens 50 us over an f16 cache, 82 us over f32 (153, 100 with FMAs on the CUDA cores); 2047
-// tokens 345, 576 us (1125, 1366).  Error against 64 bits 3.0e-7 and 3.7e-7 (4.0e-7, 5.7e-7).
+// 32 heads of 128 in groups of 4: 512 tokens 50 us (153 with FMAs on the CUDA cores), 2047 tokens 345 us (1125).  Error against 64
+// bits 3.0e-7 (4.0e-7).
+//
+// f32: a split into f16 halves would need scales, and one value far from the others' size - a key that the query does not even
+// see, where a tile shares the scale - would cost the rest their bits.  These products stay in f32 (attn_prefill_tiled_kernel).
+//
+// Infinities and NaN: a row that ends without finite values - a probability of zero times an infinite value of a key it does not
+// see, or an infinity split into halves - is computed again by attend_row, which reads no key past the row's limit.
 //
 // Arithmetic contract: cera/src/backend/cpu.rs:4028-4241 (scaled dot, causal limit start_pos + j, online softmax);
 // the f32 summation order is this kernel's own.
@@ -22,6 +26,7 @@
 #include <cstring>
 
 #include "act.cuh"
+#include "attention_row.cuh"
 #include "mma.cuh"
 #include "ops.h"
 
@@ -29,16 +34,32 @@ namespace cera {
 
 namespace {
 
-template <int HD, bool F16>
+template <int HD>
 struct Pa {
-    static constexpr int TK = F16 ? 64 : 32;          // keys per tile
-    static constexpr int ROW = HD * 2 + 16;           // bytes of a staged f16 row: eight rows of an ldmatrix hit all banks
+    static constexpr int TK = 64;           // keys per tile
+    static constexpr int ROW = HD * 2 + 16; // bytes of a staged row: eight rows of an ldmatrix hit all banks
     static constexpr int TILE = TK * ROW;
-    static constexpr int RAW = TK * HD * 4;           // an f32 tile as stored
-    static constexpr int STAGES = F16 ? 2 : 3;        // tiles in flight or in use as they come from the cache
-    // f16: [stage][K, V]; f32: [K high, K low, V high, V low], [stage][raw K, raw V]
-    static constexpr size_t SMEM = F16 ? STAGES * 2 * TILE : 4 * TILE + STAGES * 2 * RAW;
+    static constexpr size_t SMEM = 2 * 2 * TILE;  // [stage][K, V]
 };
+
+// Nothing infinite, no NaN?
+template <int N>
+__device__ __forceinline__ bool pa_finite(const float (&v)[N], float l) {
+    float z = l * 0.0f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) z = fmaf(v[i], 0.0f, z);
+    return z == 0.0f;
+}
+
+// The warp's rows whose bit is set in `again` once more.
+template <int VEC, bool F16>
+__device__ __forceinline__ void pa_again(uint32_t again, uint32_t r_first, uint32_t G, const float *q, const uint8_t *kc, const uint8_t *vc, uint32_t n_heads,
+                                      uint32_t n_kv_heads, uint32_t start_pos, float scale, float *out) {
+    for (; again; again &= again - 1) {
+        const uint32_t r = r_first + __ffs(again) - 1;
+        attend_row<VEC, F16>(q, kc, vc, n_heads, n_kv_heads, r / G, blockIdx.x * G + r % G, start_pos, scale, out);
+    }
+}
 
 // Biased exponent of the power of two that brings values up to mx (its float's bits) below 2^14; 254 - it is the inverse's.
 __device__ __forceinline__ uint32_t pa_up(uint32_t mx_bits) {
@@ -47,15 +68,14 @@ __device__ __forceinline__ uint32_t pa_up(uint32_t mx_bits) {
 }
 __device__ __forceinline__ float pa_pow2(uint32_t biased) { return __uint_as_float(biased << 23); }
 
-template <int HD, bool F16, int WARPS>
+template <int HD, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) attn_prefill_mma_kernel(const float *__restrict__ q, const uint8_t *__restrict__ kc,
                                                                       const uint8_t *__restrict__ vc, uint32_t n_heads, uint32_t n_kv_heads, uint32_t n,
                                                                       uint32_t start_pos, float scale, float *__restrict__ out) {
-    using S = Pa<HD, F16>;
+    using S = Pa<HD>;
     extern __shared__ __align__(16) uint8_t pa_smem[];
-    __shared__ uint32_t tile_max[2][2];  // f32: bits of the largest |k| and |v| of a tile, by parity
-    constexpr int TK = S::TK, NT = TK / 8, KS = HD / 16, KK = TK / 16, ND = HD / 8, THREADS = WARPS * 32, ES = F16 ? 2 : 4;
-    constexpr int PIECES = HD * ES / 16;  // 16-byte pieces of a cache row
+    constexpr int TK = S::TK, NT = TK / 8, KS = HD / 16, KK = TK / 16, ND = HD / 8, THREADS = WARPS * 32;
+    constexpr int PIECES = HD * 2 / 16;  // 16-byte pieces of a cache row
     pdl_trigger();
     pdl_wait();
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kvh = blockIdx.x, G = n_heads / n_kv_heads;
@@ -63,25 +83,19 @@ __global__ void __launch_bounds__(WARPS * 32) attn_prefill_mma_kernel(const floa
     const size_t kv_dim = (size_t)n_kv_heads * HD, q_dim = (size_t)n_heads * HD;
     const uint32_t cta_kv = start_pos + (min(r_cta + WARPS * 16, rows) - 1) / G + 1;  // keys the CTA's last query sees
     const uint32_t n_tiles = (cta_kv + TK - 1) / TK;
-    const uint8_t *k_src = kc + (size_t)kvh * HD * ES, *v_src = vc + (size_t)kvh * HD * ES;
+    const uint8_t *k_src = kc + (size_t)kvh * HD * 2, *v_src = vc + (size_t)kvh * HD * 2;
 
     auto issue = [&](uint32_t t) {
-        uint8_t *kd = F16 ? pa_smem + (t & 1) * 2 * S::TILE : pa_smem + 4 * S::TILE + t % S::STAGES * 2 * S::RAW, *vd = kd + (F16 ? S::TILE : S::RAW);
-        constexpr int ROW = F16 ? S::ROW : HD * 4;
-        for (uint32_t i = tid; i < TK * PIECES && t < n_tiles; i += THREADS) {
+        uint8_t *kd = pa_smem + (t & 1) * 2 * S::TILE, *vd = kd + S::TILE;
+        for (uint32_t i = tid; i < TK * PIECES; i += THREADS) {
             const uint32_t r = i / PIECES, pc = i % PIECES;
-            const size_t src = (size_t)min(t * TK + r, cta_kv - 1) * kv_dim * ES + pc * 16;  // rows past the limit are masked; keep the read in range
-            tma::cp_async16(kd + r * ROW + pc * 16, k_src + src);
-            tma::cp_async16(vd + r * ROW + pc * 16, v_src + src);
+            const size_t src = (size_t)min(t * TK + r, cta_kv - 1) * kv_dim * 2 + pc * 16;  // rows past the limit are masked; keep the read in range
+            tma::cp_async16(kd + r * S::ROW + pc * 16, k_src + src);
+            tma::cp_async16(vd + r * S::ROW + pc * 16, v_src + src);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     issue(0);
-    if constexpr (!F16) {
-        issue(1);
-        issue(2);
-    }
-    if (tid < 4) tile_max[tid >> 1][tid & 1] = 0;
 
     // ---- queries of the warp's rows, as A fragments: rows g and g + 8, columns 16 ks + 2 c + {0, 1, 8, 9}
     const uint32_t g = lane >> 2, c = lane & 3, r_warp = r_cta + warp * 16;
@@ -122,60 +136,14 @@ __global__ void __launch_bounds__(WARPS * 32) attn_prefill_mma_kernel(const floa
     const uint32_t warp_kv = live ? start_pos + (min(r_warp + 16, rows) - 1) / G + 1 : 0;
 
     for (uint32_t t = 0; t < n_tiles; ++t) {
-        float kf = 1.0f, vf = 1.0f / 16384.0f;  // 2^-u of the tile's K; of its V and of the probabilities
-        const uint8_t *kt, *vt;
-        if constexpr (F16) {
-            if (t + 1 < n_tiles) {
-                issue(t + 1);
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
-            } else {
-                asm volatile("cp.async.wait_group 0;" ::: "memory");
-            }
-            __syncthreads();
-            kt = pa_smem + (t & 1) * 2 * S::TILE;
-            vt = kt + S::TILE;
+        if (t + 1 < n_tiles) {
+            issue(t + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
         } else {
-            asm volatile("cp.async.wait_group 2;" ::: "memory");
-            __syncthreads();  // the raw tile is there, and everyone is done with the halves of the tile before
-            const float4 *raw = reinterpret_cast<const float4 *>(pa_smem + 4 * S::TILE + t % S::STAGES * 2 * S::RAW);
-            constexpr int QUADS = TK * HD / 4;
-            float mx[2] = {0.0f, 0.0f};
-#pragma unroll
-            for (int w = 0; w < 2; ++w) {
-#pragma unroll 4
-                for (uint32_t i = tid; i < QUADS; i += THREADS) {
-                    const float4 x = raw[w * QUADS + i];
-                    mx[w] = fmaxf(mx[w], fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
-                }
-#pragma unroll
-                for (int s = 16; s > 0; s >>= 1) mx[w] = fmaxf(mx[w], __shfl_xor_sync(0xffffffffu, mx[w], s));
-                if (lane == 0) atomicMax(&tile_max[t & 1][w], __float_as_uint(mx[w]));  // magnitudes order like their bits
-            }
-            __syncthreads();
-#pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                const uint32_t up = pa_up(tile_max[t & 1][w]);
-                const float f = pa_pow2(up);
-                if (w == 0) kf = pa_pow2(254u - up);
-                else vf = pa_pow2(254u - up) * (1.0f / 16384.0f);
-                uint8_t *hi_t = pa_smem + w * 2 * S::TILE, *lo_t = hi_t + S::TILE;
-#pragma unroll 4
-                for (uint32_t i = tid; i < QUADS; i += THREADS) {
-                    const float4 x = raw[w * QUADS + i];
-                    uint2 hi, lo;
-                    split_f16(x.x * f, x.y * f, hi.x, lo.x);
-                    split_f16(x.z * f, x.w * f, hi.y, lo.y);
-                    const uint32_t off = i / (HD / 4) * S::ROW + i % (HD / 4) * 8;
-                    *reinterpret_cast<uint2 *>(hi_t + off) = hi;
-                    *reinterpret_cast<uint2 *>(lo_t + off) = lo;
-                }
-            }
-            __syncthreads();
-            if (tid < 2) tile_max[t & 1][tid] = 0;  // for the tile after the next
-            issue(t + 3);
-            kt = pa_smem;
-            vt = pa_smem + 2 * S::TILE;
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
+        __syncthreads();
+        const uint8_t *kt = pa_smem + (t & 1) * 2 * S::TILE, *vt = kt + S::TILE;
         if (t * TK < warp_kv) {
             // ---- scores: keys 8 nt + 2 c + {0, 1} of rows g (0, 1) and g + 8 (2, 3)
             float s[NT][4];
@@ -189,16 +157,6 @@ __global__ void __launch_bounds__(WARPS * 32) attn_prefill_mma_kernel(const floa
 #pragma unroll
                     for (int j = 0; j < 4; ++j) s[nt + p][j] = u[p][j] = 0.0f;
                 uint32_t b[2][KS / 2][4];
-                if constexpr (!F16) {
-#pragma unroll
-                    for (int k2 = 0; k2 < KS / 2; ++k2)
-#pragma unroll
-                        for (int p = 0; p < 2; ++p) ldsm4(b[p][k2], kl + S::TILE + (nt + p) * 8 * S::ROW + k2 * 64);
-#pragma unroll
-                    for (int ks = 0; ks < KS; ++ks)
-#pragma unroll
-                        for (int p = 0; p < 2; ++p) mma_f16(s[nt + p], qh[ks], b[p][ks / 2][2 * (ks & 1)], b[p][ks / 2][2 * (ks & 1) + 1]);
-                }
 #pragma unroll
                 for (int k2 = 0; k2 < KS / 2; ++k2)
 #pragma unroll
@@ -228,7 +186,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_prefill_mma_kernel(const floa
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const bool seen = key0 + 8 * nt + (j & 1) <= lim[j >> 1];
-                    s[nt][j] = seen ? __fmul_rn(s[nt][j] * qf[j >> 1] * kf, scale) : -INFINITY;
+                    s[nt][j] = seen ? __fmul_rn(s[nt][j] * qf[j >> 1], scale) : -INFINITY;
                     mx[j >> 1] = fmaxf(mx[j >> 1], s[nt][j]);
                 }
 #pragma unroll
@@ -265,16 +223,6 @@ __global__ void __launch_bounds__(WARPS * 32) attn_prefill_mma_kernel(const floa
 #pragma unroll
                     for (int j = 0; j < 4; ++j) a[p][j] = 0.0f;
                 uint32_t b[W][KK / 2][4];
-                if constexpr (!F16) {
-#pragma unroll
-                    for (int k2 = 0; k2 < KK / 2; ++k2)
-#pragma unroll
-                        for (int p = 0; p < W; ++p) ldsm4_trans(b[p][k2], vl + S::TILE + k2 * 32 * S::ROW + (nd + p) * 16);
-#pragma unroll
-                    for (int kk = 0; kk < KK; ++kk)
-#pragma unroll
-                        for (int p = 0; p < W; ++p) mma_f16(a[p], ph[kk], b[p][kk / 2][2 * (kk & 1)], b[p][kk / 2][2 * (kk & 1) + 1]);
-                }
 #pragma unroll
                 for (int k2 = 0; k2 < KK / 2; ++k2)
 #pragma unroll
@@ -290,52 +238,62 @@ __global__ void __launch_bounds__(WARPS * 32) attn_prefill_mma_kernel(const floa
 #pragma unroll
                 for (int p = 0; p < W; ++p)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) o[nd + p][j] = fmaf(a[p][j], vf, o[nd + p][j] * corr[j >> 1]);
+                    for (int j = 0; j < 4; ++j) o[nd + p][j] = fmaf(a[p][j], 1.0f / 16384.0f, o[nd + p][j] * corr[j >> 1]);
             }
         }
-        if constexpr (F16) __syncthreads();  // the stage is refilled by the copy issued in the next iteration
+        __syncthreads();  // the stage is refilled by the copy issued in the next iteration
     }
 
+    uint32_t again = 0;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 1);
         l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 2);
         const uint32_t r = r_warp + g + 8 * h;
+        float v[2 * ND];
+#pragma unroll
+        for (int nd = 0; nd < ND; ++nd) v[2 * nd] = o[nd][2 * h], v[2 * nd + 1] = o[nd][2 * h + 1];
+        uint32_t bad = r < rows && !pa_finite(v, l_run[h]) ? 1u << (g + 8 * h) : 0;
+        again |= __reduce_or_sync(0xffffffffu, bad);
         if (r >= rows) continue;
         const float inv = 1.0f / l_run[h];
         float *dst = out + (size_t)(r / G) * q_dim + ((size_t)kvh * G + r % G) * HD + 2 * c;
 #pragma unroll
-        for (int nd = 0; nd < ND; ++nd) *reinterpret_cast<float2 *>(dst + 8 * nd) = make_float2(o[nd][2 * h] * inv, o[nd][2 * h + 1] * inv);
+        for (int nd = 0; nd < ND; ++nd) *reinterpret_cast<float2 *>(dst + 8 * nd) = make_float2(v[2 * nd] * inv, v[2 * nd + 1] * inv);
     }
+    __syncwarp();  // a row's first values are not stored after its second
+    if (again) pa_again<HD / 32, true>(again, r_warp, G, q, kc, vc, n_heads, n_kv_heads, start_pos, scale, out);
 }
 
-template <int HD, bool F16, int WARPS>
+template <int HD>
 int32_t launch_mma(const float *q, const uint8_t *kc, const uint8_t *vc, uint32_t nh, uint32_t nkv, uint32_t n, uint32_t sp, float scale, float *out,
                    cudaStream_t st) {
-    constexpr size_t smem = Pa<HD, F16>::SMEM;
+    constexpr size_t smem = Pa<HD>::SMEM;
+    constexpr int WARPS = 4;  // 64 rows per CTA, two CTAs on an SM
     static thread_local int configured_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_dev != dev) {
-        CERA_CUDA_TRY(cudaFuncSetAttribute(attn_prefill_mma_kernel<HD, F16, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CERA_CUDA_TRY(cudaFuncSetAttribute(attn_prefill_mma_kernel<HD, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured_dev = dev;
     }
     const dim3 grid(nkv, (unsigned)(((size_t)n * (nh / nkv) + WARPS * 16 - 1) / (WARPS * 16)));
     count_launch();
-    return check_cuda(launch_k(attn_prefill_mma_kernel<HD, F16, WARPS>, grid, dim3(WARPS * 32), smem, st, q, kc, vc, nh, nkv, n, sp, scale, out),
+    return check_cuda(launch_k(attn_prefill_mma_kernel<HD, WARPS>, grid, dim3(WARPS * 32), smem, st, q, kc, vc, nh, nkv, n, sp, scale, out),
                       "prefill attention (tensor cores) launch");
 }
 
-// ---- few rows over an f32 cache -----------------------------------------------------------------------------------------
-// With one or two warps' worth of rows the splitting of every tile above costs more than its MMAs save (32 heads in groups of 4, 5
-// queries after 4000 positions: 450 against 420 us; 2 after 3000: 334 against 275).  Here a CTA owns one KV head and PA_BQ
-// consecutive queries; warp w owns query w with all G heads of the group.  Keys go by in tiles of 32, double-buffered with cp.async:
+// ---- f32 cache ----------------------------------------------------------------------------------------------------------
+// A CTA owns one KV head and PA_BQ consecutive queries; warp w owns query w with all G heads of the group.  Keys go by in tiles of
+// 32, double-buffered with cp.async:
 //   scores : lane = key.  The lane keeps 32 dims of its K row in registers at a time and reads the queries as
 //            shared-memory broadcasts: no shuffle per key, four FMAs per broadcast load.
-//   softmax: one running maximum / sum per (query, head), updated once per tile.
+//   softmax: one running maximum / sum per (query, head), updated once per tile (two warp reductions and ONE expf per
+//            key, against a reduction and two expf per key in the one-warp-per-row kernel).
 //   P.V    : lane = four output dims.  The tile's probabilities sit in shared memory, V rows are read as float4 and
 //            shared by the G heads.
 // Rows are padded to 132 floats, so the lane = key reads (stride one row) hit all 32 banks.
+// 32 heads of 128 in groups of 4: 512 tokens 100 us, 2047 tokens 1366 us.  Error against 64 bits 5.7e-7.
 constexpr int PA_WARPS = 8, PA_THREADS = PA_WARPS * 32, PA_BQ = PA_WARPS;
 constexpr int PA_TK = 32;        // keys per tile
 constexpr int PA_HD = 128;       // head dim
@@ -482,14 +440,15 @@ __global__ void __launch_bounds__(PA_THREADS) attn_prefill_tiled_kernel(const fl
         __syncthreads();    // the stage is refilled by the copy issued in the next iteration
     }
 
-    if (live) {
+    if (!live) return;
+    uint32_t again = 0;
 #pragma unroll
-        for (int g = 0; g < G; ++g) {
-            const float inv = 1.0f / l_run[g];
-            float4 o = make_float4(acc[g].x * inv, acc[g].y * inv, acc[g].z * inv, acc[g].w * inv);
-            *reinterpret_cast<float4 *>(out + j * q_dim + ((size_t)kvh * G + g) * PA_HD + 4 * lane) = o;
-        }
+    for (int g = 0; g < G; ++g) {
+        const float v[4] = {acc[g].x, acc[g].y, acc[g].z, acc[g].w}, inv = 1.0f / l_run[g];
+        if (__any_sync(0xffffffffu, !pa_finite(v, l_run[g]))) again |= 1u << g;
+        *reinterpret_cast<float4 *>(out + j * q_dim + ((size_t)kvh * G + g) * PA_HD + 4 * lane) = make_float4(v[0] * inv, v[1] * inv, v[2] * inv, v[3] * inv);
     }
+    if (again) pa_again<PA_HD / 32, false>(again, j * G, G, q, kc, vc, n_heads, n_kv_heads, start_pos, scale, out);
 }
 
 template <int G>
@@ -511,8 +470,8 @@ int32_t launch_tiled(const float *q, const uint8_t *kc, const uint8_t *vc, uint3
 
 }  // namespace
 
-// f32 or f16 cache, head_dim 64 or 128, 16-byte aligned operands; anything else: *taken = false and the caller runs the
-// one-warp-per-row kernel.  CERA_CUDA_PREFILL_ATTN=rows turns this kernel off.
+// f16 cache: head_dim 64 or 128, any group size; f32 cache: head_dim 128, group size 1, 2, 4 or 8.  16-byte aligned operands; anything
+// else: *taken = false and the caller runs the one-warp-per-row kernel.  CERA_CUDA_PREFILL_ATTN=rows turns these kernels off.
 int32_t launch_prefill_attention_tiled(const float *q, const void *kc, const void *vc, int kv_f16, size_t n_heads,
                                        size_t n_kv_heads, size_t head_dim, size_t n, size_t start_pos, float scale, float *out,
                                        cudaStream_t st, bool *taken) {
@@ -521,24 +480,21 @@ int32_t launch_prefill_attention_tiled(const float *q, const void *kc, const voi
         const char *e = getenv("CERA_CUDA_PREFILL_ATTN");
         return e && strcmp(e, "rows") == 0;
     }();
-    if (off || (head_dim != 64 && head_dim != 128) || n == 0) return CERA_CUDA_OK;
+    if (off || n == 0) return CERA_CUDA_OK;
     if (((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc | (uintptr_t)out) % 16) return CERA_CUDA_OK;
     const uint32_t nh = (uint32_t)n_heads, nkv = (uint32_t)n_kv_heads, nn = (uint32_t)n, sp = (uint32_t)start_pos;
     const uint8_t *kf = (const uint8_t *)kc, *vf = (const uint8_t *)vc;
     *taken = true;
-    const size_t G = n_heads / n_kv_heads;
-    if (!kv_f16 && head_dim == PA_HD && n * G <= 32) {
-        switch (G) {
+    if (kv_f16 && head_dim == 128) return launch_mma<128>(q, kf, vf, nh, nkv, nn, sp, scale, out, st);
+    if (kv_f16 && head_dim == 64) return launch_mma<64>(q, kf, vf, nh, nkv, nn, sp, scale, out, st);
+    if (!kv_f16 && head_dim == PA_HD) switch (n_heads / n_kv_heads) {
             case 1: return launch_tiled<1>(q, kf, vf, nh, nkv, nn, sp, scale, out, st);
             case 2: return launch_tiled<2>(q, kf, vf, nh, nkv, nn, sp, scale, out, st);
             case 4: return launch_tiled<4>(q, kf, vf, nh, nkv, nn, sp, scale, out, st);
             case 8: return launch_tiled<8>(q, kf, vf, nh, nkv, nn, sp, scale, out, st);
         }
-    }
-    // f16: 64 rows per CTA, two CTAs on an SM; f32, whose tiles every CTA splits anew: 128
-    if (head_dim == 128)
-        return kv_f16 ? launch_mma<128, true, 4>(q, kf, vf, nh, nkv, nn, sp, scale, out, st) : launch_mma<128, false, 8>(q, kf, vf, nh, nkv, nn, sp, scale, out, st);
-    return kv_f16 ? launch_mma<64, true, 4>(q, kf, vf, nh, nkv, nn, sp, scale, out, st) : launch_mma<64, false, 8>(q, kf, vf, nh, nkv, nn, sp, scale, out, st);
+    *taken = false;
+    return CERA_CUDA_OK;
 }
 
 }  // namespace cera

@@ -172,7 +172,8 @@ def test_prefill_attention_tiled_shapes(nh, nkv, n, start, f16):
     (16, 4, 64, 130, 61), (4, 4, 64, 1, 0), (5, 1, 64, 70, 0), (32, 8, 128, 200, 500)])
 @pytest.mark.parametrize("f16,spread", [(False, 0), (True, 0), (False, 1), (False, 2)])
 def test_prefill_attention_products_of_halves(nh, nkv, hd, n, start, f16, spread):
-    """Edges of the 16-row and 32- / 64-key tiles, any group size; f32 caches whose rows lie far apart in size, or far from 1."""
+    """Edges of the 16-row and 32- / 64-key tiles, any group size; f32 caches whose rows lie far apart in size, or far from 1.  One norm over
+    all rows, which the large ones make up: the small ones are looked at by the next test."""
     torch = need_gpu()
     import cera_b200 as cb
     total = start + n
@@ -192,9 +193,50 @@ def test_prefill_attention_products_of_halves(nh, nkv, hd, n, start, f16, spread
     s = torch.einsum("nhd,thd->hnt", qd, kd.repeat_interleave(g, dim=1)) * scale
     s = s.masked_fill(torch.arange(total, device="cuda")[None, :] > start + torch.arange(n, device="cuda")[:, None], float("-inf"))
     want = torch.einsum("hnt,thd->nhd", torch.softmax(s, 2), vd.repeat_interleave(g, dim=1)).reshape(n, nh * hd)
-    # 22 bits of every operand, f32 sums over hd and over the keys: a few 1e-7 of the result's size (measured up to 5e-7)
+    # f32 (f16 caches: 22 bits of q and p) and f32 sums over hd and over the keys: a few 1e-7 of the result's size (measured up to 5e-7)
     err = ((got - want).norm() / want.norm()).item()
     assert err < 2e-6, err
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(4, 1, 128), (3, 1, 128), (8, 2, 64), (3, 1, 64), (2, 2, 128)])
+@pytest.mark.parametrize("f16,which,size", [
+    (False, "k", 1e6), (False, "k", 1e9), (False, "k", 1e12), (False, "v", 1e9), (False, "v", 1e12), (False, "dims", 1e9), (False, "rows", 0.0),
+    (True, "k", 1e4), (True, "v", 1e4), (True, "rows", 0.0)] + [(f, w, x) for f in (False, True) for w in ("k", "v") for x in (math.inf, math.nan)])
+def test_prefill_attention_rows_judged_alone(nh, nkv, hd, f16, which, size):
+    """A key that a query does not see leaves the query's output alone, whatever it holds; queries that see it get what plain arithmetic gives."""
+    torch = need_gpu()
+    import cera_b200 as cb
+    n, at, g = 70, 40, nh // nkv
+    kc = cb.synth_normal(n * nkv * hd, seed=21, sigma=1.0).reshape(n, nkv * hd)
+    vc = cb.synth_normal(n * nkv * hd, seed=22, sigma=1.0).reshape(n, nkv * hd)
+    q = cb.synth_normal(n * nh * hd, seed=23, sigma=1.0).reshape(n, nh * hd)
+    odd = kc if which == "k" else vc
+    if which == "rows":  # neighbouring rows up to six orders of magnitude apart
+        step = 10.0 ** (torch.arange(n, device="cuda") % 7 - 6.0)
+        kc, vc = kc * step[:, None], vc * step[:, None]
+    elif which == "dims":
+        vc[:, 5] *= size
+    elif math.isfinite(size):
+        odd[at] *= size
+    else:
+        odd[at, 5] = size
+    scale = 1.0 / math.sqrt(hd)
+    kk, vv = (kc.half(), vc.half()) if f16 else (kc, vc)
+    got = cb.prefill_attention(q, kk, vv, nh, nkv, hd, n, 0, scale).double().reshape(n, nh, hd)
+    qd = q.double().reshape(n, nh, hd)
+    kd, vd = (x.double().reshape(n, nkv, hd).repeat_interleave(g, dim=1) for x in (kk, vv))
+    for j in range(n):
+        p = torch.softmax(torch.einsum("hd,thd->ht", qd[j], kd[:j + 1]) * scale, 1)
+        want = torch.einsum("ht,thd->hd", p, vd[:j + 1])
+        assert torch.equal(torch.isfinite(got[j]), torch.isfinite(want)), j
+        if which == "k" and j >= at and math.isfinite(size):
+            continue  # scores of that size leave no bits to compare
+        ok = torch.isfinite(want)
+        if which == "dims":
+            ok[:, [i for i in range(hd) if i != 5]], ok[:, 5] = True, False
+        err = torch.where(ok, got[j] - want, 0.0).norm(dim=1) / torch.where(ok, want, 0.0).norm(dim=1).clamp_min(1e-30)
+        # scores below 8 in f32 carry up to 8 * 2^-24 * a few into a probability; measured up to 1e-6
+        assert err.max().item() < 4e-6, (j, err)
 
 
 @pytest.mark.parametrize("f16", [False, True])
