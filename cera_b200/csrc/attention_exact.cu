@@ -713,6 +713,7 @@ int32_t launch_decode_attention_exact(const float *q, const void *kc, const void
                                       float *out, void *workspace, size_t workspace_bytes, float *scales, int8_t *quants,
                                       int16_t *sums, cudaStream_t st, const TpHook *tp) {
     if (!q || !kc || !vc || !out || !workspace) return fail(CERA_CUDA_ERR_BAD_ARG, "decode_attention: null argument");
+    if (!aligned16(vc)) return fail(CERA_CUDA_ERR_BAD_ARG, "decode_attention: the value cache does not start on a 16-byte boundary");
     const size_t cap = workspace_bytes / (2 * n_heads * sizeof(float)) / 64 * 64;  // positions the workspace holds
     if (cap == 0 || seq_len > cap)
         return fail(CERA_CUDA_ERR_BAD_ARG, "decode_attention: workspace of %zu bytes holds %zu positions, %zu needed", workspace_bytes, cap, seq_len);

@@ -167,7 +167,9 @@ CERA_API int32_t cera_cuda_rope(float *q_dev, float *k_dev, size_t pos, size_t n
 /* position-ordered value sums) and is bit-identical to it.  With the           */
 /* environment variable CERA_CUDA_ATTN set the online-softmax kernels run       */
 /* instead (groups of 4 or 8, head_dim 64 or 128; agreement within 1e-3         */
-/* relative).  Any other shape: CERA_CUDA_ERR_UNSUPPORTED.                      */
+/* relative).  Any other shape: CERA_CUDA_ERR_UNSUPPORTED.  v_cache_dev starts   */
+/* on a 16-byte boundary (CERA_CUDA_ERR_BAD_ARG otherwise); k_cache_dev may     */
+/* start anywhere.                                                            */
 CERA_API size_t cera_cuda_decode_attention_workspace_bytes(size_t n_heads, size_t head_dim,
                                                           size_t seq_len);
 CERA_API int32_t cera_cuda_decode_attention(const float *q_dev, const void *k_cache_dev,

@@ -112,6 +112,24 @@ def test_decode_attention_bits_at_tile_edges(nh, nkv, hd, seq, off, kv_f16):
 
 
 @pytest.mark.parametrize("kv_f16", [0, 1])
+@pytest.mark.parametrize("seq", [100, 2000])
+def test_value_cache_off_a_16_byte_boundary_is_refused(seq, kv_f16):
+    """By the host, ahead of any launch; the next call finds nothing amiss."""
+    torch = need_gpu()
+    import cera_b200 as cb
+    nh, nkv, hd = 4, 1, 128
+    dt = torch.float16 if kv_f16 else torch.float32
+    base, kc = torch.ones(seq * hd + 8, device="cuda", dtype=dt), torch.ones(seq, hd, device="cuda", dtype=dt)
+    q = torch.ones(nh * hd, device="cuda")
+    for off in (1, 2, 3):
+        with pytest.raises(cb.CeraCudaError) as e:
+            cb.decode_attention(q, kc, base[off:off + seq * hd].reshape(seq, hd), nh, nkv, hd, seq, 0.1)
+        assert e.value.code == 1 and "16-byte" in str(e.value)
+    out = cb.decode_attention(q, kc, base[8:].reshape(seq, hd), nh, nkv, hd, seq, 0.1)
+    assert torch.allclose(out, torch.ones_like(out), atol=1e-5)
+
+
+@pytest.mark.parametrize("kv_f16", [0, 1])
 def test_model_logits_bit_identical_to_the_oracle(kv_f16):
     """A llama-architecture model whose matrices are K-quants with row lengths that are multiples of 512 runs every
     projection, norm, rotation and attention on reference-order kernels: logits equal the oracle's bits at every
