@@ -379,9 +379,10 @@ attn_chain_exact_kernel(const __grid_constant__ CUtensorMap v_map, const float *
             for (uint32_t i = 0; i < boxes; ++i)
                 tma::tensor_g2s_2d(ring + slot * C::STAGE + i * AXC_BOX * C::ROW, &v_map, (int)(kvh * hd + d0), (int)(tile * AXC_T + i * AXC_BOX), full + slot);
         }
-        // no copy may be in flight into this CTA's memory once it is gone
+        // no copy may be in flight into this CTA's memory once it is gone, also when something gave up (the slot's other arrival may then be
+        // missing: the limit, some milliseconds, is what the copy itself has)
         for (uint32_t t = tile > C::STAGES ? tile - C::STAGES : 0; t < tile; ++t)
-            for (uint32_t i = 0; i < (tma::SPIN_LIMIT >> 4) && !tma::mbar_try(full + t % C::STAGES, (t / C::STAGES) & 1) && !*(volatile uint32_t *)&gave_up; ++i) {}
+            for (uint32_t i = 0; i < (1u << 16) && !tma::mbar_test(full + t % C::STAGES, (t / C::STAGES) & 1); ++i) __nanosleep(40);
         return;
     }
     if (warp >= AXC_HEADS) {
