@@ -26,7 +26,9 @@
 // the source rank's return buffer at the pair index, and the source adds its picks in pick order.
 // Both all-to-alls are peer stores issued by the kernels themselves, with the flag protocol of
 // tp.cu between the phases.  Every (token, expert) product and the combine order are those of the
-// single-GPU path, so results are bit-identical for any number of ranks.
+// single-GPU path, so results are bit-identical for any number of ranks from 16 tokens on: which kernel forms
+// the products follows from the tokens of the call (moe_tcq_entries), here as counted on the device over all
+// ranks.  (Fewer: a single GPU runs dp4a, ranks the tensor-core kernel where the type has one.)
 #include <cstdlib>
 #include <cstring>
 #include <new>
@@ -139,15 +141,17 @@ constexpr uint32_t EP_STATUS_OVERFLOW = 0x40000000u;  // | destination rank << 2
 
 // One CTA.  counts_all[G][E] (every rank's per-expert entry counts) -> my_base[e] = first slot, in the
 // receive buffer of e's owner, of this rank's entries for expert e; the work list over what THIS rank
-// receives for its local experts; *n_recv.  Zeroes this rank's own count row for the next call.
+// receives for its local experts, in n_tiles[0] items of nc columns and n_tiles[1] narrow ones, or, if all ranks
+// together have at least tcq_from entries, in n_tiles[2] items of TCQ_COLUMNS; *n_recv.  Zeroes this rank's own count row for the next call.
 // Every receive buffer holds `limit` entries.  If the counts of any destination add up to more (the
 // ranks' token counts exceed what the layer was created for), or an earlier exchange of this layer ran
 // out of time (the table may then mix rows of different calls), nothing may be stored into a peer:
 // *skip is set, the work list and *n_recv are emptied, and the status word names the cause.
 __global__ void moe_ep_plan_kernel(TpCtx c, EpLayout lay, uint32_t n_expert, uint32_t nc, uint32_t small_nc, uint32_t cap,
-                                   uint32_t limit, uint32_t *my_base, uint32_t *cursor, MoeTile *tiles, uint32_t *n_tiles,
+                                   uint32_t limit, uint32_t tcq_from, uint32_t *my_base, uint32_t *cursor, MoeTile *tiles, uint32_t *n_tiles,
                                    uint32_t *n_recv, uint32_t *skip) {
     if (threadIdx.x != 0) return;
+    uint64_t total = 0;
     uint32_t *counts = (uint32_t *)(c.peer[c.rank] + lay.counts);
     const uint32_t per = n_expert / c.size;
     uint32_t t = 0, ts = 0;
@@ -160,7 +164,9 @@ __global__ void moe_ep_plan_kernel(TpCtx c, EpLayout lay, uint32_t n_expert, uin
             atomicCAS(c.status, 0u, EP_STATUS_OVERFLOW | (d << 24));
             bad = true;
         }
+        total += tot_d;
     }
+    const bool tcq = total >= tcq_from;
     for (uint32_t d = 0; d < c.size && !bad; ++d) {
         uint32_t off = 0;  // running slot in rank d's receive buffer
         for (uint32_t e = d * per; e < (d + 1) * per; ++e) {
@@ -172,7 +178,7 @@ __global__ void moe_ep_plan_kernel(TpCtx c, EpLayout lay, uint32_t n_expert, uin
             }
             my_base[e] = off + before_me;
             cursor[e] = 0;
-            if (d == c.rank) moe_emit_items(tiles, cap, t, ts, e - d * per, off, tot, nc, small_nc);
+            if (d == c.rank) moe_emit_items(tiles, cap, t, ts, e - d * per, off, tot, tcq ? TCQ_COLUMNS : nc, tcq ? 0 : small_nc);
             off += tot;
         }
         if (d == c.rank) *n_recv = off;
@@ -182,8 +188,9 @@ __global__ void moe_ep_plan_kernel(TpCtx c, EpLayout lay, uint32_t n_expert, uin
         *n_recv = 0;
     }
     *skip = bad ? 1u : 0u;
-    n_tiles[0] = t;
+    n_tiles[0] = tcq ? 0 : t;
     n_tiles[1] = ts;
+    n_tiles[2] = tcq ? t : 0;
     for (uint32_t e = 0; e < n_expert; ++e) counts[c.rank * n_expert + e] = 0;
 }
 
@@ -305,6 +312,8 @@ struct cera_cuda_moe {
     int16_t *xsum = nullptr, *g_sums = nullptr, *f_sums = nullptr;
     uint32_t *ids = nullptr, *counts = nullptr, *cursor = nullptr, *entry_of = nullptr, *n_tiles = nullptr;
     MoeTile *tiles = nullptr;
+    uint32_t tcq_from = UINT32_MAX;  // entries of a call from which the products run on gemm_tcq.cu
+    void *tcq_scratch = nullptr;     // its operands, for the largest call
     // expert parallelism
     uint32_t ep_rank = 0, ep_size = 1;
     size_t max_total = 0;     // tokens of all ranks in one call
@@ -319,6 +328,18 @@ struct cera_cuda_moe {
 };
 
 namespace {
+
+// Entries ((token, pick) pairs, of all ranks) from which a call's projections go straight from the quantized bytes, in items of 128
+// columns; UINT32_MAX: never.  That kernel converts an expert's weights whatever the number of its tokens; measured (whole layer, us, it /
+// the other): Q8_0 (else on dp4a) 448 / 426 at 8 entries per expert, 453 / 759 at 16 (32 experts, 4 used, 2048 x 1792); Q4_0 (else on
+// mma.sync) 361 / 347 at 32, 424 / 540 at 64; 16 experts: 202 / 158 at 16, 221 / 291 at 32.
+uint32_t moe_tcq_entries(const cera_cuda_moe *h) {
+    const int gt = h->gate->v.type, dt = h->down->v.type;
+    if (moe_force_dp4a() || !gemm_tcq_supports(gt, h->hidden) || !gemm_tcq_supports(dt, h->ff)) return UINT32_MAX;
+    const bool mma = gemm_mma_supports(gt, h->hidden) && gemm_mma_supports(dt, h->ff);
+    const uint32_t least = 16 * h->n_used, want = h->n_expert * (mma ? 40 : 12);
+    return least > want ? least : want;
+}
 
 int32_t moe_create_impl(uint32_t n_expert, uint32_t n_used, uint32_t hidden, uint32_t ff, int32_t ggml_type,
                         const void *gate_exps, const void *up_exps, const void *down_exps, size_t gate_up_bytes,
@@ -372,8 +393,12 @@ int32_t moe_create_impl(uint32_t n_expert, uint32_t n_used, uint32_t hidden, uin
                  o_fq = take((entries + pad) * ff), o_fsum = take((entries + pad) * (ff / 16) * 2), o_w = take(entries * 4),
                  o_g = take(entries * ff * 4), o_u = take(entries * ff * 4), o_eo = take(entries * hidden * 4),
                  o_ids = take(entries * 4), o_counts = take((size_t)n_expert * 4), o_cursor = take((size_t)n_expert * 4),
-                 o_entry = take(entries * 4), o_nt = take(8), o_tiles = take(2 * (entries + n_expert) * sizeof(MoeTile)),
+                 o_entry = take(entries * 4), o_nt = take(12), o_tiles = take(2 * (entries + n_expert) * sizeof(MoeTile)),
                  o_words = take(64 * 4), o_base = take((size_t)n_expert * 4);
+    if (st == CERA_CUDA_OK) h->tcq_from = moe_tcq_entries(h);
+    const bool tcq = entries >= h->tcq_from;  // a call may get there
+    const size_t o_tcq = take(tcq ? gemm_tcq_grouped_scratch(hidden > ff ? hidden : ff, (uint32_t)(entries / TCQ_COLUMNS + n_local)) : 0);
+    if (!tcq) h->tcq_from = UINT32_MAX;
     h->bytes = off;
     if (st == CERA_CUDA_OK) st = check_cuda(cudaMalloc((void **)&h->base, off), "cudaMalloc(moe scratch)");
     if (st == CERA_CUDA_OK) st = check_cuda(cudaMemset(h->base, 0, off), "cudaMemset(moe scratch)");
@@ -402,6 +427,7 @@ int32_t moe_create_impl(uint32_t n_expert, uint32_t n_used, uint32_t hidden, uin
         h->tiles = (MoeTile *)(b + o_tiles);
         h->ep_words = (uint32_t *)(b + o_words);
         h->my_base = (uint32_t *)(b + o_base);
+        h->tcq_scratch = b + o_tcq;
         st = check_cuda(cudaMemcpy(h->router, router, (size_t)n_expert * hidden * 4, cudaMemcpyDefault), "cudaMemcpy(router)");
         if (st == CERA_CUDA_OK && exp_probs_b)
             st = check_cuda(cudaMemcpy(h->bias, exp_probs_b, (size_t)n_expert * 4, cudaMemcpyDefault), "cudaMemcpy(exp_probs_b)");
@@ -444,35 +470,30 @@ int32_t moe_create_impl(uint32_t n_expert, uint32_t n_used, uint32_t hidden, uin
     return CERA_CUDA_OK;
 }
 
-// How a call of n tokens with `entries` (token, pick) pairs runs, and the scratch that takes (null or to be freed in stream order); the
-// work list covers `experts` of the layer's experts.  A handful of tokens: dp4a work items of 8 columns (1 for a single token); a
-// batch: tensor-core items of 64, or of 128 straight from the quantized bytes.  The latter converts an expert's weights whatever
-// the number of its tokens; measured (whole layer, us, it / the other): Q8_0 (else on dp4a) 448 / 426 at 8 entries per expert, 453 / 759
-// at 16 (32 experts, 4 used, 2048 x 1792); Q4_0 (else on mma.sync) 361 / 347 at 32, 424 / 540 at 64; 16 experts: 202 / 158 at 16,
-// 221 / 291 at 32.
-MoePlan moe_pick_plan(const cera_cuda_moe *h, size_t n, size_t entries, uint32_t experts, cudaStream_t st, void **scratch) {
-    *scratch = nullptr;
-    if (n < 16 || moe_force_dp4a()) return MoePlan::DP4A;
-    const int gt = h->gate->v.type, dt = h->down->v.type;
-    const bool mma = gemm_mma_supports(gt, h->hidden) && gemm_mma_supports(dt, h->ff);
-    if (entries >= (size_t)h->n_expert * (mma ? 40 : 12) && gemm_tcq_supports(gt, h->hidden) && gemm_tcq_supports(dt, h->ff)) {
-        const uint32_t items = (uint32_t)(entries / TCQ_COLUMNS + experts);
-        keep_stream_pool();
-        if (cudaMallocAsync(scratch, gemm_tcq_grouped_scratch(h->hidden > h->ff ? h->hidden : h->ff, items), st) == cudaSuccess) return MoePlan::TCQ;
-        cudaGetLastError();
-        *scratch = nullptr;
-    }
-    return mma ? MoePlan::MMA : MoePlan::DP4A;
+// How a call below tcq_from runs: a handful of tokens in dp4a items of 8 columns (1 for a single token), otherwise in tensor-core items of
+// 64 where the type has them.
+MoePlan moe_small_plan(const cera_cuda_moe *h) {
+    return gemm_mma_supports(h->gate->v.type, h->hidden) && gemm_mma_supports(h->down->v.type, h->ff) && !moe_force_dp4a() ? MoePlan::MMA : MoePlan::DP4A;
 }
 
 // The expert-parallel call: see the file header.
 int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softmax_gate, float *out_dev, uint32_t *ids_out_dev,
-                   float *weights_out_dev, MoePlan plan, void *scratch, cudaStream_t st) {
+                   float *weights_out_dev, cudaStream_t st) {
     if (!h->connected) return fail(CERA_CUDA_ERR_STATE, "moe_ffn: expert-parallel layer is not connected to its peers");
     const uint32_t hs = h->hidden, ff = h->ff, ku = h->n_used, E = h->n_expert;
     const size_t entries = n * ku, rmax = h->max_total * ku;
-    const uint32_t nc = moe_columns(plan);
-    const uint32_t max_tiles = (uint32_t)(rmax / nc + E / h->ep_size);
+    // Only the device knows the tokens of all ranks: its plan fills the list of one kernel and leaves the other's empty.
+    const MoePlan plan = moe_small_plan(h);
+    const bool may_tcq = h->tcq_from != UINT32_MAX;
+    const uint32_t nc = moe_columns(plan), per = E / h->ep_size;
+    const uint32_t max_tiles = (uint32_t)((may_tcq ? h->tcq_from - 1 : rmax) / nc + per), max_tcq = (uint32_t)(rmax / TCQ_COLUMNS + per);
+    auto projection = [&](const MoeGemmParams &p) -> int32_t {
+        CERA_TRY(grouped_projection(plan, p, max_tiles, (uint32_t)(rmax + E), per, false, nullptr, st));
+        if (!may_tcq) return CERA_CUDA_OK;
+        MoeGemmParams q = p;
+        q.n_tiles = h->n_tiles + 2;
+        return grouped_projection(MoePlan::TCQ, q, max_tcq, 0, 0, false, h->tcq_scratch, st);
+    };
     uint32_t *counts_mine = (uint32_t *)(h->region + h->lay.counts) + (size_t)h->ep_rank * E;
     uint32_t *n_recv = h->ep_words + 32;
     CERA_TRY(launch_tp_tick(h->ep_words, st));
@@ -483,10 +504,9 @@ int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softm
     // all ranks learn all counts
     const TpRange cr{(uint32_t)((char *)counts_mine - h->region), E * 4};
     CERA_TRY(launch_tp_exchange(h->ep, &cr, 1, 0, st));
-    const uint32_t cap = (uint32_t)(rmax + E), max_small = E / h->ep_size;
     uint32_t *skip = h->ep_words + 33;
-    moe_ep_plan_kernel<<<1, 32, 0, st>>>(h->ep, h->lay, E, nc, plan == MoePlan::MMA ? nc / 2 : 0, cap, (uint32_t)rmax, h->my_base, h->cursor, h->tiles,
-                                         h->n_tiles, n_recv, skip);
+    moe_ep_plan_kernel<<<1, 32, 0, st>>>(h->ep, h->lay, E, nc, plan == MoePlan::MMA ? nc / 2 : 0, (uint32_t)(rmax + E), (uint32_t)rmax, h->tcq_from,
+                                         h->my_base, h->cursor, h->tiles, h->n_tiles, n_recv, skip);
     if (n)
         moe_ep_dispatch_kernel<<<(unsigned)entries, 128, 0, st>>>(h->ep, h->lay, h->ids, ku, hs, E, ActView{h->xs, h->xq, h->xsum},
                                                                    h->my_base, h->cursor, skip);
@@ -506,7 +526,7 @@ int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softm
     p.ldc = ff;
     p.tiles = h->tiles;
     p.n_tiles = h->n_tiles;
-    CERA_TRY(grouped_projection(plan, p, max_tiles, cap, max_small, false, scratch, st));
+    CERA_TRY(projection(p));
     const size_t worst = rmax * ff;
     moe_silu_q8_kernel<<<(unsigned)((worst + 255) / 256), 256, 0, st>>>(h->g, h->u, ff, n_recv, h->f_scales, h->f_quants, h->f_sums);
     count_launch();
@@ -520,7 +540,7 @@ int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softm
     d.ldc = hs;
     d.tiles = h->tiles;
     d.n_tiles = h->n_tiles;
-    CERA_TRY(grouped_projection(plan, d, max_tiles, cap, max_small, false, scratch, st));
+    CERA_TRY(projection(d));
     moe_ep_return_kernel<<<(unsigned)rmax, 128, 0, st>>>(h->ep, h->lay, h->expert_out, hs, n_recv);
     count_launch();
     CERA_CUDA_TRY(cudaGetLastError());
@@ -538,11 +558,12 @@ int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softm
 }
 
 // The layer on one GPU, n >= 1.
-int32_t moe_ffn_planned(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softmax_gate, float *out_dev, uint32_t *ids_out_dev, float *weights_out_dev,
-                        MoePlan plan, void *scratch, cudaStream_t st) {
+int32_t moe_ffn_one(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softmax_gate, float *out_dev, uint32_t *ids_out_dev, float *weights_out_dev,
+                    cudaStream_t st) {
     const uint32_t hs = h->hidden, ff = h->ff, ku = h->n_used;
     const size_t entries = n * ku;
     const bool single = n == 1;
+    const MoePlan plan = entries >= h->tcq_from ? MoePlan::TCQ : n < 16 ? MoePlan::DP4A : moe_small_plan(h);
     const uint32_t nc = single ? 1 : moe_columns(plan);
     const uint32_t max_tiles = (uint32_t)(entries / nc + (single ? 0 : h->n_expert));
     CERA_TRY(launch_quantize(x_dev, hs, n, false, h->xs, h->xq, h->xsum, st));
@@ -565,7 +586,7 @@ int32_t moe_ffn_planned(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t 
     p.ldc = ff;
     p.tiles = h->tiles;
     p.n_tiles = h->n_tiles;
-    CERA_TRY(grouped_projection(plan, p, max_tiles, cap, max_small, single, scratch, st));
+    CERA_TRY(grouped_projection(plan, p, max_tiles, cap, max_small, single, h->tcq_scratch, st));
     CERA_TRY(launch_silu_mul(h->g, h->u, ff, entries, h->f_scales, h->f_quants, h->f_sums, st));
     MoeGemmParams d{};
     d.w[0] = h->down->v;
@@ -577,7 +598,7 @@ int32_t moe_ffn_planned(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t 
     d.ldc = hs;
     d.tiles = h->tiles;
     d.n_tiles = h->n_tiles;
-    CERA_TRY(grouped_projection(plan, d, max_tiles, cap, max_small, single, scratch, st));
+    CERA_TRY(grouped_projection(plan, d, max_tiles, cap, max_small, single, h->tcq_scratch, st));
     const size_t total = n * hs;
     moe_combine_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(h->expert_out, h->entry_of, h->weights, ku, hs, n, out_dev);
     count_launch();
@@ -659,19 +680,9 @@ int32_t cera_cuda_moe_ffn(cera_cuda_moe *h, const float *x_dev, size_t n, int32_
     if (!h || (n && (!x_dev || !out_dev))) return fail(CERA_CUDA_ERR_BAD_ARG, "moe_ffn: null argument");
     if (n > h->max_tokens) return fail(CERA_CUDA_ERR_BAD_ARG, "moe_ffn: %zu tokens, created for at most %zu", n, h->max_tokens);
     cudaStream_t st = (cudaStream_t)stream;
-    if (h->ep_size > 1) {  // n == 0 still takes part; the plan follows from the tokens of a full call, alike on every rank
-        void *scratch = nullptr;
-        const MoePlan plan = moe_pick_plan(h, 16, h->max_total * h->n_used, h->n_expert / h->ep_size, st, &scratch);
-        const int32_t rc = moe_ffn_ep(h, x_dev, n, softmax_gate, out_dev, ids_out_dev, weights_out_dev, plan, scratch, st);
-        if (scratch) cudaFreeAsync(scratch, st);  // after the kernels above, in stream order
-        return rc;
-    }
+    if (h->ep_size > 1) return moe_ffn_ep(h, x_dev, n, softmax_gate, out_dev, ids_out_dev, weights_out_dev, st);  // n == 0 still takes part
     if (n == 0) return CERA_CUDA_OK;
-    void *scratch = nullptr;
-    const MoePlan plan = moe_pick_plan(h, n, n * h->n_used, h->n_expert, st, &scratch);
-    const int32_t rc = moe_ffn_planned(h, x_dev, n, softmax_gate, out_dev, ids_out_dev, weights_out_dev, plan, scratch, st);
-    if (scratch) cudaFreeAsync(scratch, st);  // after the kernels above, in stream order
-    return rc;
+    return moe_ffn_one(h, x_dev, n, softmax_gate, out_dev, ids_out_dev, weights_out_dev, st);
 }
 
 size_t cera_cuda_moe_memory_bytes(const cera_cuda_moe *h) {

@@ -511,7 +511,8 @@ CERA_API int32_t cera_cuda_moe_ffn(cera_cuda_moe *moe, const float *x_dev, size_
  * (cera_cuda_moe_ep_handle -> gather in rank order -> cera_cuda_moe_ep_connect).  Every
  * cera_cuda_moe_ffn call is then collective: all ranks call it (n may differ per rank, 0 included);
  * tokens are dispatched to the ranks that own their experts and the results combined back, all by
- * peer stores from the kernels.  Outputs are bit-identical to the single-GPU layer.  A peer that does
+ * peer stores from the kernels.  Outputs are bit-identical to the single-GPU layer for calls of 16
+ * tokens and more, all ranks together (fewer: within f32 rounding).  A peer that does
  * not arrive within CERA_CUDA_TP_TIMEOUT_MS leaves a status word that cera_cuda_moe_ep_status
  * (call it after synchronising the stream) turns into CERA_CUDA_ERR_TIMEOUT.  If the ranks together
  * route more entries to one rank than max_total_tokens x n_used, the call stores nothing into any

@@ -22,7 +22,7 @@ def main():
     from cera_b200 import tp
     report = {"world": world, "cases": []}
     ok = True
-    for name, (t, E, used, hs, ff, n_total) in CASES.items():
+    for name, (t, E, used, hs, ff, n_total, capacity) in CASES.items():
         t = getattr(cb, t)
         q = lambda n, seed: cb.quantize_weights(t, cb.synth_normal(n, seed=seed, sigma=0.02))
         gate, up, down = q(E * ff * hs, 1), q(E * ff * hs, 2), q(E * hs * ff, 3)
@@ -34,8 +34,8 @@ def main():
         if world > 2:
             cut[-2] = n_total
         mine = x[cut[rank]:cut[rank + 1]]
-        moe = cb.MoeFfn(E, used, hs, ff, t, gate, up, down, router, exp_probs_b=bias, max_tokens=max(1, n_total),
-                        ep=(rank, world), max_total_tokens=n_total)
+        moe = cb.MoeFfn(E, used, hs, ff, t, gate, up, down, router, exp_probs_b=bias, max_tokens=capacity,
+                        ep=(rank, world), max_total_tokens=capacity)
         tp.connect(moe)
         outs = []
         for _ in range(3):  # repeated calls reuse counters, cursors and flags
@@ -89,10 +89,15 @@ def main():
     sys.exit(0 if int(flag) else 1)
 
 
+# type, experts, used, hidden, width, tokens of the call, tokens that the expert-parallel layer is made for
 CASES = {
-    "small_q4_0": ("Q4_0", 8, 2, 256, 128, 37),
-    "k_quant": ("Q4_K", 8, 3, 512, 256, 21),
-    "lfm2moe_shape": ("Q4_0", 32, 4, 2048, 1792, 96),
+    "small_q4_0": ("Q4_0", 8, 2, 256, 128, 37, 37),
+    "k_quant": ("Q4_K", 8, 3, 512, 256, 21, 21),
+    "lfm2moe_shape": ("Q4_0", 32, 4, 2048, 1792, 96, 96),
+    "few_of_many": ("Q4_0", 8, 2, 256, 256, 64, 512),  # below the 160 tokens from which the kernel changes, on a layer that gets there
+    "many": ("Q4_0", 8, 2, 256, 256, 400, 512),
+    "few_of_many_q8_0": ("Q8_0", 8, 2, 256, 128, 40, 512),
+    "many_q8_0": ("Q8_0", 8, 2, 256, 128, 60, 512),
 }
 
 if __name__ == "__main__":

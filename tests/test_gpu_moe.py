@@ -112,6 +112,24 @@ def test_routed_ffn_from_quantized_bytes(t_name, hidden, ff, n):
     _run(getattr(cb, t_name), n_expert=8, n_used=2, hidden=hidden, ff=ff, n=n, seed=71)
 
 
+@pytest.mark.parametrize("t_name", ["Q4_0", "Q8_0"])
+def test_a_call_runs_by_its_own_tokens(t_name):
+    """Not by those the layer was made for: the same bits as a layer made for just this call, on both sides of every change of kernel."""
+    torch = need_gpu()
+    import cera_b200 as cb
+    E, used, hs, ff = 8, 2, 256, 256
+    t = getattr(cb, t_name)
+    q = lambda n, seed: cb.quantize_weights(t, cb.synth_normal(n, seed=seed, sigma=0.02))  # noqa: E731
+    parts = (E, used, hs, ff, t, q(E * ff * hs, 1), q(E * ff * hs, 2), q(E * hs * ff, 3), cb.synth_normal(E * hs, seed=4, sigma=0.05))
+    x = cb.synth_normal(400 * hs, seed=5, sigma=1.0).view(400, hs)
+    large = cb.MoeFfn(*parts, max_tokens=400)
+    for n in (400, 160, 159, 49, 48, 47, 16, 15, 1, 400):
+        own = cb.MoeFfn(*parts, max_tokens=n)
+        assert torch.equal(large(x[:n]).view(torch.int32), own(x[:n]).view(torch.int32)), n
+        own.close()
+    large.close()
+
+
 def test_selection_bias_steers_rank_not_weight():
     """exp_probs_b changes which experts are picked; the combine weights stay the unbiased probabilities."""
     need_gpu()
