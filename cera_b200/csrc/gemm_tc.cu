@@ -1199,22 +1199,6 @@ static const bool g_tc_status_registered = register_kernel_status([] {
     return (uint32_t)v << 8;
 });
 
-// By default a stream-ordered pool hands everything back to the driver at every synchronise, and the next prompt's first
-// allocations pay for mapping it again; up to 1 GB of scratch stays cached.  Once per device and thread.
-void keep_stream_pool() {
-    static thread_local int pooled_dev = -1;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (pooled_dev == dev) return;
-    cudaMemPool_t pool = nullptr;
-    if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
-        uint64_t keep = 1ull << 30;
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    }
-    cudaGetLastError();
-    pooled_dev = dev;
-}
-
 // One activation matrix against up to three weights (q / k / v, gate / up): the activation operands are converted once
 // and, when every weight has its image, ONE kernel launch covers all of them (the small matrices' CTAs run beside the
 // large one's instead of after them).  *taken = false: not these kernels' case, nothing launched.
@@ -1244,11 +1228,8 @@ int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, s
     const bool borrowed = lent.p && lent.bytes >= need;
     uint8_t *scratch = (uint8_t *)lent.p;
     if (!borrowed) {
-        keep_stream_pool();
-        if (cudaMallocAsync((void **)&scratch, need, st) != cudaSuccess) {
-            cudaGetLastError();  // no room for the operand scratch: leave the GEMM to the kernels that need none
-            return CERA_CUDA_OK;
-        }
+        scratch = (uint8_t *)scratch_alloc(need, st);
+        if (!scratch) return CERA_CUDA_OK;  // no room for the operand scratch: leave the GEMM to the kernels that need none
     }
     uint8_t *xm = scratch + img_bytes + min_bytes;
     float *g_tab = reinterpret_cast<float *>(xm + xm_bytes), *ginv_tab = g_tab + n_pad;

@@ -554,9 +554,57 @@ __global__ void __launch_bounds__(256) tq_reduce_kernel(const __grid_constant__ 
         if (j < nc) o[(size_t)j * ldc] = p.epilogue == EPI_ADD ? __fadd_rn(o[(size_t)j * ldc], v[j]) : v[j];
 }
 
+// Splits of k for a product of so many 128-row x BN-column tiles, `pairs` 128s of k each: those expected to finish first, in rounds of
+// units on the SMs plus the reduction's launch and traffic.
+uint32_t tcq_splits(uint64_t whole, uint32_t pairs, uint32_t bn) {
+    const uint32_t sms = (uint32_t)sm_count();
+    const double tp = 0.25 + 0.0045 * bn, cells = (double)whole * bn * TQ_BM;
+    double best = 1e30;
+    uint32_t splits = 1;
+    for (uint32_t s = 1; s <= 16 && 2 * s <= pairs + 1; ++s) {
+        const double rounds = (double)((whole * s + sms - 1) / sms);
+        const double t = rounds * (((pairs + s - 1) / s) * tp + 1.0) + (s > 1 ? 2.5 + cells * 4 * (s + 1) / 3e6 : 0.0);
+        if (t < best) {
+            best = t;
+            splits = s;
+        }
+    }
+    return splits;
+}
+
+// A plain product whose converted activations would take more than this goes through them in parts of the columns.
+constexpr size_t TQ_IMG_LIMIT = 256ull << 20;
+
+// The scratch of col_tiles column tiles: activations, then the partial tiles of a split.
+template <int BN>
+size_t tcq_bytes(const TqParams &p, uint32_t col_tiles, size_t *img_bytes, uint32_t *splits) {
+    const uint64_t whole = (uint64_t)p.row_tiles * col_tiles;
+    *splits = p.tiles ? 1 : tcq_splits(whole, (p.n_it + 1) / 2, BN);
+    *img_bytes = (size_t)col_tiles * p.n_it * BN * TQ_COL;
+    return *img_bytes + (*splits > 1 ? (size_t)*splits * whole * BN * TQ_BM * 4 : 0);
+}
+
+template <int T, int BN>
+int32_t launch_tcq_part(TqParams p, const ActView &x, uint8_t *scratch, cudaStream_t st) {
+    size_t img_bytes;
+    tcq_bytes<BN>(p, p.col_tiles, &img_bytes, &p.splits);
+    p.img = scratch;
+    p.partial = reinterpret_cast<float *>(scratch + img_bytes);
+    count_launch(2);
+    CERA_TRY(check_cuda(launch_k(tq_image_kernel<BN>, dim3(p.col_tiles, (p.k + 255) / 256), dim3(TQ_IMG_THREADS), 0, st, x, p.n, p.k, p.n_it, p.tiles,
+                                 p.n_tiles, scratch),
+                        "gemm (quantized, tcgen05) activation launch"));
+    const uint64_t whole = (uint64_t)p.row_tiles * p.col_tiles, units = whole * p.splits, sms = (uint64_t)sm_count();
+    CERA_TRY(check_cuda(launch_k(gemm_tcq_kernel<T, BN>, dim3((unsigned)(units < sms ? units : sms)), dim3(TQ_THREADS), (size_t)Tq<T, BN>::SMEM, st, p),
+                        "gemm (quantized, tcgen05) launch"));
+    if (p.splits == 1) return CERA_CUDA_OK;
+    count_launch();
+    return check_cuda(launch_k(tq_reduce_kernel<BN>, dim3((unsigned)((whole * (BN / 4) * TQ_BM + 255) / 256)), dim3(256), 0, st, p),
+                      "gemm (quantized, tcgen05) reduction launch");
+}
+
 template <int T, int BN>
 int32_t launch_tcq_bn(TqParams p, int segs, const ActView &x, uint32_t max_col_tiles, uint8_t *given, cudaStream_t st, bool *taken) {
-    using S = Tq<T, BN>;
     p.row_tiles = 0;
     for (int i = 0; i < TQ_SEGS; ++i) {
         if (i < segs) p.row_tiles += (p.m[i] + TQ_BM - 1) / TQ_BM;
@@ -564,56 +612,36 @@ int32_t launch_tcq_bn(TqParams p, int segs, const ActView &x, uint32_t max_col_t
     }
     p.n_it = (p.k + TQ_KS - 1) / TQ_KS;
     p.nb = p.k / 32;
-    p.col_tiles = max_col_tiles;
-    const uint32_t sms = (uint32_t)sm_count(), pairs = (p.n_it + 1) / 2;
-    const uint64_t whole = (uint64_t)p.row_tiles * max_col_tiles;
-    p.splits = 1;
-    if (!p.tiles) {
-        // the split of k that is expected to finish first: rounds x 128s of k of a unit, plus the reduction's launch and traffic
-        const double tp = 0.25 + 0.0045 * BN, cells = (double)whole * BN * TQ_BM;
-        double best = 1e30;
-        for (uint32_t s = 1; s <= 16 && 2 * s <= pairs + 1; ++s) {
-            const double rounds = (double)((whole * s + sms - 1) / sms);
-            const double t = rounds * (((pairs + s - 1) / s) * tp + 1.0) + (s > 1 ? 2.5 + cells * 4 * (s + 1) / 3e6 : 0.0);
-            if (t < best) {
-                best = t;
-                p.splits = s;
-            }
-        }
-    }
-    const size_t img_bytes = (size_t)max_col_tiles * p.n_it * BN * TQ_COL, part_bytes = p.splits > 1 ? (size_t)p.splits * whole * BN * TQ_BM * 4 : 0;
     static thread_local int configured_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_dev != dev) {
-        CERA_CUDA_TRY(cudaFuncSetAttribute(gemm_tcq_kernel<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
+        CERA_CUDA_TRY(cudaFuncSetAttribute(gemm_tcq_kernel<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tq<T, BN>::SMEM));
         configured_dev = dev;
     }
-    uint8_t *scratch = given;
-    if (!given) {
-        keep_stream_pool();
-        if (cudaMallocAsync((void **)&scratch, img_bytes + part_bytes, st) != cudaSuccess) {
-            cudaGetLastError();  // no room for the operands: leave the product to the kernels that need none
-            return CERA_CUDA_OK;
-        }
+    if (given) {
+        *taken = true;
+        p.col_tiles = max_col_tiles;
+        return launch_tcq_part<T, BN>(p, x, given, st);
     }
+    const size_t most = TQ_IMG_LIMIT / ((size_t)p.n_it * BN * TQ_COL);
+    const uint32_t part = most < 1 ? 1 : most < max_col_tiles ? (uint32_t)most : max_col_tiles, last = (max_col_tiles - 1) % part + 1;
+    size_t img;
+    uint32_t splits;
+    const size_t bytes = tcq_bytes<BN>(p, part, &img, &splits), bytes_last = tcq_bytes<BN>(p, last, &img, &splits);
+    uint8_t *scratch = (uint8_t *)scratch_alloc(bytes > bytes_last ? bytes : bytes_last, st);
+    if (!scratch) return CERA_CUDA_OK;  // no room for the operands: leave the product to the kernels that need none
     *taken = true;
-    p.img = scratch;
-    p.partial = reinterpret_cast<float *>(scratch + img_bytes);
-    count_launch(2);
-    int32_t rc = check_cuda(launch_k(tq_image_kernel<BN>, dim3(max_col_tiles, (p.k + 255) / 256), dim3(TQ_IMG_THREADS), 0, st, x, p.n, p.k, p.n_it, p.tiles,
-                                     p.n_tiles, scratch),
-                            "gemm (quantized, tcgen05) activation launch");
-    const uint64_t units = whole * p.splits;
-    if (rc == CERA_CUDA_OK)
-        rc = check_cuda(launch_k(gemm_tcq_kernel<T, BN>, dim3((unsigned)(units < sms ? units : sms)), dim3(TQ_THREADS), (size_t)S::SMEM, st, p),
-                        "gemm (quantized, tcgen05) launch");
-    if (rc == CERA_CUDA_OK && p.splits > 1) {
-        count_launch();
-        rc = check_cuda(launch_k(tq_reduce_kernel<BN>, dim3((unsigned)((whole * (BN / 4) * TQ_BM + 255) / 256)), dim3(256), 0, st, p),
-                        "gemm (quantized, tcgen05) reduction launch");
+    int32_t rc = CERA_CUDA_OK;
+    for (uint32_t t = 0; t < max_col_tiles && rc == CERA_CUDA_OK; t += part) {
+        TqParams q = p;
+        const size_t first = (size_t)t * BN;
+        q.col_tiles = max_col_tiles - t < part ? max_col_tiles - t : part;
+        q.n = p.n - first < (size_t)q.col_tiles * BN ? (uint32_t)(p.n - first) : q.col_tiles * BN;
+        q.out[0] = p.out[0] + first * p.ldc[0];
+        rc = launch_tcq_part<T, BN>(q, ActView{x.scales + first * p.nb, x.quants + first * p.k, x.sums + first * (p.k / 16)}, scratch, st);
     }
-    if (!given) cudaFreeAsync(scratch, st);  // after the kernels above, in stream order
+    cudaFreeAsync(scratch, st);  // after the kernels above, in stream order
     return rc;
 }
 
@@ -651,6 +679,12 @@ static size_t tcq_min_columns(const WeightView &w) {
 int32_t launch_gemm_tcq(const WeightView &w, const ActView &x, size_t n, float *out, size_t ldy, size_t ldc, int epilogue, cudaStream_t st, bool *taken) {
     *taken = false;
     if ((uintptr_t)x.quants % 16 || n < tcq_min_columns(w) || !gemm_tcq_supports(w.type, w.k)) return CERA_CUDA_OK;
+    // A graph that is being captured stays one without allocation nodes, which may be cloned and nested: the other kernels need none.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return CERA_CUDA_OK;
+    }
     TqParams p{};
     p.w[0] = w;
     p.out[0] = out;

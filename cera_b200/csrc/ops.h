@@ -47,6 +47,11 @@ struct GemvFusion {
 // (EPI_STORE / EPI_ADD, single column) into the peers' regions.
 int32_t launch_gemv(const GemvSeg *segs, int n_segs, const ActView &x, size_t n_cols, size_t ldy, int epilogue,
                     cudaStream_t st, size_t ldc = 1, bool batch_tile = false, const TpHook *tp = nullptr);
+// Stream-ordered memory for the launches of one call (cudaFreeAsync after them), from a pool of the library's own on the current device, which
+// keeps up to 1 GB of what was freed - by default a pool hands everything back at every synchronisation, and the next call pays for
+// mapping it again - and 64 MB after scratch_trim, which every freed weight calls.  Null: no room.  Captured, it becomes an allocation node.
+void *scratch_alloc(size_t bytes, cudaStream_t st);
+void scratch_trim();
 // Device memory a caller lends a product for its converted operands, from launch to launch on one stream (256-byte aligned); too
 // small or none: a stream-ordered allocation for the call.
 struct GemmScratch {
@@ -107,8 +112,6 @@ int32_t launch_gemm_tcq(const WeightView &w, const ActView &x, size_t n, float *
 size_t gemm_tcq_grouped_scratch(size_t k, uint32_t max_tiles);  // bytes
 int32_t launch_gemm_tcq_grouped(const WeightView *ws, float *const *outs, int n_segs, const ActView &x, const MoeTile *tiles, const uint32_t *n_tiles,
                                 uint32_t max_tiles, uint32_t rows_per_expert, size_t ldc, void *scratch, cudaStream_t st);
-// Keeps the current device's stream-ordered pool from handing its memory back at every synchronisation (gemm_tc.cu).
-void keep_stream_pool();
 // The tensor-core GEMM over a device-side list of such items (one column tile of up to `bn` = 64 or 32 columns per item):
 // w stacks `rows_per_expert` rows per expert; cell (row i of the expert, column c) goes to out[c * ldc + i].
 // *taken = false: no tensor-core path for this weight type / shape.

@@ -7,7 +7,10 @@
 
 #include <cudaTypedefs.h>
 
+#include <mutex>
+
 #include "common.cuh"
+#include "ops.h"
 #include "tensor_map.h"
 
 namespace cera {
@@ -60,6 +63,50 @@ int sm_count() {
         cached_dev = dev;
     }
     return cached;
+}
+
+namespace {
+constexpr int MAX_DEVICES = 64;
+// What the scratch pool keeps while it is in use, and once a weight has been freed: the small products of whatever is left (with nothing kept
+// the next call of 64 columns of 4096 x 14336 took 360 us, mapping it again, instead of 115).
+constexpr uint64_t POOL_IN_USE = 1ull << 30, POOL_KEPT = 64ull << 20;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pools[MAX_DEVICES] = {};
+}  // namespace
+
+void *scratch_alloc(size_t bytes, cudaStream_t st) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= MAX_DEVICES) return nullptr;
+    cudaMemPool_t pool;
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        if (!g_pools[dev]) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            uint64_t keep = POOL_IN_USE;
+            if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            g_pools[dev] = pool;
+        }
+        pool = g_pools[dev];
+    }
+    void *p = nullptr;
+    if (cudaMallocFromPoolAsync(&p, bytes, pool, st) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
+}
+
+void scratch_trim() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= MAX_DEVICES) return;
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    if (g_pools[dev]) cudaMemPoolTrimTo(g_pools[dev], POOL_KEPT);
+    cudaGetLastError();
 }
 
 int32_t tensor_map_2d(CUtensorMap *map, CUtensorMapDataType type, uint32_t elem_bytes, const void *base, uint64_t rows, uint64_t ld, uint32_t box_cols,

@@ -3,6 +3,7 @@
 #include <new>
 
 #include "formats.cuh"
+#include "ops.h"
 #include "weight.h"
 
 namespace cera {
@@ -200,6 +201,7 @@ void cera_cuda_weight_free(cera_cuda_weight *w) {
     if (!w) return;
     if (w->base) cudaFree(w->base);
     if (w->tc_image) cudaFree(w->tc_image);
+    scratch_trim();
     delete w;
 }
 

@@ -125,7 +125,11 @@ CERA_API int32_t cera_cuda_gemv_q5k_f32(const cera_cuda_weight *w, const float *
                                         void *stream);
 /* cera/src/model/transformer.rs:710-788 gemm_preq -> cpu.rs:1437-1557:
  * out_dev[m x n] = W * X for pre-quantized columns.  sums_dev as produced by
- * cera_cuda_quantize_q8_0 (required). */
+ * cera_cuda_quantize_q8_0 (required).  Many columns (more than 32 of Q4_K / Q5_K and of Q6_K with an
+ * operand image, 16 or 48 and more of the others, by size) take stream-ordered scratch, from a pool of
+ * the library's own that keeps up to 1 GB, and 64 MB once a weight is freed; where there is no room, kernels without
+ * scratch run, and the last bits differ.  In a stream that is being captured the former types' scratch is
+ * an allocation node of the graph, the latter run without. */
 CERA_API int32_t cera_cuda_gemm_preq(const cera_cuda_weight *w, const float *scales_dev,
                                      const int8_t *quants_dev, const int16_t *sums_dev,
                                      float *out_dev, size_t m, size_t n, size_t k, void *stream);

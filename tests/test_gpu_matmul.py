@@ -193,8 +193,8 @@ def test_gemm_tensor_core_shapes(t, m, n, k):
     (O.Q4_0, 2050, 48, 2080), (O.Q4_0, 2049, 64, 2048), (O.Q4_0, 131, 65, 32800), (O.Q4_0, 4096, 128, 1056), (O.Q4_0, 4097, 257, 1024),
     (O.Q6_K, 2049, 48, 2048), (O.Q6_K, 300, 63, 14336), (O.Q6_K, 4223, 130, 1024), (O.Q6_K, 4096, 300, 2816)])
 def test_gemm_from_quantized_bytes(t, m, n, k):
-    """The tcgen05 product that converts the weights itself, at the edges of its rows, columns, stages and of its rule; both cell layouts
-    that its splits of k and its direct stores write."""
+    """The tcgen05 product that converts the weights itself, at the edges of its rows, columns, stages and of its rule, with k split and not.
+    Cells row-major: the token-major ones and those added to a residual are a model's (test_gpu_model.py)."""
     torch = need_gpu()
     import cera_b200 as cb
     raw = cb.quantize_weights(t, cb.synth_normal(m * k, seed=7 * t + m + n, sigma=0.02)).cpu().numpy()
@@ -208,6 +208,56 @@ def test_gemm_from_quantized_bytes(t, m, n, k):
     err = np.linalg.norm((got - want).astype(np.float64)) / np.linalg.norm(want.astype(np.float64))
     assert err < 2e-6, f"{O.NAMES[t]} {m}x{n}x{k}: {err}"
     assert_close(got, want, f"{O.NAMES[t]} {m}x{n}x{k}")
+
+
+def test_gemm_scratch_is_bounded_and_given_back():
+    """20000 columns of k = 14336 would take 645 MB of converted activations: they go through 256 MB, in parts whose bits are those of calls of
+    their own, and a freed weight hands the memory back."""
+    torch = need_gpu()
+    import cera_b200 as cb
+    t, m, n, k, part = O.Q8_0, 128, 20000, 14336, 65 * 128
+    cb.QuantWeight(t, 1, 32, cb.quantize_weights(t, cb.synth_normal(32, seed=1, sigma=1.0))).close()  # hands back what earlier calls kept
+    w = cb.QuantWeight(t, m, k, cb.quantize_weights(t, cb.synth_normal(m * k, seed=1, sigma=0.02)))
+    acts = cb.quantize_q8_0(cb.synth_normal(n * k, seed=2, sigma=1.0), k=k, n=n)
+    out = torch.empty(m, n, device="cuda")
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    cb.gemm_preq(w, acts, out)
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] < 320 << 20
+    for first in range(0, n, part):
+        c = min(part, n - first)
+        x = cb.quantize_q8_0(cb.synth_normal(c * k, seed=2, sigma=1.0, offset=first * k), k=k, n=c)
+        assert torch.equal(cb.gemm_preq(w, x, torch.empty(m, c, device="cuda")).view(torch.int32), out[:, first:first + c].view(torch.int32)), first
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    w.close()
+    assert torch.cuda.mem_get_info()[0] - free >= 180 << 20
+
+
+@pytest.mark.parametrize("t,m,k", [(O.Q8_0, 2048, 2048), (O.Q6_K, 2048, 2048)])
+def test_captured_gemm_leaves_a_graph_that_can_be_cloned(t, m, k):
+    """A captured product allocates nothing (allocation nodes bar a graph from being cloned or nested)."""
+    torch = need_gpu()
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    import cera_b200 as cb
+    n = 64
+    w = cb.QuantWeight(t, m, k, cb.quantize_weights(t, cb.synth_normal(m * k, seed=1, sigma=0.02)))
+    acts, out = cb.quantize_q8_0(cb.synth_normal(n * k, seed=2, sigma=1.0), k=k, n=n), torch.empty(m, n, device="cuda")
+    want = cb.gemm_preq(w, acts, out).clone()
+    out.zero_()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        cb.gemm_preq(w, acts, out)
+    err, clone = rt.cudaGraphClone(rt.cudaGraph_t(g.raw_cuda_graph()))
+    assert err == rt.cudaError_t.cudaSuccess, err
+    assert rt.cudaGraphDestroy(clone)[0] == rt.cudaError_t.cudaSuccess
+    g.instantiate()
+    g.replay()
+    torch.cuda.synchronize()
+    assert ((out - want).norm() / want.norm()).item() < 2e-6  # another order of the same f32 sums
 
 
 def test_gemm_on_reference_fixtures():
