@@ -108,9 +108,9 @@ def test_wide_llama_matches_oracle(kv_f16):
     assert compare_greedy_streams(stream_g, stream_o, lambda i: logits_o[i]) >= 4
 
 
-def test_batched_prefill_matches_oracle_and_crosses_a_chunk_boundary():
-    """600 prompt tokens = one full 512-token chunk + a ragged one, through the batched kernels; the last-token logits
-    against the oracle's per-token forward, then decode continues from the batched KV cache."""
+def test_batched_prefill_matches_oracle():
+    """600 prompt tokens through the batched kernels (one chunk: see below for two); the last-token logits against the
+    oracle's per-token forward, then decode continues from the batched KV cache."""
     need_gpu()
     from cera_b200 import synth
     gpu, oracle = _pair(SMALL, seed=13, max_seq_len=620, threads=4)
@@ -121,6 +121,59 @@ def test_batched_prefill_matches_oracle_and_crosses_a_chunk_boundary():
     assert_model_logits(lp, lo, "batched prefill, 600 tokens")
     tok = int(O.argmax(lo))
     assert_model_logits(gpu.forward(tok, 600), oracle.forward(tok, 600), "decode after batched prefill")
+
+
+@pytest.mark.parametrize("kv_f16", [0, 1])
+@pytest.mark.parametrize("wide", [False, True])
+def test_batched_prefill_crosses_chunk_boundaries(wide, kv_f16):
+    """4170 prompt tokens = two chunks of 2048 and a ragged one, the converted activations of the wide model's products in lent buffers; the
+    last logits against the same prompt in portions of at most 500 tokens, then decode from either cache.  A shorter prompt of a chunk and a
+    token against the oracle."""
+    need_gpu()
+    from cera_b200 import synth
+    cfg, n = WIDE if wide else SMALL, 2049
+    gpu, oracle = _pair(cfg, seed=13, max_seq_len=4200, threads=8, kv_f16=kv_f16)
+    prompt = synth.prompt_tokens(4170, cfg["vocab_size"], seed=6)
+    whole = gpu.forward_prefill(prompt, 0)
+    after = gpu.forward(7, 4170)
+    gpu.truncate_kv(0)
+    for at in range(0, 4170, 500):
+        parts = gpu.forward_prefill(prompt[at:at + 500], at)
+    assert_model_logits(whole, parts, "4170 tokens at once and in portions")
+    assert_model_logits(after, gpu.forward(7, 4170), "decode after either")
+    if not wide:
+        gpu.truncate_kv(0)
+        lp = gpu.forward_prefill(prompt[:n], 0)
+        for pos, t in enumerate(prompt[:n]):
+            lo = oracle.forward(int(t), pos)
+        assert_model_logits(lp, lo, "2049 tokens")
+        assert_model_logits(gpu.forward(7, n), oracle.forward(7, n), "decode after 2049 tokens")
+
+
+# the projections' types, by role; 4096 x 1024 is the smallest size at which Q4_0 and Q6_K leave the mma.sync kernel
+PROMPT_TYPES = {
+    "a": dict(ATTN_Q="Q8_0", ATTN_K="Q4_1", ATTN_V="Q8_0", ATTN_OUTPUT="Q8_0", FFN_GATE="Q4_0", FFN_UP="Q4_1", FFN_DOWN="Q8_0"),
+    "b": dict(ATTN_Q="Q4_0", ATTN_K="Q8_0", ATTN_V="Q4_1", ATTN_OUTPUT="Q4_1", FFN_GATE="Q8_0", FFN_UP="Q4_0", FFN_DOWN="Q4_0"),
+    "c": dict(ATTN_Q="Q4_1", ATTN_K="Q4_0", ATTN_V="Q8_0", ATTN_OUTPUT="Q8_0", FFN_GATE="Q4_1", FFN_UP="Q8_0", FFN_DOWN="Q6_K"),
+}
+
+
+@pytest.mark.parametrize("n", [48, 64, 130])
+@pytest.mark.parametrize("types", sorted(PROMPT_TYPES))
+def test_batched_prefill_from_quantized_bytes(types, n):
+    """Prompts through the tcgen05 product that converts the weights itself: token-major stores, added to the residual by the attention's and
+    the feed-forward's output matrices, with k split (8 row tiles for 148 SMs) and not."""
+    need_gpu()
+    import cera_b200 as cb
+    from cera_b200 import synth
+    cfg = dict(WIDE, intermediate_size=4096)
+    gpu, oracle = _pair(cfg, seed=23, max_seq_len=160, threads=8, types={getattr(cb.Role, r): getattr(cb, t) for r, t in PROMPT_TYPES[types].items()})
+    prompt = synth.prompt_tokens(n, cfg["vocab_size"], seed=9)
+    lp = gpu.forward_prefill(prompt, 0)
+    for pos, t in enumerate(prompt):
+        lo = oracle.forward(int(t), pos)
+    assert_model_logits(lp, lo, f"{n} tokens")
+    assert_model_logits(gpu.forward(7, n), oracle.forward(7, n), "decode after the prompt")
 
 
 def test_batched_prefill_wide_model_and_f16_kv():
