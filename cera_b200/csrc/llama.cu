@@ -59,8 +59,11 @@ struct Layer {
 };
 
 constexpr size_t PREFILL_CHUNK = 512;
-// A prompt that needs only its last logits goes through the layers this many tokens at a time on one GPU.  At 512 the wide tcgen05
-// product of the 8B shape's gate and up matrices has 448 tiles for 148 SMs, 3.03 rounds, and pays for 4; at 2048 12.1, and 13.
+// A prompt that needs only its last logits goes through the layers this many tokens at a time on one GPU.  Wider products have fewer
+// nearly empty last rounds of tiles (the 8B shape's gate and up matrices: 3.03 rounds paid as 4 at 512, 12.1 as 13 at 2048), and everything
+// else fewer launches.  Two layers, ms, chunks of 512 / 1024 / 2048 / 4096: width 1024 and 1000 tokens 1.29 / 0.87 / 0.87 / 0.86; 2047
+// tokens 2.78 / 2.06 / 1.55 / 1.55, width 4096 9.01 / 8.24 / 7.68 / 7.68; 4096 tokens 7.4 / 5.6 / 4.6 / 4.2, width 4096 24.0 / 21.8 / 20.6 /
+// 19.9, for twice the buffers (1.2 GB).
 constexpr size_t PROMPT_CHUNK = 2048;
 
 struct LlamaModel : cera_cuda_model {
@@ -607,7 +610,7 @@ int32_t LlamaModel::build() {
     CERA_TRY(m->dev_alloc((void **)&m->u, m->l_ff * 4));
     CERA_TRY(alloc_act(m, m->act_hs, hs));
     if (m->tp_size == 1 && c.max_seq_len > PREFILL_CHUNK) {
-        // (rounded so that the longest prompt fits one chunk; 512 where the device is nearly full)
+        // (rounded so that the longest prompt fits one chunk; 512 where the device is nearly full: its rest is for the weight images)
         const size_t want = std::min(PROMPT_CHUNK, ((size_t)c.max_seq_len + 127) / 128 * 128), more = (want - PREFILL_CHUNK) * 4 * (3 * hs + 4 * qd + 3 * ff);
         size_t free_b = 0, total_b = 0;
         if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b > more + (4ull << 30)) m->pf_chunk = want;

@@ -422,7 +422,11 @@ CERA_API int32_t cera_cuda_forward_greedy(cera_cuda_model *m, uint32_t token, si
 CERA_API int32_t cera_cuda_generate_greedy(cera_cuda_model *m, uint32_t first_token, size_t start_pos,
                                            size_t n, uint32_t *tokens_out, float *device_ms);
 /* Model::forward_prefill (cera/src/model/llama.rs:1607-1649): start_pos must
- * equal seq_len; logits of the last token (may be NULL). */
+ * equal seq_len; logits of the last token (may be NULL).  The batched kernels take a dense model's
+ * portion in chunks: of 2048 tokens on one GPU, or the longest sequence rounded up to 128 if that is
+ * less, provided 4 GB of the device stay free beside their buffers when the model is finalized; of 512
+ * otherwise, and where logits of chosen positions are asked for (below).  The last bits depend on the
+ * chunk, as on whether a weight's operand image found room. */
 CERA_API int32_t cera_cuda_forward_prefill(cera_cuda_model *m, const uint32_t *tokens, size_t n,
                                            size_t start_pos, float *logits_out);
 /* Model::truncate_kv (mod.rs:251-283).  A model with recurrent layers can only be truncated to 0 (a new sequence):
