@@ -7,7 +7,8 @@
 // six-bit (Q6_K: int8) sub-block scale - and so is every partial sum of a block in f32 (below 2^24), so two tcgen05.mma of
 // K = 16 leave the block's exact sum in TMEM.  Q6_K's products have 13 bits: a rounded part and the remainder, two operands.
 // The epilogue adds (d * xs) * sum to f32 registers, packed in pairs, and subtracts the minimum's term m * (xs * A), A the block's sum
-// of quants.  Same operations, same precision as the kernels that form the sums with integer instructions.
+// of quants.  Same operations and types as the kernels that form the sums with integer instructions, in the order of k: error against 64 bits
+// 1.6e-7 to 2e-7 at k of 4096 to 14336 (mma.sync 2e-7; eight columns at a time, whose 32 lanes have shorter chains, 0.8e-7 to 1.1e-7).
 //
 // What bounds it: the shared-memory data path.  Per stage of 64 k, 128 rows and 128 columns the products read 32 KB of operands (256
 // cycles), the epilogue's column scales are 256 broadcasts, and a thread per weight row makes every 16-byte weight load of a
@@ -554,11 +555,13 @@ __global__ void __launch_bounds__(256) tq_reduce_kernel(const __grid_constant__ 
         if (j < nc) o[(size_t)j * ldc] = p.epilogue == EPI_ADD ? __fadd_rn(o[(size_t)j * ldc], v[j]) : v[j];
 }
 
-// Splits of k for a product of so many 128-row x BN-column tiles, `pairs` 128s of k each: those expected to finish first, in rounds of
-// units on the SMs plus the reduction's launch and traffic.
+// Splits of k for a product of so many 128-row x BN-column tiles, `pairs` 128s of k each: those expected to finish first, us: rounds of units on
+// the SMs, each its share of k (measured per 128 of k: 2.15 with 128 columns, 1.7 with 64, 1.47 with 32), plus the reduction's launch and
+// traffic.  Against every split from 1 to 16, at eight shapes from 1024 x 1024 x 64 to 4096 x 14336 x 512, the choice is within 1 % of the
+// fastest, once within 4 % (4096 x 4096 x 128 Q8_0: 86 us whole, 35.3 in four as chosen, 49.7 in five).
 uint32_t tcq_splits(uint64_t whole, uint32_t pairs, uint32_t bn) {
     const uint32_t sms = (uint32_t)sm_count();
-    const double tp = 0.25 + 0.0045 * bn, cells = (double)whole * bn * TQ_BM;
+    const double tp = 1.25 + 0.007 * bn, cells = (double)whole * bn * TQ_BM;
     double best = 1e30;
     uint32_t splits = 1;
     for (uint32_t s = 1; s <= 16 && 2 * s <= pairs + 1; ++s) {
@@ -661,17 +664,21 @@ bool gemm_tcq_supports(int type, size_t k) {
 }
 
 // Fewer columns than this, and the kernels that need no operands in scratch are faster (device times of all launches, us, this
-// kernel / the other): Q8_0 and Q4_1, whose other kernel reads the weights once per eight columns, 4096 x 4096: 27 / 17 at 8
-// columns, 27 / 33 at 16, 90 / 1082 at 512; 1024 x 1024: 24 / 21 at 32, 14 / 33 at 48.  Q4_0 and Q6_K, whose other kernel is the
-// mma.sync one, 4096 x 14336: 54 / 45 and 60 / 56 at 32, 59 / 77 and 64 / 102 at 48, 253 / 491 and 278 / 604 at 512; 1024 x 1024: 16 / 18
-// at 128 but 27 / 19 at 512.
+// kernel / the other).
+//   Q8_0 and Q4_1, whose other kernel reads the weights once per eight columns.  4096 x 4096: 27 / 17 at 8 columns, 27 / 33 at 16, 92 /
+//   1077 at 512; 2048 x 2048: 14 / 18 and 13 / 13 at 16; 2048 x 1024: 22 / 17 at 24, 22 / 22 at 32, 24 / 33 at 48; 1024 x 1024: 23 / 22 at 32,
+//   13 / 33 at 48.
+//   Q4_0 and Q6_K, whose other kernel is the mma.sync one, in tiles of 64 columns.  4096 x 4096: 23 / 16 at 32, 25 / 28 at 48, 26 / 30 at 64, 66 /
+//   143 at 384; 2048 x 4096 and 4096 x 2048: 20 / 14 and 19 / 14 at 64, 22 / 24 and 22 / 27 at 96, 39 / 79 and 47 / 74 at 384; 2048 x 2048: 16 / 11 at
+//   64, 18 / 20 at 96, 20 / 17 at 128, 23 / 33 at 160, 28 / 44 at 384; 1024 x 1024: 16 / 18 at 128 but 27 / 19 at 512 (Q6_K up to a tenth better
+//   throughout).
 static size_t tcq_min_columns(const WeightView &w) {
-    const bool large = (uint64_t)w.m * w.k >= (1u << 22);
+    const uint64_t weights = (uint64_t)w.m * w.k;
     switch (w.type) {
         case CERA_TYPE_Q4_1:
-        case CERA_TYPE_Q8_0: return large ? 16 : 48;
+        case CERA_TYPE_Q8_0: return weights >= 1u << 22 ? 16 : 48;
         case CERA_TYPE_Q4_0:
-        case CERA_TYPE_Q6_K: return large ? 48 : SIZE_MAX;
+        case CERA_TYPE_Q6_K: return weights >= 1u << 24 ? 48 : weights >= 1u << 23 ? 65 : weights >= 1u << 22 ? 129 : SIZE_MAX;
         default: return SIZE_MAX;  // Q4_K, Q5_K: gemm_tc.cu (14336 x 4096 x 512 without an image: 216 us, here 358)
     }
 }

@@ -189,9 +189,10 @@ def test_gemm_tensor_core_shapes(t, m, n, k):
     # Q8_0 / Q4_1: 16 columns up (48 for small matrices), any k: half a stage, one stage, ragged 128s, a split of k, one row
     (O.Q8_0, 1, 48, 32), (O.Q8_0, 127, 64, 96), (O.Q8_0, 129, 65, 320), (O.Q8_0, 300, 129, 64), (O.Q8_0, 130, 16, 32800), (O.Q8_0, 2048, 17, 2080),
     (O.Q8_0, 4100, 33, 1024), (O.Q4_1, 128, 48, 160), (O.Q4_1, 200, 200, 2048), (O.Q4_1, 2100, 31, 2016), (O.Q4_1, 33, 128, 4096),
-    # Q4_0 / Q6_K: 48 columns up, from 2^22 weights on
-    (O.Q4_0, 2050, 48, 2080), (O.Q4_0, 2049, 64, 2048), (O.Q4_0, 131, 65, 32800), (O.Q4_0, 4096, 128, 1056), (O.Q4_0, 4097, 257, 1024),
-    (O.Q6_K, 2049, 48, 2048), (O.Q6_K, 300, 63, 14336), (O.Q6_K, 4223, 130, 1024), (O.Q6_K, 4096, 300, 2816)])
+    # Q4_0 / Q6_K: 48 columns up from 2^24 weights on, 65 from 2^23, 129 from 2^22
+    (O.Q4_0, 2050, 48, 2080), (O.Q4_0, 2049, 64, 2048), (O.Q4_0, 131, 65, 32800), (O.Q4_0, 4096, 128, 1056), (O.Q6_K, 2049, 48, 2048), (O.Q6_K, 300, 63, 14336),
+    (O.Q4_0, 8070, 48, 2080), (O.Q4_0, 8193, 64, 2048), (O.Q4_0, 257, 65, 32800), (O.Q4_0, 4099, 129, 1024), (O.Q4_0, 4097, 257, 1024),
+    (O.Q6_K, 8193, 48, 2048), (O.Q6_K, 1175, 63, 14336), (O.Q6_K, 4223, 130, 1024), (O.Q6_K, 2999, 65, 2816), (O.Q6_K, 4096, 300, 2816)])
 def test_gemm_from_quantized_bytes(t, m, n, k):
     """The tcgen05 product that converts the weights itself, at the edges of its rows, columns, stages and of its rule, with k split and not.
     Cells row-major: the token-major ones and those added to a residual are a model's (test_gpu_model.py)."""

@@ -150,7 +150,7 @@ def test_batched_prefill_crosses_chunk_boundaries(wide, kv_f16):
         assert_model_logits(gpu.forward(7, n), oracle.forward(7, n), "decode after 2049 tokens")
 
 
-# the projections' types, by role; 4096 x 1024 is the smallest size at which Q4_0 and Q6_K leave the mma.sync kernel
+# the projections' types, by role; at 4096 x 1024 Q4_0 and Q6_K leave the mma.sync kernel from 129 columns on
 PROMPT_TYPES = {
     "a": dict(ATTN_Q="Q8_0", ATTN_K="Q4_1", ATTN_V="Q8_0", ATTN_OUTPUT="Q8_0", FFN_GATE="Q4_0", FFN_UP="Q4_1", FFN_DOWN="Q8_0"),
     "b": dict(ATTN_Q="Q4_0", ATTN_K="Q8_0", ATTN_V="Q4_1", ATTN_OUTPUT="Q4_1", FFN_GATE="Q8_0", FFN_UP="Q4_0", FFN_DOWN="Q4_0"),
@@ -158,7 +158,7 @@ PROMPT_TYPES = {
 }
 
 
-@pytest.mark.parametrize("n", [48, 64, 130])
+@pytest.mark.parametrize("n", [48, 64, 127, 130])
 @pytest.mark.parametrize("types", sorted(PROMPT_TYPES))
 def test_batched_prefill_from_quantized_bytes(types, n):
     """Prompts through the tcgen05 product that converts the weights itself: token-major stores, added to the residual by the attention's and
