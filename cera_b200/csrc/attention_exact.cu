@@ -13,7 +13,7 @@
 //   scores  : sixteen positions per warp, two lanes per position: lane bit 0 picks the accumulator (a), a lane holds its
 //             eight chains, so a K row arrives in 128-bit loads and is read once for all heads of the group; five shuffles
 //             add the chains in the reference's order.
-//   up to 1024 positions, ONE launch (attn_fused_exact_kernel): the hd / 32 CTAs of a KV head are a cluster, each scores a
+//   up to 1024 positions and heads of 64, 128 or 256, ONE launch (attn_fused_exact_kernel): the hd / 32 CTAs of a KV head are a cluster, each scores a
 //             share of the positions into the tables of all, then runs the softmax and the value chains of its 32 dims.
 //   beyond  : attn_scores_exact_kernel writes scores and the maximum of every sixteen; attn_exp_exact_kernel turns them into
 //             exponentials in place and leaves one f64 sum per 1024 positions; attn_chain_exact_kernel multiplies by
@@ -444,6 +444,8 @@ attn_chain_exact_kernel(const __grid_constant__ CUtensorMap v_map, const float *
 // the share's K rows come the same way, in whole lines, padded by 16 bytes so that eight rows are read without bank conflicts.
 // 32 heads of 128 in groups of 4, f32, 512 / 1024 positions: 9.5 / 12.9 us alone (12.4 / 18 with four heads per CTA, K rows read
 // in 32-byte pieces and chains that waited for their loads).
+// f32 heads of 256 in groups of 7 or 8 do not fit its shared memory and take three launches: 13.8 / 16.3 us at 300 / 1000 positions, 16 heads
+// of 2 KV heads (with half the K rows staged they fit, 9.8 / 24.1 us).
 // grid = n_kv * cluster size CTAs, AX_VTHREADS threads; dynamic shared memory: AxFused.
 template <int HD, bool F16>
 struct AxFused {
@@ -726,7 +728,7 @@ int32_t launch_decode_attention_exact(const float *q, const void *kc, const void
     if (reach > cap) reach = cap;
     if (seq_len > reach) return fail(CERA_CUDA_ERR_BAD_ARG, "decode_attention: plan 0x%x does not cover %zu positions", plan, seq_len);
     float *ws = (float *)workspace, *aux = ws + n_heads * (size_t)ld;
-    // ---- one launch when the scores fit shared memory (CERA_CUDA_ATTN_EXACT=split keeps the two-kernel form)
+    // ---- one launch when the scores fit shared memory (CERA_CUDA_ATTN_EXACT=split keeps the three-kernel form)
     static const bool no_fused = [] { const char *e = getenv("CERA_CUDA_ATTN_EXACT"); return e && strcmp(e, "split") == 0; }();
     if (!no_fused && b == 1 && (hd == 64 || hd == 128 || hd == 256)) {  // up to 1024 positions
         const uint32_t fpos = (uint32_t)reach, sl = (uint32_t)seq_len;

@@ -92,7 +92,7 @@ def test_decode_attention_bits(nh, nkv, hd, seq, kv_f16):
     (4, 1, 128, 15, 0), (4, 1, 128, 17, 0), (8, 2, 64, 255, 0), (8, 2, 64, 257, 0), (4, 1, 256, 272, 0), (32, 8, 128, 1023, 0),
     (32, 8, 128, 1024, 0), (32, 8, 128, 1025, 0), (6, 2, 128, 1041, 0), (8, 1, 64, 2048, 0), (8, 1, 128, 2049, 0), (3, 1, 256, 1300, 0),
     (5, 1, 32, 40, 0), (2, 2, 160, 1291, 0), (4, 2, 192, 513, 0), (4, 1, 224, 16, 0), (24, 3, 128, 4200, 0), (64, 8, 128, 3075, 0),
-    (4, 1, 128, 300, 2), (4, 1, 64, 1500, 1), (2, 1, 96, 100, 3)])
+    (4, 1, 128, 300, 2), (4, 1, 64, 1500, 1), (2, 1, 96, 100, 3), (8, 1, 256, 1000, 0), (7, 1, 256, 130, 0), (16, 2, 256, 1024, 1)])
 def test_decode_attention_bits_at_tile_edges(nh, nkv, hd, seq, off, kv_f16):
     torch = need_gpu()
     import cera_b200 as cb
