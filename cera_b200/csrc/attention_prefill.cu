@@ -7,8 +7,9 @@
 // low f16, 22 bits, so that a product is two MMAs, the low one first, and its sums are truncated at full size by the second half
 // only.  Queries are scaled by a power of two per row, probabilities by 2^14; what f16 then cannot tell from zero is 2^-39 of the row's
 // largest |q| and of 1.  A tile's weighted values start from zero and are added to the running output in f32.
-// What bounds it: the tensor pipe at the rate of mma.sync, 256 MMAs per 16 rows x 64 keys beside 32 exponentials a lane.  It stays
-// on mma.sync because scores, probabilities and their halves live in registers between the two products.
+// What bounds it: the latency of a warp's own MMAs and exponentials, 256 and 32 a lane per 16 rows x 64 keys, with two warps per scheduler - 255
+// registers - to hide it (tensor pipe 37 % active at 2047 tokens).  It stays on mma.sync because scores, probabilities and their halves
+// live in registers between the two products.
 // 32 heads of 128 in groups of 4: 512 tokens 50 us (153 with FMAs on the CUDA cores), 2047 tokens 345 us (1125).  Error against 64
 // bits 3.0e-7 (4.0e-7).
 //

@@ -10,11 +10,11 @@
 // of quants.  Same operations and types as the kernels that form the sums with integer instructions, in the order of k: error against 64 bits
 // 1.6e-7 to 2e-7 at k of 4096 to 14336 (mma.sync 2e-7; eight columns at a time, whose 32 lanes have shorter chains, 0.8e-7 to 1.1e-7).
 //
-// What bounds it: the shared-memory data path.  Per stage of 64 k, 128 rows and 128 columns the products read 32 KB of operands (256
-// cycles), the epilogue's column scales are 256 broadcasts, and a thread per weight row makes every 16-byte weight load of a
-// warp touch 32 lines; the rescale itself is two packed f32 instructions per pair of cells (three with a minimum) and the
-// conversion about 1.3 per weight.  4096 x 14336 Q6_K, 64 columns: 62 us (110 with mma.sync, which also spends the issue slots
-// of its fragments); 14336 x 4096 Q8_0, 2048 columns: 1.08 ms (12.9 ms by eight columns at a time).
+// What bounds it: no unit's rate (tensor pipe 8 to 14 % active, issue slots 41 to 43 %, DRAM 10 %), but the hands a stage passes through: four warps convert its
+// weights, and a thread per weight row makes each of their 16-byte loads touch 32 lines; then the products; then the rescale, two packed
+// f32 instructions per pair of cells (three with a minimum) and 256 broadcasts of column scales.  4096 x 14336 Q6_K, 64 columns: 60 us
+// (110 with mma.sync, which also spends the issue slots of its fragments); 14336 x 4096 Q8_0, 2048 columns: 1.08 ms (12.9 ms by eight
+// columns at a time).
 //
 // A CTA is persistent: it walks units (128 rows x up to BN columns x a share of k), one thread issuing the products, one
 // requesting activation tiles by bulk copies, four warps converting weights into the operand tiles, eight draining finished
