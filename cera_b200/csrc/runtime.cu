@@ -77,6 +77,14 @@ cudaMemPool_t g_pools[MAX_DEVICES] = {};
 void *scratch_alloc(size_t bytes, cudaStream_t st) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev >= MAX_DEVICES) return nullptr;
+    void *p = nullptr;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        if (cudaMallocAsync(&p, bytes, st) == cudaSuccess) return p;  // the graph's own memory, whatever the pool
+        cudaGetLastError();
+        return nullptr;
+    }
     cudaMemPool_t pool;
     {
         std::lock_guard<std::mutex> lock(g_pool_mu);
@@ -86,7 +94,11 @@ void *scratch_alloc(size_t bytes, cudaStream_t st) {
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = dev;
             uint64_t keep = POOL_IN_USE;
-            if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // another thread may be capturing
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            const cudaError_t e = cudaMemPoolCreate(&pool, &props);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (e != cudaSuccess) {
                 cudaGetLastError();
                 return nullptr;
             }
@@ -95,7 +107,6 @@ void *scratch_alloc(size_t bytes, cudaStream_t st) {
         }
         pool = g_pools[dev];
     }
-    void *p = nullptr;
     if (cudaMallocFromPoolAsync(&p, bytes, pool, st) == cudaSuccess) return p;
     cudaGetLastError();
     return nullptr;

@@ -261,6 +261,30 @@ def test_captured_gemm_leaves_a_graph_that_can_be_cloned(t, m, k):
     assert ((out - want).norm() / want.norm()).item() < 2e-6  # another order of the same f32 sums
 
 
+def test_captured_k_quant_gemm_is_the_first_call_of_a_process():
+    """Its scratch is a node of the graph; nothing that a capture forbids happens on the way, and a replay gives an eager call's bits."""
+    need_gpu()
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch, cera_b200 as cb
+w = cb.QuantWeight(cb.Q4_K, 512, 1024, cb.quantize_weights(cb.Q4_K, cb.synth_normal(512 * 1024, seed=1, sigma=0.02)))
+acts, out = cb.quantize_q8_0(cb.synth_normal(64 * 1024, seed=2, sigma=1.0), k=1024, n=64), torch.zeros(512, 64, device="cuda")
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    cb.gemm_preq(w, acts, out)
+for _ in range(3):
+    g.replay()
+torch.cuda.synchronize()
+got = out.clone()
+assert torch.equal(cb.gemm_preq(w, acts).view(torch.int32), got.view(torch.int32)) and got.abs().max() > 0
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 def test_gemm_on_reference_fixtures():
     """The reference's own extreme fixtures (-128 weights, +/-127 activations)."""
     torch = need_gpu()
