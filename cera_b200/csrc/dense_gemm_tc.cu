@@ -124,6 +124,11 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dense_gemm_tc_kernel(const __gr
             bool ok = true;
             for (uint32_t t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++j) {
                 const uint32_t b = j & 1, acc = tmem + b * S::ACC;
+                const DtTile o = dt_tile<BN, NA>(p, t);
+                // a ragged tile's products stop at its last column (in whole 32s, as the epilogue reads them): an expert's last item.
+                // 2048 tokens through four layers of routed experts at width 4096: 4.50 -> 4.42 ms, 1.4 to 2.4 % in three pairs of runs that
+                // repeat within 1 %
+                const uint32_t idesc = tc_idesc_bf16(DT_BM, min((uint32_t)BN, (o.end - o.first + 31) & ~31u));
                 if (!(ok = tma::mbar_wait_blocking(acc_empty + b, (j >> 1 & 1) ^ 1, abort_flag, &g_dense_tc_status, 2u))) break;
                 tc_fence_after();
                 for (uint32_t k = 0; k < n_k; ++k, ++it) {
@@ -134,8 +139,8 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dense_gemm_tc_kernel(const __gr
                     const uint64_t da = smem_desc_sw128(st), db = smem_desc_sw128(st + NA * DT_A_BYTES);
 #pragma unroll
                     for (int kk = 0; kk < DT_KS / 16; ++kk) {
-                        tc_mma_f16(acc, da + 2 * kk, db + 2 * kk, tc_idesc_bf16(DT_BM, BN), k | kk);
-                        if (NA == 2) tc_mma_f16(acc + BN, smem_desc_sw128(st + DT_A_BYTES) + 2 * kk, db + 2 * kk, tc_idesc_bf16(DT_BM, BN), k | kk);
+                        tc_mma_f16(acc, da + 2 * kk, db + 2 * kk, idesc, k | kk);
+                        if (NA == 2) tc_mma_f16(acc + BN, smem_desc_sw128(st + DT_A_BYTES) + 2 * kk, db + 2 * kk, idesc, k | kk);
                     }
                     tc_commit(empty + s);
                 }
