@@ -22,9 +22,9 @@
 // The chain of an output element is one dependent FMA per position, 4 cycles: 2.1 ns per position at 1.96 GHz bounds a long
 // context (34 us at 16384).  What a chain warp adds to that is the issue of its loads, which do not overlap the FMAs they stand
 // between, and the wait for them when other warps keep the load / store unit busy: V therefore arrives by TMA, probabilities
-// are multiplied by 1 / sum beforehand and fetched four at a time, and operands are loaded 32 positions ahead of their FMAs.  Alone
-// on an SM: 6.5 cycles per position (f32; f16 6.7); eight positions ahead it is 10.8 cycles in either form, and V transposed
-// to [dim][position] by copying warps - 5.1 alone - costs 9 to 13 beside those warps.
+// are multiplied by 1 / sum beforehand and fetched four at a time, and values four or eight positions a load, 32 positions ahead of
+// their FMAs.  Alone on an SM: 5.1 cycles per position (f32; f16 6.0), 6.5 and 6.7 with a load per position, 10.8 eight positions
+// ahead; V transposed to [dim][position] by copying warps - 5.1 alone - costs 9 to 13 beside those warps.
 //
 // The f64 sum of the exponentials is a tree, the reference's a left-to-right loop: the two can differ
 // in the last bits of the f64 sum, which survive the narrowing to f32 only in about one softmax in
@@ -211,79 +211,77 @@ __device__ __forceinline__ void ax_commit() { asm volatile("cp.async.commit_grou
 template <int N>
 __device__ __forceinline__ void ax_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// cnt positions of one lane's chain: out = fma(p, V, out) in position order.  va: the lane's element of the first of cnt rows of 32
-// dims; pa: the head's probabilities, 16-byte aligned (shared-memory addresses).  The loads are volatile so that the compiler
-// leaves them 32 positions ahead of their FMAs.
+// Which of a slice's 32 dims a lane's chain is, and a warp's chains in the order of the dims.
 template <bool F16>
-__device__ __forceinline__ float ax_chain(uint32_t va, uint32_t pa, uint32_t cnt, float acc) {
-    constexpr int R = 8, ROW = F16 ? 64 : 128;  // quads of positions in registers
-    auto ld_v = [](uint32_t &r, uint32_t a) {
-        if constexpr (F16) asm volatile("ld.shared.u16 %0, [%1];" : "=r"(r) : "r"(a) : "memory");
-        else asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(a) : "memory");
+__device__ __forceinline__ uint32_t ax_dim(uint32_t lane) { return F16 ? lane % 4 * 8 + lane / 4 : lane; }
+template <bool F16>
+__device__ __forceinline__ float ax_by_dim(float acc, uint32_t lane) { return F16 ? __shfl_sync(0xffffffffu, acc, lane % 8 * 4 + lane / 8) : acc; }
+
+// cnt positions of one lane's chain: out = fma(p, V, out) in position order.  v: the first of cnt rows of 32 dims; pa: the head's
+// probabilities (shared-memory addresses, 16-byte aligned).  Values come by ldmatrix, whose eight 16-byte rows may lie anywhere: f32, a
+// row of 32 dims is one 8 x 8 matrix of 32-bit words, word l of it lane l's; f16, the four pieces of two rows in turn, transposed, are
+// lane (g, j)'s dim 8 j + g of both.  So one load brings four positions (f16: eight), where one load per position cost the chain 7.9 cycles
+// beside the TMA thread.  The loads are volatile so that the compiler leaves them 32 positions ahead of their FMAs.
+template <bool F16>
+__device__ __forceinline__ float ax_chain(uint32_t v, uint32_t pa, uint32_t cnt, float acc) {
+    constexpr int R = 8, ROW = F16 ? 64 : 128, PER = F16 ? 2 : 1, N = R / PER;  // quads of positions in registers; of a load; loads
+    const uint32_t lane = threadIdx.x & 31;
+    // the matrix row whose address this lane gives: position, piece
+    const uint32_t at = F16 ? (lane >> 3) * 2 + (lane & 1) : lane >> 3, piece = F16 ? (lane >> 1) & 3 : lane & 7;
+    uint32_t va = v + at * ROW + piece * 16;
+    auto ld_v = [](uint32_t (&r)[4], uint32_t a) {
+        if constexpr (F16)
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+        else
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
     };
     auto ld_p = [](float4 &r, uint32_t a) {
         asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "r"(a) : "memory");
     };
-    auto val = [](uint32_t r) -> float {
-        if constexpr (F16) return h2f((uint16_t)r);
-        else return __uint_as_float(r);
+    // four positions, the q-th quad of a load
+    auto quad = [&](const uint32_t (&r)[4], int q, const float4 &p) {
+        if constexpr (F16) {
+            const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&r[2 * q])), b = __half22float2(*reinterpret_cast<const __half2 *>(&r[2 * q + 1]));
+            acc = fmaf(p.w, b.y, fmaf(p.z, b.x, fmaf(p.y, a.y, fmaf(p.x, a.x, acc))));
+        } else {
+            acc = fmaf(p.w, __uint_as_float(r[3]), fmaf(p.z, __uint_as_float(r[2]), fmaf(p.y, __uint_as_float(r[1]), fmaf(p.x, __uint_as_float(r[0]), acc))));
+        }
     };
     const uint32_t full = cnt / (4 * R);
     if (full) {
-        uint32_t v[R][4];
+        uint32_t x[N][4];
         float4 p[R];
 #pragma unroll
-        for (int i = 0; i < R; ++i) {
+        for (int i = 0; i < N; ++i) ld_v(x[i], va + i * 4 * PER * ROW);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) ld_v(v[i][j], va + (4 * i + j) * ROW);
-            ld_p(p[i], pa + 16 * i);
-        }
+        for (int i = 0; i < R; ++i) ld_p(p[i], pa + 16 * i);
 #pragma unroll 1
         for (uint32_t b = 1; b < full; ++b) {
             va += 4 * R * ROW;
             pa += 16 * R;
 #pragma unroll
-            for (int i = 0; i < R; ++i) {
-                acc = fmaf(p[i].x, val(v[i][0]), acc);
-                ld_v(v[i][0], va + (4 * i) * ROW);
-                acc = fmaf(p[i].y, val(v[i][1]), acc);
-                ld_v(v[i][1], va + (4 * i + 1) * ROW);
-                acc = fmaf(p[i].z, val(v[i][2]), acc);
-                ld_v(v[i][2], va + (4 * i + 2) * ROW);
-                acc = fmaf(p[i].w, val(v[i][3]), acc);
-                ld_v(v[i][3], va + (4 * i + 3) * ROW);
-                ld_p(p[i], pa + 16 * i);
+            for (int i = 0; i < N; ++i) {
+#pragma unroll
+                for (int q = 0; q < PER; ++q) {
+                    quad(x[i], q, p[i * PER + q]);
+                    ld_p(p[i * PER + q], pa + 16 * (i * PER + q));
+                }
+                ld_v(x[i], va + i * 4 * PER * ROW);
             }
         }
 #pragma unroll
-        for (int i = 0; i < R; ++i) {
-            acc = fmaf(p[i].x, val(v[i][0]), acc);
-            acc = fmaf(p[i].y, val(v[i][1]), acc);
-            acc = fmaf(p[i].z, val(v[i][2]), acc);
-            acc = fmaf(p[i].w, val(v[i][3]), acc);
-        }
-        va += 4 * R * ROW;
+        for (int i = 0; i < R; ++i) quad(x[i / PER], i % PER, p[i]);
         pa += 16 * R;
     }
-    const uint32_t rest = cnt % (4 * R);
-#pragma unroll 1
-    for (uint32_t i = 0; i < rest / 4; ++i) {
-        uint32_t v[4];
-        float4 p;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) ld_v(v[j], va + (4 * i + j) * ROW);
-        ld_p(p, pa + 16 * i);
-        acc = fmaf(p.x, val(v[0]), acc);
-        acc = fmaf(p.y, val(v[1]), acc);
-        acc = fmaf(p.z, val(v[2]), acc);
-        acc = fmaf(p.w, val(v[3]), acc);
-    }
-#pragma unroll 1
-    for (uint32_t i = rest & ~3u; i < rest; ++i) {
-        uint32_t v, p;
-        ld_v(v, va + i * ROW);
-        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(p) : "r"(pa + 4 * i) : "memory");
-        acc = fmaf(__uint_as_float(p), val(v), acc);
+    // the rest one by one
+    const uint32_t done = full * 4 * R, el = v + ax_dim<F16>(lane) * (F16 ? 2 : 4);
+#pragma unroll 4
+    for (uint32_t i = done; i < cnt; ++i, pa += 4) {
+        uint32_t x, p;
+        if constexpr (F16) asm volatile("ld.shared.u16 %0, [%1];" : "=r"(x) : "r"(el + i * ROW) : "memory");
+        else asm volatile("ld.shared.u32 %0, [%1];" : "=r"(x) : "r"(el + i * ROW) : "memory");
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(p) : "r"(pa) : "memory");
+        acc = fmaf(__uint_as_float(p), F16 ? h2f((uint16_t)x) : __uint_as_float(x), acc);
     }
     return acc;
 }
@@ -328,7 +326,7 @@ __device__ __forceinline__ void ax_emit(float acc, size_t o, uint32_t d, float *
 // of every third tile.  Slots of the ring are handed over through mbarriers, every wait bounded.  The positions of a last,
 // incomplete box are copied by the probability warp: a box may not reach past the cache.  Two heads per CTA: one would read
 // every V slice from L2 once per head, four would share one load / store unit among four chains.
-// 16384 f16 positions, 32 heads of 128 in groups of 4: 66 us, and 86 us with the two kernels ahead (218 and 254 us before; f32 61 and 87).
+// 16384 f16 positions, 32 heads of 128 in groups of 4: 57.6 us, and 77 us with the two kernels ahead.
 constexpr int AXC_HEADS = 2, AXC_PWARPS = 3, AXC_T = 512, AXC_BOX = 256;
 constexpr uint32_t AXC_THREADS = (AXC_HEADS + AXC_PWARPS + 1) * 32;
 template <bool F16>
@@ -430,10 +428,11 @@ attn_chain_exact_kernel(const __grid_constant__ CUtensorMap v_map, const float *
         const uint32_t slot = tile % C::STAGES;
         if (!tma::mbar_wait_blocking(full + slot, (tile / C::STAGES) & 1, &gave_up, &g_ax_status, 1u)) return;
         const uint32_t base = tma::smem_u32(ring + slot * C::STAGE);
-        acc = ax_chain<F16>(base + lane * (F16 ? 2 : 4), base + C::V_BYTES + warp * AXC_T * 4, min((uint32_t)AXC_T, seq - tile * AXC_T), acc);
+        acc = ax_chain<F16>(base, base + C::V_BYTES + warp * AXC_T * 4, min((uint32_t)AXC_T, seq - tile * AXC_T), acc);
         __syncwarp();
         if (lane == 0) tma::mbar_arrive(empty + slot);
     }
+    acc = ax_by_dim<F16>(acc, lane);
     ax_emit(acc, (size_t)(kvh * G + h0 + warp) * hd + d0 + lane, lane, out, scales, quants, sums, tp);
 }
 
@@ -596,7 +595,7 @@ attn_fused_exact_kernel(const float *__restrict__ q, const void *__restrict__ kc
 
     // ---- out[d] = fma(p[t], V[t][d], out[d]) in position order: warp h walks head h, a lane per output dim
     if (warp >= nh) return;
-    const float acc = ax_chain<F16>(tma::smem_u32(vt) + lane * ES, tma::smem_u32(ax_p + (size_t)warp * pstride), seq, 0.0f);
+    const float acc = ax_by_dim<F16>(ax_chain<F16>(tma::smem_u32(vt), tma::smem_u32(ax_p + (size_t)warp * pstride), seq, 0.0f), lane);
     ax_emit(acc, (size_t)(kvh * G + h0 + warp) * HD + d0 + lane, lane, out, scales, quants, sums, tp);
 }
 
