@@ -66,4 +66,33 @@ __device__ __forceinline__ int quantize_lane(float v, float &scale, int &half_su
     return q;
 }
 
+// The same block with four consecutive elements per lane: eight neighbouring lanes hold it, all of them in the call.
+struct QuantQuad {
+    uint32_t quants;  // four int8, the first lowest
+    float scale;      // same on the eight lanes
+    int half_sum;     // sum of the 16-element half this lane is in
+};
+__device__ __forceinline__ QuantQuad quantize_quad(const float (&e)[4]) {
+    float amax = fmaxf(fmaxf(fabsf(e[0]), fabsf(e[1])), fmaxf(fabsf(e[2]), fabsf(e[3])));  // fmaxf, like f32::max, ignores NaN
+    amax = amax == amax ? amax : 0.0f;                                                     // (four of them)
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const float d = __fdiv_rn(amax, 127.0f);
+    const float r = __fdiv_rn(1.0f, d);
+    const float id = (d != 0.0f && isfinite(r)) ? r : 0.0f;
+    // |e * id| is at most 127 and a few roundings, or NaN: added to 1.5 * 2^23 it is rounded to the nearest integer, ties to even, in the
+    // low bits - without the conversions' slow pipe and with nothing to clamp
+    uint32_t q[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float p = __fadd_rn(__fmul_rn(e[i], id), 12582912.0f);
+        q[i] = p == p ? __float_as_uint(p) : 0x4B400000u;
+    }
+    const uint32_t quants = __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
+    int s4 = __dp4a((int)quants, 0x01010101, 0);
+    s4 += __shfl_xor_sync(0xffffffffu, s4, 1);
+    s4 += __shfl_xor_sync(0xffffffffu, s4, 2);
+    return {quants, __half2float(__float2half_rn(d)), s4};
+}
+
 }  // namespace cera

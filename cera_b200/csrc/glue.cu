@@ -71,6 +71,38 @@ __global__ void rope_kernel(float *q, float *k, const float *__restrict__ v, uin
     }
 }
 
+// The same for a batch with adjacent pairs and a table: a thread per two pairs, or per four values of v, in 128-bit accesses.
+// grid (ceil(values of a token / 4 / 256), tokens); every pointer 16-byte aligned, hd a multiple of 4.
+__global__ void __launch_bounds__(256) rope_quad_kernel(float *q, float *k, const float *__restrict__ v, uint32_t start, uint32_t q_dim, uint32_t kv_dim,
+                                                        uint32_t hd, void *k_cache, void *v_cache, int kv_f16, const float *__restrict__ table) {
+    pdl_trigger();
+    pdl_wait();
+    const uint32_t at = (blockIdx.x * 256 + threadIdx.x) * 4, pos = start + blockIdx.y;
+    const size_t t = blockIdx.y;
+    auto store = [&](void *cache, uint32_t e, const float4 &x) {
+        const size_t o = (size_t)pos * kv_dim + e;
+        if (kv_f16) {
+            const __half2 a = __floats2half2_rn(x.x, x.y), b = __floats2half2_rn(x.z, x.w);
+            *reinterpret_cast<uint2 *>((__half *)cache + o) = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+        } else {
+            *reinterpret_cast<float4 *>((float *)cache + o) = x;
+        }
+    };
+    if (at < q_dim + kv_dim) {
+        const bool is_k = at >= q_dim;
+        const uint32_t e = is_k ? at - q_dim : at;
+        float4 *p = reinterpret_cast<float4 *>(is_k ? k + t * kv_dim + e : q + t * q_dim + e);
+        const float4 x = *p, c = *reinterpret_cast<const float4 *>(table + (size_t)pos * hd + e % hd);  // cos, sin of both pairs
+        const float4 r = make_float4(__fsub_rn(__fmul_rn(x.x, c.x), __fmul_rn(x.y, c.y)), __fadd_rn(__fmul_rn(x.x, c.y), __fmul_rn(x.y, c.x)),
+                                     __fsub_rn(__fmul_rn(x.z, c.z), __fmul_rn(x.w, c.w)), __fadd_rn(__fmul_rn(x.z, c.w), __fmul_rn(x.w, c.z)));
+        *p = r;
+        if (is_k && k_cache) store(k_cache, e, r);
+    } else if (v_cache && at < q_dim + 2 * kv_dim) {
+        const uint32_t e = at - q_dim - kv_dim;
+        store(v_cache, e, *reinterpret_cast<const float4 *>(v + t * kv_dim + e));
+    }
+}
+
 // LoRA delta of one projection for one token: y += B (scale * (A x))  (cera/src/lora.rs:794-821 apply_decode; A is
 // [rank x k], B is [d x rank], row-major, f32).  Every CTA recomputes the rank-sized vector (A is small and stays in
 // L2) and then finishes 256 outputs; each B-row dot product is summed from zero and added to y once, as the
@@ -160,7 +192,8 @@ __global__ void embed_kernel(WeightView w, uint32_t token_imm, const uint32_t *_
     HalfRef h0, h1;
     Fmt<T>::decode(raw, item, lo, hi, h0, h1);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i) {
+        float e0[4], e1[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
             int q0 = (lo[i] >> (8 * t)) & 0xFF, q1 = (hi[i] >> (8 * t)) & 0xFF;
@@ -168,9 +201,12 @@ __global__ void embed_kernel(WeightView w, uint32_t token_imm, const uint32_t *_
                 q0 = (int8_t)q0;
                 q1 = (int8_t)q1;
             }
-            out[h0.off + 4 * i + t] = Fmt<T>::deq(q0, h0);
-            out[h1.off + 4 * i + t] = Fmt<T>::deq(q1, h1);
+            e0[t] = Fmt<T>::deq(q0, h0);
+            e1[t] = Fmt<T>::deq(q1, h1);
         }
+        *reinterpret_cast<float4 *>(out + h0.off + 4 * i) = make_float4(e0[0], e0[1], e0[2], e0[3]);  // rows are 16-byte aligned (ops.h)
+        *reinterpret_cast<float4 *>(out + h1.off + 4 * i) = make_float4(e1[0], e1[1], e1[2], e1[3]);
+    }
 }
 
 }  // namespace
@@ -227,6 +263,13 @@ int32_t launch_rope_batch(float *q, float *k, const float *v, size_t start_pos, 
     const uint32_t total = (uint32_t)((n_heads + n_kv_heads) * (head_dim / 2));
     const int threads = 128;
     count_launch();
+    const uintptr_t all = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)table;
+    if (table && rope_type != 1 && head_dim % 4 == 0 && all % 16 == 0) {
+        const uint32_t q_dim = (uint32_t)(n_heads * head_dim), kv_dim = (uint32_t)(n_kv_heads * head_dim);
+        return check_cuda(launch_k(rope_quad_kernel, dim3((q_dim + 2 * kv_dim + 1023) / 1024, (unsigned)n), dim3(256), 0, st, q, k, v, (uint32_t)start_pos, q_dim,
+                                   kv_dim, (uint32_t)head_dim, k_cache, v_cache, kv_f16, table),
+                          "rope launch");
+    }
     return check_cuda(launch_k(rope_kernel, dim3((total + threads - 1) / threads, (unsigned)n), dim3(threads), 0, st, q, k, v,
                                (uint32_t)start_pos, (const uint32_t *)nullptr, (uint32_t)n_heads, (uint32_t)n_kv_heads,
                                (uint32_t)head_dim, theta_scale, freq_factors, rope_type == 1 ? 1 : 0, k_cache, v_cache, kv_f16, table),

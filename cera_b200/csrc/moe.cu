@@ -118,17 +118,25 @@ __global__ void __launch_bounds__(MOE_WARPS * 32) moe_gemm_kernel(const MoeGemmP
 
 // out[j][i] = sum over picks in pick order of weight * expert_out[entry][i]; multiply and add rounded
 // separately, as the reference's `*acc += weight * v` is (lfm2.rs:891-897).
-__global__ void moe_combine_kernel(const float *__restrict__ expert_out, const uint32_t *__restrict__ entry_of,
-                                   const float *__restrict__ weights, uint32_t n_used, uint32_t hidden, size_t n, float *out) {
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= n * hidden) return;
-    const size_t j = idx / hidden, i = idx - j * hidden;
-    float acc = 0.0f;
+// grid tokens x ceil(hidden / 1024): thread = four outputs of a token.
+__global__ void __launch_bounds__(256) moe_combine_kernel(const float *__restrict__ expert_out, const uint32_t *__restrict__ entry_of,
+                                                          const float *__restrict__ weights, uint32_t n_used, uint32_t hidden, float *out) {
+    const uint32_t parts = (hidden + 1023) / 1024, i = (blockIdx.x % parts * 256 + threadIdx.x) * 4;
+    const size_t j = blockIdx.x / parts;
+    if (i >= hidden) return;
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (uint32_t s = 0; s < n_used; ++s) {
         const size_t e = entry_of ? entry_of[j * n_used + s] : j * n_used + s;
-        acc = __fadd_rn(acc, __fmul_rn(weights[j * n_used + s], expert_out[e * hidden + i]));
+        const float w = weights[j * n_used + s];
+        const float4 v = *reinterpret_cast<const float4 *>(expert_out + e * hidden + i);
+        acc.x = __fadd_rn(acc.x, __fmul_rn(w, v.x));
+        acc.y = __fadd_rn(acc.y, __fmul_rn(w, v.y));
+        acc.z = __fadd_rn(acc.z, __fmul_rn(w, v.z));
+        acc.w = __fadd_rn(acc.w, __fmul_rn(w, v.w));
     }
-    out[idx] = acc;
+    float *o = out + j * hidden + i;
+    if ((uintptr_t)out % 16 == 0) *reinterpret_cast<float4 *>(o) = acc;
+    else o[0] = acc.x, o[1] = acc.y, o[2] = acc.z, o[3] = acc.w;
 }
 
 // ---- expert-parallel pieces ------------------------------------------------------------------------
@@ -546,9 +554,7 @@ int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softm
     CERA_CUDA_TRY(cudaGetLastError());
     CERA_TRY(launch_tp_exchange(h->ep, nullptr, 0, 2, st));  // every result row has come back
     if (n) {
-        const size_t total = n * hs;
-        moe_combine_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>((const float *)(rg + h->lay.ret_out), nullptr, h->weights, ku, hs, n,
-                                                                            out_dev);
+        moe_combine_kernel<<<(unsigned)(n * ((hs + 1023) / 1024)), 256, 0, st>>>((const float *)(rg + h->lay.ret_out), nullptr, h->weights, ku, hs, out_dev);
         count_launch();
         CERA_CUDA_TRY(cudaGetLastError());
         if (ids_out_dev) CERA_CUDA_TRY(cudaMemcpyAsync(ids_out_dev, h->ids, entries * 4, cudaMemcpyDeviceToDevice, st));
@@ -587,7 +593,7 @@ int32_t moe_ffn_one(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t soft
     p.tiles = h->tiles;
     p.n_tiles = h->n_tiles;
     CERA_TRY(grouped_projection(plan, p, max_tiles, cap, max_small, single, h->tcq_scratch, st));
-    CERA_TRY(launch_silu_mul(h->g, h->u, ff, entries, h->f_scales, h->f_quants, h->f_sums, st));
+    CERA_TRY(launch_silu_mul(h->g, h->u, ff, entries, h->f_scales, h->f_quants, h->f_sums, st, nullptr, false));
     MoeGemmParams d{};
     d.w[0] = h->down->v;
     d.y[0] = h->expert_out;
@@ -599,8 +605,7 @@ int32_t moe_ffn_one(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t soft
     d.tiles = h->tiles;
     d.n_tiles = h->n_tiles;
     CERA_TRY(grouped_projection(plan, d, max_tiles, cap, max_small, single, h->tcq_scratch, st));
-    const size_t total = n * hs;
-    moe_combine_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(h->expert_out, h->entry_of, h->weights, ku, hs, n, out_dev);
+    moe_combine_kernel<<<(unsigned)(n * ((hs + 1023) / 1024)), 256, 0, st>>>(h->expert_out, h->entry_of, h->weights, ku, hs, out_dev);
     count_launch();
     CERA_CUDA_TRY(cudaGetLastError());
     if (ids_out_dev) CERA_CUDA_TRY(cudaMemcpyAsync(ids_out_dev, h->ids, entries * 4, cudaMemcpyDeviceToDevice, st));

@@ -11,11 +11,11 @@ int32_t launch_quantize(const float *x, size_t k, size_t n, bool strided, float 
                         int16_t *sums, cudaStream_t st);
 // out_f32 and the quantized outputs are each optional (null = skip).
 // tp (optional, tensor-parallel decode step): rmsnorm waits for the exchange that completes x; silu_mul mirrors its
-// quantized output into the peers' regions.
+// quantized output into the peers' regions.  keep = false: the product is needed in quantized form only, and gate's content is undefined afterwards.
 int32_t launch_rmsnorm(const float *x, const float *weight, size_t n_elem, size_t n_cols, float eps, float *out_f32,
                        float *scales, int8_t *quants, int16_t *sums, cudaStream_t st, const TpHook *tp = nullptr);
 int32_t launch_silu_mul(float *gate, const float *up, size_t n_elem, size_t n_cols, float *scales, int8_t *quants,
-                        int16_t *sums, cudaStream_t st, const TpHook *tp = nullptr);
+                        int16_t *sums, cudaStream_t st, const TpHook *tp = nullptr, bool keep = true);
 
 // Up to three weight matrices of one type sharing the same activations
 // (q/k/v, gate/up), handled by one launch.
@@ -162,6 +162,7 @@ int32_t launch_decode_attention_ex(const float *q, const void *kc, const void *v
                                    float *scales, int8_t *quants, int16_t *sums, cudaStream_t st,
                                    const TpHook *tp = nullptr);  // tp: mirror the Q8_0 output into the peers' regions
 
+// out: rows of w.k floats, 16-byte aligned.
 int32_t launch_embed(const WeightView &w, uint32_t token, const uint32_t *token_dev, float *out, cudaStream_t st);
 // n rows: out[j][k] = row tokens_dev[j] of the table.
 // x[i] *= s, and y[i] += x[i] * s (product rounded, then the sum: cera/src/backend/cpu.rs scale_inplace + add_inplace)

@@ -26,6 +26,22 @@ __global__ void quantize_kernel(const float *__restrict__ x, size_t k, size_t n,
     if (sums && (lane & 15) == 0) sums[j * (k / 16) + b * 2 + (lane >> 4)] = (int16_t)hs;
 }
 
+// The same for contiguous columns, a thread per four consecutive elements: one 128-bit load and eight lanes a block, where a warp per
+// block had one 4-byte load in flight per thread.  n_vec = k / 4 * n, a multiple of 8.
+__global__ void __launch_bounds__(256) quantize_quad_kernel(const float *__restrict__ x, size_t n_vec, float *scales, int8_t *quants, int16_t *sums) {
+    pdl_trigger();
+    pdl_wait();
+    const size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = v < n_vec;  // a block's eight lanes are all in or all out
+    const float4 x4 = in ? reinterpret_cast<const float4 *>(x)[v] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float e[4] = {x4.x, x4.y, x4.z, x4.w};
+    const QuantQuad o = quantize_quad(e);
+    if (!in) return;
+    reinterpret_cast<uint32_t *>(quants)[v] = o.quants;
+    if ((threadIdx.x & 7) == 0) scales[v >> 3] = o.scale;
+    if (sums && (threadIdx.x & 3) == 0) sums[v >> 2] = (int16_t)o.half_sum;
+}
+
 // RMSNorm of one column per CTA (cera/src/backend/cpu.rs:2479-2496: f64 sum of
 // squares, inv = (float)(1/sqrt(mean+eps)), x*inv*w left to right), then
 // optionally the Q8_0 quantizer on the normed values.  Latency-bound and on the critical path of
@@ -101,37 +117,56 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_kernel(const float *__rest
     }
 }
 
-// The same operation for columns whose length is a multiple of 32, laid out for latency: every thread owns FOUR
-// consecutive elements (one 128-bit load of x and of the weights), so a 32-element Q8_0 block is eight neighbouring
-// lanes: its amax takes three shuffle steps, its two 16-element sums two, and all blocks of the column are quantized
-// at the same time instead of four per warp one after another.  Up to 4096 elements stay in registers between the
-// sum of squares and the scaling; longer columns re-read x.
-__global__ void __launch_bounds__(RN_THREADS) rmsnorm_q8_kernel(const float *__restrict__ x, const float *__restrict__ weight,
-                                                                 size_t n_elem, double inv_n, float eps, float *out_f32,
-                                                                 float *scales, int8_t *quants, int16_t *sums, const TpHook tp) {
+// The same operation for columns whose length is a multiple of 32.  1024 virtual threads own FOUR consecutive elements each (one 128-bit
+// load of x and of the weights), so a 32-element Q8_0 block is eight neighbouring lanes and all blocks of the column are quantized at the same
+// time.  Up to 4096 elements stay in registers between the sum of squares and the scaling; longer columns re-read x.
+// The CTA's warps share the 32 virtual ones; sums are added in the same order whatever their number.  One column is latency: 32 warps (eight:
+// 0.6 us more in a decode step).  Many columns are throughput, and a CTA of 32 warps holds two of an SM's columns at a time while most of its warps
+// wait for the scale: eight warps, five columns.  2047 x 4096: 64 -> 21 us.
+template <int RQ_WARPS>
+__global__ void __launch_bounds__(RQ_WARPS * 32, RQ_WARPS == RN_WARPS ? 1 : 5) rmsnorm_q8_kernel(const float *__restrict__ x, const float *__restrict__ weight, size_t n_elem, float eps,
+                                                                float *out_f32, float *scales, int8_t *quants, int16_t *sums, const TpHook tp) {
+    constexpr int VT = RN_THREADS, PER = RN_WARPS / RQ_WARPS;  // virtual threads; of a thread
     __shared__ double red[RN_WARPS];
     __shared__ float inv_s;
     pdl_trigger();
     const size_t col = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t nvec = (uint32_t)(n_elem >> 2);
-    const bool single = nvec <= RN_THREADS;
-    float4 wv = make_float4(0.f, 0.f, 0.f, 0.f), xv = wv;
-    if (single && threadIdx.x < nvec) wv = reinterpret_cast<const float4 *>(weight)[threadIdx.x];  // independent of the previous kernel
+    const bool single = nvec <= VT;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 wv[PER], xv[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const uint32_t v = threadIdx.x + j * RQ_WARPS * 32;
+        wv[j] = single && v < nvec ? reinterpret_cast<const float4 *>(weight)[v] : zero;  // independent of the previous kernel
+    }
     pdl_wait();
     tp_arrive_wait(tp.ctx, tp.wait_slot);
     const float4 *xc = reinterpret_cast<const float4 *>(x + col * n_elem);
-    double ss = 0.0;
-    for (uint32_t v = threadIdx.x; v < nvec; v += RN_THREADS) {
-        xv = xc[v];
-        ss += (double)xv.x * (double)xv.x;
-        ss += (double)xv.y * (double)xv.y;
-        ss += (double)xv.z * (double)xv.z;
-        ss += (double)xv.w * (double)xv.w;
+    double ss[PER] = {};
+    for (uint32_t v0 = 0; v0 < nvec; v0 += VT) {
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            const uint32_t v = v0 + threadIdx.x + j * RQ_WARPS * 32;
+            xv[j] = v < nvec ? xc[v] : zero;
+        }
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            if (v0 + threadIdx.x + j * RQ_WARPS * 32 >= nvec) continue;
+            ss[j] += (double)xv[j].x * (double)xv[j].x;
+            ss[j] += (double)xv[j].y * (double)xv[j].y;
+            ss[j] += (double)xv[j].z * (double)xv[j].z;
+            ss[j] += (double)xv[j].w * (double)xv[j].w;
+        }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (lane == 0) red[warp] = ss;
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < PER; ++j) ss[j] += __shfl_xor_sync(0xffffffffu, ss[j], o);
+    if (lane == 0)
+#pragma unroll
+        for (int j = 0; j < PER; ++j) red[warp + j * RQ_WARPS] = ss[j];
     __syncthreads();
     if (warp == 0) {
         double t = red[lane];
@@ -142,45 +177,22 @@ __global__ void __launch_bounds__(RN_THREADS) rmsnorm_q8_kernel(const float *__r
     __syncthreads();
     const float inv = inv_s;
     // whole warps iterate together: nvec is a multiple of 8, so a block's eight lanes are all in or all out
-    for (uint32_t v0 = 0; v0 < nvec; v0 += RN_THREADS) {
-        const uint32_t v = v0 + threadIdx.x;
-        const bool in = v < nvec;
-        if (!single) {
-            xv = in ? xc[v] : make_float4(0.f, 0.f, 0.f, 0.f);
-            wv = in ? reinterpret_cast<const float4 *>(weight)[v] : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        float e[4] = {__fmul_rn(__fmul_rn(xv.x, inv), wv.x), __fmul_rn(__fmul_rn(xv.y, inv), wv.y),
-                      __fmul_rn(__fmul_rn(xv.z, inv), wv.z), __fmul_rn(__fmul_rn(xv.w, inv), wv.w)};
-        if (out_f32 && in) reinterpret_cast<float4 *>(out_f32 + col * n_elem)[v] = make_float4(e[0], e[1], e[2], e[3]);
-        // Q8_0 of the block these eight lanes share (cera/src/backend/cpu.rs:942-958)
-        float amax = 0.0f;
+    for (uint32_t v0 = 0; v0 < nvec; v0 += VT)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float a = fabsf(e[i]);
-            amax = fmaxf(amax, a == a ? a : 0.0f);  // f32::max ignores NaN
+        for (int j = 0; j < PER; ++j) {
+            const uint32_t v = v0 + threadIdx.x + j * RQ_WARPS * 32;
+            const bool in = v < nvec;
+            const float4 xi = single ? xv[j] : in ? xc[v] : zero, wi = single ? wv[j] : in ? reinterpret_cast<const float4 *>(weight)[v] : zero;
+            const float e[4] = {__fmul_rn(__fmul_rn(xi.x, inv), wi.x), __fmul_rn(__fmul_rn(xi.y, inv), wi.y), __fmul_rn(__fmul_rn(xi.z, inv), wi.z),
+                                __fmul_rn(__fmul_rn(xi.w, inv), wi.w)};
+            if (out_f32 && in) reinterpret_cast<float4 *>(out_f32 + col * n_elem)[v] = make_float4(e[0], e[1], e[2], e[3]);
+            const QuantQuad o = quantize_quad(e);
+            if (in) {
+                reinterpret_cast<uint32_t *>(quants + col * n_elem)[v] = o.quants;
+                if ((lane & 7) == 0) scales[col * (n_elem / 32) + (v >> 3)] = o.scale;
+                if ((lane & 3) == 0) sums[col * (n_elem / 16) + (v >> 2)] = (int16_t)o.half_sum;
+            }
         }
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-        const float d = __fdiv_rn(amax, 127.0f);
-        const float r = __fdiv_rn(1.0f, d);
-        const float id = (d != 0.0f && isfinite(r)) ? r : 0.0f;
-        int q[4], s4 = 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float pq = rintf(__fmul_rn(e[i], id));
-            q[i] = pq != pq ? 0 : (int)fminf(fmaxf(pq, -128.0f), 127.0f);
-            s4 += q[i];
-        }
-        s4 += __shfl_xor_sync(0xffffffffu, s4, 1);
-        s4 += __shfl_xor_sync(0xffffffffu, s4, 2);  // sum of the 16 elements of lanes 4j .. 4j+3
-        if (in) {
-            const uint32_t packed = (uint32_t)(uint8_t)q[0] | ((uint32_t)(uint8_t)q[1] << 8) | ((uint32_t)(uint8_t)q[2] << 16) |
-                                    ((uint32_t)(uint8_t)q[3] << 24);
-            reinterpret_cast<uint32_t *>(quants + col * n_elem)[v] = packed;
-            if ((lane & 7) == 0) scales[col * (n_elem / 32) + (v >> 3)] = __half2float(__float2half_rn(d));
-            if ((lane & 3) == 0) sums[col * (n_elem / 16) + (v >> 2)] = (int16_t)s4;
-        }
-    }
 }
 
 __global__ void silu_mul_kernel(float *gate, const float *__restrict__ up, size_t n_elem, size_t n_cols,
@@ -208,8 +220,9 @@ __global__ void silu_mul_kernel(float *gate, const float *__restrict__ up, size_
 }
 
 // SiLU*mul with the Q8_0 quantizer, four consecutive elements per thread (one 128-bit load of gate and of up): a
-// 32-element block is eight neighbouring lanes, so its amax takes three shuffle steps and its 16-element sums two.
-__global__ void __launch_bounds__(256) silu_mul_q8_kernel(float *gate, const float *__restrict__ up, size_t n_vec, float *scales,
+// 32-element block is eight neighbouring lanes, so its amax takes three shuffle steps and its 16-element sums two.  keep: the
+// product replaces gate (a third of the traffic, which a prompt's product on the quants alone does without).
+__global__ void __launch_bounds__(256) silu_mul_q8_kernel(float *gate, const float *__restrict__ up, size_t n_vec, int keep, float *scales,
                                                           int8_t *quants, int16_t *sums, const TpHook tp) {
     pdl_trigger();
     pdl_wait();
@@ -222,38 +235,16 @@ __global__ void __launch_bounds__(256) silu_mul_q8_kernel(float *gate, const flo
         u4 = reinterpret_cast<const float4 *>(up)[v];
     }
     const float e[4] = {silu_mul(g4.x, u4.x), silu_mul(g4.y, u4.y), silu_mul(g4.z, u4.z), silu_mul(g4.w, u4.w)};
-    if (in) reinterpret_cast<float4 *>(gate)[v] = make_float4(e[0], e[1], e[2], e[3]);
-    float amax = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float a = fabsf(e[i]);
-        amax = fmaxf(amax, a == a ? a : 0.0f);
-    }
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float d = __fdiv_rn(amax, 127.0f);
-    const float r = __fdiv_rn(1.0f, d);
-    const float id = (d != 0.0f && isfinite(r)) ? r : 0.0f;
-    int q[4], s4 = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float pq = rintf(__fmul_rn(e[i], id));
-        q[i] = pq != pq ? 0 : (int)fminf(fmaxf(pq, -128.0f), 127.0f);
-        s4 += q[i];
-    }
-    s4 += __shfl_xor_sync(0xffffffffu, s4, 1);
-    s4 += __shfl_xor_sync(0xffffffffu, s4, 2);
+    if (in && keep) reinterpret_cast<float4 *>(gate)[v] = make_float4(e[0], e[1], e[2], e[3]);
+    const QuantQuad o = quantize_quad(e);
     if (!in) return;
-    const uint32_t packed = (uint32_t)(uint8_t)q[0] | ((uint32_t)(uint8_t)q[1] << 8) | ((uint32_t)(uint8_t)q[2] << 16) |
-                            ((uint32_t)(uint8_t)q[3] << 24);
-    const float scale = __half2float(__float2half_rn(d));
-    reinterpret_cast<uint32_t *>(quants)[v] = packed;
-    if ((lane & 7) == 0) scales[v >> 3] = scale;
-    if ((lane & 3) == 0) sums[v >> 2] = (int16_t)s4;
+    reinterpret_cast<uint32_t *>(quants)[v] = o.quants;
+    if ((lane & 7) == 0) scales[v >> 3] = o.scale;
+    if ((lane & 3) == 0) sums[v >> 2] = (int16_t)o.half_sum;
     if (tp.push) {
-        tp_push(tp.ctx, reinterpret_cast<uint32_t *>(quants) + v, packed);
-        if ((lane & 7) == 0) tp_push(tp.ctx, scales + (v >> 3), scale);
-        if ((lane & 3) == 0) tp_push(tp.ctx, sums + (v >> 2), (int16_t)s4);
+        tp_push(tp.ctx, reinterpret_cast<uint32_t *>(quants) + v, o.quants);
+        if ((lane & 7) == 0) tp_push(tp.ctx, scales + (v >> 3), o.scale);
+        if ((lane & 3) == 0) tp_push(tp.ctx, sums + (v >> 2), (int16_t)o.half_sum);
     }
 }
 
@@ -264,8 +255,14 @@ int32_t launch_quantize(const float *x, size_t k, size_t n, bool strided, float 
     if (!x || !scales || !quants) return fail(CERA_CUDA_ERR_BAD_ARG, "quantize_q8_0: null argument");
     if (k == 0 || k % 32) return fail(CERA_CUDA_ERR_BAD_ARG, "quantize_q8_0: k=%zu must be a positive multiple of 32", k);
     if (n == 0) return CERA_CUDA_OK;
-    const size_t warps = (k / 32) * n;
     const int threads = 256;
+    if (!strided && (uintptr_t)x % 16 == 0 && (uintptr_t)quants % 4 == 0) {
+        const size_t n_vec = k / 4 * n;
+        CERA_CUDA_TRY(launch_k(quantize_quad_kernel, dim3((unsigned)((n_vec + threads - 1) / threads)), dim3(threads), 0, st, x, n_vec, scales, quants, sums));
+        count_launch();
+        return check_cuda(cudaGetLastError(), "quantize launch");
+    }
+    const size_t warps = (k / 32) * n;
     const size_t grid = (warps * 32 + threads - 1) / threads;
     CERA_CUDA_TRY(launch_k(quantize_kernel, dim3((unsigned)grid), dim3(threads), 0, st, x, k, n, strided ? 1 : 0, scales, quants, sums));
     count_launch();
@@ -281,8 +278,12 @@ int32_t launch_rmsnorm(const float *x, const float *weight, size_t n_elem, size_
     const int threads = RN_THREADS;
     if (quants && ((uintptr_t)x % 16 == 0) && ((uintptr_t)weight % 16 == 0) && (!out_f32 || (uintptr_t)out_f32 % 16 == 0) &&
         (uintptr_t)quants % 4 == 0) {
-        CERA_CUDA_TRY(launch_k(rmsnorm_q8_kernel, dim3((unsigned)n_cols), dim3(threads), 0, st, x, weight, n_elem, 1.0 / (double)n_elem, eps,
-                               out_f32, scales, quants, sums, tp ? *tp : TpHook{}));
+        const TpHook hook = tp ? *tp : TpHook{};
+        if (n_cols > (size_t)sm_count())
+            CERA_CUDA_TRY(launch_k(rmsnorm_q8_kernel<8>, dim3((unsigned)n_cols), dim3(256), 0, st, x, weight, n_elem, eps, out_f32, scales, quants, sums, hook));
+        else
+            CERA_CUDA_TRY(launch_k(rmsnorm_q8_kernel<RN_WARPS>, dim3((unsigned)n_cols), dim3(threads), 0, st, x, weight, n_elem, eps, out_f32, scales, quants,
+                                   sums, hook));
         count_launch();
         return check_cuda(cudaGetLastError(), "rmsnorm launch");
     }
@@ -293,7 +294,7 @@ int32_t launch_rmsnorm(const float *x, const float *weight, size_t n_elem, size_
 }
 
 int32_t launch_silu_mul(float *gate, const float *up, size_t n_elem, size_t n_cols, float *scales, int8_t *quants,
-                        int16_t *sums, cudaStream_t st, const TpHook *tp) {
+                        int16_t *sums, cudaStream_t st, const TpHook *tp, bool keep) {
     if (!gate || !up) return fail(CERA_CUDA_ERR_BAD_ARG, "silu_mul: null argument");
     if (quants && n_elem % 32) return fail(CERA_CUDA_ERR_BAD_ARG, "silu_mul+quantize: n=%zu must be a multiple of 32", n_elem);
     const size_t total = n_elem * n_cols;
@@ -302,7 +303,7 @@ int32_t launch_silu_mul(float *gate, const float *up, size_t n_elem, size_t n_co
     if (quants && (uintptr_t)gate % 16 == 0 && (uintptr_t)up % 16 == 0 && (uintptr_t)quants % 4 == 0) {
         const size_t n_vec = total / 4;
         CERA_CUDA_TRY(launch_k(silu_mul_q8_kernel, dim3((unsigned)((n_vec + threads - 1) / threads)), dim3(threads), 0, st, gate, up, n_vec,
-                               scales, quants, sums, tp ? *tp : TpHook{}));
+                               keep ? 1 : 0, scales, quants, sums, tp ? *tp : TpHook{}));
         count_launch();
         return check_cuda(cudaGetLastError(), "silu_mul launch");
     }
