@@ -253,16 +253,13 @@ __global__ void __launch_bounds__(128) moe_ep_return_kernel(TpCtx c, EpLayout la
 }
 
 template <int T>
-int32_t launch_moe_gemm(const MoeGemmParams &p, uint32_t max_tiles, bool single, cudaStream_t st) {
+int32_t launch_moe_gemm(const MoeGemmParams &p, uint32_t max_tiles, cudaStream_t st) {
     const uint32_t rows = p.m * p.n_segs;
     uint32_t gx = (rows + MOE_WARPS - 1) / MOE_WARPS;
     const uint32_t want = (uint32_t)sm_count() * 8 / (max_tiles ? max_tiles : 1) + 1;  // a few waves over all items
     if (gx > want) gx = want;
     if (gx < 1) gx = 1;
-    if (single)
-        moe_gemm_kernel<T, 1><<<dim3(gx, max_tiles), MOE_WARPS * 32, 0, st>>>(p);
-    else
-        moe_gemm_kernel<T, MOE_NC><<<dim3(gx, max_tiles), MOE_WARPS * 32, 0, st>>>(p);
+    moe_gemm_kernel<T, MOE_NC><<<dim3(gx, max_tiles), MOE_WARPS * 32, 0, st>>>(p);
     count_launch();
     return check_cuda(cudaGetLastError(), "moe grouped gemm launch");
 }
@@ -284,7 +281,7 @@ uint32_t moe_columns(MoePlan plan) { return plan == MoePlan::TCQ ? TCQ_COLUMNS :
 
 // One grouped projection over the work list, by the kernel that the plan was made for.  cap / max_small: where the list of narrow
 // items starts inside p.tiles and how many it can hold (MMA only); scratch: the TCQ kernel's.
-int32_t grouped_projection(MoePlan plan, const MoeGemmParams &p, uint32_t max_tiles, uint32_t cap, uint32_t max_small, bool single, void *scratch,
+int32_t grouped_projection(MoePlan plan, const MoeGemmParams &p, uint32_t max_tiles, uint32_t cap, uint32_t max_small, void *scratch,
                            cudaStream_t st) {
     if (plan == MoePlan::TCQ)
         return launch_gemm_tcq_grouped(p.w, p.y, p.n_segs, p.x, p.tiles, p.n_tiles, max_tiles, p.m, p.ldc, scratch, st);
@@ -299,7 +296,7 @@ int32_t grouped_projection(MoePlan plan, const MoeGemmParams &p, uint32_t max_ti
         }
         return CERA_CUDA_OK;
     }
-    CERA_DISPATCH_BLOCK_TYPE(p.w[0].type, return (launch_moe_gemm<TT>(p, max_tiles, single, st)));
+    CERA_DISPATCH_BLOCK_TYPE(p.w[0].type, return (launch_moe_gemm<TT>(p, max_tiles, st)));
     return CERA_CUDA_OK;
 }
 
@@ -478,7 +475,7 @@ int32_t moe_create_impl(uint32_t n_expert, uint32_t n_used, uint32_t hidden, uin
     return CERA_CUDA_OK;
 }
 
-// How a call below tcq_from runs: a handful of tokens in dp4a items of 8 columns (1 for a single token), otherwise in tensor-core items of
+// How a call below tcq_from runs: a handful of tokens in dp4a items of 8 columns, otherwise in tensor-core items of
 // 64 where the type has them.
 MoePlan moe_small_plan(const cera_cuda_moe *h) {
     return gemm_mma_supports(h->gate->v.type, h->hidden) && gemm_mma_supports(h->down->v.type, h->ff) && !moe_force_dp4a() ? MoePlan::MMA : MoePlan::DP4A;
@@ -496,11 +493,11 @@ int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softm
     const uint32_t nc = moe_columns(plan), per = E / h->ep_size;
     const uint32_t max_tiles = (uint32_t)((may_tcq ? h->tcq_from - 1 : rmax) / nc + per), max_tcq = (uint32_t)(rmax / TCQ_COLUMNS + per);
     auto projection = [&](const MoeGemmParams &p) -> int32_t {
-        CERA_TRY(grouped_projection(plan, p, max_tiles, (uint32_t)(rmax + E), per, false, nullptr, st));
+        CERA_TRY(grouped_projection(plan, p, max_tiles, (uint32_t)(rmax + E), per, nullptr, st));
         if (!may_tcq) return CERA_CUDA_OK;
         MoeGemmParams q = p;
         q.n_tiles = h->n_tiles + 2;
-        return grouped_projection(MoePlan::TCQ, q, max_tcq, 0, 0, false, h->tcq_scratch, st);
+        return grouped_projection(MoePlan::TCQ, q, max_tcq, 0, 0, h->tcq_scratch, st);
     };
     uint32_t *counts_mine = (uint32_t *)(h->region + h->lay.counts) + (size_t)h->ep_rank * E;
     uint32_t *n_recv = h->ep_words + 32;
@@ -563,17 +560,21 @@ int32_t moe_ffn_ep(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softm
     return CERA_CUDA_OK;
 }
 
-// The layer on one GPU, n >= 1.
+// The layer on one GPU, n >= 1: a single token in three launches of its own.
 int32_t moe_ffn_one(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t softmax_gate, float *out_dev, uint32_t *ids_out_dev, float *weights_out_dev,
                     cudaStream_t st) {
     const uint32_t hs = h->hidden, ff = h->ff, ku = h->n_used;
+    if (n == 1)
+        return launch_moe_token(MoeToken{x_dev, h->router, h->bias, hs, ff, h->n_expert, ku, softmax_gate, h->gate->v, h->up->v, h->down->v,
+                                         {h->xs, h->xq, h->xsum}, {h->f_scales, h->f_quants, h->f_sums}, h->ids, h->weights, ids_out_dev, weights_out_dev, out_dev},
+                                st);
     const size_t entries = n * ku;
-    const bool single = n == 1;
     const MoePlan plan = entries >= h->tcq_from ? MoePlan::TCQ : n < 16 ? MoePlan::DP4A : moe_small_plan(h);
-    const uint32_t nc = single ? 1 : moe_columns(plan);
-    const uint32_t max_tiles = (uint32_t)(entries / nc + (single ? 0 : h->n_expert));
+    const uint32_t nc = moe_columns(plan);
+    const uint32_t max_tiles = (uint32_t)(entries / nc + h->n_expert);
     CERA_TRY(launch_quantize(x_dev, hs, n, false, h->xs, h->xq, h->xsum, st));
-    CERA_TRY(launch_moe_route(x_dev, hs, n, h->router, h->bias, hs, h->n_expert, ku, softmax_gate, 1, h->ids, h->weights, h->counts, st));
+    CERA_TRY(launch_moe_route(x_dev, hs, n, h->router, h->bias, hs, h->n_expert, ku, softmax_gate, 1, h->ids, h->weights, h->counts, st, ids_out_dev,
+                              weights_out_dev));
     const uint32_t cap = (uint32_t)(h->max_total * ku + h->n_expert), max_small = h->n_expert;
     CERA_TRY(launch_moe_plan(h->counts, h->n_expert, nc, plan == MoePlan::MMA ? nc / 2 : 0, cap, h->cursor, h->tiles, h->n_tiles, st));
     moe_scatter_kernel<<<(unsigned)entries, 128, 0, st>>>(h->ids, ku, hs, ActView{h->xs, h->xq, h->xsum}, h->cursor, h->entry_of,
@@ -592,7 +593,7 @@ int32_t moe_ffn_one(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t soft
     p.ldc = ff;
     p.tiles = h->tiles;
     p.n_tiles = h->n_tiles;
-    CERA_TRY(grouped_projection(plan, p, max_tiles, cap, max_small, single, h->tcq_scratch, st));
+    CERA_TRY(grouped_projection(plan, p, max_tiles, cap, max_small, h->tcq_scratch, st));
     CERA_TRY(launch_silu_mul(h->g, h->u, ff, entries, h->f_scales, h->f_quants, h->f_sums, st, nullptr, false));
     MoeGemmParams d{};
     d.w[0] = h->down->v;
@@ -604,12 +605,10 @@ int32_t moe_ffn_one(cera_cuda_moe *h, const float *x_dev, size_t n, int32_t soft
     d.ldc = hs;
     d.tiles = h->tiles;
     d.n_tiles = h->n_tiles;
-    CERA_TRY(grouped_projection(plan, d, max_tiles, cap, max_small, single, h->tcq_scratch, st));
+    CERA_TRY(grouped_projection(plan, d, max_tiles, cap, max_small, h->tcq_scratch, st));
     moe_combine_kernel<<<(unsigned)(n * ((hs + 1023) / 1024)), 256, 0, st>>>(h->expert_out, h->entry_of, h->weights, ku, hs, out_dev);
     count_launch();
     CERA_CUDA_TRY(cudaGetLastError());
-    if (ids_out_dev) CERA_CUDA_TRY(cudaMemcpyAsync(ids_out_dev, h->ids, entries * 4, cudaMemcpyDeviceToDevice, st));
-    if (weights_out_dev) CERA_CUDA_TRY(cudaMemcpyAsync(weights_out_dev, h->weights, entries * 4, cudaMemcpyDeviceToDevice, st));
     return CERA_CUDA_OK;
 }
 

@@ -12,7 +12,7 @@ template <int T>
 __global__ void __launch_bounds__(256) moe_route_kernel(const float *x, const float *__restrict__ router,
                                                         const float *__restrict__ bias, uint32_t hidden, uint32_t ld_x, uint32_t n, uint32_t n_expert,
                                                         uint32_t n_used, int softmax_gate, int renorm, uint32_t *ids, float *weights,
-                                                        uint32_t *counts) {
+                                                        uint32_t *counts, uint32_t *ids_out, float *weights_out) {
     __shared__ float probs[T][MOE_MAX_EXPERTS];
     __shared__ uint32_t picked[T][MOE_MAX_USED];
     __shared__ float w[T][MOE_MAX_USED];
@@ -58,6 +58,8 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const float *x, const fl
     if (lane < n_used) {
         ids[(size_t)j * n_used + lane] = picked[warp][lane];
         weights[(size_t)j * n_used + lane] = w[warp][lane];
+        if (ids_out) ids_out[(size_t)j * n_used + lane] = picked[warp][lane];
+        if (weights_out) weights_out[(size_t)j * n_used + lane] = w[warp][lane];
         atomicAdd(counts + picked[warp][lane], 1u);
     }
 }
@@ -89,14 +91,15 @@ __global__ void moe_plan_kernel(uint32_t *counts, uint32_t n_expert, uint32_t nc
 }  // namespace
 
 int32_t launch_moe_route(const float *x, size_t ld_x, size_t n, const float *router, const float *bias, uint32_t hidden, uint32_t n_expert,
-                         uint32_t n_used, int softmax_gate, int renorm, uint32_t *ids, float *weights, uint32_t *counts, cudaStream_t st) {
+                         uint32_t n_used, int softmax_gate, int renorm, uint32_t *ids, float *weights, uint32_t *counts, cudaStream_t st,
+                         uint32_t *ids_out, float *weights_out) {
     if (n_expert == 0 || n_expert > MOE_MAX_EXPERTS || n_used == 0 || n_used > MOE_MAX_USED || n_used > n_expert)
         return fail(CERA_CUDA_ERR_BAD_ARG, "moe route: %u experts, %u used (limits %d, %d)", n_expert, n_used, MOE_MAX_EXPERTS, MOE_MAX_USED);
     if (n == 0) return CERA_CUDA_OK;
     count_launch();
     auto go = [&](auto kernel, uint32_t per) {
         return check_cuda(launch_k(kernel, dim3((unsigned)((n + per - 1) / per)), dim3(256), 0, st, x, router, bias, hidden, (uint32_t)ld_x, (uint32_t)n, n_expert,
-                                   n_used, softmax_gate, renorm, ids, weights, counts),
+                                   n_used, softmax_gate, renorm, ids, weights, counts, ids_out, weights_out),
                           "moe route launch");
     };
     return n < (size_t)sm_count() * 4 ? go(moe_route_kernel<1>, 1) : go(moe_route_kernel<8>, 8);

@@ -3,7 +3,7 @@
 // Reference: cera/src/model/lfm2.rs:177-226 (select_experts), 673-715 (route_experts).
 #pragma once
 
-#include "common.cuh"
+#include "act.cuh"
 #include "ops.h"
 
 namespace cera {
@@ -11,22 +11,29 @@ namespace cera {
 constexpr int MOE_MAX_EXPERTS = 256;  // the reference's stack buffer (lfm2.rs:180)
 constexpr int MOE_MAX_USED = 16;
 
-// probs[0..n_expert) hold the router logits on entry (shared memory, visible to the whole CTA) and the scores on exit.
-__device__ __forceinline__ void moe_scores(float *probs, uint32_t n_expert, int softmax_gate) {
-    if (softmax_gate) {
-        if (threadIdx.x == 0) {
-            float mx = probs[0];
-            for (uint32_t e = 1; e < n_expert; ++e) mx = fmaxf(mx, probs[e]);
-            float sum = 0.0f;
-            for (uint32_t e = 0; e < n_expert; ++e) {
-                probs[e] = expf(probs[e] - mx);
-                sum += probs[e];
-            }
-            for (uint32_t e = 0; e < n_expert; ++e) probs[e] = probs[e] / sum;
-        }
+// One warp: probs[0..n_expert) hold the router logits on entry (shared memory, visible to the warp) and the scores on exit.
+__device__ __forceinline__ void moe_scores_warp(float *probs, uint32_t n_expert, int softmax_gate) {
+    const uint32_t lane = threadIdx.x & 31;
+    if (softmax_gate) {  // the sum in the order of the experts
+        float mx = -INFINITY;
+        for (uint32_t e = lane; e < n_expert; e += 32) mx = fmaxf(mx, probs[e]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        for (uint32_t e = lane; e < n_expert; e += 32) probs[e] = expf(probs[e] - mx);
+        __syncwarp();
+        float sum = 0.0f;
+        for (uint32_t e = 0; e < n_expert; ++e) sum += probs[e];
+        __syncwarp();
+        for (uint32_t e = lane; e < n_expert; e += 32) probs[e] = probs[e] / sum;
     } else {
-        for (uint32_t e = threadIdx.x; e < n_expert; e += blockDim.x) probs[e] = 1.0f / (1.0f + expf(-probs[e]));
+        for (uint32_t e = lane; e < n_expert; e += 32) probs[e] = 1.0f / (1.0f + expf(-probs[e]));
     }
+    __syncwarp();
+}
+
+// The same for a CTA, which is synchronised on exit.
+__device__ __forceinline__ void moe_scores(float *probs, uint32_t n_expert, int softmax_gate) {
+    if (threadIdx.x < 32) moe_scores_warp(probs, n_expert, softmax_gate);
     __syncthreads();
 }
 
@@ -83,5 +90,24 @@ __device__ __forceinline__ void moe_emit_items(MoeTile *tiles, uint32_t cap, uin
         else tiles[t++] = MoeTile{e, off + f, n};
     }
 }
+
+// One token's call (moe_token.cu): the layer's weights and its scratch.
+struct MoeToken {
+    struct Act {
+        float *scales;
+        int8_t *quants;
+        int16_t *sums;
+    };
+    const float *x, *router, *bias;  // bias: null without one
+    uint32_t hidden, ff, n_expert, n_used;
+    int softmax_gate;
+    WeightView gate, up, down;
+    Act in, mid;  // the token, [hidden]; the gated units of the picks, [n_used][ff]
+    uint32_t *ids;
+    float *weights;
+    uint32_t *ids_out;  // the caller's copies, or null
+    float *weights_out, *out;
+};
+int32_t launch_moe_token(const MoeToken &p, cudaStream_t st);
 
 }  // namespace cera

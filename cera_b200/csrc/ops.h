@@ -98,9 +98,11 @@ struct MoeTile {
     uint32_t expert, first, count;
 };
 // Routing of a batch (moe_route.cu): x rows of ld_x floats; counts[e] += entries of expert e; and the work lists over the
-// buckets (counts is zeroed, n_tiles[0] main list, n_tiles[1] the list of items of at most small_nc columns at tiles + cap).
+// buckets (counts is zeroed, n_tiles[0] main list, n_tiles[1] the list of items of at most small_nc columns at tiles + cap).  ids_out, weights_out:
+// a caller's copies, or null.
 int32_t launch_moe_route(const float *x, size_t ld_x, size_t n, const float *router, const float *bias, uint32_t hidden, uint32_t n_expert,
-                         uint32_t n_used, int softmax_gate, int renorm, uint32_t *ids, float *weights, uint32_t *counts, cudaStream_t st);
+                         uint32_t n_used, int softmax_gate, int renorm, uint32_t *ids, float *weights, uint32_t *counts, cudaStream_t st,
+                         uint32_t *ids_out = nullptr, float *weights_out = nullptr);
 int32_t launch_moe_plan(uint32_t *counts, uint32_t n_expert, uint32_t nc, uint32_t small_nc, uint32_t cap, uint32_t *cursor, MoeTile *tiles,
                         uint32_t *n_tiles, cudaStream_t st);
 // tcgen05 product straight from the quantized bytes (gemm_tcq.cu).  The plain form takes Q4_0, Q4_1, Q8_0 and Q6_K where it is the

@@ -3,7 +3,8 @@ import numpy as np
 import pytest
 
 import oracle_lib as O
-from gpu_util import need_gpu
+from gpu_util import assert_bits, need_gpu
+from test_gpu_moe import _layer
 
 pytestmark = pytest.mark.gpu
 
@@ -31,3 +32,25 @@ def test_contiguous_quantizer_equals_the_strided_one(k, n):
     for c in (b, cb.quantize_q8_0(odd, k=k, n=n)):
         for f in ("quants", "scales", "sums"):
             assert torch.equal(getattr(a, f).view(torch.uint8), getattr(c, f).view(torch.uint8)), f
+
+
+# experts: fewer, as many and more than the cluster has warps; widths whose items do not fill a warp, and that take several rounds
+@pytest.mark.parametrize("t,experts,used,hidden,ff,softmax", [
+    (O.Q4_0, 1, 1, 32, 32, False), (O.Q4_0, 8, 2, 96, 160, True), (O.Q8_0, 33, 4, 2080, 64, False), (O.Q4_1, 64, 16, 256, 96, True),
+    (O.Q4_0, 65, 5, 512, 2112, False), (O.Q8_0, 256, 16, 64, 32, True), (O.Q4_K, 8, 3, 512, 256, False), (O.Q5_K, 16, 4, 256, 768, True),
+    (O.Q6_K, 12, 2, 1280, 512, False), (O.Q4_0, 4, 2, 8224, 64, False)])
+@pytest.mark.parametrize("biased", [False, True])
+def test_one_token_equals_the_first_of_two(t, experts, used, hidden, ff, softmax, biased):
+    torch = need_gpu()
+    import cera_b200 as cb
+    gate, up, down, router = _layer(t, experts, hidden, ff, 100 + experts)
+    bias = O.synth_normal(experts, 5, 0.3) if biased else None
+    moe = cb.MoeFfn(experts, used, hidden, ff, t, gate, up, down, router, exp_probs_b=bias, max_tokens=4)
+    x = torch.from_numpy(O.synth_normal(2 * hidden, 7, 1.0).reshape(2, hidden)).cuda()
+    two = moe(x, softmax_gate=softmax, want_routing=True)
+    one = moe(x[:1], softmax_gate=softmax, want_routing=True)
+    plain = moe(x[:1], softmax_gate=softmax)
+    for a, b, what in zip(one, two, ("out", "ids", "weights")):
+        assert_bits(a[0].cpu().numpy(), b[0].cpu().numpy(), what)
+    assert_bits(plain.cpu().numpy(), one[0].cpu().numpy(), "without routing")
+    moe.close()
