@@ -167,6 +167,22 @@ int32_t launch_gemv_fused(const GemvSeg *segs, int n_segs, const ActView &x, int
     return launch_gemv_rows(segs, n_segs, x, epilogue, fusion, st, taken, tp);
 }
 
+// The column is quantized by every CTA for itself while its first weights are on their way, where a launch of its own came before.  us, both
+// launches / one, back to back: Q4_0 4096 x 4096 6.4 / 4.6, Q4_K 4096 x 4096 8.9 / 6.8, 10240 x 1024 5.6 / 3.8, 28672 x 4096 17.5 / 15.3, Q6_K
+// 4096 x 14336 17.8 / 16.8.
+int32_t launch_gemv_from_f32(const GemvSeg &seg, const float *x, cudaStream_t st, bool *taken) {
+    *taken = false;
+    static const bool chosen = getenv("CERA_CUDA_GEMV") != nullptr;  // A/B runs
+    // a result over its own operand needs the operand quantized first
+    const uintptr_t x0 = (uintptr_t)x, x1 = x0 + (size_t)seg.w.k * 4, y0 = (uintptr_t)seg.y, y1 = y0 + (size_t)seg.w.m * 4;
+    if (chosen || (x0 < y1 && y0 < x1)) return CERA_CUDA_OK;
+    GemvFusion f;
+    f.quant_x = x;
+    CERA_TRY(launch_gemv_exact(&seg, 1, ActView{}, EPI_STORE, &f, st, taken));
+    if (*taken) return CERA_CUDA_OK;
+    return launch_gemv_rows(&seg, 1, ActView{}, EPI_STORE, &f, st, taken);
+}
+
 // All segments must share the type and k.  n_cols in {1,2,4,8}.
 int32_t launch_gemv(const GemvSeg *segs, int n_segs, const ActView &x, size_t n_cols, size_t ldy, int epilogue,
                     cudaStream_t st, size_t ldc, bool batch_tile, const TpHook *tp) {
@@ -254,8 +270,11 @@ int32_t cera_cuda_gemv(const cera_cuda_weight *w, const float *x_dev, float *y_d
     if (!w || !x_dev || !y_dev) return fail(CERA_CUDA_ERR_BAD_ARG, "gemv: null argument");
     if (!w->xq) return fail(CERA_CUDA_ERR_STATE, "gemv: weight was created without activation scratch");
     cudaStream_t st = (cudaStream_t)stream;
-    CERA_TRY(launch_quantize(x_dev, w->v.k, 1, false, w->xs, w->xq, w->xsum, st));
     GemvSeg seg{w->v, y_dev};
+    bool taken = false;
+    CERA_TRY(launch_gemv_from_f32(seg, x_dev, st, &taken));
+    if (taken) return CERA_CUDA_OK;
+    CERA_TRY(launch_quantize(x_dev, w->v.k, 1, false, w->xs, w->xq, w->xsum, st));
     ActView x{w->xs, w->xq, w->xsum};
     return launch_gemv(&seg, 1, x, 1, 1, EPI_STORE, st);
 }

@@ -50,6 +50,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "act.cuh"
 #include "gemv_task.cuh"
 #include "tma.cuh"
 
@@ -278,6 +279,19 @@ __global__ void __launch_bounds__((TEAM ? XG_MAX_WARPS : XG_LONE_MAX_WARPS) * 32
                 a32[v >> 3] = (float)s8;
             }
             if ((lane & 3) == 0) a16[v >> 2] = (float)(int)(int16_t)s4;
+        }
+    } else if (p.f.quant_x) {
+        for (uint32_t v = tid; v < k / 4; v += nthreads) {  // whole warps: k is a multiple of 512
+            const float4 xv = reinterpret_cast<const float4 *>(p.f.quant_x)[v];
+            const float e[4] = {xv.x, xv.y, xv.z, xv.w};
+            const QuantQuad o = quantize_quad(e);
+            const int s32 = o.half_sum + __shfl_xor_sync(0xffffffffu, o.half_sum, 4);
+            reinterpret_cast<uint32_t *>(aq)[v] = o.quants;
+            if ((lane & 7) == 0) {
+                xs[v >> 3] = o.scale;
+                a32[v >> 3] = (float)s32;
+            }
+            if ((lane & 3) == 0) a16[v >> 2] = (float)o.half_sum;
         }
     } else {
         // stage the activation column
@@ -662,7 +676,9 @@ int32_t launch_gemv_exact(const GemvSeg *segs, int n_segs, const ActView &x, int
         if (segs[i].w.ilv != 8) return CERA_CUDA_OK;
     if (xg_cta_smem(k) + xg_warp_smem(2, 4096) > XG_SMEM_LIMIT) return CERA_CUDA_OK;
     const bool norm = fusion && fusion->norm_x;
-    if (norm ? ((uintptr_t)fusion->norm_x % 16 || (uintptr_t)fusion->norm_w % 16 || !fusion->norm_w) : ((uintptr_t)x.quants % 16 != 0)) return CERA_CUDA_OK;
+    if (norm ? ((uintptr_t)fusion->norm_x % 16 || (uintptr_t)fusion->norm_w % 16 || !fusion->norm_w)
+             : (uintptr_t)(fusion && fusion->quant_x ? (const void *)fusion->quant_x : x.quants) % 16 != 0)
+        return CERA_CUDA_OK;
     ExactParams p{};
     if (fusion) p.f = *fusion;
     if (tp) p.tp = *tp;

@@ -19,6 +19,7 @@
 //
 // Arithmetic contract: cera/src/backend/simd.rs:4593-4637 (Q4_0/Q8_0),
 // 5693-5878 (Q4_K), 5893-5976 (Q4_1), 5988-6195 (Q6_K).
+#include "act.cuh"
 #include "gemv_task.cuh"
 
 namespace cera {
@@ -28,6 +29,7 @@ namespace {
 constexpr int RW_WARPS = 8;
 constexpr int RW_THREADS = RW_WARPS * 32;
 constexpr int RW_MAX_SEGS = 3;
+constexpr uint32_t RW_TASK = 144;  // bytes a task's quants take in shared memory
 
 struct RowsParams {
     WeightView w[RW_MAX_SEGS];
@@ -75,7 +77,25 @@ __global__ void __launch_bounds__(RW_THREADS) gemv_rows_kernel(const RowsParams 
             pdl_trigger();
             pdl_wait();
             tp_arrive_wait(p.tp.ctx, p.tp.wait_slot);
-            if (active) load_act<T>(p.x, tau, act);
+            if (p.f.quant_x) {
+                // Every CTA quantizes the column for itself, into shared memory: four elements a thread, and a lane task's 128 quants 16 bytes
+                // further than they need, so that the lanes' 16-byte reads do not meet in one bank.
+                extern __shared__ __align__(16) uint8_t rw_x[];
+                float *scales = reinterpret_cast<float *>(rw_x + (size_t)p.t128 * RW_TASK);
+                int16_t *sums = reinterpret_cast<int16_t *>(scales + 4 * p.t128);
+                for (uint32_t v = threadIdx.x; v < p.k / 4; v += RW_THREADS) {  // whole warps: k is a multiple of 128
+                    const float4 x4 = reinterpret_cast<const float4 *>(p.f.quant_x)[v];
+                    const float e[4] = {x4.x, x4.y, x4.z, x4.w};
+                    const QuantQuad o = quantize_quad(e);
+                    *reinterpret_cast<uint32_t *>(rw_x + v / 32 * RW_TASK + v % 32 * 4) = o.quants;
+                    if ((v & 7) == 0) scales[v >> 3] = o.scale;
+                    if ((v & 3) == 0) sums[v >> 2] = (int16_t)o.half_sum;
+                }
+                __syncthreads();
+                if (active) load_act<T>(ActView{scales, reinterpret_cast<const int8_t *>(rw_x), sums}, tau, act, RW_TASK);
+            } else if (active) {
+                load_act<T>(p.x, tau, act);
+            }
             first = false;
         }
         float acc[UNR];
@@ -178,7 +198,8 @@ int32_t launch_rows_typed(const RowsParams &p, cudaStream_t st) {
     const uint32_t rows_per_pass = (RW_WARPS / p.wpr) * UNR;
     const uint32_t passes = (p.total_rows + rows_per_pass - 1) / rows_per_pass;
     count_launch();
-    return check_cuda(launch_k(gemv_rows_kernel<T, UNR>, dim3(passes < cap ? passes : cap), dim3(RW_THREADS), 0, st, p),
+    return check_cuda(launch_k(gemv_rows_kernel<T, UNR>, dim3(passes < cap ? passes : cap), dim3(RW_THREADS),
+                               p.f.quant_x ? (size_t)p.t128 * (RW_TASK + 32) : 0, st, p),
                       "gemv launch");
 }
 
@@ -197,7 +218,7 @@ int32_t launch_gemv_rows(const GemvSeg *segs, int n_segs, const ActView &x, int 
     RowsParams p{};
     if (fusion) p.f = *fusion;
     if (tp) p.tp = *tp;
-    if ((uintptr_t)x.quants % 16 || (uintptr_t)x.scales % 16 || (uintptr_t)x.sums % 16) return CERA_CUDA_OK;
+    if (p.f.quant_x ? (uintptr_t)p.f.quant_x % 16 : (uintptr_t)x.quants % 16 || (uintptr_t)x.scales % 16 || (uintptr_t)x.sums % 16) return CERA_CUDA_OK;
     uint32_t rows = 0;
     for (int i = 0; i < n_segs; ++i) {
         if (segs[i].w.type != type || segs[i].w.k != k) return CERA_CUDA_OK;

@@ -47,9 +47,10 @@ struct ActRegs {
     float xb[8];   // Q6_K: -32 * xs_j * (sum of 16 quants) per half; others: xb[j] = xs_j * (sum of 32 quants)
 };
 
+// q_stride: bytes from a task's quants to the next one's.
 template <int T>
-__device__ __forceinline__ void load_act(const ActView &x, uint32_t tau, ActRegs<T> &r) {
-    const int4 *q = reinterpret_cast<const int4 *>(x.quants + (size_t)tau * 128);
+__device__ __forceinline__ void load_act(const ActView &x, uint32_t tau, ActRegs<T> &r, uint32_t q_stride = 128) {
+    const int4 *q = reinterpret_cast<const int4 *>(x.quants + (size_t)tau * q_stride);
 #pragma unroll
     for (int i = 0; i < 8; ++i) r.a[i] = q[i];
     const float4 s = *reinterpret_cast<const float4 *>(x.scales + (size_t)tau * 4);

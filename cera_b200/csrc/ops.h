@@ -42,7 +42,11 @@ struct GemvFusion {
     const float *norm_x = nullptr, *norm_w = nullptr;
     float norm_eps = 0.0f;
     float *norm_out = nullptr;
+    // Quantizing prologue: the kernel forms the activation column from this f32 vector (16-byte aligned) instead of reading `x`.
+    const float *quant_x = nullptr;
 };
+// y = Wx from the f32 column in one launch.  *taken = false: no kernel with a quantizing prologue takes the shape; nothing launched.
+int32_t launch_gemv_from_f32(const GemvSeg &seg, const float *x, cudaStream_t st, bool *taken);
 // tp (optional): wait for the exchange that completes x before reading it and / or mirror the output stores
 // (EPI_STORE / EPI_ADD, single column) into the peers' regions.
 int32_t launch_gemv(const GemvSeg *segs, int n_segs, const ActView &x, size_t n_cols, size_t ldy, int epilogue,

@@ -34,6 +34,36 @@ def test_contiguous_quantizer_equals_the_strided_one(k, n):
             assert torch.equal(getattr(a, f).view(torch.uint8), getattr(c, f).view(torch.uint8)), f
 
 
+@pytest.mark.parametrize("t", O.QUANT_TYPES)
+@pytest.mark.parametrize("m,k", [(1, 256), (9, 512), (70, 768), (33, 4096), (300, 1024), (20, 14336)])
+def test_gemv_equals_quantizer_and_product(t, m, k):
+    torch = need_gpu()
+    import cera_b200 as cb
+    w = cb.QuantWeight(t, m, k, cb.quantize_weights(t, cb.synth_normal(m * k, seed=m + k, sigma=0.05)))
+    x = torch.from_numpy(O.synth_normal(k, k, 1.0)).cuda()
+    odd = torch.cat([torch.zeros(1, device="cuda"), x])[1:]
+    want = cb.gemm_preq(w, cb.quantize_q8_0(x))[:, 0]
+    for v in (x, odd):
+        assert_bits(cb.gemv(w, v).cpu().numpy(), want.cpu().numpy(), f"{O.NAMES[t]} {m} x {k}")
+
+
+@pytest.mark.parametrize("t", O.QUANT_TYPES)
+def test_gemv_over_its_own_operand(t):
+    torch = need_gpu()
+    import cera_b200 as cb
+    n = 4096
+    w = cb.QuantWeight(t, n, n, cb.quantize_weights(t, cb.synth_normal(n * n, seed=3, sigma=0.05)))
+    x = torch.from_numpy(O.synth_normal(n, 4, 1.0)).cuda()
+    want = cb.gemv(w, x)
+    assert_bits(cb.gemv(w, x, x).cpu().numpy(), want.cpu().numpy(), O.NAMES[t])
+
+
+@pytest.mark.parametrize("t", [O.Q4_0, O.Q4_1, O.Q8_0])
+@pytest.mark.parametrize("m,k", [(5, 128), (17, 384), (3, 32768), (11, 160)])
+def test_gemv_of_32_element_formats_equals_quantizer_and_product(t, m, k):
+    test_gemv_equals_quantizer_and_product(t, m, k)
+
+
 # experts: fewer, as many and more than the cluster has warps; widths whose items do not fill a warp, and that take several rounds
 @pytest.mark.parametrize("t,experts,used,hidden,ff,softmax", [
     (O.Q4_0, 1, 1, 32, 32, False), (O.Q4_0, 8, 2, 96, 160, True), (O.Q8_0, 33, 4, 2080, 64, False), (O.Q4_1, 64, 16, 256, 96, True),
