@@ -61,7 +61,11 @@ __device__ unsigned int g_xg_status = 0;
 namespace {
 
 constexpr int XG_MAX_WARPS = 16;                     // warps per CTA when they form teams (picked per launch)
-constexpr int XG_LONE_MAX_WARPS = 32;                // ... when every warp walks its groups alone (64 registers per thread)
+constexpr int XG_LONE_MAX_WARPS = 32;                // ... when every warp walks its groups alone
+// Registers of a lone warp's thread: 72, what the kernel wants, up to 21 warps (LM head 84.1 -> 78.5 us, Q5_K 14336 x 4096 13.0 -> 12.2), beyond
+// that 64.  (25 warps, the gate / up product, would be 1 us faster with 72 as well, but the next kernel of a decode step, launched early
+// to wait beside this one, then finds no registers left on any SM and starts 2 us late.)
+constexpr int XG_WIDE_WARPS = 21, XG_WIDE_BOUND = 800;  // the launch bound that gives these registers
 constexpr int XG_MAX_SEGS = 3;
 constexpr int XG_SEG_TASKS = 4;                      // tasks (of 128 weights) per segment: two super-blocks
 constexpr int XG_MAX_STAGES = 8;
@@ -131,8 +135,8 @@ __host__ __device__ inline size_t xg_warp_smem(uint32_t stages, uint32_t seg_byt
     return (size_t)stages * seg_bytes + 2 * XG_SCT_BYTES + 2 * XG_TERM_BYTES;
 }
 
-template <int T, bool TEAM>
-__global__ void __launch_bounds__((TEAM ? XG_MAX_WARPS : XG_LONE_MAX_WARPS) * 32) gemv_exact_kernel(const ExactParams p) {
+template <int T, bool TEAM, int BOUND>
+__global__ void __launch_bounds__(BOUND, 1) gemv_exact_kernel(const ExactParams p) {
     using L = SegLayout<T>;
     extern __shared__ __align__(128) uint8_t xg_smem[];
     const uint32_t k = p.k, nb32 = k >> 5, nb = k >> 8, n_seg = k / (128 * XG_SEG_TASKS);
@@ -352,10 +356,12 @@ __global__ void __launch_bounds__((TEAM ? XG_MAX_WARPS : XG_LONE_MAX_WARPS) * 32
 #pragma unroll
             for (int jp = 0; jp < 2; ++jp) {
                 const float2 x2 = make_float2(xv[2 * jp], xv[2 * jp + 1]), a2 = make_float2(av[2 * jp], av[2 * jp + 1]);
-                const float2 scf = __fadd2_rn(make_float2(__uint_as_float(0x4B000000u | ((scp >> (16 * jp)) & 0xFF)),
-                                                          __uint_as_float(0x4B000000u | ((scp >> (16 * jp + 8)) & 0xFF))), nb23);
-                const float2 mnf = __fadd2_rn(make_float2(__uint_as_float(0x4B000000u | ((mnp >> (16 * jp)) & 0xFF)),
-                                                          __uint_as_float(0x4B000000u | ((mnp >> (16 * jp + 8)) & 0xFF))), nb23);
+                // a byte into the low bits of 2^23: its value, exactly, once 2^23 is subtracted
+                auto bytes = [&](uint32_t w) {
+                    return __fadd2_rn(make_float2(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + 2 * jp)),
+                                                  __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7441 + 2 * jp))), nb23);
+                };
+                const float2 scf = bytes(scp), mnf = bytes(mnp);
                 const float2 ee = __fmul2_rn(x2, __fmul2_rn(d2, scf));
                 const float2 tt = __fmul2_rn(__fmul2_rn(x2, __fmul2_rn(dm2, mnf)), a2);
                 e[2 * jp] = ee.x, e[2 * jp + 1] = ee.y;
@@ -577,7 +583,7 @@ int32_t launch_exact_typed(const ExactParams &p0, cudaStream_t st) {
     const uint32_t share = (groups + grid - 1) / grid;
     const size_t cta = xg_cta_smem(p.k);
     static const int env_cap = [] { const char *e = getenv("CERA_CUDA_XG_CAP"); return e ? atoi(e) : 0; }();
-    // lone warps: up to 32 per CTA (28 672 gate / up rows give an SM 24 groups: one round of 25 warps instead of two of 16;
+    // lone warps: up to 32 per CTA (28 672 gate / up rows give an SM 24.2 groups: one round of 25 warps instead of two of 16;
     // CERA_CUDA_XG_CAP lowers the cap for A/B runs)
     const uint32_t warp_cap = env_cap >= 1 && env_cap <= XG_LONE_MAX_WARPS ? (uint32_t)env_cap : (uint32_t)XG_LONE_MAX_WARPS;
     auto max_warps = [&](uint32_t stages) -> uint32_t {
@@ -629,17 +635,17 @@ int32_t launch_exact_typed(const ExactParams &p0, cudaStream_t st) {
     p.stages = (int)s_log;
     p.team = (int)t_log;
     const size_t smem = cta + (size_t)P * xg_warp_smem(1u << s_log, L::BYTES) + (t_log ? (size_t)(P >> t_log) * xg_mail_bytes(t_log) : 0);
+    void (*const team)(ExactParams) = gemv_exact_kernel<T, true, XG_MAX_WARPS * 32>, (*const wide)(ExactParams) = gemv_exact_kernel<T, false, XG_WIDE_BOUND>,
+                 (*const full)(ExactParams) = gemv_exact_kernel<T, false, XG_LONE_MAX_WARPS * 32>;
     static thread_local int raised_dev = -1;  // per instantiation: opt in to more than 48 KB once per device
     int dev = 0;
     cudaGetDevice(&dev);
     if (raised_dev != dev) {
-        CERA_CUDA_TRY(cudaFuncSetAttribute(gemv_exact_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XG_SMEM_LIMIT));
-        CERA_CUDA_TRY(cudaFuncSetAttribute(gemv_exact_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XG_SMEM_LIMIT));
+        for (auto k : {team, wide, full}) CERA_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XG_SMEM_LIMIT));
         raised_dev = dev;
     }
     count_launch();
-    if (t_log) return check_cuda(launch_k(gemv_exact_kernel<T, true>, dim3(grid), dim3(P * 32), smem, st, p), "gemv (reference order, teams) launch");
-    return check_cuda(launch_k(gemv_exact_kernel<T, false>, dim3(grid), dim3(P * 32), smem, st, p), "gemv (reference order) launch");
+    return check_cuda(launch_k(t_log ? team : P <= (uint32_t)XG_WIDE_WARPS ? wide : full, dim3(grid), dim3(P * 32), smem, st, p), "gemv (reference order) launch");
 }
 
 }  // namespace
