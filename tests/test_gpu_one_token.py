@@ -84,3 +84,19 @@ def test_one_token_equals_the_first_of_two(t, experts, used, hidden, ff, softmax
         assert_bits(a[0].cpu().numpy(), b[0].cpu().numpy(), what)
     assert_bits(plain.cpu().numpy(), one[0].cpu().numpy(), "without routing")
     moe.close()
+
+
+@pytest.mark.parametrize("t", [O.Q4_K, O.Q5_K, O.Q6_K])
+@pytest.mark.parametrize("k", [256, 1280])
+@pytest.mark.parametrize("warps", [20, 21, 22, 32])  # warps of a CTA, around the line between the two register budgets
+def test_gemv_of_many_rows_equals_its_parts(t, k, warps):
+    torch = need_gpu()
+    import cera_b200 as cb
+    m, part = torch.cuda.get_device_properties(0).multi_processor_count * 8 * warps - 3, 1000
+    raw = cb.quantize_weights(t, cb.synth_normal(m * k, seed=warps, sigma=0.02)).cpu().numpy()
+    x = torch.from_numpy(O.synth_normal(k, 5, 1.0)).cuda()
+    got = cb.gemv(cb.QuantWeight(t, m, k, raw), x).cpu().numpy()
+    per_row = raw.size // m
+    for a in (0, m // 2, m - part):
+        rows = np.ascontiguousarray(raw.reshape(-1)[a * per_row:(a + part) * per_row])
+        assert_bits(got[a:a + part], cb.gemv(cb.QuantWeight(t, part, k, rows), x).cpu().numpy(), f"{O.NAMES[t]} rows from {a}")
