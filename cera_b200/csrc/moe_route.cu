@@ -6,10 +6,33 @@ namespace cera {
 
 namespace {
 
+// Sums of N values over a warp, each by the tree of warp_sum, N a power of two: every step halves the values a lane still carries, which takes
+// 31 shuffles for 32 values where one at a time takes 160.  Lane l ends with value l / (32 / N).
+template <int N>
+__device__ __forceinline__ float warp_sums(float (&v)[N]) {
+    const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16, n = N; o > 0; o >>= 1) {
+        if (n > 1) {
+            n >>= 1;
+#pragma unroll
+            for (int i = 0; i < N / 2; ++i)
+                if (i < n) {
+                    const float keep = lane & o ? v[i + n] : v[i], send = lane & o ? v[i] : v[i + n];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    return v[0];
+}
+
 // One CTA per T tokens.  A warp takes four experts at a time: lane-strided float4 dots in f32, every router and token
-// vector loaded once for the 4 T products it enters; shuffle tree; then warp t picks for token t.
-template <int T>
-__global__ void __launch_bounds__(256) moe_route_kernel(const float *x, const float *__restrict__ router,
+// vector loaded once for the 4 T products it enters, those of U steps under way together; then warp t scores and picks for token t.
+// What bounds it: L1 reads, twelve for 32 products at T = 8.  2048 tokens, 32 experts, width 2048: 65-73 us before, 37 now.
+template <int T, int U>
+__global__ void __launch_bounds__(256, 2) moe_route_kernel(const float *x, const float *__restrict__ router,
                                                         const float *__restrict__ bias, uint32_t hidden, uint32_t ld_x, uint32_t n, uint32_t n_expert,
                                                         uint32_t n_used, int softmax_gate, int renorm, uint32_t *ids, float *weights,
                                                         uint32_t *counts, uint32_t *ids_out, float *weights_out) {
@@ -19,41 +42,49 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const float *x, const fl
     pdl_trigger();
     pdl_wait();
     const uint32_t j0 = blockIdx.x * T;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const float *xj[T];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nv = hidden / 4;
+    const float4 *xj[T];
 #pragma unroll
-    for (int t = 0; t < T; ++t) xj[t] = x + (size_t)min(j0 + t, n - 1) * ld_x;
+    for (int t = 0; t < T; ++t) xj[t] = reinterpret_cast<const float4 *>(x + (size_t)min(j0 + t, n - 1) * ld_x);
     constexpr int EG = 4;
     for (uint32_t e0 = warp * EG; e0 < n_expert; e0 += (blockDim.x >> 5) * EG) {
         const float4 *r[EG];
 #pragma unroll
         for (int g = 0; g < EG; ++g) r[g] = reinterpret_cast<const float4 *>(router + (size_t)min(e0 + g, n_expert - 1) * hidden);
-        float acc[EG][T] = {};
-        for (uint32_t i = lane; i < hidden / 4; i += 32) {
-            float4 rv[EG];
+        float acc[EG * T] = {};  // (token, expert): t * EG + g
+        float4 rv[U][EG], xv[U][T];
+        auto load = [&](int u, uint32_t i) {
+            if (i >= nv) return;
 #pragma unroll
-            for (int g = 0; g < EG; ++g) rv[g] = __ldg(r[g] + i);
+            for (int g = 0; g < EG; ++g) rv[u][g] = __ldg(r[g] + i);
 #pragma unroll
-            for (int t = 0; t < T; ++t) {
-                const float4 xv = reinterpret_cast<const float4 *>(xj[t])[i];
+            for (int t = 0; t < T; ++t) xv[u][t] = xj[t][i];
+        };
 #pragma unroll
-                for (int g = 0; g < EG; ++g)
-                    acc[g][t] = fmaf(rv[g].w, xv.w, fmaf(rv[g].z, xv.z, fmaf(rv[g].y, xv.y, fmaf(rv[g].x, xv.x, acc[g][t]))));
+        for (int u = 0; u < U; ++u) load(u, lane + 32 * u);
+        for (uint32_t i = lane; i < nv; i += 32 * U) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (i + 32 * u < nv) {
+#pragma unroll
+                    for (int t = 0; t < T; ++t)
+#pragma unroll
+                        for (int g = 0; g < EG; ++g)
+                            acc[t * EG + g] = fmaf(rv[u][g].w, xv[u][t].w,
+                                                   fmaf(rv[u][g].z, xv[u][t].z, fmaf(rv[u][g].y, xv[u][t].y, fmaf(rv[u][g].x, xv[u][t].x, acc[t * EG + g]))));
+                }
+                load(u, i + 32 * (u + U));
             }
         }
-#pragma unroll
-        for (int g = 0; g < EG; ++g)
-#pragma unroll
-            for (int t = 0; t < T; ++t) {
-                const float v = warp_sum(acc[g][t]);
-                if (lane == 0 && e0 + g < n_expert) probs[t][e0 + g] = v;
-            }
+        const float v = warp_sums(acc);
+        constexpr uint32_t SHARE = 32 / (EG * T);  // lanes that hold the same sum
+        const uint32_t k = lane / SHARE, g = k % EG;
+        if (lane % SHARE == 0 && e0 + g < n_expert) probs[k / EG][e0 + g] = v;
     }
     __syncthreads();
-#pragma unroll 1
-    for (int t = 0; t < T; ++t) moe_scores(probs[t], n_expert, softmax_gate);
     if (warp >= T || j0 + warp >= n) return;
     const uint32_t j = j0 + warp;
+    moe_scores_warp(probs[warp], n_expert, softmax_gate);
     moe_pick(probs[warp], bias, n_expert, n_used, renorm, picked[warp], w[warp]);
     if (lane < n_used) {
         ids[(size_t)j * n_used + lane] = picked[warp][lane];
@@ -102,7 +133,7 @@ int32_t launch_moe_route(const float *x, size_t ld_x, size_t n, const float *rou
                                    n_used, softmax_gate, renorm, ids, weights, counts, ids_out, weights_out),
                           "moe route launch");
     };
-    return n < (size_t)sm_count() * 4 ? go(moe_route_kernel<1>, 1) : go(moe_route_kernel<8>, 8);
+    return n < (size_t)sm_count() * 4 ? go(moe_route_kernel<1, 4>, 1) : go(moe_route_kernel<8, 1>, 8);
 }
 
 int32_t launch_moe_plan(uint32_t *counts, uint32_t n_expert, uint32_t nc, uint32_t small_nc, uint32_t cap, uint32_t *cursor, MoeTile *tiles,
