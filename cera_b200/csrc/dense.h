@@ -88,11 +88,12 @@ struct RouterRule {
     uint32_t n_expert = 0, n_used = 0;
     int softmax = 0, renorm = 0, weight_input = 0;
 };
-// Routed feed-forward of one token: picks from the router logits, gate / up rows of the chosen experts through the gated
-// unit into act [n_used][ff_p]; the second call y = sum over picks of down rows.  w_gate_up stacks per expert ff_p gate
+// Routed feed-forward of one token: router logits (an f32 matrix) and picks; gate / up rows of the picked experts through the gated
+// unit into act [n_used][ff_p]; y = sum over picks of down rows.  w_gate_up stacks per expert ff_p gate
 // rows then ff_p up rows, w_down `rows_per_expert` rows per expert.
-int32_t launch_expert_gate_up_step(const DenseView &w_gate_up, const void *x, const float *router_logits, const RouterRule &r, uint32_t ff_p,
-                                   const ExpertAct &a, uint32_t *ids, float *weights, void *act, cudaStream_t st);
+int32_t launch_router_pick_step(const DenseView &router, const float *x, const RouterRule &r, uint32_t *ids, float *weights, cudaStream_t st);
+int32_t launch_expert_gate_up_step(const DenseView &w_gate_up, const void *x, const uint32_t *ids, const float *weights, const RouterRule &r, uint32_t ff_p,
+                                   const ExpertAct &a, void *act, cudaStream_t st);
 int32_t launch_expert_down_step(const DenseView &w_down, uint32_t rows_per_expert, const void *act, const RouterRule &r, const uint32_t *ids,
                                 const float *weights, float *y, cudaStream_t st);
 

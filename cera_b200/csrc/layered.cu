@@ -12,8 +12,8 @@
 // latent attention: [input products] [norm, rotation, cache append] [W_uk on the query] [split attention] [merge, W_uv, gate]
 // [output product]; grouped attention: [input products] [bias, rotation, norm, cache append] [split attention] [merge] [output
 // product]; real-gated recurrence: [input products] [convolution, gates, state, output gate] [output product]; state-space
-// recurrence: [input products] [convolution, state] [gate, norm] [output product]; experts: [boundary] [router logits] [pick,
-// gate / up, gated unit] [down, sum over picks]; one gated unit: [boundary] [gate / up, gated unit] [down].
+// recurrence: [input products] [convolution, state] [gate, norm] [output product]; experts: [boundary] [router logits,
+// pick] [gate / up, gated unit] [down, sum over picks]; one gated unit: [boundary] [gate / up, gated unit] [down].
 // A prompt portion takes the same steps with many-column products, scans for the recurrences, and experts grouped by a
 // device-built work list.
 #include <cmath>
@@ -166,7 +166,7 @@ struct LayeredModel : cera_cuda_model {
     std::vector<Rope> ropes;
     // scratch; chunk buffers have LAYERED_CHUNK rows, the decode step uses row 0
     size_t rows_alloc = 0;
-    float *x = nullptr, *emb = nullptr, *y = nullptr, *h32 = nullptr, *aux = nullptr, *pre = nullptr, *q32 = nullptr, *gate = nullptr, *logits_r = nullptr;
+    float *x = nullptr, *emb = nullptr, *y = nullptr, *h32 = nullptr, *aux = nullptr, *pre = nullptr, *q32 = nullptr, *gate = nullptr;
     void *h = nullptr, *mix = nullptr, *qt = nullptr, *conv = nullptr;
     LatentScratch lat;
     void *k_exp = nullptr, *v_exp = nullptr;
@@ -651,7 +651,6 @@ int32_t LayeredModel::build() {
     }
     if (eo_rows) {
         eo_rows = C * used;
-        CERA_TRY(dev_alloc((void **)&logits_r, experts * 4));
         CERA_TRY(dev_alloc((void **)&ids, eo_rows * 4));
         CERA_TRY(dev_alloc((void **)&pick_w, eo_rows * 4));
         CERA_TRY(dev_alloc((void **)&col_scale, eo_rows * 4));
@@ -724,8 +723,8 @@ int32_t LayeredModel::enqueue_step(int kind, uint32_t splits) {
             rn.h32 = h32;
             CERA_TRY(launch_residual_norm(rn, hidden_size, ld, 1, cfg.norm_eps, st));
             rn.h32 = nullptr;
-            CERA_TRY(launch_dense_gemv(L.ffn.router, h32, logits_r, st));
-            CERA_TRY(launch_expert_gate_up_step(L.ffn.gate_up, h, logits_r, rule, L.ffn.ff_p, ea, ids, pick_w, act, st));
+            CERA_TRY(launch_router_pick_step(L.ffn.router, h32, rule, ids, pick_w, st));
+            CERA_TRY(launch_expert_gate_up_step(L.ffn.gate_up, h, ids, pick_w, rule, L.ffn.ff_p, ea, act, st));
             CERA_TRY(launch_expert_down_step(L.ffn.down, ld, act, rule, ids, pick_w, y, st));
             rn.post = L.ff_post;
         } else if (L.d.ff == CERA_FF_GATED) {

@@ -31,12 +31,6 @@ __device__ __forceinline__ void moe_scores_warp(float *probs, uint32_t n_expert,
     __syncwarp();
 }
 
-// The same for a CTA, which is synchronised on exit.
-__device__ __forceinline__ void moe_scores(float *probs, uint32_t n_expert, int softmax_gate) {
-    if (threadIdx.x < 32) moe_scores_warp(probs, n_expert, softmax_gate);
-    __syncthreads();
-}
-
 // One warp: the n_used experts with the largest probs + bias, ties to the lower index, in order; lane 0 writes picked /
 // weight (shared memory).  Weights are the unbiased scores, divided by max(their sum, 2^-14) when `renorm`.
 __device__ __forceinline__ void moe_pick(const float *probs, const float *bias, uint32_t n_expert, uint32_t n_used, int renorm, uint32_t *picked,
