@@ -119,39 +119,38 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(const __gri
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t id_s = tc_idesc_bf16(AT_Q, AT_K), id_o = tc_idesc_bf16(AT_Q, s.vdim_p);
-            auto scores = [&](uint32_t j) -> bool {
-                const uint32_t b = j & 1, par = j >> 1 & 1;
-                if (!tma::mbar_wait_blocking(k_full + b, par, abort_flag, status, 2u)) return false;
-                if (!tma::mbar_wait_blocking(s_free + b, par ^ 1, abort_flag, status, 2u)) return false;
-                tc_fence_after();
-                const uint32_t qa = tma::smem_u32(qs), ka = tma::smem_u32(ks + b * k_stage);
-                uint32_t acc = 0;
-                for (uint32_t part = 0; part < 2; ++part) {
-                    const uint32_t steps = (part ? s.rot_p : s.dim_p) / 16, blk0 = part ? p.nb_dim : 0;
-                    for (uint32_t k = 0; k < steps; ++k, acc = 1) {
-                        const uint32_t blk = blk0 + (k >> 2), kk = k & 3;
-                        tc_mma_f16(tmem + b * AT_K, smem_desc_sw128(qa + blk * AT_QBLK) + 2 * kk, smem_desc_sw128(ka + blk * AT_KBLK) + 2 * kk, id_s, acc);
-                    }
+        // the whole warp, one lane issues
+        const uint32_t id_s = tc_idesc_bf16(AT_Q, AT_K), id_o = tc_idesc_bf16(AT_Q, s.vdim_p), me = elect_one();
+        auto arrived = [&](uint64_t *bar, uint32_t parity) { return warp_all(tma::mbar_wait_blocking(bar, parity, abort_flag, status, 2u)); };
+        auto scores = [&](uint32_t j) -> bool {
+            const uint32_t b = j & 1, par = j >> 1 & 1;
+            if (!arrived(k_full + b, par) || !arrived(s_free + b, par ^ 1)) return false;
+            tc_fence_after();
+            const uint64_t qd = smem_desc_sw128(tma::smem_u32(qs)), kd = smem_desc_sw128(tma::smem_u32(ks + b * k_stage));
+            uint32_t acc = 0;
+            for (uint32_t part = 0; part < 2; ++part) {
+                const uint32_t steps = (part ? s.rot_p : s.dim_p) / 16, blk0 = part ? p.nb_dim : 0;
+                for (uint32_t k = 0; k < steps; ++k, acc = 1) {
+                    const uint32_t blk = blk0 + (k >> 2), kk = k & 3;
+                    tc_mma_f16(tmem + b * AT_K, qd + blk * (AT_QBLK / 16) + 2 * kk, kd + blk * (AT_KBLK / 16) + 2 * kk, id_s, acc, me);  // address fields count 16 bytes
                 }
-                tc_commit(k_empty + b);
-                tc_commit(s_full + b);
-                return true;
-            };
-            bool ok = tma::mbar_wait_blocking(q_full, 0, abort_flag, status, 2u) && scores(0);
-            for (uint32_t j = 0; j < n_kv && ok; ++j) {
-                if (j + 1 < n_kv && !(ok = scores(j + 1))) break;
-                const uint32_t b = j & 1, par = j >> 1 & 1;
-                ok = tma::mbar_wait_blocking(p_full + b, par, abort_flag, status, 2u) && tma::mbar_wait_blocking(v_full + b, par, abort_flag, status, 2u);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t pa = tma::smem_u32(ps + b * AT_P_BYTES), va = tma::smem_u32(vs + b * v_stage);
-#pragma unroll
-                for (int k = 0; k < AT_K / 16; ++k) tc_mma_f16(tm_o, smem_desc_sw128(pa) + 2 * k, smem_desc_sw128(va) + 2 * k, id_o, j | k);
-                tc_commit(v_empty + b);
-                tc_commit(pv_done + b);
             }
+            tc_commit(k_empty + b, me);
+            tc_commit(s_full + b, me);
+            return true;
+        };
+        bool ok = arrived(q_full, 0) && scores(0);
+        for (uint32_t j = 0; j < n_kv && ok; ++j) {
+            if (j + 1 < n_kv && !(ok = scores(j + 1))) break;
+            const uint32_t b = j & 1, par = j >> 1 & 1;
+            ok = arrived(p_full + b, par) && arrived(v_full + b, par);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t pd = smem_desc_sw128(tma::smem_u32(ps + b * AT_P_BYTES)), vd = smem_desc_sw128(tma::smem_u32(vs + b * v_stage));
+#pragma unroll
+            for (int k = 0; k < AT_K / 16; ++k) tc_mma_f16(tm_o, pd + 2 * k, vd + 2 * k, id_o, j | k, me);
+            tc_commit(v_empty + b, me);
+            tc_commit(pv_done + b, me);
         }
     } else {
         const uint32_t quad = warp & 3, r = quad * 32 + lane, lanes = quad * 32 << 16, pos = p.start_pos + q0 + r;

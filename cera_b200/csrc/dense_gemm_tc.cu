@@ -96,56 +96,60 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dense_gemm_tc_kernel(const __gr
     const uint32_t tmem = *tmem_at;
     pdl_wait();
     const uint32_t n_tiles = p.g.tiles ? *p.g.n_tiles * p.row_tiles : p.row_tiles * p.col_tiles, n_k = p.g.w.ld / DT_KS;
-    if (warp == 0) {
-        if (lane == 0) {
-            uint32_t it = 0;
-            bool ok = true;
-            for (uint32_t t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-                const DtTile o = dt_tile<BN, NA>(p, t);
-                const uint32_t x0 = p.g.block_rows ? o.a_row / p.g.block_rows * p.g.w.ld : 0;
-                for (uint32_t k = 0; k < n_k; ++k, ++it) {
-                    const uint32_t s = it % S::STAGES;
-                    if (!(ok = tma::mbar_wait_blocking(empty + s, (it / S::STAGES & 1) ^ 1, abort_flag, &g_dense_tc_status, 1u))) break;
-                    uint8_t *st = stages + s * S::STAGE;
-                    tma::mbar_expect_tx(full + s, S::STAGE);
-                    tma::tensor_g2s_2d(st, &map_w, k * DT_KS, o.a_row, full + s);
-                    if (NA == 2) tma::tensor_g2s_2d(st + DT_A_BYTES, &map_w, k * DT_KS, o.a_row + o.rows, full + s);
-                    tma::tensor_g2s_2d(st + NA * DT_A_BYTES, &map_x, x0 + k * DT_KS, o.first, full + s);
-                }
+    // a ragged tile's products stop at its last column (in whole 32s, as the epilogue reads them): an expert's last item.
+    // 2048 tokens through four layers of routed experts at width 4096: 4.50 -> 4.42 ms, 1.4 to 2.4 % in three pairs of runs that
+    // repeat within 1 %
+    auto columns = [](const DtTile &o) { return min((uint32_t)BN, (o.end - o.first + 31) & ~31u); };
+    if (warp == 0) {  // the whole warp, one lane requests
+        const uint32_t me = elect_one();
+        uint32_t it = 0;
+        bool ok = true;
+        for (uint32_t t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+            const DtTile o = dt_tile<BN, NA>(p, t);
+            const uint32_t x0 = p.g.block_rows ? o.a_row / p.g.block_rows * p.g.w.ld : 0;
+            for (uint32_t k = 0; k < n_k; ++k, ++it) {
+                const uint32_t s = it % S::STAGES;
+                if (!(ok = warp_all(tma::mbar_wait_blocking(empty + s, (it / S::STAGES & 1) ^ 1, abort_flag, &g_dense_tc_status, 1u)))) break;
+                uint8_t *st = stages + s * S::STAGE;
+                tma::mbar_expect_tx_if(full + s, S::STAGE, me);
+                tma::tensor_g2s_2d_if(st, &map_w, k * DT_KS, o.a_row, full + s, me);
+                if (NA == 2) tma::tensor_g2s_2d_if(st + DT_A_BYTES, &map_w, k * DT_KS, o.a_row + o.rows, full + s, me);
+                tma::tensor_g2s_2d_if(st + NA * DT_A_BYTES, &map_x, x0 + k * DT_KS, o.first, full + s, me);
             }
-            // given up: this CTA's shared memory must outlive the copies in flight
-            if (*abort_flag)
-                for (uint32_t i = it > S::STAGES ? it - S::STAGES : 0; i < it; ++i)
-                    for (uint32_t n = 0; n < tma::SPIN_LIMIT && !tma::mbar_test(full + i % S::STAGES, i / S::STAGES & 1); ++n) __nanosleep(40);
         }
+        // given up: this CTA's shared memory must outlive the copies in flight
+        if (*abort_flag)
+            for (uint32_t i = it > S::STAGES ? it - S::STAGES : 0; i < it; ++i)
+                for (uint32_t n = 0; n < tma::SPIN_LIMIT && !tma::mbar_test(full + i % S::STAGES, i / S::STAGES & 1); ++n) __nanosleep(40);
     } else if (warp == 1) {
-        if (lane == 0) {
-            uint32_t it = 0, j = 0;
-            bool ok = true;
-            for (uint32_t t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++j) {
-                const uint32_t b = j & 1, acc = tmem + b * S::ACC;
-                const DtTile o = dt_tile<BN, NA>(p, t);
-                // a ragged tile's products stop at its last column (in whole 32s, as the epilogue reads them): an expert's last item.
-                // 2048 tokens through four layers of routed experts at width 4096: 4.50 -> 4.42 ms, 1.4 to 2.4 % in three pairs of runs that
-                // repeat within 1 %
-                const uint32_t idesc = tc_idesc_bf16(DT_BM, min((uint32_t)BN, (o.end - o.first + 31) & ~31u));
-                if (!(ok = tma::mbar_wait_blocking(acc_empty + b, (j >> 1 & 1) ^ 1, abort_flag, &g_dense_tc_status, 2u))) break;
+        // the whole warp, one lane issues
+        const uint32_t me = elect_one();
+        uint32_t it = 0, j = 0;
+        bool ok = true;
+        auto arrived = [&](uint64_t *bar, uint32_t parity) {
+            return warp_all(tma::mbar_wait_blocking(bar, parity, abort_flag, &g_dense_tc_status, 2u));
+        };
+        for (uint32_t t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++j) {
+            const uint32_t b = j & 1, acc = tmem + b * S::ACC;
+            const DtTile o = dt_tile<BN, NA>(p, t);
+            const uint32_t idesc = tc_idesc_bf16(DT_BM, columns(o));
+            if (!(ok = arrived(acc_empty + b, (j >> 1 & 1) ^ 1))) break;
+            tc_fence_after();
+            for (uint32_t k = 0; k < n_k; ++k, ++it) {
+                const uint32_t s = it % S::STAGES;
+                if (!(ok = arrived(full + s, it / S::STAGES & 1))) break;
                 tc_fence_after();
-                for (uint32_t k = 0; k < n_k; ++k, ++it) {
-                    const uint32_t s = it % S::STAGES;
-                    if (!(ok = tma::mbar_wait_blocking(full + s, it / S::STAGES & 1, abort_flag, &g_dense_tc_status, 2u))) break;
-                    tc_fence_after();
-                    const uint32_t st = tma::smem_u32(stages + s * S::STAGE);
-                    const uint64_t da = smem_desc_sw128(st), db = smem_desc_sw128(st + NA * DT_A_BYTES);
+                const uint32_t st = tma::smem_u32(stages + s * S::STAGE);
+                const uint64_t da = smem_desc_sw128(st), da2 = smem_desc_sw128(st + DT_A_BYTES), db = smem_desc_sw128(st + NA * DT_A_BYTES);
 #pragma unroll
-                    for (int kk = 0; kk < DT_KS / 16; ++kk) {
-                        tc_mma_f16(acc, da + 2 * kk, db + 2 * kk, idesc, k | kk);
-                        if (NA == 2) tc_mma_f16(acc + BN, smem_desc_sw128(st + DT_A_BYTES) + 2 * kk, db + 2 * kk, idesc, k | kk);
-                    }
-                    tc_commit(empty + s);
-                }
-                if (ok) tc_commit(acc_full + b);
+                for (int kk = 0; kk < DT_KS / 16; ++kk)
+#pragma unroll
+                    for (int a = 0; a < NA; ++a)
+                        tc_mma_f16(acc + a * BN, (a ? da2 : da) + 2 * kk, db + 2 * kk, idesc, k | kk, me);
+                tc_commit(empty + s, me);
             }
+            if (!ok) break;
+            tc_commit(acc_full + b, me);
         }
     } else {
         const uint32_t quad = warp & 3;  // the TMEM lanes this warp may read: [32 quad, + 32)

@@ -431,62 +431,55 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
     pdl_wait();
 
     if (warp == 0) {
-        // ---------------------------------------------------------------- MMA issue (one thread)
-        if (lane == 0) {
-            const uint32_t idesc = tc_idesc(TC_BM, TC_BN);
-            bool ok = true;
-            uint32_t it = 0;
-            for (uint32_t sb = 0; sb <= n_sb && ok; ++sb) {  // super-block n_sb is the min GEMM
-                const uint32_t buf = sb & 1, d0 = tmem + buf * 2 * TC_BN;
-                if (!tma::mbar_wait_blocking(empty_d + buf, ((sb >> 1) & 1) ^ 1, abort_flag, &g_tc_status, 2u)) break;
+        // ---------------------------------------------------------------- MMA issue (the whole warp, one lane issues)
+        const uint32_t idesc = tc_idesc(TC_BM, TC_BN), me = elect_one();
+        bool ok = true;
+        uint32_t it = 0;
+        for (uint32_t sb = 0; sb <= n_sb && ok; ++sb) {  // super-block n_sb is the min GEMM
+            const uint32_t buf = sb & 1, d0 = tmem + buf * 2 * TC_BN;
+            if (!warp_all(tma::mbar_wait_blocking(empty_d + buf, ((sb >> 1) & 1) ^ 1, abort_flag, &g_tc_status, 2u))) break;
+            tc_fence_after();
+            const uint32_t n_st = sb < n_sb ? 4u : n_mit;
+            for (uint32_t st = 0; st < n_st; ++st, ++it) {
+                const uint32_t s = it % TCW_STAGES;
+                ok = warp_all(tma::mbar_wait_blocking(full_ab + s, (it / TCW_STAGES) & 1, abort_flag, &g_tc_status, 1u));
+                if (!ok) break;
                 tc_fence_after();
-                const uint32_t n_st = sb < n_sb ? 4u : n_mit;
-                for (uint32_t st = 0; st < n_st; ++st, ++it) {
-                    const uint32_t s = it % TCW_STAGES;
-                    if (!tma::mbar_wait_blocking(full_ab + s, (it / TCW_STAGES) & 1, abort_flag, &g_tc_status, 1u)) {
-                        ok = false;
-                        break;
+                const uint32_t base = tma::smem_u32(tc_smem + s * TCW_STAGE_BYTES);
+                if (sb < n_sb) {
+                    const uint64_t ah = smem_desc(base, TC_KC_STRIDE, 128), al = smem_desc(base + TC_OP_BYTES, TC_KC_STRIDE, 128),
+                                   bd0 = smem_desc(base + 2 * TC_OP_BYTES, TC_KC_STRIDE, 128), bd1 = smem_desc(base + 3 * TC_OP_BYTES, TC_KC_STRIDE, 128);
+#pragma unroll
+                    for (uint32_t ks = 0; ks < TC_KS / 16; ++ks) {
+                        const uint32_t o = 2 * ks * TC_KC_STRIDE / 16, acc = (st | ks) != 0;  // address fields count 16 bytes
+                        tc_mma_f16(d0, ah + o, bd0 + o, idesc, acc, me);
+                        tc_mma_f16(d0 + TC_BN, ah + o, bd1 + o, idesc, acc, me);
+                        tc_mma_f16(d0, al + o, bd0 + o, idesc, 1, me);
+                        tc_mma_f16(d0 + TC_BN, al + o, bd1 + o, idesc, 1, me);
                     }
-                    tc_fence_after();
-                    const uint32_t base = tma::smem_u32(tc_smem + s * TCW_STAGE_BYTES);
-                    if (sb < n_sb) {
-                        const uint32_t a_hi = base, a_lo = base + TC_OP_BYTES, b0 = a_lo + TC_OP_BYTES, b1 = b0 + TC_OP_BYTES;
+                } else {
+                    // min GEMM: [x high | x low | w high, w low of rows [0,128) | the same of rows [128,256)], 32 blocks = two steps
+                    const uint64_t xh = smem_desc(base, TC_KC_STRIDE, 128), xl = smem_desc(base + TCW_MINT_BYTES, TC_KC_STRIDE, 128);
 #pragma unroll
-                        for (uint32_t ks = 0; ks < TC_KS / 16; ++ks) {
-                            const uint32_t o = 2 * ks * TC_KC_STRIDE;
-                            const uint64_t ah = smem_desc(a_hi + o, TC_KC_STRIDE, 128), al = smem_desc(a_lo + o, TC_KC_STRIDE, 128);
-                            const uint64_t bd0 = smem_desc(b0 + o, TC_KC_STRIDE, 128), bd1 = smem_desc(b1 + o, TC_KC_STRIDE, 128);
-                            const uint32_t acc = (st | ks) != 0;
-                            tc_mma_f16(d0, ah, bd0, idesc, acc);
-                            tc_mma_f16(d0 + TC_BN, ah, bd1, idesc, acc);
-                            tc_mma_f16(d0, al, bd0, idesc, 1);
-                            tc_mma_f16(d0 + TC_BN, al, bd1, idesc, 1);
-                        }
-                    } else {
-                        // min GEMM: [x high | x low | w high, w low of rows [0,128) | the same of rows [128,256)], 32 blocks = two steps
-                        const uint32_t x_hi = base, x_lo = base + TCW_MINT_BYTES;
+                    for (uint32_t ks = 0; ks < TCW_MIN_J / 16; ++ks) {
+                        const uint32_t o = 2 * ks * TC_KC_STRIDE / 16;
 #pragma unroll
-                        for (uint32_t ks = 0; ks < TCW_MIN_J / 16; ++ks) {
-                            const uint32_t o = 2 * ks * TC_KC_STRIDE;
-                            const uint64_t xh = smem_desc(x_hi + o, TC_KC_STRIDE, 128), xl = smem_desc(x_lo + o, TC_KC_STRIDE, 128);
-#pragma unroll
-                            for (uint32_t h = 0; h < 2; ++h) {
-                                const uint32_t w_hi = base + (2 + 2 * h) * TCW_MINT_BYTES, w_lo = w_hi + TCW_MINT_BYTES;
-                                const uint64_t wh = smem_desc(w_hi + o, TC_KC_STRIDE, 128), wl = smem_desc(w_lo + o, TC_KC_STRIDE, 128);
-                                tc_mma_f16(d0 + h * TC_BN, xh, wh, idesc, (st | ks) != 0);
-                                tc_mma_f16(d0 + h * TC_BN, xl, wh, idesc, 1);
-                                tc_mma_f16(d0 + h * TC_BN, xh, wl, idesc, 1);
-                            }
+                        for (uint32_t h = 0; h < 2; ++h) {
+                            const uint64_t wh = xh + (2 + 2 * h) * TCW_MINT_BYTES / 16, wl = wh + TCW_MINT_BYTES / 16;
+                            tc_mma_f16(d0 + h * TC_BN, xh + o, wh + o, idesc, (st | ks) != 0, me);
+                            tc_mma_f16(d0 + h * TC_BN, xl + o, wh + o, idesc, 1, me);
+                            tc_mma_f16(d0 + h * TC_BN, xh + o, wl + o, idesc, 1, me);
                         }
                     }
-                    tc_commit(empty_ab + s);
                 }
-                if (ok) tc_commit(full_d + buf);
+                tc_commit(empty_ab + s, me);
             }
+            if (ok) tc_commit(full_d + buf, me);
         }
     } else if (warp == 1) {
-        // ---------------------------------------------------------------- operands: one thread asks for them (bulk asynchronous copies)
-        if (lane == 0) {
+        // ---------------------------------------------------------------- operands: the whole warp, one lane asks for them (bulk asynchronous copies)
+        {
+            const uint32_t me = elect_one();
             const uint32_t t0 = min(2 * sub.by, L.tiles - 1), t1 = min(2 * sub.by + 1, L.tiles - 1);  // (an odd last tile is read twice)
             const uint8_t *img = p.img + (size_t)blockIdx.x * n_it * (2 * TC_OP_BYTES);
             const uint8_t *w0 = sub.tc + (size_t)t0 * n_it * TC_OP_BYTES, *w1 = sub.tc + (size_t)t1 * n_it * TC_OP_BYTES;
@@ -497,24 +490,24 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
             for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
                 for (uint32_t st = 0; st < 4; ++st, ++it) {
                     const uint32_t s = it % TCW_STAGES;
-                    if (!tma::mbar_wait_blocking(empty_ab + s, ((it / TCW_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u)) {
+                    if (!warp_all(tma::mbar_wait_blocking(empty_ab + s, ((it / TCW_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u))) {
                         ok = false;
                         break;
                     }
                     // the d slot of this super-block was last read by the epilogue of super-block sb - 2
-                    if (st == 0 && sb >= 2 && !tma::mbar_wait_blocking(empty_d + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u)) {
+                    if (st == 0 && sb >= 2 && !warp_all(tma::mbar_wait_blocking(empty_d + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u))) {
                         ok = false;
                         break;
                     }
                     uint8_t *dst = tc_smem + s * TCW_STAGE_BYTES;
-                    tma::mbar_expect_tx(full_ab + s, TCW_STAGE_BYTES + (st == 0 ? 2 * TC_BN * 4 : 0));
-                    tma::bulk_g2s(dst, img + (size_t)it * (2 * TC_OP_BYTES), 2 * TC_OP_BYTES, full_ab + s);
-                    tma::bulk_g2s(dst + 2 * TC_OP_BYTES, w0 + (size_t)it * TC_OP_BYTES, TC_OP_BYTES, full_ab + s);
-                    tma::bulk_g2s(dst + 3 * TC_OP_BYTES, w1 + (size_t)it * TC_OP_BYTES, TC_OP_BYTES, full_ab + s);
+                    tma::mbar_expect_tx_if(full_ab + s, TCW_STAGE_BYTES + (st == 0 ? 2 * TC_BN * 4 : 0), me);
+                    tma::bulk_g2s_if(dst, img + (size_t)it * (2 * TC_OP_BYTES), 2 * TC_OP_BYTES, full_ab + s, me);
+                    tma::bulk_g2s_if(dst + 2 * TC_OP_BYTES, w0 + (size_t)it * TC_OP_BYTES, TC_OP_BYTES, full_ab + s, me);
+                    tma::bulk_g2s_if(dst + 3 * TC_OP_BYTES, w1 + (size_t)it * TC_OP_BYTES, TC_OP_BYTES, full_ab + s, me);
                     if (st == 0) {
                         uint8_t *dv = tc_smem + TCW_DVAL_OFF + (sb & 1) * (2 * TC_BN * 4);
-                        tma::bulk_g2s(dv, sd0 + (size_t)sb * TC_SIDE_BYTES, TC_BN * 4, full_ab + s);
-                        tma::bulk_g2s(dv + TC_BN * 4, sd1 + (size_t)sb * TC_SIDE_BYTES, TC_BN * 4, full_ab + s);
+                        tma::bulk_g2s_if(dv, sd0 + (size_t)sb * TC_SIDE_BYTES, TC_BN * 4, full_ab + s, me);
+                        tma::bulk_g2s_if(dv + TC_BN * 4, sd1 + (size_t)sb * TC_SIDE_BYTES, TC_BN * 4, full_ab + s, me);
                     }
                 }
             }
@@ -522,15 +515,15 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
             const uint8_t *m0 = sub.tc + L.wmin + (size_t)t0 * n_mit * (2 * TCW_MINT_BYTES), *m1 = sub.tc + L.wmin + (size_t)t1 * n_mit * (2 * TCW_MINT_BYTES);
             for (uint32_t mi = 0; mi < n_mit && ok; ++mi, ++it) {
                 const uint32_t s = it % TCW_STAGES;
-                if (!tma::mbar_wait_blocking(empty_ab + s, ((it / TCW_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u)) break;
+                if (!warp_all(tma::mbar_wait_blocking(empty_ab + s, ((it / TCW_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u))) break;
                 uint8_t *dst = tc_smem + s * TCW_STAGE_BYTES;
-                tma::mbar_expect_tx(full_ab + s, 6 * TCW_MINT_BYTES + (mi == 0 ? 2 * TC_BN * 4 : 0));
-                tma::bulk_g2s(dst, xm + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s);
-                tma::bulk_g2s(dst + 2 * TCW_MINT_BYTES, m0 + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s);
-                tma::bulk_g2s(dst + 4 * TCW_MINT_BYTES, m1 + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s);
+                tma::mbar_expect_tx_if(full_ab + s, 6 * TCW_MINT_BYTES + (mi == 0 ? 2 * TC_BN * 4 : 0), me);
+                tma::bulk_g2s_if(dst, xm + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s, me);
+                tma::bulk_g2s_if(dst + 2 * TCW_MINT_BYTES, m0 + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s, me);
+                tma::bulk_g2s_if(dst + 4 * TCW_MINT_BYTES, m1 + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s, me);
                 if (mi == 0) {  // 2^-s of the CTA's rows (read by the epilogue after the min GEMM)
-                    tma::bulk_g2s(tc_smem + TCW_RS_OFF, sub.tc + L.rscale + (size_t)t0 * TC_BN * 4, TC_BN * 4, full_ab + s);
-                    tma::bulk_g2s(tc_smem + TCW_RS_OFF + TC_BN * 4, sub.tc + L.rscale + (size_t)t1 * TC_BN * 4, TC_BN * 4, full_ab + s);
+                    tma::bulk_g2s_if(tc_smem + TCW_RS_OFF, sub.tc + L.rscale + (size_t)t0 * TC_BN * 4, TC_BN * 4, full_ab + s, me);
+                    tma::bulk_g2s_if(tc_smem + TCW_RS_OFF + TC_BN * 4, sub.tc + L.rscale + (size_t)t1 * TC_BN * 4, TC_BN * 4, full_ab + s, me);
                 }
             }
         }
@@ -650,45 +643,38 @@ __global__ void __launch_bounds__(IMG ? TC_THREADS_IMG : TC_THREADS, 1) gemm_tc_
     pdl_wait();
 
     if (warp == 0) {
-        // ---------------------------------------------------------------- MMA issue (one thread)
-        if (lane == 0) {
-            const uint32_t idesc = tc_idesc(TC_BM, TC_BN);
-            bool ok = true;
-            for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
-                const uint32_t buf = sb & 1;
-                // the epilogue has left this D buffer (super-block sb - 2)
-                if (!tma::mbar_wait_blocking(empty_d + buf, ((sb >> 1) & 1) ^ 1, abort_flag, &g_tc_status, 2u)) break;
+        // ---------------------------------------------------------------- MMA issue (the whole warp, one lane issues)
+        const uint32_t idesc = tc_idesc(TC_BM, TC_BN), me = elect_one();
+        bool ok = true;
+        for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
+            const uint32_t buf = sb & 1, d0 = tmem + buf * TC_BN;
+            // the epilogue has left this D buffer (super-block sb - 2)
+            if (!warp_all(tma::mbar_wait_blocking(empty_d + buf, ((sb >> 1) & 1) ^ 1, abort_flag, &g_tc_status, 2u))) break;
+            tc_fence_after();
+            for (uint32_t st = 0; st < (uint32_t)TC_STAGES; ++st) {
+                const uint32_t it = sb * TC_STAGES + st;
+                const bool last = st + 1 == (uint32_t)TC_STAGES;
+                ok = warp_all(tma::mbar_wait_blocking(full_ab + st, (it / TC_STAGES) & 1, abort_flag, &g_tc_status, 1u));
+                // with the last stage goes the super-block's min term.  Without the weight image Dm has one buffer (the fourth TMEM region
+                // holds the running output): the epilogue must have read super-block sb - 1's
+                if (ok && last && !IMG && sb)
+                    ok = warp_all(tma::mbar_wait_blocking(empty_d + (buf ^ 1), ((sb - 1) >> 1) & 1, abort_flag, &g_tc_status, 2u));
+                if (!ok) break;
                 tc_fence_after();
-                for (uint32_t st = 0; st < (uint32_t)TC_STAGES; ++st) {
-                    const uint32_t it = sb * TC_STAGES + st;
-                    if (!tma::mbar_wait_blocking(full_ab + st, (it / TC_STAGES) & 1, abort_flag, &g_tc_status, 1u)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t a_hi = tma::smem_u32(tc_smem + st * TC_STAGE_BYTES), a_lo = a_hi + TC_OP_BYTES, b_base = a_lo + TC_OP_BYTES;
+                const uint32_t base = tma::smem_u32(tc_smem + st * TC_STAGE_BYTES), slot = tma::smem_u32(slots + buf * TC_SLOT_BYTES);
+                const uint64_t ah = smem_desc(base, TC_KC_STRIDE, 128), al = smem_desc(base + TC_OP_BYTES, TC_KC_STRIDE, 128),
+                               bd = smem_desc(base + 2 * TC_OP_BYTES, TC_KC_STRIDE, 128);
+                const uint64_t xm = smem_desc(slot, TC_KC_STRIDE, 128), wm = smem_desc(slot + TC_MINOP_BYTES, TC_KC_STRIDE, 128);
 #pragma unroll
-                    for (uint32_t ks = 0; ks < TC_KS / 16; ++ks) {
-                        const uint64_t bd = smem_desc(b_base + 2 * ks * TC_KC_STRIDE, TC_KC_STRIDE, 128);
-                        tc_mma_f16(tmem + buf * TC_BN, smem_desc(a_hi + 2 * ks * TC_KC_STRIDE, TC_KC_STRIDE, 128), bd, idesc, (st | ks) != 0);
-                        tc_mma_f16(tmem + buf * TC_BN, smem_desc(a_lo + 2 * ks * TC_KC_STRIDE, TC_KC_STRIDE, 128), bd, idesc, 1);
-                    }
-                    if (st + 1 == (uint32_t)TC_STAGES) {
-                        // the super-block's min term.  Without the weight image Dm has one buffer (the fourth TMEM region holds
-                        // the running output): the epilogue must have read super-block sb - 1's
-                        if (!IMG && sb && !tma::mbar_wait_blocking(empty_d + (buf ^ 1), ((sb - 1) >> 1) & 1, abort_flag, &g_tc_status, 2u)) {
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after();
-                        const uint32_t slot = tma::smem_u32(slots + buf * TC_SLOT_BYTES);
-                        tc_mma_f16(tmem + (IMG ? 2 + buf : 2) * TC_BN, smem_desc(slot, TC_KC_STRIDE, 128), smem_desc(slot + TC_MINOP_BYTES, TC_KC_STRIDE, 128),
-                                   idesc, 0);
-                    }
-                    tc_commit(empty_ab + st);
+                for (uint32_t ks = 0; ks < TC_KS / 16; ++ks) {
+                    const uint32_t o = 2 * ks * TC_KC_STRIDE / 16;  // address fields count 16 bytes
+                    tc_mma_f16(d0, ah + o, bd + o, idesc, (st | ks) != 0, me);
+                    tc_mma_f16(d0, al + o, bd + o, idesc, 1, me);
                 }
-                if (ok) tc_commit(full_d + buf);
+                tc_mma_f16(tmem + (IMG ? 2 + buf : 2) * TC_BN, xm, wm, idesc, 0, last ? me : 0);
+                tc_commit(empty_ab + st, me);
             }
+            if (ok) tc_commit(full_d + buf, me);
         }
     } else if (!IMG && warp <= TC_W_WARPS) {
         // ---------------------------------------------------------------- weight operand: thread = (weight row, half of the stage's bytes)
@@ -713,8 +699,9 @@ __global__ void __launch_bounds__(IMG ? TC_THREADS_IMG : TC_THREADS, 1) gemm_tc_
     } else if (warp == TC_LOADER_WARP) {
         // ---------------------------------------------------------------- activation operands: one thread asks for them
         // (bulk asynchronous copies of the tiles tc_token_image_kernel wrote in this layout; 32 KB per stage, and the token
-        // side of the min operand with a super-block's first stage)
-        if (lane == 0) {
+        // side of the min operand with a super-block's first stage; the whole warp, one lane asks)
+        {
+            const uint32_t me = elect_one();
             const uint8_t *img = p.img + (size_t)blockIdx.x * n_it * (2 * TC_OP_BYTES);
             const uint8_t *img_min = p.img_min + (size_t)blockIdx.x * n_sb * TC_MINOP_BYTES;
             // the resident weight image of this row tile (null without one): operand tiles, then the per-super-block sides
@@ -723,15 +710,15 @@ __global__ void __launch_bounds__(IMG ? TC_THREADS_IMG : TC_THREADS, 1) gemm_tc_
             const uint8_t *wside = IMG ? sub.tc + (size_t)tiles_m * n_it * TC_OP_BYTES + (size_t)sub.by * n_sb * TC_SIDE_BYTES : nullptr;
             for (uint32_t it = 0; it < n_it; ++it) {
                 const uint32_t st = it % TC_STAGES, sb = it / TC_STAGES;
-                if (!tma::mbar_wait_blocking(empty_ab + st, ((it / TC_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u)) break;
-                if (st == 0 && sb >= 2 && !tma::mbar_wait_blocking(empty_d + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u)) break;
-                tma::mbar_expect_tx(full_ab + st, (IMG ? 3 : 2) * TC_OP_BYTES + (st == 0 ? TC_MINOP_BYTES + (IMG ? TC_SIDE_BYTES : 0) : 0));
-                tma::bulk_g2s(tc_smem + st * TC_STAGE_BYTES, img + (size_t)it * (2 * TC_OP_BYTES), 2 * TC_OP_BYTES, full_ab + st);
-                if (IMG) tma::bulk_g2s(tc_smem + st * TC_STAGE_BYTES + 2 * TC_OP_BYTES, wimg + (size_t)it * TC_OP_BYTES, TC_OP_BYTES, full_ab + st);
+                if (!warp_all(tma::mbar_wait_blocking(empty_ab + st, ((it / TC_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u))) break;
+                if (st == 0 && sb >= 2 && !warp_all(tma::mbar_wait_blocking(empty_d + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u))) break;
+                tma::mbar_expect_tx_if(full_ab + st, (IMG ? 3 : 2) * TC_OP_BYTES + (st == 0 ? TC_MINOP_BYTES + (IMG ? TC_SIDE_BYTES : 0) : 0), me);
+                tma::bulk_g2s_if(tc_smem + st * TC_STAGE_BYTES, img + (size_t)it * (2 * TC_OP_BYTES), 2 * TC_OP_BYTES, full_ab + st, me);
+                if (IMG) tma::bulk_g2s_if(tc_smem + st * TC_STAGE_BYTES + 2 * TC_OP_BYTES, wimg + (size_t)it * TC_OP_BYTES, TC_OP_BYTES, full_ab + st, me);
                 if (st == 0) {
                     uint8_t *slot = slots + (sb & 1) * TC_SLOT_BYTES;
-                    tma::bulk_g2s(slot, img_min + (size_t)sb * TC_MINOP_BYTES, TC_MINOP_BYTES, full_ab + st);
-                    if (IMG) tma::bulk_g2s(slot + TC_MINOP_BYTES, wside + (size_t)sb * TC_SIDE_BYTES, TC_SIDE_BYTES, full_ab + st);
+                    tma::bulk_g2s_if(slot, img_min + (size_t)sb * TC_MINOP_BYTES, TC_MINOP_BYTES, full_ab + st, me);
+                    if (IMG) tma::bulk_g2s_if(slot + TC_MINOP_BYTES, wside + (size_t)sb * TC_SIDE_BYTES, TC_SIDE_BYTES, full_ab + st, me);
                 }
             }
         }
@@ -983,52 +970,51 @@ __global__ void __launch_bounds__(TC_THREADS_IMG, 1) gemm_tc6_kernel(const TcPar
     pdl_wait();
 
     if (warp == 0) {
-        if (lane == 0) {  // ---- MMA issue
-            const uint32_t idesc = tc_idesc(TC_BM, TC_BN);
-            bool ok = true;
-            uint32_t it = 0;
-            for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
-                const uint32_t buf = sb & 1, d0 = tmem + buf * TC_BN;
-                if (!tma::mbar_wait_blocking(empty_d + buf, ((sb >> 1) & 1) ^ 1, abort_flag, &g_tc_status, 2u)) break;
+        // ---- MMA issue (the whole warp, one lane issues)
+        const uint32_t idesc = tc_idesc(TC_BM, TC_BN), me = elect_one();
+        bool ok = true;
+        uint32_t it = 0;
+        for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
+            const uint32_t buf = sb & 1, d0 = tmem + buf * TC_BN;
+            if (!warp_all(tma::mbar_wait_blocking(empty_d + buf, ((sb >> 1) & 1) ^ 1, abort_flag, &g_tc_status, 2u))) break;
+            tc_fence_after();
+            for (uint32_t st = 0; st < 8; ++st, ++it) {
+                const uint32_t s = it % TC6_STAGES;
+                ok = warp_all(tma::mbar_wait_blocking(full_ab + s, (it / TC6_STAGES) & 1, abort_flag, &g_tc_status, 1u));
+                if (!ok) break;
                 tc_fence_after();
-                for (uint32_t st = 0; st < 8; ++st, ++it) {
-                    const uint32_t s = it % TC6_STAGES;
-                    if (!tma::mbar_wait_blocking(full_ab + s, (it / TC6_STAGES) & 1, abort_flag, &g_tc_status, 1u)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t a_hi = tma::smem_u32(tc_smem + s * TC6_STAGE_BYTES), a_lo = a_hi + TC6_HALF, b_ev = a_lo + TC6_HALF, b_lo = b_ev + TC6_HALF;
+                const uint32_t base = tma::smem_u32(tc_smem + s * TC6_STAGE_BYTES);
+                const uint64_t ah = smem_desc(base, TC_KC_STRIDE, 128), al = smem_desc(base + TC6_HALF, TC_KC_STRIDE, 128),
+                               be = smem_desc(base + 2 * TC6_HALF, TC_KC_STRIDE, 128), bl = smem_desc(base + 3 * TC6_HALF, TC_KC_STRIDE, 128);
 #pragma unroll
-                    for (uint32_t ks = 0; ks < TC6_KS / 16; ++ks) {
-                        const uint32_t o = 2 * ks * TC_KC_STRIDE;
-                        const uint64_t ah = smem_desc(a_hi + o, TC_KC_STRIDE, 128), be = smem_desc(b_ev + o, TC_KC_STRIDE, 128);
-                        tc_mma_f16(d0, ah, be, idesc, (st | ks) != 0);
-                        tc_mma_f16(d0, smem_desc(a_lo + o, TC_KC_STRIDE, 128), be, idesc, 1);
-                        tc_mma_f16(d0, ah, smem_desc(b_lo + o, TC_KC_STRIDE, 128), idesc, 1);
-                    }
-                    tc_commit(empty_ab + s);
+                for (uint32_t ks = 0; ks < TC6_KS / 16; ++ks) {
+                    const uint32_t o = 2 * ks * TC_KC_STRIDE / 16;  // address fields count 16 bytes
+                    tc_mma_f16(d0, ah + o, be + o, idesc, (st | ks) != 0, me);
+                    tc_mma_f16(d0, al + o, be + o, idesc, 1, me);
+                    tc_mma_f16(d0, ah + o, bl + o, idesc, 1, me);
                 }
-                if (ok) tc_commit(full_d + buf);
+                tc_commit(empty_ab + s, me);
             }
+            if (ok) tc_commit(full_d + buf, me);
         }
     } else if (warp == 1) {
-        if (lane == 0) {  // ---- operands (bulk asynchronous copies)
+        {  // ---- operands (bulk asynchronous copies; the whole warp, one lane asks)
+            const uint32_t me = elect_one();
             const uint8_t *img = p.img + (size_t)blockIdx.x * (p.k / TC_KS) * (2 * TC_OP_BYTES);
             const uint8_t *wimg = p.w.tc + (size_t)blockIdx.y * n_it * (2 * TC6_HALF);
             const uint8_t *dv = p.w.tc + (size_t)tiles_m * n_it * (2 * TC6_HALF) + (size_t)blockIdx.y * n_sb * (TC_BN * 4);
             for (uint32_t it = 0; it < n_it; ++it) {
                 const uint32_t s = it % TC6_STAGES, sb = it >> 3, st = it & 7;
-                if (!tma::mbar_wait_blocking(empty_ab + s, ((it / TC6_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u)) break;
-                if (st == 0 && sb >= 2 && !tma::mbar_wait_blocking(empty_d + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u)) break;
+                if (!warp_all(tma::mbar_wait_blocking(empty_ab + s, ((it / TC6_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u))) break;
+                if (st == 0 && sb >= 2 && !warp_all(tma::mbar_wait_blocking(empty_d + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u))) break;
                 uint8_t *dst = tc_smem + s * TC6_STAGE_BYTES;
                 // the 64-k activation stage it / 2 holds [high 16 KB | low 16 KB]; its k half it % 2 is 8 contiguous KB of each
                 const uint8_t *a = img + (size_t)(it >> 1) * (2 * TC_OP_BYTES) + (it & 1) * TC6_HALF;
-                tma::mbar_expect_tx(full_ab + s, TC6_STAGE_BYTES + (st == 0 ? TC_BN * 4 : 0));
-                tma::bulk_g2s(dst, a, TC6_HALF, full_ab + s);
-                tma::bulk_g2s(dst + TC6_HALF, a + TC_OP_BYTES, TC6_HALF, full_ab + s);
-                tma::bulk_g2s(dst + 2 * TC6_HALF, wimg + (size_t)it * (2 * TC6_HALF), 2 * TC6_HALF, full_ab + s);
-                if (st == 0) tma::bulk_g2s(tc_smem + TC6_DVAL_OFF + (sb & 1) * (TC_BN * 4), dv + (size_t)sb * (TC_BN * 4), TC_BN * 4, full_ab + s);
+                tma::mbar_expect_tx_if(full_ab + s, TC6_STAGE_BYTES + (st == 0 ? TC_BN * 4 : 0), me);
+                tma::bulk_g2s_if(dst, a, TC6_HALF, full_ab + s, me);
+                tma::bulk_g2s_if(dst + TC6_HALF, a + TC_OP_BYTES, TC6_HALF, full_ab + s, me);
+                tma::bulk_g2s_if(dst + 2 * TC6_HALF, wimg + (size_t)it * (2 * TC6_HALF), 2 * TC6_HALF, full_ab + s, me);
+                if (st == 0) tma::bulk_g2s_if(tc_smem + TC6_DVAL_OFF + (sb & 1) * (TC_BN * 4), dv + (size_t)sb * (TC_BN * 4), TC_BN * 4, full_ab + s, me);
             }
         }
     } else {

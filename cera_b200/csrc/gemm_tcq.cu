@@ -323,54 +323,50 @@ __global__ void __launch_bounds__(TQ_THREADS, 1) gemm_tcq_kernel(const __grid_co
     uint32_t it = 0;  // stages so far, over all units
 
     if (warp == 0) {
-        if (lane == 0) {  // ---- products
-            bool ok = true;
-            for (uint32_t u = blockIdx.x; u < units && ok; u += gridDim.x) {
-                const TqUnit o = tq_unit<BN>(p, u);
-                const uint32_t idesc = (1u << 4) | ((o.nc >> 3) << 17) | ((TQ_BM >> 4) << 24);  // f16 x f16 -> f32, K-major
-                for (uint32_t st = o.s0; st < o.s1; ++st, ++it) {
-                    const uint32_t s = it % S::STAGES, b = it % S::ACC, nblk = min(2u, p.nb - 2 * st);
-                    if (!tma::mbar_wait_blocking(empty_d + b, ((it / S::ACC) & 1) ^ 1, abort_flag, &g_tcq_status, 1u) ||
-                        !tma::mbar_wait_blocking(full + s, (it / S::STAGES) & 1, abort_flag, &g_tcq_status, 1u)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t a = tma::smem_u32(tq_smem + s * S::STAGE), x = a + S::NA * S::OP, d = tmem + b * 2 * BN;
-                    const uint64_t ad = smem_desc(a, S::KC, 128), xd = smem_desc(x, o.nc * 16, 128);  // address fields count 16 bytes
+        // ---- products: the whole warp, one lane issues
+        const uint32_t me = elect_one();
+        bool ok = true;
+        for (uint32_t u = blockIdx.x; u < units && ok; u += gridDim.x) {
+            const TqUnit o = tq_unit<BN>(p, u);
+            const uint32_t idesc = (1u << 4) | ((o.nc >> 3) << 17) | ((TQ_BM >> 4) << 24);  // f16 x f16 -> f32, K-major
+            for (uint32_t st = o.s0; st < o.s1; ++st, ++it) {
+                const uint32_t s = it % S::STAGES, b = it % S::ACC, nblk = min(2u, p.nb - 2 * st);
+                ok = warp_all(tma::mbar_wait_blocking(empty_d + b, ((it / S::ACC) & 1) ^ 1, abort_flag, &g_tcq_status, 1u) &&
+                              tma::mbar_wait_blocking(full + s, (it / S::STAGES) & 1, abort_flag, &g_tcq_status, 1u));
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t a = tma::smem_u32(tq_smem + s * S::STAGE), x = a + S::NA * S::OP, d = tmem + b * 2 * BN;
+                const uint64_t ad = smem_desc(a, S::KC, 128), xd = smem_desc(x, o.nc * 16, 128);  // address fields count 16 bytes
 #pragma unroll
-                    for (uint32_t ks = 0; ks < 4; ++ks) {
-                        if (ks / 2 >= nblk) break;
-                        tc_mma_f16(d + ks / 2 * BN, ad + 2 * ks * S::KC / 16, xd + 2 * ks * o.nc, idesc, ks & 1);
-                        if (S::NA == 2) tc_mma_f16(d + ks / 2 * BN, ad + (S::OP + 2 * ks * S::KC) / 16, xd + 2 * ks * o.nc, idesc, 1);
-                    }
-                    tc_commit(full_d + b);
-                    tc_commit(empty + s);
+                for (uint32_t ks = 0; ks < 4; ++ks) {
+                    const uint32_t on = ks / 2 < nblk ? me : 0;
+                    tc_mma_f16(d + ks / 2 * BN, ad + 2 * ks * S::KC / 16, xd + 2 * ks * o.nc, idesc, ks & 1, on);
+                    if (S::NA == 2) tc_mma_f16(d + ks / 2 * BN, ad + (S::OP + 2 * ks * S::KC) / 16, xd + 2 * ks * o.nc, idesc, 1, on);
                 }
+                tc_commit(full_d + b, me);
+                tc_commit(empty + s, me);
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {  // ---- activations
-            bool ok = true;
-            for (uint32_t u = blockIdx.x; u < units && ok; u += gridDim.x) {
-                const TqUnit o = tq_unit<BN>(p, u);
-                const uint8_t *src = p.img + (size_t)o.ct * p.n_it * BN * TQ_COL;
-                const uint32_t bytes = o.nc * TQ_COL;
-                for (uint32_t st = o.s0; st < o.s1; ++st, ++it) {
-                    const uint32_t s = it % S::STAGES;
-                    if (!tma::mbar_wait_blocking(empty + s, ((it / S::STAGES) & 1) ^ 1, abort_flag, &g_tcq_status, 2u)) {
-                        ok = false;
-                        break;
-                    }
-                    tma::mbar_expect_tx(full + s, bytes);  // (of a last half stage no product and no sum reads the second block)
-                    tma::bulk_g2s(tq_smem + s * S::STAGE + S::NA * S::OP, src + (size_t)st * bytes, bytes, full + s);
-                }
+        // ---- activations: the whole warp, one lane requests
+        const uint32_t me = elect_one();
+        bool ok = true;
+        for (uint32_t u = blockIdx.x; u < units && ok; u += gridDim.x) {
+            const TqUnit o = tq_unit<BN>(p, u);
+            const uint8_t *src = p.img + (size_t)o.ct * p.n_it * BN * TQ_COL;
+            const uint32_t bytes = o.nc * TQ_COL;
+            for (uint32_t st = o.s0; st < o.s1; ++st, ++it) {
+                const uint32_t s = it % S::STAGES;
+                ok = warp_all(tma::mbar_wait_blocking(empty + s, ((it / S::STAGES) & 1) ^ 1, abort_flag, &g_tcq_status, 2u));
+                if (!ok) break;
+                tma::mbar_expect_tx_if(full + s, bytes, me);  // (of a last half stage no product and no sum reads the second block)
+                tma::bulk_g2s_if(tq_smem + s * S::STAGE + S::NA * S::OP, src + (size_t)st * bytes, bytes, full + s, me);
             }
-            // this CTA's shared memory must outlive the copies in flight (they only are when something gave up)
-            if (*abort_flag)
-                for (uint32_t i = it > S::STAGES ? it - S::STAGES : 0; i < it; ++i)
-                    for (uint32_t n = 0; n < (1u << 16) && !tma::mbar_test(full + i % S::STAGES, (i / S::STAGES) & 1); ++n) __nanosleep(40);
         }
+        // this CTA's shared memory must outlive the copies in flight (they only are when something gave up)
+        if (*abort_flag)
+            for (uint32_t i = it > S::STAGES ? it - S::STAGES : 0; i < it; ++i)
+                for (uint32_t n = 0; n < (1u << 16) && !tma::mbar_test(full + i % S::STAGES, (i / S::STAGES) & 1); ++n) __nanosleep(40);
     } else if (warp < 2 + TQ_EPI) {
         // ---- epilogue: lane = row, half of the columns, the running sums in registers
         const uint32_t quad = warp & 3, ch = (warp - 2) >> 2, c_base = ch * (BN / 2);

@@ -87,6 +87,24 @@ __device__ __forceinline__ void tensor_g2s_2d(void *dst, const void *map, int32_
                  : "memory");
 }
 
+// ---- for a warp that runs a loop of requests together, issued by the lane for which `me` is true (see tc_mma_f16) ----
+__device__ __forceinline__ void mbar_expect_tx_if(uint64_t *bar, uint32_t bytes, uint32_t me) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)), "r"(bytes), "r"(me)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_g2s_if(void *dst, const void *src, uint32_t bytes, uint64_t *bar, uint32_t me) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t}" ::"r"(smem_u32(dst)),
+        "l"(src), "r"(bytes), "r"(smem_u32(bar)), "r"(me)
+        : "memory");
+}
+__device__ __forceinline__ void tensor_g2s_2d_if(void *dst, const void *map, int32_t x, int32_t y, uint64_t *bar, uint32_t me) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t@q cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}" ::"r"(
+            smem_u32(dst)),
+        "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(me)
+        : "memory");
+}
 // 16 bytes global -> shared through the LSU's asynchronous copy path (L1-bypassing).
 __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
