@@ -87,7 +87,34 @@ __device__ __forceinline__ void tensor_g2s_2d(void *dst, const void *map, int32_
                  : "memory");
 }
 
-// ---- for a warp that runs a loop of requests together, issued by the lane for which `me` is true (see tc_mma_f16) ----
+// ---- barriers of another CTA of the cluster ----
+__device__ __forceinline__ uint32_t smem_of_rank(const void *p, uint32_t rank) {  // the same object in that CTA's shared memory
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// mbar_wait_blocking for a barrier that threads of other CTAs arrive on.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity, volatile uint32_t *abort_flag, unsigned int *status, unsigned int who) {
+    for (uint32_t i = 0; i < (SPIN_LIMIT >> 4); ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        if (*abort_flag) return false;
+    }
+    *abort_flag = 1;
+    atomicOr(status, who);
+    return false;
+}
+// ---- the same for a warp that runs a loop of requests together, issued by the lane for which `me` is true (see tc_mma_f16) ----
 __device__ __forceinline__ void mbar_expect_tx_if(uint64_t *bar, uint32_t bytes, uint32_t me) {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)), "r"(bytes), "r"(me)
                  : "memory");
@@ -105,6 +132,15 @@ __device__ __forceinline__ void tensor_g2s_2d_if(void *dst, const void *map, int
         "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(me)
         : "memory");
 }
+// Its bytes counted on a barrier (cluster address) of this CTA or its cta_group::2 peer.
+__device__ __forceinline__ void tensor_g2s_2d_pair_if(void *dst, const void *map, int32_t x, int32_t y, uint32_t bar, uint32_t me) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(bar), "r"(x), "r"(y), "r"(me)
+        : "memory");
+}
+
 // 16 bytes global -> shared through the LSU's asynchronous copy path (L1-bypassing).
 __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
