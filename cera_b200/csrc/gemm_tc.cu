@@ -36,8 +36,8 @@
 //    the min term is one more GEMM over the k / 32 blocks after the k loop.
 //  * gemm_tc_kernel<T, IMG>: 128 x 128 per CTA.  IMG: the loader thread fetches all three operands, the min term is the
 //    16-column MMA above into its own double-buffered accumulator, output in registers.  !IMG: 18 warps - warp 0
-//    issues the MMAs from one thread, warps 1-8 build the weight operand (thread = weight row x half of the stage's
-//    bytes), one thread of warp 9 requests the activation operands, warps 10-17 are the epilogue (thread = token lane x
+//    issues the MMAs, warps 1-8 build the weight operand (thread = weight row x half of the stage's
+//    bytes), warp 9 requests the activation operands, warps 10-17 are the epilogue (thread = token lane x
 //    64 rows) with the running output in a fourth TMEM region.
 //  * gemm_tc6_kernel (Q6_K, image only): sc * (q - 32) needs 13 bits, so the image holds it as two exact f16 operands
 //    and a k-step is three MMAs; no min term.
@@ -46,6 +46,7 @@
 // TMEM is freed and a status word reports it (cera_cuda_kernel_status).
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 
@@ -132,7 +133,23 @@ struct TcParams {
     const uint8_t *tc_x[2];
     float *out_x[2];
     uint32_t m_x[2], ldc_x[2];
+    // CTA b < whole: tile b (x = b % x_tiles fastest); beyond it `parts` CTAs per tile, each over its share of the super-blocks, leave partial sums
+    // [row of the tile][token] at partial + slot * tile size for tc_parts_kernel.
+    uint32_t x_tiles, whole, parts;
+    float *partial;
 };
+
+// A CTA's tile and its super-blocks [sb0, sb0 + n_sb); slot: where its partial sum goes, TC_WHOLE if it does the tile alone.
+constexpr uint32_t TC_WHOLE = 0xffffffffu;
+struct TcTile {
+    uint32_t x, y, sb0, n_sb, slot;
+};
+__device__ __forceinline__ TcTile tc_tile(const TcParams &p) {
+    const uint32_t b = blockIdx.x, n_sb = p.k / 256;
+    if (b < p.whole) return {b % p.x_tiles, b / p.x_tiles, 0, n_sb, TC_WHOLE};
+    const uint32_t i = b - p.whole, t = p.whole + i / p.parts, part = i % p.parts, sb0 = n_sb * part / p.parts;
+    return {t % p.x_tiles, t / p.x_tiles, sb0, n_sb * (part + 1) / p.parts - sb0, i};
+}
 
 // The weight a CTA works for and its y tile inside that weight.
 struct TcSub {
@@ -140,15 +157,15 @@ struct TcSub {
     float *out;
     uint32_t m, ldc, by;
 };
-__device__ __forceinline__ TcSub tc_select(const TcParams &p) {
-    TcSub s{p.w.tc, p.out, p.m, p.ldc, blockIdx.y};
-    if (p.n_w > 1 && blockIdx.y >= p.y_end[0]) {
-        const int i = (p.n_w > 2 && blockIdx.y >= p.y_end[1]) ? 1 : 0;
+__device__ __forceinline__ TcSub tc_select(const TcParams &p, uint32_t y) {
+    TcSub s{p.w.tc, p.out, p.m, p.ldc, y};
+    if (p.n_w > 1 && y >= p.y_end[0]) {
+        const int i = (p.n_w > 2 && y >= p.y_end[1]) ? 1 : 0;
         s.tc = p.tc_x[i];
         s.out = p.out_x[i];
         s.m = p.m_x[i];
         s.ldc = p.ldc_x[i];
-        s.by = blockIdx.y - p.y_end[i];
+        s.by = y - p.y_end[i];
     }
     return s;
 }
@@ -395,7 +412,7 @@ __global__ void __launch_bounds__(TC_BN) tc_weight_min_kernel(const WeightView w
 //    blocks of the whole row after the k loop - weights dmin * mn * 2^s[row] (tc_weight_min_kernel) and activations
 //    g * xs_b * A_b, each as high and low f16 parts, three MMAs per step (the low x low product is below 2^-22) - into
 //    the accumulator buffer of a virtual last super-block.
-// Warps: 0 MMA issue (one thread), 1 operand loader (one thread), 2-9 epilogue.
+// Warps: 0 MMA issue, 1 operand loader, 2-9 epilogue.
 __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams p) {
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(tc_smem + TCW_TAIL_OFF);
@@ -403,10 +420,12 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * TCW_STAGES + 4);
     volatile uint32_t *abort_flag = tmem_slot + 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const TcSub sub = tc_select(p);
-    const uint32_t col0 = blockIdx.x * TC_BM, row0 = sub.by * 2 * TC_BN;
+    const TcTile tile = tc_tile(p);
+    const TcSub sub = tc_select(p, tile.y);
+    const uint32_t col0 = tile.x * TC_BM, row0 = sub.by * 2 * TC_BN;
     const TcImage L = tc_image_layout(sub.m, p.k);
-    const uint32_t n_sb = L.n_sb, n_it = L.n_it, n_mit = L.n_mit;
+    // loops count the super-blocks of this CTA; the min GEMM goes with the last share
+    const uint32_t n_sb = tile.n_sb, n_it = L.n_it, n_mit = L.n_mit, n_rounds = n_sb + (tile.sb0 + n_sb == L.n_sb);
     if (tid == 0) {
         for (int s = 0; s < TCW_STAGES; ++s) {
             tma::mbar_init(full_ab + s, 1);   // the loader's expect_tx
@@ -435,7 +454,7 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
         const uint32_t idesc = tc_idesc(TC_BM, TC_BN), me = elect_one();
         bool ok = true;
         uint32_t it = 0;
-        for (uint32_t sb = 0; sb <= n_sb && ok; ++sb) {  // super-block n_sb is the min GEMM
+        for (uint32_t sb = 0; sb < n_rounds && ok; ++sb) {  // super-block n_sb is the min GEMM
             const uint32_t buf = sb & 1, d0 = tmem + buf * 2 * TC_BN;
             if (!warp_all(tma::mbar_wait_blocking(empty_d + buf, ((sb >> 1) & 1) ^ 1, abort_flag, &g_tc_status, 2u))) break;
             tc_fence_after();
@@ -481,10 +500,11 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
         {
             const uint32_t me = elect_one();
             const uint32_t t0 = min(2 * sub.by, L.tiles - 1), t1 = min(2 * sub.by + 1, L.tiles - 1);  // (an odd last tile is read twice)
-            const uint8_t *img = p.img + (size_t)blockIdx.x * n_it * (2 * TC_OP_BYTES);
-            const uint8_t *w0 = sub.tc + (size_t)t0 * n_it * TC_OP_BYTES, *w1 = sub.tc + (size_t)t1 * n_it * TC_OP_BYTES;
-            const uint8_t *sd0 = sub.tc + L.side + (size_t)t0 * n_sb * TC_SIDE_BYTES + TC_MINOP_BYTES;  // d[128] of a super-block
-            const uint8_t *sd1 = sub.tc + L.side + (size_t)t1 * n_sb * TC_SIDE_BYTES + TC_MINOP_BYTES;
+            const uint32_t it0 = tile.sb0 * (256 / TC_KS);
+            const uint8_t *img = p.img + ((size_t)tile.x * n_it + it0) * (2 * TC_OP_BYTES);
+            const uint8_t *w0 = sub.tc + ((size_t)t0 * n_it + it0) * TC_OP_BYTES, *w1 = sub.tc + ((size_t)t1 * n_it + it0) * TC_OP_BYTES;
+            const uint8_t *sd0 = sub.tc + L.side + ((size_t)t0 * L.n_sb + tile.sb0) * TC_SIDE_BYTES + TC_MINOP_BYTES;  // d[128] of a super-block
+            const uint8_t *sd1 = sub.tc + L.side + ((size_t)t1 * L.n_sb + tile.sb0) * TC_SIDE_BYTES + TC_MINOP_BYTES;
             uint32_t it = 0;
             bool ok = true;
             for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
@@ -511,9 +531,9 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
                     }
                 }
             }
-            const uint8_t *xm = p.xm + (size_t)blockIdx.x * n_mit * (2 * TCW_MINT_BYTES);
+            const uint8_t *xm = p.xm + (size_t)tile.x * n_mit * (2 * TCW_MINT_BYTES);
             const uint8_t *m0 = sub.tc + L.wmin + (size_t)t0 * n_mit * (2 * TCW_MINT_BYTES), *m1 = sub.tc + L.wmin + (size_t)t1 * n_mit * (2 * TCW_MINT_BYTES);
-            for (uint32_t mi = 0; mi < n_mit && ok; ++mi, ++it) {
+            for (uint32_t mi = 0; mi < n_mit && ok && n_rounds > n_sb; ++mi, ++it) {
                 const uint32_t s = it % TCW_STAGES;
                 if (!warp_all(tma::mbar_wait_blocking(empty_ab + s, ((it / TCW_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u))) break;
                 uint8_t *dst = tc_smem + s * TCW_STAGE_BYTES;
@@ -537,7 +557,7 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
         for (int i = 0; i < TC_BN; ++i) acc[i] = 0.0f;
         float ginv = 1.0f;
         bool ok = true;
-        for (uint32_t sb = 0; sb <= n_sb && ok; ++sb) {
+        for (uint32_t sb = 0; sb < n_rounds && ok; ++sb) {
             const uint32_t buf = sb & 1;
             if (!tma::mbar_wait_blocking(full_d + buf, (sb >> 1) & 1, abort_flag, &g_tc_status, 16u)) {
                 ok = false;
@@ -572,7 +592,11 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
             __syncwarp();
             if (lane == 0) tma::mbar_arrive(empty_d + buf);  // the accumulator buffer and the d slot are free again
         }
-        if (ok && col0 + tl < p.n) {
+        if (ok && tile.slot != TC_WHOLE) {
+            float *o = p.partial + (size_t)tile.slot * (2 * TC_BN * TC_BM) + hh * TC_BN * TC_BM + tl;
+#pragma unroll
+            for (int i = 0; i < TC_BN; ++i) o[i * TC_BM] = acc[i];
+        } else if (ok && col0 + tl < p.n) {
             // ---- the thread's 128 cells -> global memory: cell (row i, token j) at out[i * ldy + j * ldc]
             const uint32_t r0 = row0 + hh * TC_BN;
             float *o = sub.out + (size_t)r0 * p.ldy + (size_t)(col0 + tl) * sub.ldc;
@@ -615,9 +639,10 @@ __global__ void __launch_bounds__(IMG ? TC_THREADS_IMG : TC_THREADS, 1) gemm_tc_
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * TC_STAGES + 4);
     volatile uint32_t *abort_flag = tmem_slot + 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const TcSub sub = tc_select(p);
-    const uint32_t col0 = blockIdx.x * TC_BM, row0 = sub.by * TC_BN;
-    const uint32_t n_sb = p.k / 256, n_it = n_sb * TC_STAGES;
+    const TcTile tile = tc_tile(p);
+    const TcSub sub = tc_select(p, tile.y);
+    const uint32_t col0 = tile.x * TC_BM, row0 = sub.by * TC_BN;
+    const uint32_t k_sb = p.k / 256, n_sb = tile.n_sb, n_it = n_sb * TC_STAGES;  // loops count the super-blocks of this CTA
     constexpr int TC_LOADER_WARP = IMG ? 1 : TC_W_WARPS + 1;  // the epilogue warps follow it
     if (tid == 0) {
         for (int s = 0; s < TC_STAGES; ++s) {
@@ -697,17 +722,18 @@ __global__ void __launch_bounds__(IMG ? TC_THREADS_IMG : TC_THREADS, 1) gemm_tc_
             tma::mbar_arrive(full_ab + st);
         }
     } else if (warp == TC_LOADER_WARP) {
-        // ---------------------------------------------------------------- activation operands: one thread asks for them
+        // ---------------------------------------------------------------- activation operands: the whole warp, one lane asks
         // (bulk asynchronous copies of the tiles tc_token_image_kernel wrote in this layout; 32 KB per stage, and the token
-        // side of the min operand with a super-block's first stage; the whole warp, one lane asks)
+        // side of the min operand with a super-block's first stage)
         {
             const uint32_t me = elect_one();
-            const uint8_t *img = p.img + (size_t)blockIdx.x * n_it * (2 * TC_OP_BYTES);
-            const uint8_t *img_min = p.img_min + (size_t)blockIdx.x * n_sb * TC_MINOP_BYTES;
+            const size_t x_sb = (size_t)tile.x * k_sb + tile.sb0, w_sb = (size_t)sub.by * k_sb + tile.sb0;
+            const uint8_t *img = p.img + x_sb * TC_STAGES * (2 * TC_OP_BYTES);
+            const uint8_t *img_min = p.img_min + x_sb * TC_MINOP_BYTES;
             // the resident weight image of this row tile (null without one): operand tiles, then the per-super-block sides
             const uint32_t tiles_m = (sub.m + TC_BN - 1) / TC_BN;
-            const uint8_t *wimg = IMG ? sub.tc + (size_t)sub.by * n_it * TC_OP_BYTES : nullptr;
-            const uint8_t *wside = IMG ? sub.tc + (size_t)tiles_m * n_it * TC_OP_BYTES + (size_t)sub.by * n_sb * TC_SIDE_BYTES : nullptr;
+            const uint8_t *wimg = IMG ? sub.tc + w_sb * TC_STAGES * TC_OP_BYTES : nullptr;
+            const uint8_t *wside = IMG ? sub.tc + (size_t)tiles_m * k_sb * TC_STAGES * TC_OP_BYTES + w_sb * TC_SIDE_BYTES : nullptr;
             for (uint32_t it = 0; it < n_it; ++it) {
                 const uint32_t st = it % TC_STAGES, sb = it / TC_STAGES;
                 if (!warp_all(tma::mbar_wait_blocking(empty_ab + st, ((it / TC_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u))) break;
@@ -772,7 +798,11 @@ __global__ void __launch_bounds__(IMG ? TC_THREADS_IMG : TC_THREADS, 1) gemm_tc_
                 __syncwarp();
                 if (lane == 0) tma::mbar_arrive(empty_d + buf);  // D and Dm of this parity and the slot's tables are free again
             }
-            if (ok && col0 + tl < p.n) {
+            if (ok && tile.slot != TC_WHOLE) {
+                float *o = p.partial + (size_t)tile.slot * (TC_BN * TC_BM) + ch * 64 * TC_BM + tl;
+#pragma unroll
+                for (int i = 0; i < 64; ++i) o[i * TC_BM] = acc[i];
+            } else if (ok && col0 + tl < p.n) {
                 // ---- the thread's 64 cells -> global memory: cell (row i, token j) at out[i * ldy + j * ldc]
                 float *o = sub.out + (size_t)(row0 + ch * 64) * p.ldy + (size_t)(col0 + tl) * sub.ldc;
                 if (p.ldy == 1 && row0 + ch * 64 + 64 <= sub.m && ((uintptr_t)o & 15) == 0) {  // token-major output: 256 contiguous bytes
@@ -871,7 +901,7 @@ __global__ void __launch_bounds__(IMG ? TC_THREADS_IMG : TC_THREADS, 1) gemm_tc_
 }
 
 template <int T, bool IMG>
-int32_t launch_tc_typed(const TcParams &p, uint32_t y_tiles, cudaStream_t st) {
+int32_t launch_tc_typed(const TcParams &p, uint32_t ctas, cudaStream_t st) {
     static thread_local int configured_dev = -1;  // (one per instantiation)
     int dev = 0;
     cudaGetDevice(&dev);
@@ -879,9 +909,8 @@ int32_t launch_tc_typed(const TcParams &p, uint32_t y_tiles, cudaStream_t st) {
         CERA_CUDA_TRY(cudaFuncSetAttribute(gemm_tc_kernel<T, IMG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_BYTES));
         configured_dev = dev;
     }
-    const dim3 grid((p.n + TC_BM - 1) / TC_BM, y_tiles);
     count_launch();
-    return check_cuda(launch_k(gemm_tc_kernel<T, IMG>, grid, dim3(IMG ? TC_THREADS_IMG : TC_THREADS), (size_t)TC_SMEM_BYTES, st, p),
+    return check_cuda(launch_k(gemm_tc_kernel<T, IMG>, dim3(ctas), dim3(IMG ? TC_THREADS_IMG : TC_THREADS), (size_t)TC_SMEM_BYTES, st, p),
                       "gemm (tcgen05) launch");
 }
 
@@ -944,8 +973,9 @@ __global__ void __launch_bounds__(TC_THREADS_IMG, 1) gemm_tc6_kernel(const TcPar
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * TC6_STAGES + 4);
     volatile uint32_t *abort_flag = tmem_slot + 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t col0 = blockIdx.x * TC_BM, row0 = blockIdx.y * TC_BN;
-    const uint32_t n_sb = p.k / 256, n_it = p.k / TC6_KS, tiles_m = (p.m + TC_BN - 1) / TC_BN;
+    const TcTile tile = tc_tile(p);
+    const uint32_t col0 = tile.x * TC_BM, row0 = tile.y * TC_BN;
+    const uint32_t k_sb = p.k / 256, n_sb = tile.n_sb, n_it = n_sb * 8, tiles_m = (p.m + TC_BN - 1) / TC_BN;
     if (tid == 0) {
         for (int s = 0; s < TC6_STAGES; ++s) {
             tma::mbar_init(full_ab + s, 1);
@@ -1000,9 +1030,10 @@ __global__ void __launch_bounds__(TC_THREADS_IMG, 1) gemm_tc6_kernel(const TcPar
     } else if (warp == 1) {
         {  // ---- operands (bulk asynchronous copies; the whole warp, one lane asks)
             const uint32_t me = elect_one();
-            const uint8_t *img = p.img + (size_t)blockIdx.x * (p.k / TC_KS) * (2 * TC_OP_BYTES);
-            const uint8_t *wimg = p.w.tc + (size_t)blockIdx.y * n_it * (2 * TC6_HALF);
-            const uint8_t *dv = p.w.tc + (size_t)tiles_m * n_it * (2 * TC6_HALF) + (size_t)blockIdx.y * n_sb * (TC_BN * 4);
+            const size_t w_sb = (size_t)tile.y * k_sb + tile.sb0;
+            const uint8_t *img = p.img + ((size_t)tile.x * k_sb + tile.sb0) * (256 / TC_KS) * (2 * TC_OP_BYTES);
+            const uint8_t *wimg = p.w.tc + w_sb * 8 * (2 * TC6_HALF);
+            const uint8_t *dv = p.w.tc + (size_t)tiles_m * k_sb * 8 * (2 * TC6_HALF) + w_sb * (TC_BN * 4);
             for (uint32_t it = 0; it < n_it; ++it) {
                 const uint32_t s = it % TC6_STAGES, sb = it >> 3, st = it & 7;
                 if (!warp_all(tma::mbar_wait_blocking(empty_ab + s, ((it / TC6_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u))) break;
@@ -1060,7 +1091,11 @@ __global__ void __launch_bounds__(TC_THREADS_IMG, 1) gemm_tc6_kernel(const TcPar
             __syncwarp();
             if (lane == 0) tma::mbar_arrive(empty_d + buf);
         }
-        if (ok && col0 + tl < p.n) {
+        if (ok && tile.slot != TC_WHOLE) {
+            float *o = p.partial + (size_t)tile.slot * (TC_BN * TC_BM) + ch * 64 * TC_BM + tl;
+#pragma unroll
+            for (int i = 0; i < 64; ++i) o[i * TC_BM] = acc[i];
+        } else if (ok && col0 + tl < p.n) {
             float *o = p.out + (size_t)(row0 + ch * 64) * p.ldy + (size_t)(col0 + tl) * p.ldc;
             if (p.ldy == 1 && row0 + ch * 64 + 64 <= p.m && ((uintptr_t)o & 15) == 0) {
 #pragma unroll
@@ -1092,7 +1127,7 @@ __global__ void __launch_bounds__(TC_THREADS_IMG, 1) gemm_tc6_kernel(const TcPar
     }
 }
 
-int32_t launch_tc6(const TcParams &p, cudaStream_t st) {
+int32_t launch_tc6(const TcParams &p, uint32_t ctas, cudaStream_t st) {
     static thread_local int configured_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1100,12 +1135,51 @@ int32_t launch_tc6(const TcParams &p, cudaStream_t st) {
         CERA_CUDA_TRY(cudaFuncSetAttribute(gemm_tc6_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC6_SMEM_BYTES));
         configured_dev = dev;
     }
-    const dim3 grid((p.n + TC_BM - 1) / TC_BM, (p.m + TC_BN - 1) / TC_BN);
     count_launch();
-    return check_cuda(launch_k(gemm_tc6_kernel, grid, dim3(TC_THREADS_IMG), (size_t)TC6_SMEM_BYTES, st, p), "gemm (tcgen05, Q6_K) launch");
+    return check_cuda(launch_k(gemm_tc6_kernel, dim3(ctas), dim3(TC_THREADS_IMG), (size_t)TC6_SMEM_BYTES, st, p), "gemm (tcgen05, Q6_K) launch");
 }
 
-int32_t launch_tc_wide(const TcParams &p, uint32_t y_tiles, cudaStream_t st) {
+// Adds the parts of the tiles that several CTAs share, in order, and stores as those kernels do.  CTA = 32 rows x 32 tokens of a tile of `rows` rows,
+// turned in shared memory so that both sides are coalesced.  grid (tiles shared, rows / 32, 4).
+__global__ void __launch_bounds__(256) tc_parts_kernel(const TcParams p, uint32_t rows) {
+    __shared__ float cells[32][33];
+    pdl_trigger();
+    pdl_wait();
+    const uint32_t t = p.whole + blockIdx.x, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const TcSub sub = tc_select(p, t / p.x_tiles);
+    const uint32_t col0 = t % p.x_tiles * TC_BM + blockIdx.z * 32, row0 = sub.by * rows + blockIdx.y * 32;
+    const float *v = p.partial + (size_t)blockIdx.x * p.parts * rows * TC_BM + (size_t)blockIdx.y * 32 * TC_BM + blockIdx.z * 32 + tx;
+    float sum[4] = {};
+    for (uint32_t part = 0; part < p.parts; ++part)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[i] += v[(size_t)part * rows * TC_BM + (ty + 8 * i) * TC_BM];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) cells[ty + 8 * i][tx] = sum[i];
+    __syncthreads();
+    const bool by_rows = p.ldy < sub.ldc;  // neighbouring threads: rows or tokens
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t r = by_rows ? tx : ty + 8 * i, c = by_rows ? ty + 8 * i : tx;
+        if (row0 + r < sub.m && col0 + c < p.n) {
+            float *o = sub.out + (size_t)(row0 + r) * p.ldy + (size_t)(col0 + c) * sub.ldc;
+            *o = p.epilogue == EPI_ADD ? __fadd_rn(*o, cells[r][c]) : cells[r][c];
+        }
+    }
+}
+
+// The last round of a grid of `tiles` tiles over `sms` SMs, a CTA each: how many tiles it has and how many CTAs share one of them along k (1: no
+// sharing).  A round that fills less than half the SMs is shared out; with more in it a tile could not have two CTAs.  Each share is a
+// super-block at least.  448 tiles of k = 4096 (gate / up of 512 tokens, three rounds and four tiles): 280 us before, 212 now.
+struct TcSplit {
+    uint32_t left, parts;
+};
+TcSplit tc_split(uint32_t tiles, uint32_t n_sb, uint32_t sms) {
+    const uint32_t left = tiles % sms;
+    if (tiles < sms || left == 0 || 2 * left > sms || n_sb < 8) return {0, 1};
+    return {left, std::min(std::min(n_sb, sms / left), 16u)};
+}
+
+int32_t launch_tc_wide(const TcParams &p, uint32_t ctas, cudaStream_t st) {
     static thread_local int configured_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1113,9 +1187,8 @@ int32_t launch_tc_wide(const TcParams &p, uint32_t y_tiles, cudaStream_t st) {
         CERA_CUDA_TRY(cudaFuncSetAttribute(gemm_tcw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TCW_SMEM_BYTES));
         configured_dev = dev;
     }
-    const dim3 grid((p.n + TC_BM - 1) / TC_BM, y_tiles);
     count_launch();
-    return check_cuda(launch_k(gemm_tcw_kernel, grid, dim3(TCW_THREADS), (size_t)TCW_SMEM_BYTES, st, p), "gemm (tcgen05, wide) launch");
+    return check_cuda(launch_k(gemm_tcw_kernel, dim3(ctas), dim3(TCW_THREADS), (size_t)TCW_SMEM_BYTES, st, p), "gemm (tcgen05, wide) launch");
 }
 
 }  // namespace
@@ -1185,6 +1258,8 @@ static const bool g_tc_status_registered = register_kernel_status([] {
     return (uint32_t)v << 8;
 });
 
+size_t gemm_parts_bytes() { return (size_t)sm_count() * (2 * TC_BN * TC_BM * 4); }
+
 // One activation matrix against up to three weights (q / k / v, gate / up): the activation operands are converted once
 // and, when every weight has its image, ONE kernel launch covers all of them (the small matrices' CTAs run beside the
 // large one's instead of after them).  *taken = false: not these kernels' case, nothing launched.
@@ -1211,10 +1286,30 @@ int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, s
     const size_t img_bytes = (size_t)tiles * n_it * (2 * TC_OP_BYTES), min_bytes = (size_t)tiles * n_sb * TC_MINOP_BYTES,
                  xm_bytes = (size_t)tiles * n_mit * (2 * TCW_MINT_BYTES);
     const size_t need = img_bytes + min_bytes + xm_bytes + (size_t)n_pad * 8;
+    // with weight images: the wide kernel when its 128 x 256 tiles alone fill the device, else the 128 x 128 one
+    static const int tile_pref = [] {
+        const char *e = getenv("CERA_CUDA_GEMM_TILE");
+        return e ? atoi(e) : 0;
+    }();
+    uint32_t wide_y = 0;
+    for (int i = 0; i < count; ++i) wide_y += (t[i].w.m + 2 * TC_BN - 1) / (2 * TC_BN);
+    const bool wide = w.tc && w.type != CERA_TYPE_Q6_K && (tile_pref == 256 || (tile_pref != 128 && tiles * wide_y >= 120));
+    const uint32_t rows = wide ? 2 * TC_BN : TC_BN;
+    uint32_t y = 0;
+    for (int i = 0; i < count; ++i) y += (t[i].w.m + rows - 1) / rows;
+    // partial sums of the last round's tiles; without room for them the tiles stay whole
+    TcSplit split = w.tc ? tc_split(tiles * y, n_sb, (uint32_t)sm_count()) : TcSplit{0, 1};
+    const size_t parts_bytes = (size_t)split.left * split.parts * rows * TC_BM * 4;
     const bool borrowed = lent.p && lent.bytes >= need;
     uint8_t *scratch = (uint8_t *)lent.p;
-    if (!borrowed) {
-        scratch = (uint8_t *)scratch_alloc(need, st);
+    if (borrowed) {
+        if (lent.bytes < need + parts_bytes) split = {0, 1};
+    } else {
+        scratch = (uint8_t *)scratch_alloc(need + parts_bytes, st);
+        if (!scratch && split.left) {
+            split = {0, 1};
+            scratch = (uint8_t *)scratch_alloc(need, st);
+        }
         if (!scratch) return CERA_CUDA_OK;  // no room for the operand scratch: leave the GEMM to the kernels that need none
     }
     uint8_t *xm = scratch + img_bytes + min_bytes;
@@ -1244,18 +1339,9 @@ int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, s
     p.epilogue = epilogue;
     p.n_w = (uint32_t)count;
     *taken = true;
-    // with weight images: the wide kernel when its 128 x 256 tiles alone fill the device, else the 128 x 128 one
-    static const int tile_pref = [] {
-        const char *e = getenv("CERA_CUDA_GEMM_TILE");
-        return e ? atoi(e) : 0;
-    }();
-    uint32_t wide_y = 0;
-    for (int i = 0; i < count; ++i) wide_y += (t[i].w.m + 2 * TC_BN - 1) / (2 * TC_BN);
-    const bool wide = w.tc && (tile_pref == 256 || (tile_pref != 128 && tiles * wide_y >= 120));
-    uint32_t y = 0;
-    for (int i = 0; i < count; ++i) {
-        y += wide ? (t[i].w.m + 2 * TC_BN - 1) / (2 * TC_BN) : (t[i].w.m + TC_BN - 1) / TC_BN;
-        p.y_end[i] = y;
+    for (int i = 0, end = 0; i < count; ++i) {
+        end += (t[i].w.m + rows - 1) / rows;
+        p.y_end[i] = end;
         if (i) {
             p.tc_x[i - 1] = t[i].w.tc;
             p.out_x[i - 1] = t[i].out;
@@ -1263,15 +1349,24 @@ int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, s
             p.ldc_x[i - 1] = (uint32_t)t[i].ldc;
         }
     }
+    p.x_tiles = tiles;
+    p.whole = tiles * y - split.left;
+    p.parts = split.parts;
+    p.partial = reinterpret_cast<float *>(scratch + need);
+    const uint32_t ctas = p.whole + split.left * split.parts;
     if (rc == CERA_CUDA_OK && w.type == CERA_TYPE_Q6_K) {
-        rc = launch_tc6(p, st);
+        rc = launch_tc6(p, ctas, st);
     } else if (rc == CERA_CUDA_OK && wide) {
-        rc = launch_tc_wide(p, y, st);
+        rc = launch_tc_wide(p, ctas, st);
     } else if (rc == CERA_CUDA_OK) {
         if (w.tc)
-            rc = w.type == CERA_TYPE_Q4_K ? launch_tc_typed<CERA_TYPE_Q4_K, true>(p, y, st) : launch_tc_typed<CERA_TYPE_Q5_K, true>(p, y, st);
+            rc = w.type == CERA_TYPE_Q4_K ? launch_tc_typed<CERA_TYPE_Q4_K, true>(p, ctas, st) : launch_tc_typed<CERA_TYPE_Q5_K, true>(p, ctas, st);
         else
-            rc = w.type == CERA_TYPE_Q4_K ? launch_tc_typed<CERA_TYPE_Q4_K, false>(p, y, st) : launch_tc_typed<CERA_TYPE_Q5_K, false>(p, y, st);
+            rc = w.type == CERA_TYPE_Q4_K ? launch_tc_typed<CERA_TYPE_Q4_K, false>(p, ctas, st) : launch_tc_typed<CERA_TYPE_Q5_K, false>(p, ctas, st);
+    }
+    if (rc == CERA_CUDA_OK && split.left) {
+        count_launch();
+        rc = check_cuda(launch_k(tc_parts_kernel, dim3(split.left, rows / 32, TC_BM / 32), dim3(256), 0, st, p, rows), "gemm (tcgen05) parts launch");
     }
     if (!borrowed) cudaFreeAsync(scratch, st);  // after the kernels above, in stream order
     return rc;

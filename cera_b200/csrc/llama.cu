@@ -389,7 +389,7 @@ int32_t llama_chunk(LlamaModel *m, const uint32_t *tokens, size_t n, size_t star
     GemmScratch in_g, in_q;
     if (!tp) {
         in_g = {m->pf_g, pf_lent_bytes(m->pf_chunk, ff)};
-        in_q = {m->pf_q, pf_lent_bytes(m->pf_chunk, qd)};
+        in_q = {m->pf_q, pf_lent_bytes(m->pf_chunk, qd) + gemm_parts_bytes()};
     }
     if (tp) CERA_TRY(launch_tp_tick(m->tp_words, st));
     CERA_CUDA_TRY(cudaMemcpyAsync(m->pf_tokens, tokens, n * 4, cudaMemcpyHostToDevice, st));
@@ -618,7 +618,7 @@ int32_t LlamaModel::build() {
     }
     {
         const size_t C = m->pf_chunk;
-        CERA_TRY(m->dev_alloc((void **)&m->pf_q, pf_lent_bytes(C, m->l_qd)));
+        CERA_TRY(m->dev_alloc((void **)&m->pf_q, pf_lent_bytes(C, m->l_qd) + (m->tp_size == 1 ? gemm_parts_bytes() : 0)));
         CERA_TRY(m->dev_alloc((void **)&m->pf_k, C * m->l_kvd * 4));
         CERA_TRY(m->dev_alloc((void **)&m->pf_v, C * m->l_kvd * 4));
         if (m->tp_size == 1) {
