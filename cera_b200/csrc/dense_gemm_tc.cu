@@ -46,11 +46,6 @@ struct DtParams {
     uint32_t row_tiles, col_tiles;
 };
 
-// Every thread of both CTAs.
-__device__ __forceinline__ void dt_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 // Output tile t of this launch.
 struct DtTile {
     uint32_t a_row, row0, rows, first, end;
@@ -100,7 +95,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dense_gemm_tc_kernel(const __gr
     }
     __syncwarp();
     // A pair allocates for both of its SMs: both CTAs run by then, and have what they asked for before either goes on.
-    if constexpr (PAIR) dt_cluster_sync();
+    if constexpr (PAIR) cluster_barrier();
     if (warp == 1) {
         if constexpr (PAIR) {
             tmem_alloc_pair(tmem_at, S::TMEM);
@@ -113,7 +108,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dense_gemm_tc_kernel(const __gr
     }
     tc_fence_before();
     __syncthreads();
-    if constexpr (PAIR) dt_cluster_sync();  // (the barriers of both CTAs are there, too)
+    if constexpr (PAIR) cluster_barrier();  // (the barriers of both CTAs are there, too)
     tc_fence_after();
     const uint32_t tmem = *tmem_at;
     pdl_wait();
@@ -161,8 +156,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dense_gemm_tc_kernel(const __gr
             uint32_t it = 0, j = 0;
             bool ok = true;
             auto arrived = [&](uint64_t *bar, uint32_t parity) {
-                return warp_all(PAIR ? tma::mbar_wait_cluster(bar, parity, abort_flag, &g_dense_tc_status, 2u)
-                                     : tma::mbar_wait_blocking(bar, parity, abort_flag, &g_dense_tc_status, 2u));
+                return warp_all(tma::mbar_wait_blocking(bar, parity, abort_flag, &g_dense_tc_status, 2u));
             };
             for (uint32_t t = first_tile; t < n_tiles && ok; t += step, ++j) {
                 const uint32_t b = j & 1, acc = tmem + b * S::ACC;
@@ -261,10 +255,10 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dense_gemm_tc_kernel(const __gr
     tc_fence_before();
     __syncthreads();
     if constexpr (PAIR) {
-        dt_cluster_sync();  // the other CTA's products read this one's shared memory, its warps arrive here
+        cluster_barrier();  // the other CTA's products read this one's shared memory, its warps arrive here
         if (warp == 1) tmem_dealloc_pair(tmem, S::TMEM);
         __syncwarp();
-        dt_cluster_sync();  // neither leaves before both have given back
+        cluster_barrier();  // neither leaves before both have given back
     } else {
         if (warp == 1) tmem_dealloc(tmem, S::TMEM);
     }
@@ -281,25 +275,13 @@ int32_t launch_tc(const DenseGemm &g, cudaStream_t st) {
     const uint32_t rows = (g.tiles ? g.rows_per_expert : g.w.rows) / NA;
     p.row_tiles = (rows + S::ROWS - 1) / S::ROWS;
     p.col_tiles = g.tiles ? g.max_tiles : (g.n + BN - 1) / BN;
-    const uint64_t tiles = (uint64_t)p.row_tiles * p.col_tiles, ctas = PAIR ? 2 : 1, room = (uint64_t)sm_count() / ctas;
+    const uint64_t tiles = (uint64_t)p.row_tiles * p.col_tiles, room = (uint64_t)sm_count() / (PAIR ? 2 : 1);
+    const unsigned grid = (unsigned)(tiles < room ? tiles : room);
     auto k = dense_gemm_tc_kernel<BN, NA, PAIR>;
     CERA_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((tiles < room ? tiles : room) * ctas));
-    cfg.blockDim = dim3(DT_THREADS);
-    cfg.dynamicSmemBytes = S::SMEM;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = (unsigned)ctas;
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = PAIR ? 2 : 1;
     count_launch();
-    return check_cuda(cudaLaunchKernelEx(&cfg, k, mw, mx, p), "dense tcgen05 gemm launch");
+    if (PAIR) return check_cuda(launch_pairs(k, grid, dim3(DT_THREADS), S::SMEM, st, mw, mx, p), "dense tcgen05 gemm (pairs) launch");
+    return check_cuda(launch_k(k, dim3(grid), dim3(DT_THREADS), S::SMEM, st, mw, mx, p), "dense tcgen05 gemm launch");
 }
 
 }  // namespace

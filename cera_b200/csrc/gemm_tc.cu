@@ -30,17 +30,16 @@
 // -> one HFMA2 with the sub-block scale), same results.  Tiles use the canonical K-major no-swizzle layout (8-row x
 // 16-byte core matrices), 64 k-elements per stage.
 //
-// Three kernels:
-//  * gemm_tcw_kernel ("wide", image only): 128 tokens x 256 rows per CTA when those tiles alone fill the device.  TMEM
-//    holds two double-buffered 256-column accumulators; the running output lives in the epilogue threads' registers;
-//    the min term is one more GEMM over the k / 32 blocks after the k loop.
-//  * gemm_tc_kernel<T, IMG>: 128 x 128 per CTA.  IMG: the loader thread fetches all three operands, the min term is the
+// Two kernels:
+//  * gemm_tcw_kernel<Q6, PAIR> ("wide", image only): 128 tokens x 256 rows per CTA, or 256 x 256 per pair of CTAs, when those tiles
+//    fill the device.  TMEM holds two double-buffered 256-column accumulators; the running output lives in the epilogue
+//    threads' registers; the min term is one more GEMM over the k / 32 blocks after the k loop.  Q6_K: sc * (q - 32) needs
+//    13 bits, so the image holds it as two exact f16 operands and a k-step is three MMAs; no min term.
+//  * gemm_tc_kernel<T, IMG>: 128 x 128 per CTA.  IMG: the loader fetches all three operands, the min term is the
 //    16-column MMA above into its own double-buffered accumulator, output in registers.  !IMG: 18 warps - warp 0
 //    issues the MMAs, warps 1-8 build the weight operand (thread = weight row x half of the stage's
 //    bytes), warp 9 requests the activation operands, warps 10-17 are the epilogue (thread = token lane x
 //    64 rows) with the running output in a fourth TMEM region.
-//  * gemm_tc6_kernel (Q6_K, image only): sc * (q - 32) needs 13 bits, so the image holds it as two exact f16 operands
-//    and a k-step is three MMAs; no min term.
 // Stages and accumulator buffers are handed over through mbarriers (tcgen05.commit arrives on them when the MMAs have
 // finished).  Every wait is bounded: when a limit runs out the CTA raises an abort flag, its roles leave their loops,
 // TMEM is freed and a status word reports it (cera_cuda_kernel_status).
@@ -85,15 +84,19 @@ constexpr uint32_t TC_KC_STRIDE = TC_BM * 16;                            // byte
 // The wide variant (a CTA owns 128 tokens x 256 weight rows, weight image only): stages of the two activation operand
 // tiles and the operand tiles of two 128-row image tiles; the min term is one more GEMM at the end of the k loop (see
 // gemm_tcw_kernel), whose stages of 32 activation blocks reuse the ring.
-constexpr int TCW_STAGES = 3;
-constexpr uint32_t TCW_STAGE_BYTES = 4 * TC_OP_BYTES;                     // A high, A low, B rows [0,128), B rows [128,256): 64 KB
 constexpr uint32_t TCW_MIN_J = 32;                                        // activation blocks (k / 32 columns) per min stage
 constexpr uint32_t TCW_MINT_BYTES = TC_BM * TCW_MIN_J * 2;                // one min-GEMM operand tile: 8 KB
-constexpr uint32_t TCW_DVAL_OFF = TCW_STAGES * TCW_STAGE_BYTES;           // two slots of d[256]
-constexpr uint32_t TCW_RS_OFF = TCW_DVAL_OFF + 2 * 2 * TC_BN * 4;         // 2^-s[256] of the min GEMM's weight rows
-constexpr uint32_t TCW_TAIL_OFF = TCW_RS_OFF + 2 * TC_BN * 4;
-constexpr uint32_t TCW_SMEM_BYTES = TCW_TAIL_OFF + 256;
 constexpr int TCW_THREADS = (2 + TC_EPI_WARPS) * 32;
+// Per CTA: A high and low of its 128 tokens, and of B both row tiles or, in a pair, its own.  Q6_K: stages of 32 k, B in two operands per row tile.
+template <bool Q6, bool PAIR>
+struct Wide {
+    static constexpr int KS = Q6 ? 32 : TC_KS, SB_STAGES = 256 / KS;
+    static constexpr uint32_t OP = TC_BM * KS * 2, B_TILE = (Q6 ? 2 : 1) * OP, B_TILES = PAIR ? 1 : 2, STAGE = 2 * OP + B_TILES * B_TILE;
+    static constexpr int STAGES = 192 * 1024 / STAGE;
+    static constexpr uint32_t DVAL = STAGES * STAGE;           // two slots of d[256]
+    static constexpr uint32_t RS = DVAL + 2 * 2 * TC_BN * 4;   // 2^-s[256] of the min GEMM's weight rows
+    static constexpr uint32_t TAIL = RS + 2 * TC_BN * 4, SMEM = TAIL + 256;
+};
 
 // Regions of a weight's resident image (byte offsets): the operand tile of every (128-row tile, stage); per (tile,
 // super-block) the row side of the min operand, d[128] and dmin[128]; per (tile, min stage) the high and the low part of
@@ -144,8 +147,8 @@ constexpr uint32_t TC_WHOLE = 0xffffffffu;
 struct TcTile {
     uint32_t x, y, sb0, n_sb, slot;
 };
-__device__ __forceinline__ TcTile tc_tile(const TcParams &p) {
-    const uint32_t b = blockIdx.x, n_sb = p.k / 256;
+__device__ __forceinline__ TcTile tc_tile(const TcParams &p, uint32_t b) {
+    const uint32_t n_sb = p.k / 256;
     if (b < p.whole) return {b % p.x_tiles, b / p.x_tiles, 0, n_sb, TC_WHOLE};
     const uint32_t i = b - p.whole, t = p.whole + i / p.parts, part = i % p.parts, sb0 = n_sb * part / p.parts;
     return {t % p.x_tiles, t / p.x_tiles, sb0, n_sb * (part + 1) / p.parts - sb0, i};
@@ -402,151 +405,196 @@ __global__ void __launch_bounds__(TC_BN) tc_weight_min_kernel(const WeightView w
     }
 }
 
-// The wide variant: one CTA = 128 tokens x 256 weight rows (two 128-row tiles of the weight image), for GEMMs with enough
-// tiles to fill the device.  Against the 128 x 128 kernel the activation operands are fetched once for twice the MMAs
-// (64 KB per 1024 tensor-pipe cycles instead of 48 KB per 512) and a stage hand-over pays for sixteen MMAs, which is what
-// the 128-wide kernel is short of: its MMA thread waits a third of the time for operands.  TMEM then holds nothing but the
-// two double-buffered accumulators (2 x 256 columns), so
+// The wide kernel, over resident images.  Alone a CTA does 128 tokens x 256 weight rows (two 128-row tiles of the image); in a PAIR (cta_group::2)
+// two CTAs do 256 tokens x 256 rows, each with its own 128 tokens and one of the row tiles, which the tensor cores of both read.
+// What bounds it: shared memory, which a CTA alone reads and writes 192 KB per 64 k (its 16 products of N = 128 take 1212 cycles in a ring without an
+// epilogue and 1370 with it, 1024 being the tensor core's rate), in a pair 112 KB; and then the chip's power, which holds the clock near 1.45 GHz.
+// 512 tokens: gate / up 28672 x 4096 212 us alone, 194 in pairs; Q6_K 4096 x 14336 168 us with 128 x 128 tiles, 119 in pairs.
+// TMEM holds nothing but the two double-buffered accumulators (2 x 256 columns), so
 //  * the running output lives in the epilogue threads' registers (thread = token lane x 128 rows), and
 //  * the min term sum_b dmin * mn_b * (xs_b * A_b) is not accumulated per super-block but as ONE more GEMM over the k / 32
 //    blocks of the whole row after the k loop - weights dmin * mn * 2^s[row] (tc_weight_min_kernel) and activations
 //    g * xs_b * A_b, each as high and low f16 parts, three MMAs per step (the low x low product is below 2^-22) - into
 //    the accumulator buffer of a virtual last super-block.
-// Warps: 0 MMA issue, 1 operand loader, 2-9 epilogue.
+// Warps: 0 MMA issue, 1 operand loader, 2-9 epilogue.  In a pair the even CTA's warp 0 issues for both; the odd one's passes on that its stages are full.
+template <bool Q6, bool PAIR>
 __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams p) {
+    using S = Wide<Q6, PAIR>;
     extern __shared__ __align__(1024) uint8_t tc_smem[];
-    uint64_t *bars = reinterpret_cast<uint64_t *>(tc_smem + TCW_TAIL_OFF);
-    uint64_t *full_ab = bars, *empty_ab = bars + TCW_STAGES, *full_d = bars + 2 * TCW_STAGES, *empty_d = full_d + 2;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * TCW_STAGES + 4);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(tc_smem + S::TAIL);
+    uint64_t *full_ab = bars, *empty_ab = full_ab + S::STAGES, *peer_full = empty_ab + S::STAGES, *full_d = peer_full + S::STAGES, *empty_d = full_d + 2,
+             *slot_free = PAIR ? empty_d + 2 : empty_d;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(empty_d + 4);
     volatile uint32_t *abort_flag = tmem_slot + 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const TcTile tile = tc_tile(p);
+    const uint32_t rank = PAIR ? blockIdx.x & 1 : 0;
+    const TcTile tile = tc_tile(p, PAIR ? blockIdx.x / 2 : blockIdx.x);
     const TcSub sub = tc_select(p, tile.y);
-    const uint32_t col0 = tile.x * TC_BM, row0 = sub.by * 2 * TC_BN;
+    const uint32_t col0 = (PAIR ? 2 * tile.x + rank : tile.x) * TC_BM, row0 = sub.by * 2 * TC_BN;
     const TcImage L = tc_image_layout(sub.m, p.k);
     // loops count the super-blocks of this CTA; the min GEMM goes with the last share
-    const uint32_t n_sb = tile.n_sb, n_it = L.n_it, n_mit = L.n_mit, n_rounds = n_sb + (tile.sb0 + n_sb == L.n_sb);
+    const uint32_t n_sb = tile.n_sb, n_it = L.n_sb * S::SB_STAGES, n_mit = L.n_mit, n_rounds = n_sb + (!Q6 && tile.sb0 + n_sb == L.n_sb);
     if (tid == 0) {
-        for (int s = 0; s < TCW_STAGES; ++s) {
-            tma::mbar_init(full_ab + s, 1);   // the loader's expect_tx
-            tma::mbar_init(empty_ab + s, 1);  // the commit of the stage's MMAs
+        for (int s = 0; s < S::STAGES; ++s) {
+            tma::mbar_init(full_ab + s, 1);    // the loader's expect_tx
+            tma::mbar_init(empty_ab + s, 1);   // the commit of the stage's MMAs
+            tma::mbar_init(peer_full + s, 1);  // the odd CTA's stage is full
         }
         for (int b = 0; b < 2; ++b) {
-            tma::mbar_init(full_d + b, 1);              // the commit after a super-block's last MMA
-            tma::mbar_init(empty_d + b, TC_EPI_WARPS);  // every epilogue warp is done with the buffer and the slot
+            tma::mbar_init(full_d + b, 1);                                // the commit after a super-block's last MMA
+            tma::mbar_init(empty_d + b, (PAIR ? 2 : 1) * TC_EPI_WARPS);  // every epilogue warp (of both CTAs) is done with the buffer
+            if (PAIR) tma::mbar_init(slot_free + b, TC_EPI_WARPS);        // ... of this CTA with the d slot
         }
         *abort_flag = 0;
         tma::mbar_init_fence();
     }
-    if (warp == 0) {
-        tmem_alloc(tmem_slot, TC_TMEM_COLS);
-        tmem_relinquish();
-    }
+    __syncwarp();
     pdl_trigger();
+    // A pair allocates for both of its SMs: both CTAs run by then, and have what they asked for before either goes on.
+    if constexpr (PAIR) cluster_barrier();
+    if (warp == 0) {
+        if constexpr (PAIR) {
+            tmem_alloc_pair(tmem_slot, TC_TMEM_COLS);
+            tmem_relinquish_pair();
+        } else {
+            tmem_alloc(tmem_slot, TC_TMEM_COLS);
+            tmem_relinquish();
+        }
+        __syncwarp();
+    }
     tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) cluster_barrier();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     pdl_wait();
 
-    if (warp == 0) {
+    if (warp == 0 && rank == 0) {
         // ---------------------------------------------------------------- MMA issue (the whole warp, one lane issues)
-        const uint32_t idesc = tc_idesc(TC_BM, TC_BN), me = elect_one();
+        const uint32_t me = elect_one(), idesc = tc_idesc(PAIR ? 2 * TC_BM : TC_BM, PAIR ? 2 * TC_BN : TC_BN);
+        auto mma = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+            if constexpr (PAIR) tc_mma_f16_pair(d, a, b, idesc, acc, me);
+            else tc_mma_f16(d, a, b, idesc, acc, me);
+        };
+        auto commit = [&](uint64_t *bar) {
+            if constexpr (PAIR) tc_commit_pair(bar, me);
+            else tc_commit(bar, me);
+        };
+        auto arrived = [&](uint64_t *bar, uint32_t parity, uint32_t who) {
+            return warp_all(tma::mbar_wait_blocking(bar, parity, abort_flag, &g_tc_status, who));
+        };
         bool ok = true;
         uint32_t it = 0;
         for (uint32_t sb = 0; sb < n_rounds && ok; ++sb) {  // super-block n_sb is the min GEMM
             const uint32_t buf = sb & 1, d0 = tmem + buf * 2 * TC_BN;
-            if (!warp_all(tma::mbar_wait_blocking(empty_d + buf, ((sb >> 1) & 1) ^ 1, abort_flag, &g_tc_status, 2u))) break;
+            if (!arrived(empty_d + buf, ((sb >> 1) & 1) ^ 1, 2u)) break;
             tc_fence_after();
-            const uint32_t n_st = sb < n_sb ? 4u : n_mit;
+            const uint32_t n_st = sb < n_sb ? (uint32_t)S::SB_STAGES : n_mit;
             for (uint32_t st = 0; st < n_st; ++st, ++it) {
-                const uint32_t s = it % TCW_STAGES;
-                ok = warp_all(tma::mbar_wait_blocking(full_ab + s, (it / TCW_STAGES) & 1, abort_flag, &g_tc_status, 1u));
+                const uint32_t s = it % S::STAGES, full = (it / S::STAGES) & 1;
+                ok = arrived(full_ab + s, full, 1u) && (!PAIR || arrived(peer_full + s, full, 1u));
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t base = tma::smem_u32(tc_smem + s * TCW_STAGE_BYTES);
-                if (sb < n_sb) {
-                    const uint64_t ah = smem_desc(base, TC_KC_STRIDE, 128), al = smem_desc(base + TC_OP_BYTES, TC_KC_STRIDE, 128),
-                                   bd0 = smem_desc(base + 2 * TC_OP_BYTES, TC_KC_STRIDE, 128), bd1 = smem_desc(base + 3 * TC_OP_BYTES, TC_KC_STRIDE, 128);
+                const uint32_t base = tma::smem_u32(tc_smem + s * S::STAGE);
+                if (Q6 || sb < n_sb) {
+                    const uint64_t ah = smem_desc(base, TC_KC_STRIDE, 128), al = smem_desc(base + S::OP, TC_KC_STRIDE, 128), b = smem_desc(base + 2 * S::OP, TC_KC_STRIDE, 128);
 #pragma unroll
-                    for (uint32_t ks = 0; ks < TC_KS / 16; ++ks) {
+                    for (uint32_t ks = 0; ks < S::KS / 16; ++ks) {
                         const uint32_t o = 2 * ks * TC_KC_STRIDE / 16, acc = (st | ks) != 0;  // address fields count 16 bytes
-                        tc_mma_f16(d0, ah + o, bd0 + o, idesc, acc, me);
-                        tc_mma_f16(d0 + TC_BN, ah + o, bd1 + o, idesc, acc, me);
-                        tc_mma_f16(d0, al + o, bd0 + o, idesc, 1, me);
-                        tc_mma_f16(d0 + TC_BN, al + o, bd1 + o, idesc, 1, me);
+#pragma unroll
+                        for (uint32_t h = 0; h < S::B_TILES; ++h) mma(d0 + h * TC_BN, ah + o, b + h * (S::B_TILE / 16) + o, acc);
+#pragma unroll
+                        for (uint32_t h = 0; h < S::B_TILES; ++h) mma(d0 + h * TC_BN, al + o, b + h * (S::B_TILE / 16) + o, 1);
+                        if constexpr (Q6) mma(d0, ah + o, b + S::OP / 16 + o, 1);  // the lowest bits
                     }
                 } else {
-                    // min GEMM: [x high | x low | w high, w low of rows [0,128) | the same of rows [128,256)], 32 blocks = two steps
+                    // min GEMM: [x high | x low | per row tile w high, w low], 32 blocks = two steps
                     const uint64_t xh = smem_desc(base, TC_KC_STRIDE, 128), xl = smem_desc(base + TCW_MINT_BYTES, TC_KC_STRIDE, 128);
 #pragma unroll
                     for (uint32_t ks = 0; ks < TCW_MIN_J / 16; ++ks) {
                         const uint32_t o = 2 * ks * TC_KC_STRIDE / 16;
 #pragma unroll
-                        for (uint32_t h = 0; h < 2; ++h) {
+                        for (uint32_t h = 0; h < S::B_TILES; ++h) {
                             const uint64_t wh = xh + (2 + 2 * h) * TCW_MINT_BYTES / 16, wl = wh + TCW_MINT_BYTES / 16;
-                            tc_mma_f16(d0 + h * TC_BN, xh + o, wh + o, idesc, (st | ks) != 0, me);
-                            tc_mma_f16(d0 + h * TC_BN, xl + o, wh + o, idesc, 1, me);
-                            tc_mma_f16(d0 + h * TC_BN, xh + o, wl + o, idesc, 1, me);
+                            mma(d0 + h * TC_BN, xh + o, wh + o, (st | ks) != 0);
+                            mma(d0 + h * TC_BN, xl + o, wh + o, 1);
+                            mma(d0 + h * TC_BN, xh + o, wl + o, 1);
                         }
                     }
                 }
-                tc_commit(empty_ab + s, me);
+                commit(empty_ab + s);
             }
-            if (ok) tc_commit(full_d + buf, me);
+            if (ok) commit(full_d + buf);
+        }
+    } else if (warp == 0) {
+        // ---------------------------------------------------------------- odd CTA: its stages are full
+        const uint32_t n_all = n_sb * S::SB_STAGES + (n_rounds > n_sb ? n_mit : 0);
+        for (uint32_t it = 0; it < n_all; ++it) {
+            const uint32_t s = it % S::STAGES;
+            if (!warp_all(tma::mbar_wait_blocking(full_ab + s, (it / S::STAGES) & 1, abort_flag, &g_tc_status, 1u))) break;
+            if (lane == 0) tma::mbar_arrive_cluster(tma::smem_of_rank(peer_full + s, 0));
+            __syncwarp();
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- operands: the whole warp, one lane asks for them (bulk asynchronous copies)
-        {
-            const uint32_t me = elect_one();
-            const uint32_t t0 = min(2 * sub.by, L.tiles - 1), t1 = min(2 * sub.by + 1, L.tiles - 1);  // (an odd last tile is read twice)
-            const uint32_t it0 = tile.sb0 * (256 / TC_KS);
-            const uint8_t *img = p.img + ((size_t)tile.x * n_it + it0) * (2 * TC_OP_BYTES);
-            const uint8_t *w0 = sub.tc + ((size_t)t0 * n_it + it0) * TC_OP_BYTES, *w1 = sub.tc + ((size_t)t1 * n_it + it0) * TC_OP_BYTES;
-            const uint8_t *sd0 = sub.tc + L.side + ((size_t)t0 * L.n_sb + tile.sb0) * TC_SIDE_BYTES + TC_MINOP_BYTES;  // d[128] of a super-block
-            const uint8_t *sd1 = sub.tc + L.side + ((size_t)t1 * L.n_sb + tile.sb0) * TC_SIDE_BYTES + TC_MINOP_BYTES;
-            uint32_t it = 0;
-            bool ok = true;
-            for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
-                for (uint32_t st = 0; st < 4; ++st, ++it) {
-                    const uint32_t s = it % TCW_STAGES;
-                    if (!warp_all(tma::mbar_wait_blocking(empty_ab + s, ((it / TCW_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u))) {
-                        ok = false;
-                        break;
-                    }
-                    // the d slot of this super-block was last read by the epilogue of super-block sb - 2
-                    if (st == 0 && sb >= 2 && !warp_all(tma::mbar_wait_blocking(empty_d + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u))) {
-                        ok = false;
-                        break;
-                    }
-                    uint8_t *dst = tc_smem + s * TCW_STAGE_BYTES;
-                    tma::mbar_expect_tx_if(full_ab + s, TCW_STAGE_BYTES + (st == 0 ? 2 * TC_BN * 4 : 0), me);
+        const uint32_t me = elect_one();
+        const uint32_t t0 = min(2 * sub.by, L.tiles - 1), t1 = min(2 * sub.by + 1, L.tiles - 1);  // (an odd last tile is read twice)
+        const uint32_t x_t = min(col0, p.n - 1) / TC_BM, own = rank ? t1 : t0, it0 = tile.sb0 * S::SB_STAGES;  // (as an odd last token tile is in a pair)
+        const size_t side = Q6 ? (size_t)L.tiles * n_it * S::B_TILE : L.side, side_step = Q6 ? TC_BN * 4 : TC_SIDE_BYTES;
+        const uint8_t *img = p.img + ((size_t)x_t * L.n_sb + tile.sb0) * (256 / TC_KS) * (2 * TC_OP_BYTES);
+        const uint8_t *w0 = sub.tc + ((size_t)own * n_it + it0) * S::B_TILE, *w1 = sub.tc + ((size_t)t1 * n_it + it0) * S::B_TILE;
+        const uint8_t *sd0 = sub.tc + side + ((size_t)t0 * L.n_sb + tile.sb0) * side_step + (Q6 ? 0 : TC_MINOP_BYTES);  // d[128] of a super-block
+        const uint8_t *sd1 = sub.tc + side + ((size_t)t1 * L.n_sb + tile.sb0) * side_step + (Q6 ? 0 : TC_MINOP_BYTES);
+        uint32_t it = 0;
+        bool ok = true;
+        for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
+            for (uint32_t st = 0; st < (uint32_t)S::SB_STAGES; ++st, ++it) {
+                const uint32_t s = it % S::STAGES;
+                ok = warp_all(tma::mbar_wait_blocking(empty_ab + s, ((it / S::STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u));
+                // the d slot of this super-block was last read by the epilogue of super-block sb - 2
+                if (ok && st == 0 && sb >= 2) ok = warp_all(tma::mbar_wait_blocking(slot_free + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u));
+                if (!ok) break;
+                uint8_t *dst = tc_smem + s * S::STAGE;
+                tma::mbar_expect_tx_if(full_ab + s, S::STAGE + (st == 0 ? 2 * TC_BN * 4 : 0), me);
+                if constexpr (Q6) {
+                    // the 64-k activation stage it / 2 holds [high 16 KB | low 16 KB]; its k half it % 2 is 8 contiguous KB of each
+                    const uint8_t *a = img + (size_t)(it >> 1) * (2 * TC_OP_BYTES) + (it & 1) * S::OP;
+                    tma::bulk_g2s_if(dst, a, S::OP, full_ab + s, me);
+                    tma::bulk_g2s_if(dst + S::OP, a + TC_OP_BYTES, S::OP, full_ab + s, me);
+                } else {
                     tma::bulk_g2s_if(dst, img + (size_t)it * (2 * TC_OP_BYTES), 2 * TC_OP_BYTES, full_ab + s, me);
-                    tma::bulk_g2s_if(dst + 2 * TC_OP_BYTES, w0 + (size_t)it * TC_OP_BYTES, TC_OP_BYTES, full_ab + s, me);
-                    tma::bulk_g2s_if(dst + 3 * TC_OP_BYTES, w1 + (size_t)it * TC_OP_BYTES, TC_OP_BYTES, full_ab + s, me);
-                    if (st == 0) {
-                        uint8_t *dv = tc_smem + TCW_DVAL_OFF + (sb & 1) * (2 * TC_BN * 4);
-                        tma::bulk_g2s_if(dv, sd0 + (size_t)sb * TC_SIDE_BYTES, TC_BN * 4, full_ab + s, me);
-                        tma::bulk_g2s_if(dv + TC_BN * 4, sd1 + (size_t)sb * TC_SIDE_BYTES, TC_BN * 4, full_ab + s, me);
-                    }
                 }
-            }
-            const uint8_t *xm = p.xm + (size_t)tile.x * n_mit * (2 * TCW_MINT_BYTES);
-            const uint8_t *m0 = sub.tc + L.wmin + (size_t)t0 * n_mit * (2 * TCW_MINT_BYTES), *m1 = sub.tc + L.wmin + (size_t)t1 * n_mit * (2 * TCW_MINT_BYTES);
-            for (uint32_t mi = 0; mi < n_mit && ok && n_rounds > n_sb; ++mi, ++it) {
-                const uint32_t s = it % TCW_STAGES;
-                if (!warp_all(tma::mbar_wait_blocking(empty_ab + s, ((it / TCW_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u))) break;
-                uint8_t *dst = tc_smem + s * TCW_STAGE_BYTES;
-                tma::mbar_expect_tx_if(full_ab + s, 6 * TCW_MINT_BYTES + (mi == 0 ? 2 * TC_BN * 4 : 0), me);
-                tma::bulk_g2s_if(dst, xm + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s, me);
-                tma::bulk_g2s_if(dst + 2 * TCW_MINT_BYTES, m0 + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s, me);
-                tma::bulk_g2s_if(dst + 4 * TCW_MINT_BYTES, m1 + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s, me);
-                if (mi == 0) {  // 2^-s of the CTA's rows (read by the epilogue after the min GEMM)
-                    tma::bulk_g2s_if(tc_smem + TCW_RS_OFF, sub.tc + L.rscale + (size_t)t0 * TC_BN * 4, TC_BN * 4, full_ab + s, me);
-                    tma::bulk_g2s_if(tc_smem + TCW_RS_OFF + TC_BN * 4, sub.tc + L.rscale + (size_t)t1 * TC_BN * 4, TC_BN * 4, full_ab + s, me);
+                tma::bulk_g2s_if(dst + 2 * S::OP, w0 + (size_t)it * S::B_TILE, S::B_TILE, full_ab + s, me);
+                if constexpr (!PAIR) tma::bulk_g2s_if(dst + 2 * S::OP + S::B_TILE, w1 + (size_t)it * S::B_TILE, S::B_TILE, full_ab + s, me);
+                if (st == 0) {
+                    uint8_t *dv = tc_smem + S::DVAL + (sb & 1) * (2 * TC_BN * 4);
+                    tma::bulk_g2s_if(dv, sd0 + (size_t)sb * side_step, TC_BN * 4, full_ab + s, me);
+                    tma::bulk_g2s_if(dv + TC_BN * 4, sd1 + (size_t)sb * side_step, TC_BN * 4, full_ab + s, me);
                 }
             }
         }
+        if (!Q6 && n_rounds > n_sb) {
+            const uint8_t *xm = p.xm + (size_t)x_t * n_mit * (2 * TCW_MINT_BYTES);
+            const uint8_t *m0 = sub.tc + L.wmin + (size_t)own * n_mit * (2 * TCW_MINT_BYTES), *m1 = sub.tc + L.wmin + (size_t)t1 * n_mit * (2 * TCW_MINT_BYTES);
+            for (uint32_t mi = 0; mi < n_mit && ok; ++mi, ++it) {
+                const uint32_t s = it % S::STAGES;
+                if (!warp_all(tma::mbar_wait_blocking(empty_ab + s, ((it / S::STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u))) break;
+                uint8_t *dst = tc_smem + s * S::STAGE;
+                tma::mbar_expect_tx_if(full_ab + s, (2 + 2 * S::B_TILES) * TCW_MINT_BYTES + (mi == 0 ? 2 * TC_BN * 4 : 0), me);
+                tma::bulk_g2s_if(dst, xm + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s, me);
+                tma::bulk_g2s_if(dst + 2 * TCW_MINT_BYTES, m0 + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s, me);
+                if constexpr (!PAIR) tma::bulk_g2s_if(dst + 4 * TCW_MINT_BYTES, m1 + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s, me);
+                if (mi == 0) {  // 2^-s of the CTA's rows (read by the epilogue after the min GEMM)
+                    tma::bulk_g2s_if(tc_smem + S::RS, sub.tc + L.rscale + (size_t)t0 * TC_BN * 4, TC_BN * 4, full_ab + s, me);
+                    tma::bulk_g2s_if(tc_smem + S::RS + TC_BN * 4, sub.tc + L.rscale + (size_t)t1 * TC_BN * 4, TC_BN * 4, full_ab + s, me);
+                }
+            }
+        }
+        // This CTA's shared memory must outlive the last products' arrivals on its barriers (which come after its copies) and, where something gave
+        // up, the copies in flight: the wait then runs out.
+        if (PAIR)
+            for (uint32_t i = it > (uint32_t)S::STAGES ? it - S::STAGES : 0; i < it; ++i)
+                for (uint32_t n = 0; n < tma::SPIN_LIMIT && !tma::mbar_test(empty_ab + i % S::STAGES, (i / S::STAGES) & 1); ++n) __nanosleep(40);
     } else {
         // ---------------------------------------------------------------- epilogue: thread = (token lane, 128 rows of one image tile)
         const uint32_t e = warp - 2, quad = warp & 3, hh = e >> 2;  // a warp reaches TMEM lanes [32 (warp % 4), +32)
@@ -564,10 +612,10 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
                 break;
             }
             tc_fence_after();
-            if (sb == 0) ginv = __ldg(p.ginv + col0 + tl);
+            if (sb == 0) ginv = __ldg(p.ginv + min(col0 + tl, p.n - 1));
             // per super-block: out += d[row] * D / g; after the min GEMM: out -= 2^-s[row] * Dmin / g
-            const float *fac = sb < n_sb ? reinterpret_cast<const float *>(tc_smem + TCW_DVAL_OFF + buf * (2 * TC_BN * 4)) + hh * TC_BN
-                                         : reinterpret_cast<const float *>(tc_smem + TCW_RS_OFF) + hh * TC_BN;
+            const float *fac = sb < n_sb ? reinterpret_cast<const float *>(tc_smem + S::DVAL + buf * (2 * TC_BN * 4)) + hh * TC_BN
+                                         : reinterpret_cast<const float *>(tc_smem + S::RS) + hh * TC_BN;
             const float gs = sb < n_sb ? ginv : -ginv;
 #pragma unroll
             for (uint32_t c = 0; c < TC_BN / 32; ++c) {
@@ -590,10 +638,13 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) tma::mbar_arrive(empty_d + buf);  // the accumulator buffer and the d slot are free again
+            if (lane == 0) {  // the accumulator buffer and the d slot are free again
+                if constexpr (PAIR) tma::mbar_arrive_cluster(tma::smem_of_rank(empty_d + buf, 0));
+                tma::mbar_arrive(slot_free + buf);
+            }
         }
         if (ok && tile.slot != TC_WHOLE) {
-            float *o = p.partial + (size_t)tile.slot * (2 * TC_BN * TC_BM) + hh * TC_BN * TC_BM + tl;
+            float *o = p.partial + (size_t)(PAIR ? 2 * tile.slot + rank : tile.slot) * (2 * TC_BN * TC_BM) + hh * TC_BN * TC_BM + tl;
 #pragma unroll
             for (int i = 0; i < TC_BN; ++i) o[i * TC_BM] = acc[i];
         } else if (ok && col0 + tl < p.n) {
@@ -623,7 +674,15 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) {
+    if constexpr (PAIR) {
+        cluster_barrier();  // the other CTA's products read this one's shared memory, its warps arrive here
+        if (warp == 0) {
+            tc_fence_after();
+            tmem_dealloc_pair(tmem, TC_TMEM_COLS);
+        }
+        __syncwarp();
+        cluster_barrier();  // neither leaves before both have given back
+    } else if (warp == 0) {
         __syncwarp();
         tc_fence_after();
         tmem_dealloc(tmem, TC_TMEM_COLS);
@@ -639,7 +698,7 @@ __global__ void __launch_bounds__(IMG ? TC_THREADS_IMG : TC_THREADS, 1) gemm_tc_
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * TC_STAGES + 4);
     volatile uint32_t *abort_flag = tmem_slot + 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const TcTile tile = tc_tile(p);
+    const TcTile tile = tc_tile(p, blockIdx.x);
     const TcSub sub = tc_select(p, tile.y);
     const uint32_t col0 = tile.x * TC_BM, row0 = sub.by * TC_BN;
     const uint32_t k_sb = p.k / 256, n_sb = tile.n_sb, n_it = n_sb * TC_STAGES;  // loops count the super-blocks of this CTA
@@ -921,13 +980,8 @@ int32_t launch_tc_typed(const TcParams &p, uint32_t ctas, cudaStream_t st) {
 // activations high, even part x activations low, low bit x activations high (low bit x activations low is below 2^-22
 // of the sum) - and the epilogue is out += d * D / g per super-block (Q6_K has no min term).  128 tokens x 128 rows per
 // CTA, stages of 32 k (activations 2 x 8 KB out of the 64-k tiles of tc_token_image_kernel, weights 16 KB), six stages.
-constexpr int TC6_KS = 32, TC6_STAGES = 6;
-constexpr uint32_t TC6_HALF = TC_OP_BYTES / 2;                 // one operand tile of a 32-k stage: 8 KB
-constexpr uint32_t TC6_STAGE_BYTES = 4 * TC6_HALF;             // A high, A low, B even, B low bit
-constexpr uint32_t TC6_DVAL_OFF = TC6_STAGES * TC6_STAGE_BYTES;
-constexpr uint32_t TC6_TAIL_OFF = TC6_DVAL_OFF + 2 * TC_BN * 4;
-constexpr uint32_t TC6_SMEM_BYTES = TC6_TAIL_OFF + 256;
-constexpr uint32_t TC6_TMEM_COLS = 256;
+constexpr int TC6_KS = Wide<true, true>::KS;
+constexpr uint32_t TC6_HALF = TC_OP_BYTES / 2;  // one operand tile of a 32-k stage: 8 KB
 
 // Image of a Q6_K weight: per (128-row tile, 32-k stage) [even part 8 KB | low bit 8 KB], then per (tile, super-block)
 // d[128].  grid (k / 32, tiles), thread = row.
@@ -966,193 +1020,23 @@ __global__ void __launch_bounds__(TC_BN) tc_weight_image6_kernel(const WeightVie
     if ((xb & 7) == 0) dvals[((size_t)tile * n_sb + sb) * TC_BN + r] = h2f(__ldg(reinterpret_cast<const uint16_t *>(w.d) + sbi));
 }
 
-__global__ void __launch_bounds__(TC_THREADS_IMG, 1) gemm_tc6_kernel(const TcParams p) {
-    extern __shared__ __align__(1024) uint8_t tc_smem[];
-    uint64_t *bars = reinterpret_cast<uint64_t *>(tc_smem + TC6_TAIL_OFF);
-    uint64_t *full_ab = bars, *empty_ab = bars + TC6_STAGES, *full_d = bars + 2 * TC6_STAGES, *empty_d = full_d + 2;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * TC6_STAGES + 4);
-    volatile uint32_t *abort_flag = tmem_slot + 1;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const TcTile tile = tc_tile(p);
-    const uint32_t col0 = tile.x * TC_BM, row0 = tile.y * TC_BN;
-    const uint32_t k_sb = p.k / 256, n_sb = tile.n_sb, n_it = n_sb * 8, tiles_m = (p.m + TC_BN - 1) / TC_BN;
-    if (tid == 0) {
-        for (int s = 0; s < TC6_STAGES; ++s) {
-            tma::mbar_init(full_ab + s, 1);
-            tma::mbar_init(empty_ab + s, 1);
-        }
-        for (int b = 0; b < 2; ++b) {
-            tma::mbar_init(full_d + b, 1);
-            tma::mbar_init(empty_d + b, TC_EPI_WARPS);
-        }
-        *abort_flag = 0;
-        tma::mbar_init_fence();
-    }
-    if (warp == 0) {
-        tmem_alloc(tmem_slot, TC6_TMEM_COLS);
-        tmem_relinquish();
-    }
-    pdl_trigger();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
-    pdl_wait();
-
-    if (warp == 0) {
-        // ---- MMA issue (the whole warp, one lane issues)
-        const uint32_t idesc = tc_idesc(TC_BM, TC_BN), me = elect_one();
-        bool ok = true;
-        uint32_t it = 0;
-        for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
-            const uint32_t buf = sb & 1, d0 = tmem + buf * TC_BN;
-            if (!warp_all(tma::mbar_wait_blocking(empty_d + buf, ((sb >> 1) & 1) ^ 1, abort_flag, &g_tc_status, 2u))) break;
-            tc_fence_after();
-            for (uint32_t st = 0; st < 8; ++st, ++it) {
-                const uint32_t s = it % TC6_STAGES;
-                ok = warp_all(tma::mbar_wait_blocking(full_ab + s, (it / TC6_STAGES) & 1, abort_flag, &g_tc_status, 1u));
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t base = tma::smem_u32(tc_smem + s * TC6_STAGE_BYTES);
-                const uint64_t ah = smem_desc(base, TC_KC_STRIDE, 128), al = smem_desc(base + TC6_HALF, TC_KC_STRIDE, 128),
-                               be = smem_desc(base + 2 * TC6_HALF, TC_KC_STRIDE, 128), bl = smem_desc(base + 3 * TC6_HALF, TC_KC_STRIDE, 128);
-#pragma unroll
-                for (uint32_t ks = 0; ks < TC6_KS / 16; ++ks) {
-                    const uint32_t o = 2 * ks * TC_KC_STRIDE / 16;  // address fields count 16 bytes
-                    tc_mma_f16(d0, ah + o, be + o, idesc, (st | ks) != 0, me);
-                    tc_mma_f16(d0, al + o, be + o, idesc, 1, me);
-                    tc_mma_f16(d0, ah + o, bl + o, idesc, 1, me);
-                }
-                tc_commit(empty_ab + s, me);
-            }
-            if (ok) tc_commit(full_d + buf, me);
-        }
-    } else if (warp == 1) {
-        {  // ---- operands (bulk asynchronous copies; the whole warp, one lane asks)
-            const uint32_t me = elect_one();
-            const size_t w_sb = (size_t)tile.y * k_sb + tile.sb0;
-            const uint8_t *img = p.img + ((size_t)tile.x * k_sb + tile.sb0) * (256 / TC_KS) * (2 * TC_OP_BYTES);
-            const uint8_t *wimg = p.w.tc + w_sb * 8 * (2 * TC6_HALF);
-            const uint8_t *dv = p.w.tc + (size_t)tiles_m * k_sb * 8 * (2 * TC6_HALF) + w_sb * (TC_BN * 4);
-            for (uint32_t it = 0; it < n_it; ++it) {
-                const uint32_t s = it % TC6_STAGES, sb = it >> 3, st = it & 7;
-                if (!warp_all(tma::mbar_wait_blocking(empty_ab + s, ((it / TC6_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u))) break;
-                if (st == 0 && sb >= 2 && !warp_all(tma::mbar_wait_blocking(empty_d + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u))) break;
-                uint8_t *dst = tc_smem + s * TC6_STAGE_BYTES;
-                // the 64-k activation stage it / 2 holds [high 16 KB | low 16 KB]; its k half it % 2 is 8 contiguous KB of each
-                const uint8_t *a = img + (size_t)(it >> 1) * (2 * TC_OP_BYTES) + (it & 1) * TC6_HALF;
-                tma::mbar_expect_tx_if(full_ab + s, TC6_STAGE_BYTES + (st == 0 ? TC_BN * 4 : 0), me);
-                tma::bulk_g2s_if(dst, a, TC6_HALF, full_ab + s, me);
-                tma::bulk_g2s_if(dst + TC6_HALF, a + TC_OP_BYTES, TC6_HALF, full_ab + s, me);
-                tma::bulk_g2s_if(dst + 2 * TC6_HALF, wimg + (size_t)it * (2 * TC6_HALF), 2 * TC6_HALF, full_ab + s, me);
-                if (st == 0) tma::bulk_g2s_if(tc_smem + TC6_DVAL_OFF + (sb & 1) * (TC_BN * 4), dv + (size_t)sb * (TC_BN * 4), TC_BN * 4, full_ab + s, me);
-            }
-        }
-    } else {
-        // ---- epilogue: thread = (token lane, 64 rows), the running output in registers
-        const uint32_t e = warp - 2, quad = warp & 3, ch = e >> 2;
-        const uint32_t tl = quad * 32 + lane;
-        const uint32_t lane_addr = tmem + ((quad * 32) << 16);
-        float acc[64];
-#pragma unroll
-        for (int i = 0; i < 64; ++i) acc[i] = 0.0f;
-        float ginv = 1.0f;
-        bool ok = true;
-        for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
-            const uint32_t buf = sb & 1;
-            if (!tma::mbar_wait_blocking(full_d + buf, (sb >> 1) & 1, abort_flag, &g_tc_status, 16u)) {
-                ok = false;
-                break;
-            }
-            tc_fence_after();
-            if (sb == 0) ginv = __ldg(p.ginv + col0 + tl);
-            const float *dval = reinterpret_cast<const float *>(tc_smem + TC6_DVAL_OFF + buf * (TC_BN * 4));
-#pragma unroll
-            for (uint32_t c2 = 0; c2 < 2; ++c2) {
-                const uint32_t col = ch * 64 + c2 * 32;
-                uint32_t v0[16], v1[16];
-                tmem_ld16(lane_addr + buf * TC_BN + col, v0);
-                tmem_ld16(lane_addr + buf * TC_BN + col + 16, v1);
-                tmem_wait_ld();
-                const float4 *dq = reinterpret_cast<const float4 *>(dval + col);
-#pragma unroll
-                for (int q4 = 0; q4 < 8; ++q4) {
-                    const float4 dv = dq[q4];
-                    const float dvv[4] = {dv.x, dv.y, dv.z, dv.w};
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int j = q4 * 4 + i;
-                        const float dd = __uint_as_float(j < 16 ? v0[j & 15] : v1[j & 15]);
-                        acc[c2 * 32 + j] = fmaf(dvv[i] * dd, ginv, acc[c2 * 32 + j]);
-                    }
-                }
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) tma::mbar_arrive(empty_d + buf);
-        }
-        if (ok && tile.slot != TC_WHOLE) {
-            float *o = p.partial + (size_t)tile.slot * (TC_BN * TC_BM) + ch * 64 * TC_BM + tl;
-#pragma unroll
-            for (int i = 0; i < 64; ++i) o[i * TC_BM] = acc[i];
-        } else if (ok && col0 + tl < p.n) {
-            float *o = p.out + (size_t)(row0 + ch * 64) * p.ldy + (size_t)(col0 + tl) * p.ldc;
-            if (p.ldy == 1 && row0 + ch * 64 + 64 <= p.m && ((uintptr_t)o & 15) == 0) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    float4 v = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
-                    float4 *o4 = reinterpret_cast<float4 *>(o) + i;
-                    if (p.epilogue == EPI_ADD) {
-                        const float4 c = *o4;
-                        v = make_float4(__fadd_rn(c.x, v.x), __fadd_rn(c.y, v.y), __fadd_rn(c.z, v.z), __fadd_rn(c.w, v.w));
-                    }
-                    *o4 = v;
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 64; ++i)
-                    if (row0 + ch * 64 + i < p.m) {
-                        float *oi = o + (size_t)i * p.ldy;
-                        *oi = p.epilogue == EPI_ADD ? __fadd_rn(*oi, acc[i]) : acc[i];
-                    }
-            }
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 0) {
-        __syncwarp();
-        tc_fence_after();
-        tmem_dealloc(tmem, TC6_TMEM_COLS);
-    }
-}
-
-int32_t launch_tc6(const TcParams &p, uint32_t ctas, cudaStream_t st) {
-    static thread_local int configured_dev = -1;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (configured_dev != dev) {
-        CERA_CUDA_TRY(cudaFuncSetAttribute(gemm_tc6_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC6_SMEM_BYTES));
-        configured_dev = dev;
-    }
-    count_launch();
-    return check_cuda(launch_k(gemm_tc6_kernel, dim3(ctas), dim3(TC_THREADS_IMG), (size_t)TC6_SMEM_BYTES, st, p), "gemm (tcgen05, Q6_K) launch");
-}
-
-// Adds the parts of the tiles that several CTAs share, in order, and stores as those kernels do.  CTA = 32 rows x 32 tokens of a tile of `rows` rows,
-// turned in shared memory so that both sides are coalesced.  grid (tiles shared, rows / 32, 4).
-__global__ void __launch_bounds__(256) tc_parts_kernel(const TcParams p, uint32_t rows) {
+// Adds the parts of the tiles that several CTAs (or pairs of them, `halves` 2) share, in order, and stores as those kernels do.  CTA = 32 rows x 32
+// tokens of a tile of `rows` rows, turned in shared memory so that both sides are coalesced.  grid (tiles shared, rows / 32, 4 halves).
+__global__ void __launch_bounds__(256) tc_parts_kernel(const TcParams p, uint32_t rows, uint32_t halves) {
     __shared__ float cells[32][33];
     pdl_trigger();
     pdl_wait();
-    const uint32_t t = p.whole + blockIdx.x, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const uint32_t t = p.whole + blockIdx.x, tx = threadIdx.x & 31, ty = threadIdx.x >> 5, half = blockIdx.z / (TC_BM / 32), z = blockIdx.z % (TC_BM / 32);
     const TcSub sub = tc_select(p, t / p.x_tiles);
-    const uint32_t col0 = t % p.x_tiles * TC_BM + blockIdx.z * 32, row0 = sub.by * rows + blockIdx.y * 32;
-    const float *v = p.partial + (size_t)blockIdx.x * p.parts * rows * TC_BM + (size_t)blockIdx.y * 32 * TC_BM + blockIdx.z * 32 + tx;
+    const uint32_t col0 = (t % p.x_tiles * halves + half) * TC_BM + z * 32, row0 = sub.by * rows + blockIdx.y * 32;
+    if (col0 >= p.n || row0 >= sub.m) return;
+    const size_t tile = (size_t)rows * TC_BM;
+    const float *v = p.partial + ((size_t)blockIdx.x * p.parts * halves + half) * tile + (size_t)blockIdx.y * 32 * TC_BM + z * 32 + tx;
     float sum[4] = {};
+#pragma unroll 4
     for (uint32_t part = 0; part < p.parts; ++part)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) sum[i] += v[(size_t)part * rows * TC_BM + (ty + 8 * i) * TC_BM];
+        for (int i = 0; i < 4; ++i) sum[i] += v[part * halves * tile + (ty + 8 * i) * TC_BM];
 #pragma unroll
     for (int i = 0; i < 4; ++i) cells[ty + 8 * i][tx] = sum[i];
     __syncthreads();
@@ -1167,28 +1051,37 @@ __global__ void __launch_bounds__(256) tc_parts_kernel(const TcParams p, uint32_
     }
 }
 
-// The last round of a grid of `tiles` tiles over `sms` SMs, a CTA each: how many tiles it has and how many CTAs share one of them along k (1: no
-// sharing).  A round that fills less than half the SMs is shared out; with more in it a tile could not have two CTAs.  Each share is a
-// super-block at least.  448 tiles of k = 4096 (gate / up of 512 tokens, three rounds and four tiles): 280 us before, 212 now.
+// A grid of `tiles` tiles over `slots` SMs (or pairs), one each at a time: whole rounds first; the tiles of the last one, when it does not fill the
+// device, are each shared by `parts` along k, as many as make the round shortest: rounds of the shares / parts, and a fiftieth of a round for what
+// each share adds (its start, its partial sums).  448 tiles of 128 x 256 on 148 SMs, k = 4096 (gate / up of 512 tokens: three rounds and four tiles):
+// 280 us whole, 212 shared; 32 tiles of 128 x 128 (4096 x 64 x 4096, the whole product) 63 us whole, 35 in eight shares each.
+constexpr uint32_t TC_SHARES = 3;  // partial tiles a slot has room for
 struct TcSplit {
     uint32_t left, parts;
 };
-TcSplit tc_split(uint32_t tiles, uint32_t n_sb, uint32_t sms) {
-    const uint32_t left = tiles % sms;
-    if (tiles < sms || left == 0 || 2 * left > sms || n_sb < 8) return {0, 1};
-    return {left, std::min(std::min(n_sb, sms / left), 16u)};
+TcSplit tc_split(uint32_t tiles, uint32_t n_sb, uint32_t slots) {
+    const uint32_t left = tiles % slots;
+    uint32_t best = 50, parts = 1;  // fiftieths of a round
+    for (uint32_t s = 2; left && s <= std::min(n_sb / 2, 16u) && left * s <= TC_SHARES * slots; ++s) {
+        const uint32_t cost = (50 * ((left * s + slots - 1) / slots) + s - 1) / s + s;
+        if (cost < best) best = cost, parts = s;
+    }
+    return parts > 1 ? TcSplit{left, parts} : TcSplit{0, 1};
 }
 
-int32_t launch_tc_wide(const TcParams &p, uint32_t ctas, cudaStream_t st) {
+template <bool Q6, bool PAIR>
+int32_t launch_tc_wide(const TcParams &p, uint32_t tiles, cudaStream_t st) {
+    using S = Wide<Q6, PAIR>;
     static thread_local int configured_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_dev != dev) {
-        CERA_CUDA_TRY(cudaFuncSetAttribute(gemm_tcw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TCW_SMEM_BYTES));
+        CERA_CUDA_TRY(cudaFuncSetAttribute(gemm_tcw_kernel<Q6, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
         configured_dev = dev;
     }
     count_launch();
-    return check_cuda(launch_k(gemm_tcw_kernel, dim3(ctas), dim3(TCW_THREADS), (size_t)TCW_SMEM_BYTES, st, p), "gemm (tcgen05, wide) launch");
+    if (PAIR) return check_cuda(launch_pairs(gemm_tcw_kernel<Q6, PAIR>, tiles, dim3(TCW_THREADS), (size_t)S::SMEM, st, p), "gemm (tcgen05, pairs) launch");
+    return check_cuda(launch_k(gemm_tcw_kernel<Q6, PAIR>, dim3(tiles), dim3(TCW_THREADS), (size_t)S::SMEM, st, p), "gemm (tcgen05, wide) launch");
 }
 
 }  // namespace
@@ -1258,7 +1151,7 @@ static const bool g_tc_status_registered = register_kernel_status([] {
     return (uint32_t)v << 8;
 });
 
-size_t gemm_parts_bytes() { return (size_t)sm_count() * (2 * TC_BN * TC_BM * 4); }
+size_t gemm_parts_bytes() { return (size_t)TC_SHARES * sm_count() * (2 * TC_BN * TC_BM * 4); }
 
 // One activation matrix against up to three weights (q / k / v, gate / up): the activation operands are converted once
 // and, when every weight has its image, ONE kernel launch covers all of them (the small matrices' CTAs run beside the
@@ -1286,32 +1179,35 @@ int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, s
     const size_t img_bytes = (size_t)tiles * n_it * (2 * TC_OP_BYTES), min_bytes = (size_t)tiles * n_sb * TC_MINOP_BYTES,
                  xm_bytes = (size_t)tiles * n_mit * (2 * TCW_MINT_BYTES);
     const size_t need = img_bytes + min_bytes + xm_bytes + (size_t)n_pad * 8;
-    // with weight images: the wide kernel when its 128 x 256 tiles alone fill the device, else the 128 x 128 one
+    // With weight images: the wide kernel when its 128 x 256 tiles alone fill the device, in pairs unless they would leave a quarter of their tokens
+    // empty (one or three token tiles); else the 128 x 128 one.  Whole products, 128 x 128, wide, pairs: 28672 x 4096 x 512 255, 227, 204 us;
+    // 6144 x 2047 228, 222, 200; 4096 x 384 57, 52, 55; 4096 x 512 58, 60, 63.  Q6_K takes pairs at every size it has.
     static const int tile_pref = [] {
         const char *e = getenv("CERA_CUDA_GEMM_TILE");
         return e ? atoi(e) : 0;
     }();
     uint32_t wide_y = 0;
     for (int i = 0; i < count; ++i) wide_y += (t[i].w.m + 2 * TC_BN - 1) / (2 * TC_BN);
-    const bool wide = w.tc && w.type != CERA_TYPE_Q6_K && (tile_pref == 256 || (tile_pref != 128 && tiles * wide_y >= 120));
-    const uint32_t rows = wide ? 2 * TC_BN : TC_BN;
+    const bool q6 = w.type == CERA_TYPE_Q6_K, fills = tiles * wide_y >= 120, pair = q6 || (w.tc && tile_pref == 0 && fills && (tiles % 2 == 0 || tiles >= 5));
+    const bool wide = !pair && w.tc && (tile_pref == 256 || (tile_pref != 128 && fills));
+    const uint32_t rows = pair || wide ? 2 * TC_BN : TC_BN, halves = pair ? 2 : 1, x_tiles = (tiles + halves - 1) / halves;
     uint32_t y = 0;
     for (int i = 0; i < count; ++i) y += (t[i].w.m + rows - 1) / rows;
-    // partial sums of the last round's tiles; without room for them the tiles stay whole
-    TcSplit split = w.tc ? tc_split(tiles * y, n_sb, (uint32_t)sm_count()) : TcSplit{0, 1};
-    const size_t parts_bytes = (size_t)split.left * split.parts * rows * TC_BM * 4;
+    TcSplit split = w.tc ? tc_split(x_tiles * y, n_sb, (uint32_t)sm_count() / halves) : TcSplit{0, 1};
+    // partial sums of the tiles that are shared; without room for them the tiles stay whole
+    const size_t parts_bytes = (size_t)split.left * split.parts * halves * rows * TC_BM * 4;
     const bool borrowed = lent.p && lent.bytes >= need;
     uint8_t *scratch = (uint8_t *)lent.p;
+    float *partial = nullptr;
     if (borrowed) {
-        if (lent.bytes < need + parts_bytes) split = {0, 1};
+        if (lent.parts_bytes >= parts_bytes) partial = (float *)lent.parts;
     } else {
         scratch = (uint8_t *)scratch_alloc(need + parts_bytes, st);
-        if (!scratch && split.left) {
-            split = {0, 1};
-            scratch = (uint8_t *)scratch_alloc(need, st);
-        }
+        if (scratch) partial = reinterpret_cast<float *>(scratch + need);
+        else if (split.left) scratch = (uint8_t *)scratch_alloc(need, st);
         if (!scratch) return CERA_CUDA_OK;  // no room for the operand scratch: leave the GEMM to the kernels that need none
     }
+    if (!partial) split = {0, 1};
     uint8_t *xm = scratch + img_bytes + min_bytes;
     float *g_tab = reinterpret_cast<float *>(xm + xm_bytes), *ginv_tab = g_tab + n_pad;
     // the last min stage's columns beyond k / 32 are zero (never written by the image kernel)
@@ -1349,24 +1245,24 @@ int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, s
             p.ldc_x[i - 1] = (uint32_t)t[i].ldc;
         }
     }
-    p.x_tiles = tiles;
-    p.whole = tiles * y - split.left;
+    p.x_tiles = x_tiles;
+    p.whole = x_tiles * y - split.left;
     p.parts = split.parts;
-    p.partial = reinterpret_cast<float *>(scratch + need);
-    const uint32_t ctas = p.whole + split.left * split.parts;
-    if (rc == CERA_CUDA_OK && w.type == CERA_TYPE_Q6_K) {
-        rc = launch_tc6(p, ctas, st);
+    p.partial = partial;
+    const uint32_t work = p.whole + split.left * split.parts;
+    if (rc == CERA_CUDA_OK && pair) {
+        rc = q6 ? launch_tc_wide<true, true>(p, work, st) : launch_tc_wide<false, true>(p, work, st);
     } else if (rc == CERA_CUDA_OK && wide) {
-        rc = launch_tc_wide(p, ctas, st);
+        rc = launch_tc_wide<false, false>(p, work, st);
     } else if (rc == CERA_CUDA_OK) {
         if (w.tc)
-            rc = w.type == CERA_TYPE_Q4_K ? launch_tc_typed<CERA_TYPE_Q4_K, true>(p, ctas, st) : launch_tc_typed<CERA_TYPE_Q5_K, true>(p, ctas, st);
+            rc = w.type == CERA_TYPE_Q4_K ? launch_tc_typed<CERA_TYPE_Q4_K, true>(p, work, st) : launch_tc_typed<CERA_TYPE_Q5_K, true>(p, work, st);
         else
-            rc = w.type == CERA_TYPE_Q4_K ? launch_tc_typed<CERA_TYPE_Q4_K, false>(p, ctas, st) : launch_tc_typed<CERA_TYPE_Q5_K, false>(p, ctas, st);
+            rc = w.type == CERA_TYPE_Q4_K ? launch_tc_typed<CERA_TYPE_Q4_K, false>(p, work, st) : launch_tc_typed<CERA_TYPE_Q5_K, false>(p, work, st);
     }
     if (rc == CERA_CUDA_OK && split.left) {
         count_launch();
-        rc = check_cuda(launch_k(tc_parts_kernel, dim3(split.left, rows / 32, TC_BM / 32), dim3(256), 0, st, p, rows), "gemm (tcgen05) parts launch");
+        rc = check_cuda(launch_k(tc_parts_kernel, dim3(split.left, rows / 32, halves * (TC_BM / 32)), dim3(256), 0, st, p, rows, halves), "gemm (tcgen05) parts launch");
     }
     if (!borrowed) cudaFreeAsync(scratch, st);  // after the kernels above, in stream order
     return rc;

@@ -108,6 +108,7 @@ struct LlamaModel : cera_cuda_model {
     float *pf_hidden = nullptr, *pf_q = nullptr, *pf_k = nullptr, *pf_v = nullptr, *pf_attn = nullptr, *pf_g = nullptr,
           *pf_u = nullptr;
     float *pf_attn_local = nullptr;  // = pf_attn (every rank computes all heads)
+    void *pf_parts = nullptr;        // the products' partial sums (null: no room)
     ActBuf pf_act_hs, pf_act_q, pf_act_ff;
     bool has_lora = false;
     float *normed = nullptr;       // f32 copy of the normed hidden state, written only while adapters are attached
@@ -388,8 +389,9 @@ int32_t llama_chunk(LlamaModel *m, const uint32_t *tokens, size_t n, size_t star
     // layer's, and the queries', used up by the attention.  (Tensor parallel: peers write into the former at any time.)
     GemmScratch in_g, in_q;
     if (!tp) {
-        in_g = {m->pf_g, pf_lent_bytes(m->pf_chunk, ff)};
-        in_q = {m->pf_q, pf_lent_bytes(m->pf_chunk, qd) + gemm_parts_bytes()};
+        const size_t parts = m->pf_parts ? gemm_parts_bytes() : 0;
+        in_g = {m->pf_g, pf_lent_bytes(m->pf_chunk, ff), m->pf_parts, parts};
+        in_q = {m->pf_q, pf_lent_bytes(m->pf_chunk, qd), m->pf_parts, parts};
     }
     if (tp) CERA_TRY(launch_tp_tick(m->tp_words, st));
     CERA_CUDA_TRY(cudaMemcpyAsync(m->pf_tokens, tokens, n * 4, cudaMemcpyHostToDevice, st));
@@ -618,7 +620,7 @@ int32_t LlamaModel::build() {
     }
     {
         const size_t C = m->pf_chunk;
-        CERA_TRY(m->dev_alloc((void **)&m->pf_q, pf_lent_bytes(C, m->l_qd) + (m->tp_size == 1 ? gemm_parts_bytes() : 0)));
+        CERA_TRY(m->dev_alloc((void **)&m->pf_q, pf_lent_bytes(C, m->l_qd)));
         CERA_TRY(m->dev_alloc((void **)&m->pf_k, C * m->l_kvd * 4));
         CERA_TRY(m->dev_alloc((void **)&m->pf_v, C * m->l_kvd * 4));
         if (m->tp_size == 1) {
@@ -626,6 +628,10 @@ int32_t LlamaModel::build() {
             CERA_TRY(m->dev_alloc((void **)&m->pf_attn, C * qd * 4));
             CERA_TRY(m->dev_alloc((void **)&m->pf_g, pf_lent_bytes(C, ff)));
             CERA_TRY(m->dev_alloc((void **)&m->pf_u, C * ff * 4));
+            if (std::max(hs, ff) >= 1024 && m->dev_alloc(&m->pf_parts, gemm_parts_bytes()) != CERA_CUDA_OK) {
+                m->pf_parts = nullptr;
+                cudaGetLastError();
+            }
             m->pf_attn_local = m->pf_attn;
         } else {
             m->pf_attn_local = m->pf_attn;  // (the chunk-wide buffers sit in the exchange region)

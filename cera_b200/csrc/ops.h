@@ -61,9 +61,10 @@ void scratch_trim();
 struct GemmScratch {
     void *p = nullptr;
     size_t bytes = 0;
+    void *parts = nullptr;  // partial sums of tiles that several CTAs share; optional
+    size_t parts_bytes = 0;
 };
-// Most that the tensor-core product adds to its operands for the partial sums of tiles that several CTAs share (a tile of 128 x 256 per SM).
-size_t gemm_parts_bytes();
+size_t gemm_parts_bytes();  // as many as a tensor-core product makes
 int32_t launch_gemm_ex(const WeightView &w, const ActView &x, size_t n, float *out, size_t ldy, size_t ldc, int epilogue,
                        cudaStream_t st, GemmScratch lent = {});
 // Register-resident-activation single-column GEMV.  *taken = false: shape outside its rules,

@@ -93,28 +93,12 @@ __device__ __forceinline__ uint32_t smem_of_rank(const void *p, uint32_t rank) {
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
     return a;
 }
+// What is handed over with it is no memory that threads wrote: copies that have landed, TMEM that has been read.  So the plain form does; with
+// .release.cluster here and .acquire.cluster in the waits each hand-over of a stage took some 700 cycles (512 tokens x 4096 x 14336: 190 us, 118 so).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// mbar_wait_blocking for a barrier that threads of other CTAs arrive on.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity, volatile uint32_t *abort_flag, unsigned int *status, unsigned int who) {
-    for (uint32_t i = 0; i < (SPIN_LIMIT >> 4); ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity)
-            : "memory");
-        if (ok) return true;
-        if (*abort_flag) return false;
-    }
-    *abort_flag = 1;
-    atomicOr(status, who);
-    return false;
-}
-// ---- the same for a warp that runs a loop of requests together, issued by the lane for which `me` is true (see tc_mma_f16) ----
+// ---- for a warp that runs a loop of requests together, issued by the lane for which `me` is true (see tc_mma_f16) ----
 __device__ __forceinline__ void mbar_expect_tx_if(uint64_t *bar, uint32_t bytes, uint32_t me) {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)), "r"(bytes), "r"(me)
                  : "memory");
