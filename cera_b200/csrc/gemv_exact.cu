@@ -135,7 +135,8 @@ __host__ __device__ inline size_t xg_warp_smem(uint32_t stages, uint32_t seg_byt
     return (size_t)stages * seg_bytes + 2 * XG_SCT_BYTES + 2 * XG_TERM_BYTES;
 }
 
-template <int T, bool TEAM, int BOUND>
+// QX: the column comes as f32 and is quantized here (code of its own, which the decode step's many small launches would have to load for nothing).
+template <int T, bool TEAM, int BOUND, bool QX>
 __global__ void __launch_bounds__(BOUND, 1) gemv_exact_kernel(const ExactParams p) {
     using L = SegLayout<T>;
     extern __shared__ __align__(128) uint8_t xg_smem[];
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(BOUND, 1) gemv_exact_kernel(const ExactParams 
             }
             if ((lane & 3) == 0) a16[v >> 2] = (float)(int)(int16_t)s4;
         }
-    } else if (p.f.quant_x) {
+    } else if (QX) {
         for (uint32_t v = tid; v < k / 4; v += nthreads) {  // whole warps: k is a multiple of 512
             const float4 xv = reinterpret_cast<const float4 *>(p.f.quant_x)[v];
             const float e[4] = {xv.x, xv.y, xv.z, xv.w};
@@ -570,6 +571,21 @@ __global__ void __launch_bounds__(BOUND, 1) gemv_exact_kernel(const ExactParams 
     }
 }
 
+template <int T, bool QX>
+int32_t launch_exact_column(const ExactParams &p, uint32_t grid, uint32_t P, size_t smem, bool teams, cudaStream_t st) {
+    void (*const team)(ExactParams) = gemv_exact_kernel<T, true, XG_MAX_WARPS * 32, QX>, (*const wide)(ExactParams) = gemv_exact_kernel<T, false, XG_WIDE_BOUND, QX>,
+                 (*const full)(ExactParams) = gemv_exact_kernel<T, false, XG_LONE_MAX_WARPS * 32, QX>;
+    static thread_local int raised_dev = -1;  // per instantiation: opt in to more than 48 KB once per device
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (raised_dev != dev) {
+        for (auto k : {team, wide, full}) CERA_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XG_SMEM_LIMIT));
+        raised_dev = dev;
+    }
+    count_launch();
+    return check_cuda(launch_k(teams ? team : P <= (uint32_t)XG_WIDE_WARPS ? wide : full, dim3(grid), dim3(P * 32), smem, st, p), "gemv (reference order) launch");
+}
+
 template <int T>
 int32_t launch_exact_typed(const ExactParams &p0, cudaStream_t st) {
     using L = SegLayout<T>;
@@ -635,17 +651,7 @@ int32_t launch_exact_typed(const ExactParams &p0, cudaStream_t st) {
     p.stages = (int)s_log;
     p.team = (int)t_log;
     const size_t smem = cta + (size_t)P * xg_warp_smem(1u << s_log, L::BYTES) + (t_log ? (size_t)(P >> t_log) * xg_mail_bytes(t_log) : 0);
-    void (*const team)(ExactParams) = gemv_exact_kernel<T, true, XG_MAX_WARPS * 32>, (*const wide)(ExactParams) = gemv_exact_kernel<T, false, XG_WIDE_BOUND>,
-                 (*const full)(ExactParams) = gemv_exact_kernel<T, false, XG_LONE_MAX_WARPS * 32>;
-    static thread_local int raised_dev = -1;  // per instantiation: opt in to more than 48 KB once per device
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (raised_dev != dev) {
-        for (auto k : {team, wide, full}) CERA_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XG_SMEM_LIMIT));
-        raised_dev = dev;
-    }
-    count_launch();
-    return check_cuda(launch_k(t_log ? team : P <= (uint32_t)XG_WIDE_WARPS ? wide : full, dim3(grid), dim3(P * 32), smem, st, p), "gemv (reference order) launch");
+    return p.f.quant_x ? launch_exact_column<T, true>(p, grid, P, smem, t_log != 0, st) : launch_exact_column<T, false>(p, grid, P, smem, t_log != 0, st);
 }
 
 }  // namespace
