@@ -1052,19 +1052,21 @@ __global__ void __launch_bounds__(256) tc_parts_kernel(const TcParams p, uint32_
 }
 
 // A grid of `tiles` tiles over `slots` SMs (or pairs), one each at a time: whole rounds first; the tiles of the last one, when it does not fill the
-// device, are each shared by `parts` along k, as many as make the round shortest: rounds of the shares / parts, and a fiftieth of a round for what
-// each share adds (its start, its partial sums).  448 tiles of 128 x 256 on 148 SMs, k = 4096 (gate / up of 512 tokens: three rounds and four tiles):
-// 280 us whole, 212 shared; 32 tiles of 128 x 128 (4096 x 64 x 4096, the whole product) 63 us whole, 35 in eight shares each.
+// device, are each shared by `parts` along k, as many as make the round shortest.  Its time: rounds of the shares, `sb_ns` a super-block, then
+// for every share its partial sums written and read (`rows` x 128 floats, at 5.5 TB/s) and the launch that adds them.
+// Two layers of 2047 tokens 4.81 ms with a fiftieth of a round a share instead, 4.56 so (4.62 with the shares at 11 TB/s).
+// 448 tiles of 128 x 256 on 148 SMs, k = 4096 (gate / up of 512 tokens: three rounds and four tiles): 280 us whole, 212 shared; 32 tiles of 128 x 128
+// (4096 x 64 x 4096, the whole product) 63 us whole, 35 in eight shares each.
 constexpr uint32_t TC_SHARES = 3;  // partial tiles a slot has room for
 struct TcSplit {
     uint32_t left, parts;
 };
-TcSplit tc_split(uint32_t tiles, uint32_t n_sb, uint32_t slots) {
-    const uint32_t left = tiles % slots;
-    uint32_t best = 50, parts = 1;  // fiftieths of a round
+TcSplit tc_split(uint32_t tiles, uint32_t n_sb, uint32_t slots, uint32_t sb_ns, uint32_t rows) {
+    const uint32_t left = tiles % slots, share_ns = rows * 2 * TC_BM * 4 / 5500, launch_ns = 3000;
+    uint32_t best = n_sb * sb_ns, parts = 1;
     for (uint32_t s = 2; left && s <= std::min(n_sb / 2, 16u) && left * s <= TC_SHARES * slots; ++s) {
-        const uint32_t cost = (50 * ((left * s + slots - 1) / slots) + s - 1) / s + s;
-        if (cost < best) best = cost, parts = s;
+        const uint32_t ns = (left * s + slots - 1) / slots * ((n_sb + s - 1) / s) * sb_ns + left * s * share_ns + launch_ns;
+        if (ns < best) best = ns, parts = s;
     }
     return parts > 1 ? TcSplit{left, parts} : TcSplit{0, 1};
 }
@@ -1193,7 +1195,9 @@ int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, s
     const uint32_t rows = pair || wide ? 2 * TC_BN : TC_BN, halves = pair ? 2 : 1, x_tiles = (tiles + halves - 1) / halves;
     uint32_t y = 0;
     for (int i = 0; i < count; ++i) y += (t[i].w.m + rows - 1) / rows;
-    TcSplit split = w.tc ? tc_split(x_tiles * y, n_sb, (uint32_t)sm_count() / halves) : TcSplit{0, 1};
+    // (nanoseconds of a super-block, as measured: Q6_K in pairs, pairs, wide, 128 x 128)
+    const uint32_t sb_ns = q6 ? 4000 : pair ? 2900 : wide ? 3600 : 1650;
+    TcSplit split = w.tc ? tc_split(x_tiles * y, n_sb, (uint32_t)sm_count() / halves, sb_ns, halves * rows) : TcSplit{0, 1};
     // partial sums of the tiles that are shared; without room for them the tiles stay whole
     const size_t parts_bytes = (size_t)split.left * split.parts * halves * rows * TC_BM * 4;
     const bool borrowed = lent.p && lent.bytes >= need;
