@@ -16,7 +16,8 @@ from .types import BLOCK, row_bytes
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the current device's current stream, without the Stream object that torch.cuda.current_stream() makes (3.4 us of a 13 us gemv call)
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _ptr(t):
