@@ -292,11 +292,13 @@ int32_t launch_dense_gemm_tc(const DenseGemm &g, cudaStream_t st, bool *taken) {
     if (g.out_kind == DENSE_T_TRANSPOSED && g.ldo % 8) return CERA_CUDA_OK;
     *taken = true;
     const bool unit = g.out_kind == DENSE_GATED_UNIT;
-    // A pair of CTAs per tile where a tile has more than 64 columns, unless the last pair of row tiles would leave more than an eighth of the work
-    // for rows that are not there.  2048 tokens at width 4096, single CTAs and pairs: four layers of experts 4.22 and 4.05 ms, eight dense layers
-    // 6.65 and 6.36 (at up to 64 columns the weights are read once either way).
+    // A pair of CTAs per tile where a tile has more than 64 columns - of experts, where they fill it on average: 52 columns an expert, width 2048, 60.5 us
+    // alone and 61.4 in pairs - unless the last pair of row tiles would leave more than an eighth of the work for rows that are not there.  2048 tokens at
+    // width 4096, single CTAs and pairs: four layers of experts 4.22 and 4.05 ms, eight dense layers 6.65 and 6.36; 200 tokens through a gated unit 43.2
+    // and 41.0 us (at up to 64 columns the weights are read once either way).
     const uint32_t rows = (g.tiles ? g.rows_per_expert : g.w.rows) / (unit ? 2 : 1), whole = (rows + DT_BM - 1) / DT_BM;
-    const bool two = (whole + 1) / 2 * 16 <= whole * 9 && g.block_rows % (2 * DT_BM) == 0;
+    const bool full = !g.tiles || g.n >= g.w.rows / g.rows_per_expert * DT_BM;
+    const bool two = full && (whole + 1) / 2 * 16 <= whole * 9 && g.block_rows % (2 * DT_BM) == 0;
     if (g.tiles) {
         if (g.group_columns <= 32) return unit ? launch_tc<32, 2>(g, st) : launch_tc<32, 1>(g, st);
         if (g.group_columns <= 64) return unit ? launch_tc<64, 2>(g, st) : launch_tc<64, 1>(g, st);
