@@ -16,7 +16,7 @@
 // (110 with mma.sync, which also spends the issue slots of its fragments); 14336 x 4096 Q8_0, 2048 columns: 1.08 ms (12.9 ms by eight
 // columns at a time).
 //
-// A CTA is persistent: it walks units (128 rows x up to BN columns x a share of k), one thread issuing the products, one
+// A CTA is persistent: it walks units (128 rows x up to BN columns x a share of k), one warp issuing the products, one
 // requesting activation tiles by bulk copies, four warps converting weights into the operand tiles, eight draining finished
 // blocks.  A grid of units that would leave SMs idle splits k; the
 // partial tiles go through a scratch buffer and are added in the order of k.  Every wait is bounded (tma.cuh).
