@@ -28,6 +28,7 @@ namespace {
 
 constexpr int RW_WARPS = 8;
 constexpr int RW_THREADS = RW_WARPS * 32;
+constexpr int RW_CTAS = 2;  // an SM's at a time: the grid is sized for them
 constexpr int RW_MAX_SEGS = 3;
 constexpr uint32_t RW_TASK = 144;  // bytes a task's quants take in shared memory
 
@@ -45,8 +46,10 @@ struct RowsParams {
     TpHook tp;
 };
 
-template <int T, int UNR>
-__global__ void __launch_bounds__(RW_THREADS) gemv_rows_kernel(const RowsParams p) {
+// FORM: the kernel quantizes its column itself (GemvFusion::quant_x).  A variant of its own: beside the other prologue its code took the Q8_0 and Q5_K
+// kernels from 128 registers to 141, and with them the second CTA of every SM: a Q8_0 model of width 1024 decoded a token in 337 us instead of 279.
+template <int T, int UNR, bool FORM>
+__global__ void __launch_bounds__(RW_THREADS, RW_CTAS) gemv_rows_kernel(const RowsParams p) {
     __shared__ float partial[RW_WARPS][UNR];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wpr = p.wpr, rows_per_pass = (RW_WARPS / wpr) * UNR;
@@ -77,7 +80,7 @@ __global__ void __launch_bounds__(RW_THREADS) gemv_rows_kernel(const RowsParams 
             pdl_trigger();
             pdl_wait();
             tp_arrive_wait(p.tp.ctx, p.tp.wait_slot);
-            if (p.f.quant_x) {
+            if constexpr (FORM) {
                 // Every CTA quantizes the column for itself, into shared memory: four elements a thread, and a lane task's 128 quants 16 bytes
                 // further than they need, so that the lanes' 16-byte reads do not meet in one bank.
                 extern __shared__ __align__(16) uint8_t rw_x[];
@@ -194,13 +197,13 @@ __global__ void rope_table_kernel(const uint32_t *__restrict__ pos_dev, uint32_t
 template <int T>
 int32_t launch_rows_typed(const RowsParams &p, cudaStream_t st) {
     constexpr int UNR = 2;
-    const uint32_t cap = (uint32_t)sm_count() * 2;
+    const uint32_t cap = (uint32_t)sm_count() * RW_CTAS;
     const uint32_t rows_per_pass = (RW_WARPS / p.wpr) * UNR;
     const uint32_t passes = (p.total_rows + rows_per_pass - 1) / rows_per_pass;
     count_launch();
-    return check_cuda(launch_k(gemv_rows_kernel<T, UNR>, dim3(passes < cap ? passes : cap), dim3(RW_THREADS),
-                               p.f.quant_x ? (size_t)p.t128 * (RW_TASK + 32) : 0, st, p),
-                      "gemv launch");
+    const dim3 grid(passes < cap ? passes : cap);
+    if (p.f.quant_x) return check_cuda(launch_k(gemv_rows_kernel<T, UNR, true>, grid, dim3(RW_THREADS), (size_t)p.t128 * (RW_TASK + 32), st, p), "gemv launch");
+    return check_cuda(launch_k(gemv_rows_kernel<T, UNR, false>, grid, dim3(RW_THREADS), 0, st, p), "gemv launch");
 }
 
 }  // namespace
