@@ -453,7 +453,7 @@ struct AxFused {
     static size_t smem(uint32_t pos, uint32_t G, uint32_t HC) { return (size_t)pos * 32 * ES + K_BYTES + ((size_t)(pos + 4) * HC + (size_t)G * HD) * 4; }
 };
 template <int HD, bool F16>
-__global__ void __launch_bounds__(AX_VTHREADS)
+__global__ void __launch_bounds__(AX_VTHREADS, 1)
 attn_fused_exact_kernel(const float *__restrict__ q, const void *__restrict__ kc, const void *__restrict__ vc, int vec, uint32_t seq_len,
                         const uint32_t *__restrict__ seq_dev, uint32_t n_kv, uint32_t G, uint32_t HC, float scale, uint32_t smem_pos,
                         float *__restrict__ out, float *scales, int8_t *quants, int16_t *sums, const TpHook tp) {
