@@ -168,11 +168,14 @@ int32_t launch_gemv_fused(const GemvSeg *segs, int n_segs, const ActView &x, int
 }
 
 // The column is quantized by every CTA for itself while its first weights are on their way, where a launch of its own came before.  us, both
-// launches / one, back to back: Q4_0 4096 x 4096 6.4 / 4.6, Q4_K 4096 x 4096 8.9 / 6.8, 10240 x 1024 5.6 / 3.8, 28672 x 4096 17.5 / 15.3, Q6_K
-// 4096 x 14336 17.8 / 16.8.
+// launches / one, back to back, weights from memory: Q4_0 2048 x 4096 5.2 / 3.8, 14336 x 4096 12.2 / 10.9; Q4_K 2048 x 1024 3.9 / 2.5, 4096 x 4096 8.6 / 6.5,
+// 14336 x 4096 12.4 / 10.1; Q6_K 4096 x 14336 17.2 / 15.8.
 int32_t launch_gemv_from_f32(const GemvSeg &seg, const float *x, cudaStream_t st, bool *taken) {
     *taken = false;
     static const bool chosen = getenv("CERA_CUDA_GEMV") != nullptr;  // A/B runs
+    // Few CTAs spend on a long column what the launch costs, and with much longer ones all do.  In reference order, both launches / one: 1024 x 10240
+    // 8.5 / 8.6 (Q4_K), 64 x 14336 9.7 / 10.3, 2048 x 14336 12.9 / 12.6, 8192 x 14336 26.0 / 26.0 (Q5_K), 4096 x 20480 29.5 / 31.7 (Q6_K).
+    if (seg.w.k > 9216 && (seg.w.m < 2048 || seg.w.k > 14336)) return CERA_CUDA_OK;
     // a result over its own operand needs the operand quantized first
     const uintptr_t x0 = (uintptr_t)x, x1 = x0 + (size_t)seg.w.k * 4, y0 = (uintptr_t)seg.y, y1 = y0 + (size_t)seg.w.m * 4;
     if (chosen || (x0 < y1 && y0 < x1)) return CERA_CUDA_OK;

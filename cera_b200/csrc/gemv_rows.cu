@@ -29,6 +29,8 @@ namespace {
 constexpr int RW_WARPS = 8;
 constexpr int RW_THREADS = RW_WARPS * 32;
 constexpr int RW_CTAS = 2;  // an SM's at a time: the grid is sized for them
+// (Q8_0, forming its column: 141 registers or spills, which its small launches show: 256 x 1024 3.1 us, 3.5 with spills)
+constexpr int rw_ctas(int type, bool form) { return form && type == CERA_TYPE_Q8_0 ? 1 : RW_CTAS; }
 constexpr int RW_MAX_SEGS = 3;
 constexpr uint32_t RW_TASK = 144;  // bytes a task's quants take in shared memory
 
@@ -49,7 +51,7 @@ struct RowsParams {
 // FORM: the kernel quantizes its column itself (GemvFusion::quant_x).  A variant of its own: beside the other prologue its code took the Q8_0 and Q5_K
 // kernels from 128 registers to 141, and with them the second CTA of every SM: a Q8_0 model of width 1024 decoded a token in 337 us instead of 279.
 template <int T, int UNR, bool FORM>
-__global__ void __launch_bounds__(RW_THREADS, RW_CTAS) gemv_rows_kernel(const RowsParams p) {
+__global__ void __launch_bounds__(RW_THREADS, rw_ctas(T, FORM)) gemv_rows_kernel(const RowsParams p) {
     __shared__ float partial[RW_WARPS][UNR];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wpr = p.wpr, rows_per_pass = (RW_WARPS / wpr) * UNR;
@@ -194,10 +196,22 @@ __global__ void rope_table_kernel(const uint32_t *__restrict__ pos_dev, uint32_t
     table[2 * i + 1] = sn;
 }
 
+// Where the kernel forms its column itself.  It saves a launch of some 1.3 us, and every CTA spends 0.3 us for 1024 elements of k.  us, two launches / one,
+// weights from memory:
+//   a warp a row (k up to 4096): 64 x 4096 Q4_0 4.0 / 3.3, 14336 x 4096 12.2 / 10.9, 14336 x 256 8.8 / 8.0; the same for the others but Q8_0, whose
+//   kernel has one CTA an SM for it: 256 x 1024 3.8 / 3.1, 1024 x 4096 4.3 / 3.4, 1536 x 1024 3.9 / 3.6, 2048 x 2048 4.1 / 4.4, 4096 x 4096 5.6 / 9.8.
+//   two warps (up to 8192): 64 x 6144 Q4_0 4.0 / 4.2, 2048 x 6144 5.0 / 5.4, 8192 x 6144 12.6 / 12.1, 8192 x 8192 13.4 / 13.3.
+//   four: 64 x 14336 4.1 / 7.3, 8192 x 14336 20.9 / 23.0, 8192 x 8448 Q4_K 21.3 / 21.8.
+bool rw_forms_column(int type, uint32_t k, int wpr, uint32_t rows) {
+    const uint32_t per = RW_WARPS / wpr * 2, passes = (rows + per - 1) / per, sms = (uint32_t)sm_count();
+    if (type == CERA_TYPE_Q8_0) return wpr == 1 && passes <= sms && (2 * passes <= sms || k <= 1024);
+    return wpr == 1 || (wpr == 2 && passes >= 4 * sms);
+}
+
 template <int T>
 int32_t launch_rows_typed(const RowsParams &p, cudaStream_t st) {
     constexpr int UNR = 2;
-    const uint32_t cap = (uint32_t)sm_count() * RW_CTAS;
+    const uint32_t cap = (uint32_t)sm_count() * rw_ctas(T, p.f.quant_x != nullptr);
     const uint32_t rows_per_pass = (RW_WARPS / p.wpr) * UNR;
     const uint32_t passes = (p.total_rows + rows_per_pass - 1) / rows_per_pass;
     count_launch();
@@ -232,6 +246,7 @@ int32_t launch_gemv_rows(const GemvSeg *segs, int n_segs, const ActView &x, int 
     }
     int wpr = 1;
     while (wpr * 32u < t128) wpr <<= 1;
+    if (p.f.quant_x && !rw_forms_column(type, k, wpr, rows)) return CERA_CUDA_OK;
     if (epilogue == EPI_ROPE_KV) {
         if (n_segs != 3 || wpr != 1 || !p.f.rope_cs || !p.f.pos_dev || !p.f.k_cache || !p.f.v_cache || p.f.head_dim % 2 ||
             segs[0].w.m % 2 || segs[1].w.m % 2 || segs[2].w.m % 2)

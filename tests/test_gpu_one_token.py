@@ -58,6 +58,14 @@ def test_gemv_over_its_own_operand(t):
     assert_bits(cb.gemv(w, x, x).cpu().numpy(), want.cpu().numpy(), O.NAMES[t])
 
 
+# both sides of the lines between one launch and two: rows of one, two and four warps, few and many of them; a column of 10240 and beyond
+@pytest.mark.parametrize("t", O.QUANT_TYPES)
+@pytest.mark.parametrize("m,k", [(1184, 2048), (1200, 2048), (2400, 256), (4730, 5376), (4760, 5376), (4760, 8448), (70, 9216), (70, 9728), (2047, 14336), (2048, 14336),
+                                 (2048, 14848)])
+def test_gemv_in_one_launch_or_two(t, m, k):
+    test_gemv_equals_quantizer_and_product(t, m, k)
+
+
 @pytest.mark.parametrize("t", [O.Q4_0, O.Q4_1, O.Q8_0])
 @pytest.mark.parametrize("m,k", [(5, 128), (17, 384), (3, 32768), (11, 160)])
 def test_gemv_of_32_element_formats_equals_quantizer_and_product(t, m, k):

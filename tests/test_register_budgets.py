@@ -4,7 +4,7 @@ import os
 import re
 import subprocess
 
-import pytest
+from cera_b200 import types
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
@@ -18,8 +18,10 @@ def _registers(source, tmp_path):
     return re.findall(r"Compiling entry function '(\w+)'.*?Used (\d+) registers", text, re.S)
 
 
-@pytest.mark.parametrize("source,kernel,threads,ctas,variants", [("gemv_rows.cu", "gemv_rows_kernel", 256, 2, 12)])
-def test_ctas_of_a_decode_product_fit_an_sm(tmp_path, source, kernel, threads, ctas, variants):
-    used = [int(r) for name, r in _registers(source, tmp_path) if kernel in name]
-    assert len(used) == variants
-    assert max(used) * threads * ctas <= 65536, used
+def test_ctas_of_a_decode_product_fit_an_sm(tmp_path):
+    used = {tuple(map(int, re.search(r"gemv_rows_kernelILi(\d+)ELi\d+ELb(\d)E", name).groups())): int(r)
+            for name, r in _registers("gemv_rows.cu", tmp_path) if "gemv_rows_kernel" in name}
+    assert len(used) == 12  # six formats, the column quantized before or by the kernel
+    for (fmt, forms), r in used.items():
+        ctas = 1 if (fmt, forms) == (types.Q8_0, 1) else 2
+        assert r * 256 * ctas <= 65536, (fmt, forms, r)
