@@ -404,7 +404,7 @@ attn_chain_exact_kernel(const __grid_constant__ CUtensorMap v_map, const float *
 #pragma unroll
                 for (uint32_t i = 0; i < AXC_T / 32; ++i)
                     e[hh][i] = hh < nh && 32 * i + lane < cnt ? ws[(size_t)(kvh * G + h0 + hh) * ld + t0 + 32 * i + lane] : 0.0f;
-            if (tile >= C::STAGES && !tma::mbar_wait_blocking(empty + slot, (tile / C::STAGES - 1) & 1, &gave_up, &g_ax_status, 2u)) return;
+            if (tile >= C::STAGES && !tma::mbar_wait_warp(empty + slot, (tile / C::STAGES - 1) & 1, &gave_up, &g_ax_status, 2u)) return;
             char *dst = ring + slot * C::STAGE;
             float *pd = reinterpret_cast<float *>(dst + C::V_BYTES);
 #pragma unroll
@@ -426,7 +426,7 @@ attn_chain_exact_kernel(const __grid_constant__ CUtensorMap v_map, const float *
     float acc = 0.0f;
     for (uint32_t tile = 0; tile < n_tiles; ++tile) {
         const uint32_t slot = tile % C::STAGES;
-        if (!tma::mbar_wait_blocking(full + slot, (tile / C::STAGES) & 1, &gave_up, &g_ax_status, 1u)) return;
+        if (!tma::mbar_wait_warp(full + slot, (tile / C::STAGES) & 1, &gave_up, &g_ax_status, 1u)) return;
         const uint32_t base = tma::smem_u32(ring + slot * C::STAGE);
         acc = ax_chain<F16>(base, base + C::V_BYTES + warp * AXC_T * 4, min((uint32_t)AXC_T, seq - tile * AXC_T), acc);
         __syncwarp();

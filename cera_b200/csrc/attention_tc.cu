@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(const __gri
     } else if (warp == 1) {
         // the whole warp, one lane issues
         const uint32_t id_s = tc_idesc_bf16(AT_Q, AT_K), id_o = tc_idesc_bf16(AT_Q, s.vdim_p), me = elect_one();
-        auto arrived = [&](uint64_t *bar, uint32_t parity) { return warp_all(tma::mbar_wait_blocking(bar, parity, abort_flag, status, 2u)); };
+        auto arrived = [&](uint64_t *bar, uint32_t parity) { return tma::mbar_wait_warp(bar, parity, abort_flag, status, 2u); };
         auto scores = [&](uint32_t j) -> bool {
             const uint32_t b = j & 1, par = j >> 1 & 1;
             if (!arrived(k_full + b, par) || !arrived(s_free + b, par ^ 1)) return false;
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(const __gri
         bool ok = true;
         for (uint32_t j = 0; j < n_kv; ++j) {
             const uint32_t b = j & 1, par = j >> 1 & 1;
-            ok = __all_sync(0xffffffffu, tma::mbar_wait_blocking(s_full + b, par, abort_flag, status, 4u));
+            ok = tma::mbar_wait_warp(s_full + b, par, abort_flag, status, 4u);
             if (!ok) break;
             tc_fence_after();
             uint32_t v[4][16];
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(const __gri
             }
             if (j > 0) {
                 if (__any_sync(0xffffffffu, alpha != 1.0f)) {  // O of the tiles before must be complete to be rescaled
-                    ok = __all_sync(0xffffffffu, tma::mbar_wait_blocking(pv_done + (b ^ 1), (j - 1) >> 1 & 1, abort_flag, status, 4u));
+                    ok = tma::mbar_wait_warp(pv_done + (b ^ 1), (j - 1) >> 1 & 1, abort_flag, status, 4u);
                     if (!ok) break;
                     tc_fence_after();
                     for (uint32_t c = 0; c < s.vdim_p; c += 16) {
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(const __gri
                     tmem_wait_st();
                 }
                 if (j > 1) {  // P of two tiles ago has been read
-                    ok = __all_sync(0xffffffffu, tma::mbar_wait_blocking(pv_done + b, (j - 2) >> 1 & 1, abort_flag, status, 4u));
+                    ok = tma::mbar_wait_warp(pv_done + b, (j - 2) >> 1 & 1, abort_flag, status, 4u);
                     if (!ok) break;
                 }
             }
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(const __gri
             __syncwarp();
             if (lane == 0) tma::mbar_arrive(p_full + b);
         }
-        if (ok) ok = __all_sync(0xffffffffu, tma::mbar_wait_blocking(pv_done + ((n_kv - 1) & 1), (n_kv - 1) >> 1 & 1, abort_flag, status, 4u));
+        if (ok) ok = tma::mbar_wait_warp(pv_done + ((n_kv - 1) & 1), (n_kv - 1) >> 1 & 1, abort_flag, status, 4u);
         if (ok) {
             tc_fence_after();
             const bool live = q0 + r < p.n;

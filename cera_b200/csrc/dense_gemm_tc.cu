@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dense_gemm_tc_kernel(const __gr
             const uint32_t a_row = o.a_row + rank * DT_BM, col = o.first + rank * (columns(o) / 2);
             for (uint32_t k = 0; k < n_k; ++k, ++it) {
                 const uint32_t s = it % S::STAGES;
-                if (!(ok = warp_all(tma::mbar_wait_blocking(empty + s, (it / S::STAGES & 1) ^ 1, abort_flag, &g_dense_tc_status, 1u)))) break;
+                if (!(ok = tma::mbar_wait_warp(empty + s, (it / S::STAGES & 1) ^ 1, abort_flag, &g_dense_tc_status, 1u))) break;
                 uint8_t *st = stages + s * S::STAGE;
                 if constexpr (PAIR) {  // all bytes of both CTAs are counted on the even CTA's barrier
                     tma::mbar_expect_tx_if(full + s, 2 * S::STAGE, rank == 0 ? me : 0);
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dense_gemm_tc_kernel(const __gr
             uint32_t it = 0, j = 0;
             bool ok = true;
             auto arrived = [&](uint64_t *bar, uint32_t parity) {
-                return warp_all(tma::mbar_wait_blocking(bar, parity, abort_flag, &g_dense_tc_status, 2u));
+                return tma::mbar_wait_warp(bar, parity, abort_flag, &g_dense_tc_status, 2u);
             };
             for (uint32_t t = first_tile; t < n_tiles && ok; t += step, ++j) {
                 const uint32_t b = j & 1, acc = tmem + b * S::ACC;
@@ -191,8 +191,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dense_gemm_tc_kernel(const __gr
         uint32_t j = 0;
         for (uint32_t t = first_tile; t < n_tiles; t += step, ++j) {
             const uint32_t b = j & 1;
-            const bool ok = tma::mbar_wait_blocking(acc_full + b, j >> 1 & 1, abort_flag, &g_dense_tc_status, 4u);
-            if (!__all_sync(0xffffffffu, ok)) break;
+            if (!tma::mbar_wait_warp(acc_full + b, j >> 1 & 1, abort_flag, &g_dense_tc_status, 4u)) break;
             tc_fence_after();
             const DtTile o = dt_tile<BN, NA, PAIR>(p, t);
             const uint32_t row = o.row0 + rank * DT_BM + quad * 32 + lane, acc = tmem + b * S::ACC + (quad * 32 << 16), cols = o.end - o.first;

@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
             else tc_commit(bar, me);
         };
         auto arrived = [&](uint64_t *bar, uint32_t parity, uint32_t who) {
-            return warp_all(tma::mbar_wait_blocking(bar, parity, abort_flag, &g_tc_status, who));
+            return tma::mbar_wait_warp(bar, parity, abort_flag, &g_tc_status, who);
         };
         bool ok = true;
         uint32_t it = 0;
@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
         const uint32_t n_all = n_sb * S::SB_STAGES + (n_rounds > n_sb ? n_mit : 0);
         for (uint32_t it = 0; it < n_all; ++it) {
             const uint32_t s = it % S::STAGES;
-            if (!warp_all(tma::mbar_wait_blocking(full_ab + s, (it / S::STAGES) & 1, abort_flag, &g_tc_status, 1u))) break;
+            if (!tma::mbar_wait_warp(full_ab + s, (it / S::STAGES) & 1, abort_flag, &g_tc_status, 1u)) break;
             if (lane == 0) tma::mbar_arrive_cluster(tma::smem_of_rank(peer_full + s, 0));
             __syncwarp();
         }
@@ -550,9 +550,9 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
         for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
             for (uint32_t st = 0; st < (uint32_t)S::SB_STAGES; ++st, ++it) {
                 const uint32_t s = it % S::STAGES;
-                ok = warp_all(tma::mbar_wait_blocking(empty_ab + s, ((it / S::STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u));
+                ok = tma::mbar_wait_warp(empty_ab + s, ((it / S::STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u);
                 // the d slot of this super-block was last read by the epilogue of super-block sb - 2
-                if (ok && st == 0 && sb >= 2) ok = warp_all(tma::mbar_wait_blocking(slot_free + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u));
+                if (ok && st == 0 && sb >= 2) ok = tma::mbar_wait_warp(slot_free + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u);
                 if (!ok) break;
                 uint8_t *dst = tc_smem + s * S::STAGE;
                 tma::mbar_expect_tx_if(full_ab + s, S::STAGE + (st == 0 ? 2 * TC_BN * 4 : 0), me);
@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
             const uint8_t *m0 = sub.tc + L.wmin + (size_t)own * n_mit * (2 * TCW_MINT_BYTES), *m1 = sub.tc + L.wmin + (size_t)t1 * n_mit * (2 * TCW_MINT_BYTES);
             for (uint32_t mi = 0; mi < n_mit && ok; ++mi, ++it) {
                 const uint32_t s = it % S::STAGES;
-                if (!warp_all(tma::mbar_wait_blocking(empty_ab + s, ((it / S::STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u))) break;
+                if (!tma::mbar_wait_warp(empty_ab + s, ((it / S::STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u)) break;
                 uint8_t *dst = tc_smem + s * S::STAGE;
                 tma::mbar_expect_tx_if(full_ab + s, (2 + 2 * S::B_TILES) * TCW_MINT_BYTES + (mi == 0 ? 2 * TC_BN * 4 : 0), me);
                 tma::bulk_g2s_if(dst, xm + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s, me);
@@ -607,10 +607,8 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
         bool ok = true;
         for (uint32_t sb = 0; sb < n_rounds && ok; ++sb) {
             const uint32_t buf = sb & 1;
-            if (!tma::mbar_wait_blocking(full_d + buf, (sb >> 1) & 1, abort_flag, &g_tc_status, 16u)) {
-                ok = false;
-                break;
-            }
+            ok = tma::mbar_wait_warp(full_d + buf, (sb >> 1) & 1, abort_flag, &g_tc_status, 16u);
+            if (!ok) break;
             tc_fence_after();
             if (sb == 0) ginv = __ldg(p.ginv + min(col0 + tl, p.n - 1));
             // per super-block: out += d[row] * D / g; after the min GEMM: out -= 2^-s[row] * Dmin / g
@@ -733,16 +731,16 @@ __global__ void __launch_bounds__(IMG ? TC_THREADS_IMG : TC_THREADS, 1) gemm_tc_
         for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
             const uint32_t buf = sb & 1, d0 = tmem + buf * TC_BN;
             // the epilogue has left this D buffer (super-block sb - 2)
-            if (!warp_all(tma::mbar_wait_blocking(empty_d + buf, ((sb >> 1) & 1) ^ 1, abort_flag, &g_tc_status, 2u))) break;
+            if (!tma::mbar_wait_warp(empty_d + buf, ((sb >> 1) & 1) ^ 1, abort_flag, &g_tc_status, 2u)) break;
             tc_fence_after();
             for (uint32_t st = 0; st < (uint32_t)TC_STAGES; ++st) {
                 const uint32_t it = sb * TC_STAGES + st;
                 const bool last = st + 1 == (uint32_t)TC_STAGES;
-                ok = warp_all(tma::mbar_wait_blocking(full_ab + st, (it / TC_STAGES) & 1, abort_flag, &g_tc_status, 1u));
+                ok = tma::mbar_wait_warp(full_ab + st, (it / TC_STAGES) & 1, abort_flag, &g_tc_status, 1u);
                 // with the last stage goes the super-block's min term.  Without the weight image Dm has one buffer (the fourth TMEM region
                 // holds the running output): the epilogue must have read super-block sb - 1's
                 if (ok && last && !IMG && sb)
-                    ok = warp_all(tma::mbar_wait_blocking(empty_d + (buf ^ 1), ((sb - 1) >> 1) & 1, abort_flag, &g_tc_status, 2u));
+                    ok = tma::mbar_wait_warp(empty_d + (buf ^ 1), ((sb - 1) >> 1) & 1, abort_flag, &g_tc_status, 2u);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t base = tma::smem_u32(tc_smem + st * TC_STAGE_BYTES), slot = tma::smem_u32(slots + buf * TC_SLOT_BYTES);
@@ -795,8 +793,8 @@ __global__ void __launch_bounds__(IMG ? TC_THREADS_IMG : TC_THREADS, 1) gemm_tc_
             const uint8_t *wside = IMG ? sub.tc + (size_t)tiles_m * k_sb * TC_STAGES * TC_OP_BYTES + w_sb * TC_SIDE_BYTES : nullptr;
             for (uint32_t it = 0; it < n_it; ++it) {
                 const uint32_t st = it % TC_STAGES, sb = it / TC_STAGES;
-                if (!warp_all(tma::mbar_wait_blocking(empty_ab + st, ((it / TC_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u))) break;
-                if (st == 0 && sb >= 2 && !warp_all(tma::mbar_wait_blocking(empty_d + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u))) break;
+                if (!tma::mbar_wait_warp(empty_ab + st, ((it / TC_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u)) break;
+                if (st == 0 && sb >= 2 && !tma::mbar_wait_warp(empty_d + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u)) break;
                 tma::mbar_expect_tx_if(full_ab + st, (IMG ? 3 : 2) * TC_OP_BYTES + (st == 0 ? TC_MINOP_BYTES + (IMG ? TC_SIDE_BYTES : 0) : 0), me);
                 tma::bulk_g2s_if(tc_smem + st * TC_STAGE_BYTES, img + (size_t)it * (2 * TC_OP_BYTES), 2 * TC_OP_BYTES, full_ab + st, me);
                 if (IMG) tma::bulk_g2s_if(tc_smem + st * TC_STAGE_BYTES + 2 * TC_OP_BYTES, wimg + (size_t)it * TC_OP_BYTES, TC_OP_BYTES, full_ab + st, me);
@@ -823,10 +821,8 @@ __global__ void __launch_bounds__(IMG ? TC_THREADS_IMG : TC_THREADS, 1) gemm_tc_
             for (int i = 0; i < 64; ++i) acc[i] = 0.0f;
             for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
                 const uint32_t buf = sb & 1;
-                if (!tma::mbar_wait_blocking(full_d + buf, (sb >> 1) & 1, abort_flag, &g_tc_status, 16u)) {
-                    ok = false;
-                    break;
-                }
+                ok = tma::mbar_wait_warp(full_d + buf, (sb >> 1) & 1, abort_flag, &g_tc_status, 16u);
+                if (!ok) break;
                 tc_fence_after();
                 if (sb == 0) ginv = __ldg(p.ginv + col0 + tl);
                 const float *dval = reinterpret_cast<const float *>(slots + buf * TC_SLOT_BYTES + 2 * TC_MINOP_BYTES);
@@ -888,10 +884,8 @@ __global__ void __launch_bounds__(IMG ? TC_THREADS_IMG : TC_THREADS, 1) gemm_tc_
         }
         for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
             const uint32_t buf = sb & 1;
-            if (!tma::mbar_wait_blocking(full_d + buf, (sb >> 1) & 1, abort_flag, &g_tc_status, 16u)) {
-                ok = false;
-                break;
-            }
+            ok = tma::mbar_wait_warp(full_d + buf, (sb >> 1) & 1, abort_flag, &g_tc_status, 16u);
+            if (!ok) break;
             tc_fence_after();
             if (sb == 0) ginv = __ldg(p.ginv + col0 + tl);
             const float *dval = reinterpret_cast<const float *>(slots + buf * TC_SLOT_BYTES + 2 * TC_MINOP_BYTES);

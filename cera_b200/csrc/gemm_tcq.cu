@@ -331,8 +331,8 @@ __global__ void __launch_bounds__(TQ_THREADS, 1) gemm_tcq_kernel(const __grid_co
             const uint32_t idesc = (1u << 4) | ((o.nc >> 3) << 17) | ((TQ_BM >> 4) << 24);  // f16 x f16 -> f32, K-major
             for (uint32_t st = o.s0; st < o.s1; ++st, ++it) {
                 const uint32_t s = it % S::STAGES, b = it % S::ACC, nblk = min(2u, p.nb - 2 * st);
-                ok = warp_all(tma::mbar_wait_blocking(empty_d + b, ((it / S::ACC) & 1) ^ 1, abort_flag, &g_tcq_status, 1u) &&
-                              tma::mbar_wait_blocking(full + s, (it / S::STAGES) & 1, abort_flag, &g_tcq_status, 1u));
+                ok = tma::mbar_wait_warp(empty_d + b, ((it / S::ACC) & 1) ^ 1, abort_flag, &g_tcq_status, 1u) &&
+                     tma::mbar_wait_warp(full + s, (it / S::STAGES) & 1, abort_flag, &g_tcq_status, 1u);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t a = tma::smem_u32(tq_smem + s * S::STAGE), x = a + S::NA * S::OP, d = tmem + b * 2 * BN;
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(TQ_THREADS, 1) gemm_tcq_kernel(const __grid_co
             const uint32_t bytes = o.nc * TQ_COL;
             for (uint32_t st = o.s0; st < o.s1; ++st, ++it) {
                 const uint32_t s = it % S::STAGES;
-                ok = warp_all(tma::mbar_wait_blocking(empty + s, ((it / S::STAGES) & 1) ^ 1, abort_flag, &g_tcq_status, 2u));
+                ok = tma::mbar_wait_warp(empty + s, ((it / S::STAGES) & 1) ^ 1, abort_flag, &g_tcq_status, 2u);
                 if (!ok) break;
                 tma::mbar_expect_tx_if(full + s, bytes, me);  // (of a last half stage no product and no sum reads the second block)
                 tma::bulk_g2s_if(tq_smem + s * S::STAGE + S::NA * S::OP, src + (size_t)st * bytes, bytes, full + s, me);
@@ -380,10 +380,8 @@ __global__ void __launch_bounds__(TQ_THREADS, 1) gemm_tcq_kernel(const __grid_co
             for (int i = 0; i < BN / 4; ++i) acc[i] = make_float2(0.0f, 0.0f);
             for (uint32_t st = o.s0; st < o.s1; ++st, ++it) {
                 const uint32_t s = it % S::STAGES, b = it % S::ACC, nblk = min(2u, p.nb - 2 * st);
-                if (!tma::mbar_wait_blocking(full_d + b, (it / S::ACC) & 1, abort_flag, &g_tcq_status, 8u)) {
-                    ok = false;
-                    break;
-                }
+                ok = tma::mbar_wait_warp(full_d + b, (it / S::ACC) & 1, abort_flag, &g_tcq_status, 8u);
+                if (!ok) break;
                 tc_fence_after();
                 const uint8_t *stage = tq_smem + s * S::STAGE;
                 const float *wsc = reinterpret_cast<const float *>(stage + S::W_OFF) + rl;
@@ -487,10 +485,8 @@ __global__ void __launch_bounds__(TQ_THREADS, 1) gemm_tcq_kernel(const __grid_co
                 const uint32_t stage = 2 * cur.chunk + st;
                 if (stage >= p.n_it) break;
                 const uint32_t s = it % S::STAGES;
-                if (!tma::mbar_wait_blocking(empty + s, ((it / S::STAGES) & 1) ^ 1, abort_flag, &g_tcq_status, 4u)) {
-                    ok = false;
-                    break;
-                }
+                ok = tma::mbar_wait_warp(empty + s, ((it / S::STAGES) & 1) ^ 1, abort_flag, &g_tcq_status, 4u);
+                if (!ok) break;
 #pragma unroll
                 for (uint32_t half = 0; half < 2; ++half) {
                     float sc, mn;

@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemv_tma_kernel(const TmaParams
                         // every consumer warp) but touch nothing
     for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++i) {
         const int s = (int)(i % (uint32_t)S);
-        if (!dead && !mbar_wait(full + s, (i / S) & 1, abort_flag, 1u)) dead = true;
+        if (!dead && !__all_sync(0xffffffffu, mbar_wait(full + s, (i / S) & 1, abort_flag, 1u))) dead = true;  // (the sums below take the whole warp)
         if (dead) {
             if (wpr > 1) {
                 consumer_bar();

@@ -15,7 +15,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-// One lane of a whole warp.  A warp that issues products runs their loop together, decides together (warp_all) and hands `me`, true for one
+// One lane of a whole warp.  A warp that issues products runs their loop together, waits together (mbar_wait_warp) and hands `me`, true for one
 // lane, to every product and commit, which are predicated instructions then.  A branch around them, into one thread, costs some 230 cycles
 // each time it is taken (B200, cycles for four products of K = 16 and a commit: N 64 525 with a branch, 292 so; N 256 573 and 513, which is the tensor
 // core's rate).
@@ -24,7 +24,6 @@ __device__ __forceinline__ uint32_t elect_one() {
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
     return p;
 }
-__device__ __forceinline__ bool warp_all(bool x) { return __all_sync(0xffffffffu, x); }
 // D[tmem] (+)= A[smem desc] * B[smem desc], kind::f16, issued by the lane for which `me` is true.
 __device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t me) {
     asm volatile(

@@ -1,0 +1,30 @@
+"""Rules of the kernels' bounded waits that no run shows, because they matter once a wait is given up: read from the sources (no GPU needed)."""
+import glob
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "cera_b200", "csrc")
+
+
+def _sources():
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+        yield os.path.basename(path), re.sub(r"//[^\n]*", "", open(path).read())
+
+
+# Waits that a thread makes for itself: it is alone, or meets no instruction that reads other lanes before they are together again.
+BY_THREAD = {"attention_exact.cu": 1,  # the thread that requests V
+             "attention_tc.cu": 2,     # the thread that requests operands
+             "gemm_tc.cu": 2,          # weight producers, each with operands of its own
+             "gemv_exact.cu": 3,       # lanes stay in step: none is missing from what follows
+             "gemv_tma.cu": 1}         # the thread that requests rows
+
+
+def test_a_warp_decides_together_whether_a_wait_was_given_up():
+    alone = {}
+    for name, text in _sources():
+        for call in re.finditer(r"\bmbar_wait(_blocking)?\(", text):
+            ahead = re.split(r"[;{}]", text[:call.start()])[-1]  # the statement's beginning
+            if name == "tma.cuh" or ahead.rstrip().endswith("bool") or "__all_sync(" in ahead:
+                continue
+            alone[name] = alone.get(name, 0) + 1
+    assert alone == BY_THREAD
