@@ -590,11 +590,13 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
                 }
             }
         }
-        // This CTA's shared memory must outlive the last products' arrivals on its barriers (which come after its copies) and, where something gave
-        // up, the copies in flight: the wait then runs out.
-        if (PAIR)
+        // This CTA's shared memory must outlive the copies in flight (they only are when something gave up) and, of a pair, the last products'
+        // arrivals on its barriers: what those wait for includes its copies.
+        if (PAIR || *abort_flag) {
+            uint64_t *last = PAIR ? empty_ab : full_ab;
             for (uint32_t i = it > (uint32_t)S::STAGES ? it - S::STAGES : 0; i < it; ++i)
-                for (uint32_t n = 0; n < tma::SPIN_LIMIT && !tma::mbar_test(empty_ab + i % S::STAGES, (i / S::STAGES) & 1); ++n) __nanosleep(40);
+                for (uint32_t n = 0; n < tma::SPIN_LIMIT && !tma::mbar_test(last + i % S::STAGES, (i / S::STAGES) & 1); ++n) __nanosleep(40);
+        }
     } else {
         // ---------------------------------------------------------------- epilogue: thread = (token lane, 128 rows of one image tile)
         const uint32_t e = warp - 2, quad = warp & 3, hh = e >> 2;  // a warp reaches TMEM lanes [32 (warp % 4), +32)
@@ -791,7 +793,8 @@ __global__ void __launch_bounds__(IMG ? TC_THREADS_IMG : TC_THREADS, 1) gemm_tc_
             const uint32_t tiles_m = (sub.m + TC_BN - 1) / TC_BN;
             const uint8_t *wimg = IMG ? sub.tc + w_sb * TC_STAGES * TC_OP_BYTES : nullptr;
             const uint8_t *wside = IMG ? sub.tc + (size_t)tiles_m * k_sb * TC_STAGES * TC_OP_BYTES + w_sb * TC_SIDE_BYTES : nullptr;
-            for (uint32_t it = 0; it < n_it; ++it) {
+            uint32_t it = 0;
+            for (; it < n_it; ++it) {
                 const uint32_t st = it % TC_STAGES, sb = it / TC_STAGES;
                 if (!tma::mbar_wait_warp(empty_ab + st, ((it / TC_STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u)) break;
                 if (st == 0 && sb >= 2 && !tma::mbar_wait_warp(empty_d + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u)) break;
@@ -804,6 +807,9 @@ __global__ void __launch_bounds__(IMG ? TC_THREADS_IMG : TC_THREADS, 1) gemm_tc_
                     if (IMG) tma::bulk_g2s_if(slot + TC_MINOP_BYTES, wside + (size_t)sb * TC_SIDE_BYTES, TC_SIDE_BYTES, full_ab + st, me);
                 }
             }
+            if (*abort_flag)  // given up: this CTA's shared memory must outlive the copies in flight
+                for (uint32_t i = it > (uint32_t)TC_STAGES ? it - TC_STAGES : 0; i < it; ++i)
+                    for (uint32_t n = 0; n < tma::SPIN_LIMIT && !tma::mbar_test(full_ab + i % TC_STAGES, (i / TC_STAGES) & 1); ++n) __nanosleep(40);
         }
     } else {
         // ---------------------------------------------------------------- epilogue: thread = (token lane, 64 rows)

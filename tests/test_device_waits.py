@@ -28,3 +28,13 @@ def test_a_warp_decides_together_whether_a_wait_was_given_up():
                 continue
             alone[name] = alone.get(name, 0) + 1
     assert alone == BY_THREAD
+
+
+def test_a_loader_that_gave_up_waits_for_its_copies():
+    """Kernels with a warp that requests operands ahead: shared memory may not go to another CTA with a copy on its way into it."""
+    asked = {}
+    for name, text in _sources():
+        for body in text.split("__global__")[1:]:
+            if "tc_commit" in body and re.search(r"\b(bulk|tensor)_g2s\w*\(", body):
+                asked[re.search(r"(\w+_kernel)\(", body).group(1)] = bool(re.search(r"abort_flag\).*mbar_test\(", body, re.S))
+    assert len(asked) == 5 and all(asked.values()), asked
