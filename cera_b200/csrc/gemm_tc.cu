@@ -41,7 +41,7 @@
 //    bytes), warp 9 requests the activation operands, warps 10-17 are the epilogue (thread = token lane x
 //    64 rows) with the running output in a fourth TMEM region.
 // Stages and accumulator buffers are handed over through mbarriers (tcgen05.commit arrives on them when the MMAs have
-// finished).  Every wait is bounded: when a limit runs out the CTA raises an abort flag, its roles leave their loops,
+// finished).  Of a pair, the even CTA's products read both CTAs' stages, and both CTAs' copies count their bytes on its barrier.  Every wait is bounded: when a limit runs out the CTA raises an abort flag, its roles leave their loops,
 // TMEM is freed and a status word reports it (cera_cuda_kernel_status).
 #include <cuda_fp16.h>
 
@@ -51,6 +51,7 @@
 
 #include "gemv_task.cuh"
 #include "tc.cuh"
+#include "tensor_map.h"
 #include "tma.cuh"
 #include "weight.h"
 
@@ -93,9 +94,16 @@ struct Wide {
     static constexpr int KS = Q6 ? 32 : TC_KS, SB_STAGES = 256 / KS;
     static constexpr uint32_t OP = TC_BM * KS * 2, B_TILE = (Q6 ? 2 : 1) * OP, B_TILES = PAIR ? 1 : 2, STAGE = 2 * OP + B_TILES * B_TILE;
     static constexpr int STAGES = 192 * 1024 / STAGE;
-    static constexpr uint32_t DVAL = STAGES * STAGE;           // two slots of d[256]
-    static constexpr uint32_t RS = DVAL + 2 * 2 * TC_BN * 4;   // 2^-s[256] of the min GEMM's weight rows
-    static constexpr uint32_t TAIL = RS + 2 * TC_BN * 4, SMEM = TAIL + 256;
+    static constexpr uint32_t DVAL = STAGES * STAGE;  // two slots of d[256], or of 2^-s[256] of the min GEMM's weight rows
+    static constexpr uint32_t TAIL = DVAL + 2 * 2 * TC_BN * 4, SMEM = TAIL + 256;
+    static constexpr uint32_t X_ROWS = Q6 ? 8 : 16, W_ROWS = 16;  // of TcMaps' boxes
+};
+
+// The operand images as tensors of 1 KB rows: activations (their min GEMM tiles behind them) and up to three weights'.  Only a tensor copy can count its
+// bytes on a barrier of the other CTA of a pair; a box of whole rows lays them down as they are.
+constexpr uint32_t TC_MAP_ROW = 1024;
+struct TcMaps {
+    CUtensorMap x, w[3];
 };
 
 // Regions of a weight's resident image (byte offsets): the operand tile of every (128-row tile, stage); per (tile,
@@ -158,12 +166,13 @@ __device__ __forceinline__ TcTile tc_tile(const TcParams &p, uint32_t b) {
 struct TcSub {
     const uint8_t *tc;
     float *out;
-    uint32_t m, ldc, by;
+    uint32_t m, ldc, by, index;
 };
 __device__ __forceinline__ TcSub tc_select(const TcParams &p, uint32_t y) {
-    TcSub s{p.w.tc, p.out, p.m, p.ldc, y};
+    TcSub s{p.w.tc, p.out, p.m, p.ldc, y, 0};
     if (p.n_w > 1 && y >= p.y_end[0]) {
         const int i = (p.n_w > 2 && y >= p.y_end[1]) ? 1 : 0;
+        s.index = i + 1;
         s.tc = p.tc_x[i];
         s.out = p.out_x[i];
         s.m = p.m_x[i];
@@ -416,15 +425,15 @@ __global__ void __launch_bounds__(TC_BN) tc_weight_min_kernel(const WeightView w
 //    blocks of the whole row after the k loop - weights dmin * mn * 2^s[row] (tc_weight_min_kernel) and activations
 //    g * xs_b * A_b, each as high and low f16 parts, three MMAs per step (the low x low product is below 2^-22) - into
 //    the accumulator buffer of a virtual last super-block.
-// Warps: 0 MMA issue, 1 operand loader, 2-9 epilogue.  In a pair the even CTA's warp 0 issues for both; the odd one's passes on that its stages are full.
+// Warps: 0 MMA issue, 1 operand loader, 2-9 epilogue.  In a pair the even CTA's warp 0 issues for both.
 template <bool Q6, bool PAIR>
-__global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams p) {
+__global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams p, const __grid_constant__ TcMaps maps) {
     using S = Wide<Q6, PAIR>;
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(tc_smem + S::TAIL);
-    uint64_t *full_ab = bars, *empty_ab = full_ab + S::STAGES, *peer_full = empty_ab + S::STAGES, *full_d = peer_full + S::STAGES, *empty_d = full_d + 2,
-             *slot_free = PAIR ? empty_d + 2 : empty_d;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(empty_d + 4);
+    uint64_t *full_ab = bars, *empty_ab = full_ab + S::STAGES, *full_d = empty_ab + S::STAGES, *empty_d = full_d + 2, *full_v = empty_d + 2,
+             *slot_free = PAIR ? full_v + 2 : empty_d;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(full_v + 4);
     volatile uint32_t *abort_flag = tmem_slot + 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t rank = PAIR ? blockIdx.x & 1 : 0;
@@ -436,14 +445,14 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
     const uint32_t n_sb = tile.n_sb, n_it = L.n_sb * S::SB_STAGES, n_mit = L.n_mit, n_rounds = n_sb + (!Q6 && tile.sb0 + n_sb == L.n_sb);
     if (tid == 0) {
         for (int s = 0; s < S::STAGES; ++s) {
-            tma::mbar_init(full_ab + s, 1);    // the loader's expect_tx
-            tma::mbar_init(empty_ab + s, 1);   // the commit of the stage's MMAs
-            tma::mbar_init(peer_full + s, 1);  // the odd CTA's stage is full
+            tma::mbar_init(full_ab + s, 1);   // the loader's expect_tx; the even CTA's counts the bytes of both CTAs
+            tma::mbar_init(empty_ab + s, 1);  // the commit of the stage's MMAs
         }
         for (int b = 0; b < 2; ++b) {
             tma::mbar_init(full_d + b, 1);                                // the commit after a super-block's last MMA
             tma::mbar_init(empty_d + b, (PAIR ? 2 : 1) * TC_EPI_WARPS);  // every epilogue warp (of both CTAs) is done with the buffer
-            if (PAIR) tma::mbar_init(slot_free + b, TC_EPI_WARPS);        // ... of this CTA with the d slot
+            tma::mbar_init(full_v + b, 1);                                // the loader's expect_tx of the d slot
+            if (PAIR) tma::mbar_init(slot_free + b, TC_EPI_WARPS);        // every epilogue warp of this CTA is done with it
         }
         *abort_flag = 0;
         tma::mbar_init_fence();
@@ -469,7 +478,9 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
     const uint32_t tmem = *tmem_slot;
     pdl_wait();
 
-    if (warp == 0 && rank == 0) {
+    if (warp == 0 && rank) {
+        // (the even CTA's issues for both)
+    } else if (warp == 0) {
         // ---------------------------------------------------------------- MMA issue (the whole warp, one lane issues)
         const uint32_t me = elect_one(), idesc = tc_idesc(PAIR ? 2 * TC_BM : TC_BM, PAIR ? 2 * TC_BN : TC_BN);
         auto mma = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
@@ -492,7 +503,7 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
             const uint32_t n_st = sb < n_sb ? (uint32_t)S::SB_STAGES : n_mit;
             for (uint32_t st = 0; st < n_st; ++st, ++it) {
                 const uint32_t s = it % S::STAGES, full = (it / S::STAGES) & 1;
-                ok = arrived(full_ab + s, full, 1u) && (!PAIR || arrived(peer_full + s, full, 1u));
+                ok = arrived(full_ab + s, full, 1u);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t base = tma::smem_u32(tc_smem + s * S::STAGE);
@@ -526,15 +537,6 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
             }
             if (ok) commit(full_d + buf);
         }
-    } else if (warp == 0) {
-        // ---------------------------------------------------------------- odd CTA: its stages are full
-        const uint32_t n_all = n_sb * S::SB_STAGES + (n_rounds > n_sb ? n_mit : 0);
-        for (uint32_t it = 0; it < n_all; ++it) {
-            const uint32_t s = it % S::STAGES;
-            if (!tma::mbar_wait_warp(full_ab + s, (it / S::STAGES) & 1, abort_flag, &g_tc_status, 1u)) break;
-            if (lane == 0) tma::mbar_arrive_cluster(tma::smem_of_rank(peer_full + s, 0));
-            __syncwarp();
-        }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- operands: the whole warp, one lane asks for them (bulk asynchronous copies)
         const uint32_t me = elect_one();
@@ -545,31 +547,55 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
         const uint8_t *w0 = sub.tc + ((size_t)own * n_it + it0) * S::B_TILE, *w1 = sub.tc + ((size_t)t1 * n_it + it0) * S::B_TILE;
         const uint8_t *sd0 = sub.tc + side + ((size_t)t0 * L.n_sb + tile.sb0) * side_step + (Q6 ? 0 : TC_MINOP_BYTES);  // d[128] of a super-block
         const uint8_t *sd1 = sub.tc + side + ((size_t)t1 * L.n_sb + tile.sb0) * side_step + (Q6 ? 0 : TC_MINOP_BYTES);
+        const CUtensorMap *map_w = &maps.w[sub.index];
         uint32_t it = 0;
         bool ok = true;
+        // a stage that is free again; of a pair the even CTA announces what both ask for
+        auto stage = [&](uint32_t bytes) {
+            const uint32_t s = it % S::STAGES;
+            ok = tma::mbar_wait_warp(empty_ab + s, ((it / S::STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u);
+            if (ok) tma::mbar_expect_tx_if(full_ab + s, PAIR ? 2 * bytes : bytes, rank ? 0 : me);
+            return ok;
+        };
+        // `bytes` from `src` (an image's 1 KB row) into the stage
+        auto fetch = [&](const CUtensorMap *map, const uint8_t *base, uint32_t box_rows, uint32_t off, const uint8_t *src, uint32_t bytes) {
+            const uint32_t s = it % S::STAGES;
+            uint8_t *dst = tc_smem + s * S::STAGE + off;
+            if constexpr (PAIR) {
+                const uint32_t bar = tma::smem_of_rank(full_ab + s, 0), row = (uint32_t)((size_t)(src - base) / TC_MAP_ROW);
+                for (uint32_t r = 0; r < bytes / TC_MAP_ROW; r += box_rows) tma::tensor_g2s_2d_pair_if(dst + r * TC_MAP_ROW, map, 0, (int32_t)(row + r), bar, me);
+            } else {
+                tma::bulk_g2s_if(dst, src, bytes, full_ab + s, me);
+            }
+        };
+        auto fetch_x = [&](uint32_t off, const uint8_t *src, uint32_t bytes) { fetch(&maps.x, p.img, S::X_ROWS, off, src, bytes); };
+        auto fetch_w = [&](uint32_t off, const uint8_t *src, uint32_t bytes) { fetch(map_w, sub.tc, S::W_ROWS, off, src, bytes); };
+        // 128 factors of each row tile for this CTA's epilogue, which read the slot last for super-block sb - 2
+        auto factors = [&](uint32_t sb, const uint8_t *f0, const uint8_t *f1) {
+            if (sb >= 2) ok = tma::mbar_wait_warp(slot_free + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u);
+            if (!ok) return false;
+            uint8_t *dv = tc_smem + S::DVAL + (sb & 1) * (2 * TC_BN * 4);
+            tma::mbar_expect_tx_if(full_v + (sb & 1), 2 * TC_BN * 4, me);
+            tma::bulk_g2s_if(dv, f0, TC_BN * 4, full_v + (sb & 1), me);
+            tma::bulk_g2s_if(dv + TC_BN * 4, f1, TC_BN * 4, full_v + (sb & 1), me);
+            return true;
+        };
         for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
             for (uint32_t st = 0; st < (uint32_t)S::SB_STAGES; ++st, ++it) {
-                const uint32_t s = it % S::STAGES;
-                ok = tma::mbar_wait_warp(empty_ab + s, ((it / S::STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u);
-                // the d slot of this super-block was last read by the epilogue of super-block sb - 2
-                if (ok && st == 0 && sb >= 2) ok = tma::mbar_wait_warp(slot_free + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u);
-                if (!ok) break;
-                uint8_t *dst = tc_smem + s * S::STAGE;
-                tma::mbar_expect_tx_if(full_ab + s, S::STAGE + (st == 0 ? 2 * TC_BN * 4 : 0), me);
+                if (!stage(S::STAGE)) break;
                 if constexpr (Q6) {
                     // the 64-k activation stage it / 2 holds [high 16 KB | low 16 KB]; its k half it % 2 is 8 contiguous KB of each
                     const uint8_t *a = img + (size_t)(it >> 1) * (2 * TC_OP_BYTES) + (it & 1) * S::OP;
-                    tma::bulk_g2s_if(dst, a, S::OP, full_ab + s, me);
-                    tma::bulk_g2s_if(dst + S::OP, a + TC_OP_BYTES, S::OP, full_ab + s, me);
+                    fetch_x(0, a, S::OP);
+                    fetch_x(S::OP, a + TC_OP_BYTES, S::OP);
                 } else {
-                    tma::bulk_g2s_if(dst, img + (size_t)it * (2 * TC_OP_BYTES), 2 * TC_OP_BYTES, full_ab + s, me);
+                    fetch_x(0, img + (size_t)it * (2 * TC_OP_BYTES), 2 * TC_OP_BYTES);
                 }
-                tma::bulk_g2s_if(dst + 2 * S::OP, w0 + (size_t)it * S::B_TILE, S::B_TILE, full_ab + s, me);
-                if constexpr (!PAIR) tma::bulk_g2s_if(dst + 2 * S::OP + S::B_TILE, w1 + (size_t)it * S::B_TILE, S::B_TILE, full_ab + s, me);
-                if (st == 0) {
-                    uint8_t *dv = tc_smem + S::DVAL + (sb & 1) * (2 * TC_BN * 4);
-                    tma::bulk_g2s_if(dv, sd0 + (size_t)sb * side_step, TC_BN * 4, full_ab + s, me);
-                    tma::bulk_g2s_if(dv + TC_BN * 4, sd1 + (size_t)sb * side_step, TC_BN * 4, full_ab + s, me);
+                fetch_w(2 * S::OP, w0 + (size_t)it * S::B_TILE, S::B_TILE);
+                if constexpr (!PAIR) fetch_w(2 * S::OP + S::B_TILE, w1 + (size_t)it * S::B_TILE, S::B_TILE);
+                if (st == 0 && !factors(sb, sd0 + (size_t)sb * side_step, sd1 + (size_t)sb * side_step)) {
+                    ++it;
+                    break;
                 }
             }
         }
@@ -577,16 +603,16 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
             const uint8_t *xm = p.xm + (size_t)x_t * n_mit * (2 * TCW_MINT_BYTES);
             const uint8_t *m0 = sub.tc + L.wmin + (size_t)own * n_mit * (2 * TCW_MINT_BYTES), *m1 = sub.tc + L.wmin + (size_t)t1 * n_mit * (2 * TCW_MINT_BYTES);
             for (uint32_t mi = 0; mi < n_mit && ok; ++mi, ++it) {
-                const uint32_t s = it % S::STAGES;
-                if (!tma::mbar_wait_warp(empty_ab + s, ((it / S::STAGES) & 1) ^ 1, abort_flag, &g_tc_status, 8u)) break;
-                uint8_t *dst = tc_smem + s * S::STAGE;
-                tma::mbar_expect_tx_if(full_ab + s, (2 + 2 * S::B_TILES) * TCW_MINT_BYTES + (mi == 0 ? 2 * TC_BN * 4 : 0), me);
-                tma::bulk_g2s_if(dst, xm + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s, me);
-                tma::bulk_g2s_if(dst + 2 * TCW_MINT_BYTES, m0 + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s, me);
-                if constexpr (!PAIR) tma::bulk_g2s_if(dst + 4 * TCW_MINT_BYTES, m1 + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES, full_ab + s, me);
-                if (mi == 0) {  // 2^-s of the CTA's rows (read by the epilogue after the min GEMM)
-                    tma::bulk_g2s_if(tc_smem + S::RS, sub.tc + L.rscale + (size_t)t0 * TC_BN * 4, TC_BN * 4, full_ab + s, me);
-                    tma::bulk_g2s_if(tc_smem + S::RS + TC_BN * 4, sub.tc + L.rscale + (size_t)t1 * TC_BN * 4, TC_BN * 4, full_ab + s, me);
+                if (!stage((2 + 2 * S::B_TILES) * TCW_MINT_BYTES)) break;
+                fetch_x(0, xm + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES);
+                fetch_w(2 * TCW_MINT_BYTES, m0 + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES);
+                if constexpr (!PAIR) fetch_w(4 * TCW_MINT_BYTES, m1 + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES);
+                if (mi == 0) {  // 2^-s of the CTA's rows
+                    const uint8_t *rs = sub.tc + L.rscale;
+                    if (!factors(n_sb, rs + (size_t)t0 * TC_BN * 4, rs + (size_t)t1 * TC_BN * 4)) {
+                        ++it;
+                        break;
+                    }
                 }
             }
         }
@@ -609,13 +635,13 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
         bool ok = true;
         for (uint32_t sb = 0; sb < n_rounds && ok; ++sb) {
             const uint32_t buf = sb & 1;
-            ok = tma::mbar_wait_warp(full_d + buf, (sb >> 1) & 1, abort_flag, &g_tc_status, 16u);
+            ok = tma::mbar_wait_warp(full_v + buf, (sb >> 1) & 1, abort_flag, &g_tc_status, 16u) &&
+                 tma::mbar_wait_warp(full_d + buf, (sb >> 1) & 1, abort_flag, &g_tc_status, 16u);
             if (!ok) break;
             tc_fence_after();
             if (sb == 0) ginv = __ldg(p.ginv + min(col0 + tl, p.n - 1));
             // per super-block: out += d[row] * D / g; after the min GEMM: out -= 2^-s[row] * Dmin / g
-            const float *fac = sb < n_sb ? reinterpret_cast<const float *>(tc_smem + S::DVAL + buf * (2 * TC_BN * 4)) + hh * TC_BN
-                                         : reinterpret_cast<const float *>(tc_smem + S::RS) + hh * TC_BN;
+            const float *fac = reinterpret_cast<const float *>(tc_smem + S::DVAL + buf * (2 * TC_BN * 4)) + hh * TC_BN;
             const float gs = sb < n_sb ? ginv : -ginv;
 #pragma unroll
             for (uint32_t c = 0; c < TC_BN / 32; ++c) {
@@ -1071,9 +1097,22 @@ TcSplit tc_split(uint32_t tiles, uint32_t n_sb, uint32_t slots, uint32_t sb_ns, 
     return parts > 1 ? TcSplit{left, parts} : TcSplit{0, 1};
 }
 
+// img_bytes: the activation images.
 template <bool Q6, bool PAIR>
-int32_t launch_tc_wide(const TcParams &p, uint32_t tiles, cudaStream_t st) {
+int32_t launch_tc_wide(const TcParams &p, uint32_t tiles, size_t img_bytes, cudaStream_t st) {
     using S = Wide<Q6, PAIR>;
+    TcMaps maps{};
+    if (PAIR) {
+        auto rows = [](CUtensorMap *map, const void *base, size_t bytes, uint32_t box_rows) {
+            return tensor_map_2d(map, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, base, bytes / TC_MAP_ROW, TC_MAP_ROW / 4, TC_MAP_ROW / 4, box_rows, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+        };
+        CERA_TRY(rows(&maps.x, p.img, img_bytes, S::X_ROWS));
+        for (uint32_t i = 0; i < p.n_w; ++i) {
+            const TcImage L = tc_image_layout(i ? p.m_x[i - 1] : p.m, p.k);
+            CERA_TRY(rows(&maps.w[i], i ? p.tc_x[i - 1] : p.w.tc, Q6 ? (size_t)L.tiles * (p.k / S::KS) * S::B_TILE : L.rscale, S::W_ROWS));
+        }
+    }
     static thread_local int configured_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1082,8 +1121,8 @@ int32_t launch_tc_wide(const TcParams &p, uint32_t tiles, cudaStream_t st) {
         configured_dev = dev;
     }
     count_launch();
-    if (PAIR) return check_cuda(launch_pairs(gemm_tcw_kernel<Q6, PAIR>, tiles, dim3(TCW_THREADS), (size_t)S::SMEM, st, p), "gemm (tcgen05, pairs) launch");
-    return check_cuda(launch_k(gemm_tcw_kernel<Q6, PAIR>, dim3(tiles), dim3(TCW_THREADS), (size_t)S::SMEM, st, p), "gemm (tcgen05, wide) launch");
+    if (PAIR) return check_cuda(launch_pairs(gemm_tcw_kernel<Q6, PAIR>, tiles, dim3(TCW_THREADS), (size_t)S::SMEM, st, p, maps), "gemm (tcgen05, pairs) launch");
+    return check_cuda(launch_k(gemm_tcw_kernel<Q6, PAIR>, dim3(tiles), dim3(TCW_THREADS), (size_t)S::SMEM, st, p, maps), "gemm (tcgen05, wide) launch");
 }
 
 }  // namespace
@@ -1255,9 +1294,10 @@ int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, s
     p.partial = partial;
     const uint32_t work = p.whole + split.left * split.parts;
     if (rc == CERA_CUDA_OK && pair) {
-        rc = q6 ? launch_tc_wide<true, true>(p, work, st) : launch_tc_wide<false, true>(p, work, st);
+        const size_t images = img_bytes + min_bytes + xm_bytes;
+        rc = q6 ? launch_tc_wide<true, true>(p, work, images, st) : launch_tc_wide<false, true>(p, work, images, st);
     } else if (rc == CERA_CUDA_OK && wide) {
-        rc = launch_tc_wide<false, false>(p, work, st);
+        rc = launch_tc_wide<false, false>(p, work, 0, st);
     } else if (rc == CERA_CUDA_OK) {
         if (w.tc)
             rc = w.type == CERA_TYPE_Q4_K ? launch_tc_typed<CERA_TYPE_Q4_K, true>(p, work, st) : launch_tc_typed<CERA_TYPE_Q5_K, true>(p, work, st);

@@ -1,7 +1,8 @@
 // mbarrier, bulk-copy (TMA unit) and asynchronous-copy helpers for kernels that stage global memory through a
 // ring of shared-memory stages.  Every wait is bounded: when the limit runs out the waiter raises the CTA's
 // abort flag (so the CTA's other waits give up at once) and ORs `who` into a status word in device
-// memory that the host reads through cera_cuda_kernel_status.  No copy is addressed to another CTA.
+// memory that the host reads through cera_cuda_kernel_status.  Copies go to this CTA's shared memory; of a pair they may
+// count their bytes on the other CTA's barrier.
 #pragma once
 
 #include "common.cuh"
@@ -105,8 +106,8 @@ __device__ __forceinline__ uint32_t smem_of_rank(const void *p, uint32_t rank) {
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
     return a;
 }
-// What is handed over with it is no memory that threads wrote: copies that have landed, TMEM that has been read.  So the plain form does; with
-// .release.cluster here and .acquire.cluster in the waits each hand-over of a stage took some 700 cycles (512 tokens x 4096 x 14336: 190 us, 118 so).
+// Its scope is this CTA: what it may hand over is TMEM that has been read (tcgen05.wait::ld, and tc_fence_before ahead of it), never memory.  Operands that
+// the other CTA's products read are handed over by their own tensor copies, which count their bytes on that CTA's barrier (tensor_g2s_2d_pair_if).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }

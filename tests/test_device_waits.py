@@ -38,3 +38,13 @@ def test_a_loader_that_gave_up_waits_for_its_copies():
             if "tc_commit" in body and re.search(r"\b(bulk|tensor)_g2s\w*\(", body):
                 asked[re.search(r"(\w+_kernel)\(", body).group(1)] = bool(re.search(r"abort_flag\).*mbar_test\(", body, re.S))
     assert len(asked) == 5 and all(asked.values()), asked
+
+
+def test_a_plain_arrival_at_another_cta_hands_over_tmem_only():
+    """Its scope is the CTA it comes from: what that CTA's copies or threads wrote to memory is not part of it."""
+    seen = 0
+    for name, text in _sources():
+        for call in re.finditer(r"\bmbar_arrive_cluster\(tma::", text):
+            seen += 1
+            assert "tc_fence_before();" in text[:call.start()][-250:], name
+    assert seen == 2
