@@ -31,8 +31,8 @@
 // 16-byte core matrices), 64 k-elements per stage.
 //
 // Two kernels:
-//  * gemm_tcw_kernel<Q6, PAIR> ("wide", image only): 128 tokens x 256 rows per CTA, or 256 x 256 per pair of CTAs, when those tiles
-//    fill the device.  TMEM holds two double-buffered 256-column accumulators; the running output lives in the epilogue
+//  * gemm_tcw_kernel<Q6, PAIR, TILES> ("wide", image only): 128 tokens x 256 rows per CTA, or 256 x 256 per pair of CTAs, when those tiles
+//    fill the device (Q6_K: pairs, or 128 x 128).  TMEM holds two double-buffered 256-column accumulators; the running output lives in the epilogue
 //    threads' registers; the min term is one more GEMM over the k / 32 blocks after the k loop.  Q6_K: sc * (q - 32) needs
 //    13 bits, so the image holds it as two exact f16 operands and a k-step is three MMAs; no min term.
 //  * gemm_tc_kernel<T, IMG>: 128 x 128 per CTA.  IMG: the loader fetches all three operands, the min term is the
@@ -88,14 +88,16 @@ constexpr uint32_t TC_KC_STRIDE = TC_BM * 16;                            // byte
 constexpr uint32_t TCW_MIN_J = 32;                                        // activation blocks (k / 32 columns) per min stage
 constexpr uint32_t TCW_MINT_BYTES = TC_BM * TCW_MIN_J * 2;                // one min-GEMM operand tile: 8 KB
 constexpr int TCW_THREADS = (2 + TC_EPI_WARPS) * 32;
-// Per CTA: A high and low of its 128 tokens, and of B both row tiles or, in a pair, its own.  Q6_K: stages of 32 k, B in two operands per row tile.
-template <bool Q6, bool PAIR>
+// Per CTA: A high and low of its 128 tokens, and of B the row tiles or, in a pair, its own of the two.  Q6_K: stages of 32 k, B in two operands per row tile.
+template <bool Q6, bool PAIR, int TILES>
 struct Wide {
+    static_assert(!PAIR || TILES == 2, "a pair has a row tile each");
     static constexpr int KS = Q6 ? 32 : TC_KS, SB_STAGES = 256 / KS;
-    static constexpr uint32_t OP = TC_BM * KS * 2, B_TILE = (Q6 ? 2 : 1) * OP, B_TILES = PAIR ? 1 : 2, STAGE = 2 * OP + B_TILES * B_TILE;
+    static constexpr uint32_t ROWS = TILES * TC_BN;  // weight rows of a tile
+    static constexpr uint32_t OP = TC_BM * KS * 2, B_TILE = (Q6 ? 2 : 1) * OP, B_TILES = PAIR ? 1 : TILES, STAGE = 2 * OP + B_TILES * B_TILE;
     static constexpr int STAGES = 192 * 1024 / STAGE;
-    static constexpr uint32_t DVAL = STAGES * STAGE;  // two slots of d[256], or of 2^-s[256] of the min GEMM's weight rows
-    static constexpr uint32_t TAIL = DVAL + 2 * 2 * TC_BN * 4, SMEM = TAIL + 256;
+    static constexpr uint32_t DVAL = STAGES * STAGE;  // two slots of d[ROWS], or of 2^-s[ROWS] of the min GEMM's weight rows
+    static constexpr uint32_t TAIL = DVAL + 2 * ROWS * 4, SMEM = TAIL + 256;
     static constexpr uint32_t X_ROWS = Q6 ? 8 : 16, W_ROWS = 16;  // of TcMaps' boxes
 };
 
@@ -414,21 +416,21 @@ __global__ void __launch_bounds__(TC_BN) tc_weight_min_kernel(const WeightView w
     }
 }
 
-// The wide kernel, over resident images.  Alone a CTA does 128 tokens x 256 weight rows (two 128-row tiles of the image); in a PAIR (cta_group::2)
+// The wide kernel, over resident images.  Alone a CTA does 128 tokens x TILES row tiles (of 128) of the image; in a PAIR (cta_group::2)
 // two CTAs do 256 tokens x 256 rows, each with its own 128 tokens and one of the row tiles, which the tensor cores of both read.
 // What bounds it: shared memory, which a CTA alone reads and writes 192 KB per 64 k (its 16 products of N = 128 take 1212 cycles in a ring without an
 // epilogue and 1370 with it, 1024 being the tensor core's rate), in a pair 112 KB; and then the chip's power, which holds the clock near 1.45 GHz.
 // 512 tokens: gate / up 28672 x 4096 212 us alone, 194 in pairs; Q6_K 4096 x 14336 168 us with 128 x 128 tiles, 119 in pairs.
 // TMEM holds nothing but the two double-buffered accumulators (2 x 256 columns), so
-//  * the running output lives in the epilogue threads' registers (thread = token lane x 128 rows), and
+//  * the running output lives in the epilogue threads' registers (thread = token lane x half of the tile's rows), and
 //  * the min term sum_b dmin * mn_b * (xs_b * A_b) is not accumulated per super-block but as ONE more GEMM over the k / 32
 //    blocks of the whole row after the k loop - weights dmin * mn * 2^s[row] (tc_weight_min_kernel) and activations
 //    g * xs_b * A_b, each as high and low f16 parts, three MMAs per step (the low x low product is below 2^-22) - into
 //    the accumulator buffer of a virtual last super-block.
 // Warps: 0 MMA issue, 1 operand loader, 2-9 epilogue.  In a pair the even CTA's warp 0 issues for both.
-template <bool Q6, bool PAIR>
+template <bool Q6, bool PAIR, int TILES>
 __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams p, const __grid_constant__ TcMaps maps) {
-    using S = Wide<Q6, PAIR>;
+    using S = Wide<Q6, PAIR, TILES>;
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(tc_smem + S::TAIL);
     uint64_t *full_ab = bars, *empty_ab = full_ab + S::STAGES, *full_d = empty_ab + S::STAGES, *empty_d = full_d + 2, *full_v = empty_d + 2,
@@ -439,7 +441,7 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
     const uint32_t rank = PAIR ? blockIdx.x & 1 : 0;
     const TcTile tile = tc_tile(p, PAIR ? blockIdx.x / 2 : blockIdx.x);
     const TcSub sub = tc_select(p, tile.y);
-    const uint32_t col0 = (PAIR ? 2 * tile.x + rank : tile.x) * TC_BM, row0 = sub.by * 2 * TC_BN;
+    const uint32_t col0 = (PAIR ? 2 * tile.x + rank : tile.x) * TC_BM, row0 = sub.by * S::ROWS;
     const TcImage L = tc_image_layout(sub.m, p.k);
     // loops count the super-blocks of this CTA; the min GEMM goes with the last share
     const uint32_t n_sb = tile.n_sb, n_it = L.n_sb * S::SB_STAGES, n_mit = L.n_mit, n_rounds = n_sb + (!Q6 && tile.sb0 + n_sb == L.n_sb);
@@ -540,7 +542,7 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
     } else if (warp == 1) {
         // ---------------------------------------------------------------- operands: the whole warp, one lane asks for them (bulk asynchronous copies)
         const uint32_t me = elect_one();
-        const uint32_t t0 = min(2 * sub.by, L.tiles - 1), t1 = min(2 * sub.by + 1, L.tiles - 1);  // (an odd last tile is read twice)
+        const uint32_t t0 = min(TILES * sub.by, L.tiles - 1), t1 = min(TILES * sub.by + 1, L.tiles - 1);  // (an odd last tile is read twice)
         const uint32_t x_t = min(col0, p.n - 1) / TC_BM, own = rank ? t1 : t0, it0 = tile.sb0 * S::SB_STAGES;  // (as an odd last token tile is in a pair)
         const size_t side = Q6 ? (size_t)L.tiles * n_it * S::B_TILE : L.side, side_step = Q6 ? TC_BN * 4 : TC_SIDE_BYTES;
         const uint8_t *img = p.img + ((size_t)x_t * L.n_sb + tile.sb0) * (256 / TC_KS) * (2 * TC_OP_BYTES);
@@ -574,10 +576,10 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
         auto factors = [&](uint32_t sb, const uint8_t *f0, const uint8_t *f1) {
             if (sb >= 2) ok = tma::mbar_wait_warp(slot_free + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u);
             if (!ok) return false;
-            uint8_t *dv = tc_smem + S::DVAL + (sb & 1) * (2 * TC_BN * 4);
-            tma::mbar_expect_tx_if(full_v + (sb & 1), 2 * TC_BN * 4, me);
+            uint8_t *dv = tc_smem + S::DVAL + (sb & 1) * (S::ROWS * 4);
+            tma::mbar_expect_tx_if(full_v + (sb & 1), S::ROWS * 4, me);
             tma::bulk_g2s_if(dv, f0, TC_BN * 4, full_v + (sb & 1), me);
-            tma::bulk_g2s_if(dv + TC_BN * 4, f1, TC_BN * 4, full_v + (sb & 1), me);
+            if constexpr (TILES == 2) tma::bulk_g2s_if(dv + TC_BN * 4, f1, TC_BN * 4, full_v + (sb & 1), me);
             return true;
         };
         for (uint32_t sb = 0; sb < n_sb && ok; ++sb) {
@@ -592,7 +594,7 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
                     fetch_x(0, img + (size_t)it * (2 * TC_OP_BYTES), 2 * TC_OP_BYTES);
                 }
                 fetch_w(2 * S::OP, w0 + (size_t)it * S::B_TILE, S::B_TILE);
-                if constexpr (!PAIR) fetch_w(2 * S::OP + S::B_TILE, w1 + (size_t)it * S::B_TILE, S::B_TILE);
+                if constexpr (S::B_TILES == 2) fetch_w(2 * S::OP + S::B_TILE, w1 + (size_t)it * S::B_TILE, S::B_TILE);
                 if (st == 0 && !factors(sb, sd0 + (size_t)sb * side_step, sd1 + (size_t)sb * side_step)) {
                     ++it;
                     break;
@@ -606,7 +608,7 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
                 if (!stage((2 + 2 * S::B_TILES) * TCW_MINT_BYTES)) break;
                 fetch_x(0, xm + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES);
                 fetch_w(2 * TCW_MINT_BYTES, m0 + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES);
-                if constexpr (!PAIR) fetch_w(4 * TCW_MINT_BYTES, m1 + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES);
+                if constexpr (S::B_TILES == 2) fetch_w(4 * TCW_MINT_BYTES, m1 + (size_t)mi * (2 * TCW_MINT_BYTES), 2 * TCW_MINT_BYTES);
                 if (mi == 0) {  // 2^-s of the CTA's rows
                     const uint8_t *rs = sub.tc + L.rscale;
                     if (!factors(n_sb, rs + (size_t)t0 * TC_BN * 4, rs + (size_t)t1 * TC_BN * 4)) {
@@ -624,13 +626,14 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
                 for (uint32_t n = 0; n < tma::SPIN_LIMIT && !tma::mbar_test(last + i % S::STAGES, (i / S::STAGES) & 1); ++n) __nanosleep(40);
         }
     } else {
-        // ---------------------------------------------------------------- epilogue: thread = (token lane, 128 rows of one image tile)
+        // ---------------------------------------------------------------- epilogue: thread = (token lane, R rows of one image tile)
         const uint32_t e = warp - 2, quad = warp & 3, hh = e >> 2;  // a warp reaches TMEM lanes [32 (warp % 4), +32)
         const uint32_t tl = quad * 32 + lane;
-        const uint32_t lane_addr = tmem + ((quad * 32) << 16) + hh * TC_BN;
-        float acc[TC_BN];
+        constexpr int R = S::ROWS / 2;
+        const uint32_t lane_addr = tmem + ((quad * 32) << 16) + hh * R;
+        float acc[R];
 #pragma unroll
-        for (int i = 0; i < TC_BN; ++i) acc[i] = 0.0f;
+        for (int i = 0; i < R; ++i) acc[i] = 0.0f;
         float ginv = 1.0f;
         bool ok = true;
         for (uint32_t sb = 0; sb < n_rounds && ok; ++sb) {
@@ -641,10 +644,10 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
             tc_fence_after();
             if (sb == 0) ginv = __ldg(p.ginv + min(col0 + tl, p.n - 1));
             // per super-block: out += d[row] * D / g; after the min GEMM: out -= 2^-s[row] * Dmin / g
-            const float *fac = reinterpret_cast<const float *>(tc_smem + S::DVAL + buf * (2 * TC_BN * 4)) + hh * TC_BN;
+            const float *fac = reinterpret_cast<const float *>(tc_smem + S::DVAL + buf * (S::ROWS * 4)) + hh * R;
             const float gs = sb < n_sb ? ginv : -ginv;
 #pragma unroll
-            for (uint32_t c = 0; c < TC_BN / 32; ++c) {
+            for (uint32_t c = 0; c < R / 32; ++c) {
                 uint32_t v0[16], v1[16];
                 tmem_ld16(lane_addr + buf * 2 * TC_BN + c * 32, v0);
                 tmem_ld16(lane_addr + buf * 2 * TC_BN + c * 32 + 16, v1);
@@ -670,16 +673,16 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
             }
         }
         if (ok && tile.slot != TC_WHOLE) {
-            float *o = p.partial + (size_t)(PAIR ? 2 * tile.slot + rank : tile.slot) * (2 * TC_BN * TC_BM) + hh * TC_BN * TC_BM + tl;
+            float *o = p.partial + (size_t)(PAIR ? 2 * tile.slot + rank : tile.slot) * (S::ROWS * TC_BM) + hh * R * TC_BM + tl;
 #pragma unroll
-            for (int i = 0; i < TC_BN; ++i) o[i * TC_BM] = acc[i];
+            for (int i = 0; i < R; ++i) o[i * TC_BM] = acc[i];
         } else if (ok && col0 + tl < p.n) {
-            // ---- the thread's 128 cells -> global memory: cell (row i, token j) at out[i * ldy + j * ldc]
-            const uint32_t r0 = row0 + hh * TC_BN;
+            // ---- the thread's cells -> global memory: cell (row i, token j) at out[i * ldy + j * ldc]
+            const uint32_t r0 = row0 + hh * R;
             float *o = sub.out + (size_t)r0 * p.ldy + (size_t)(col0 + tl) * sub.ldc;
-            if (p.ldy == 1 && r0 + TC_BN <= sub.m && ((uintptr_t)o & 15) == 0) {  // token-major output: 512 contiguous bytes
+            if (p.ldy == 1 && r0 + R <= sub.m && ((uintptr_t)o & 15) == 0) {  // token-major output: 4 R contiguous bytes
 #pragma unroll
-                for (int i = 0; i < TC_BN / 4; ++i) {
+                for (int i = 0; i < R / 4; ++i) {
                     float4 v = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
                     float4 *o4 = reinterpret_cast<float4 *>(o) + i;
                     if (p.epilogue == EPI_ADD) {
@@ -690,7 +693,7 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
                 }
             } else {
 #pragma unroll
-                for (int i = 0; i < TC_BN; ++i)
+                for (int i = 0; i < R; ++i)
                     if (r0 + i < sub.m) {
                         float *oi = o + (size_t)i * p.ldy;
                         *oi = p.epilogue == EPI_ADD ? __fadd_rn(*oi, acc[i]) : acc[i];
@@ -1004,9 +1007,10 @@ int32_t launch_tc_typed(const TcParams &p, uint32_t ctas, cudaStream_t st) {
 // f16 holds exactly.  The image therefore keeps B as TWO exact f16 operands, B with its lowest bit cleared (an even
 // integer up to 4096) and that bit (0 or 1); per k-step the kernel issues three MMAs into one accumulator - even part x
 // activations high, even part x activations low, low bit x activations high (low bit x activations low is below 2^-22
-// of the sum) - and the epilogue is out += d * D / g per super-block (Q6_K has no min term).  128 tokens x 128 rows per
-// CTA, stages of 32 k (activations 2 x 8 KB out of the 64-k tiles of tc_token_image_kernel, weights 16 KB), six stages.
-constexpr int TC6_KS = Wide<true, true>::KS;
+// of the sum) - and the epilogue is out += d * D / g per super-block (Q6_K has no min term): gemm_tcw_kernel, by
+// pairs of CTAs or 128 x 128 alone (tc6_alone), in stages of 32 k (activations 2 x 8 KB out of the 64-k tiles of tc_token_image_kernel, weights 16 KB), six
+// of them.
+constexpr int TC6_KS = Wide<true, true, 2>::KS;
 constexpr uint32_t TC6_HALF = TC_OP_BYTES / 2;  // one operand tile of a 32-k stage: 8 KB
 
 // Image of a Q6_K weight: per (128-row tile, 32-k stage) [even part 8 KB | low bit 8 KB], then per (tile, super-block)
@@ -1084,6 +1088,7 @@ __global__ void __launch_bounds__(256) tc_parts_kernel(const TcParams p, uint32_
 // 448 tiles of 128 x 256 on 148 SMs, k = 4096 (gate / up of 512 tokens: three rounds and four tiles): 280 us whole, 212 shared; 32 tiles of 128 x 128
 // (4096 x 64 x 4096, the whole product) 63 us whole, 35 in eight shares each.
 constexpr uint32_t TC_SHARES = 3;  // partial tiles a slot has room for
+constexpr uint32_t TC6_PAIR_SB_NS = 4000;
 struct TcSplit {
     uint32_t left, parts;
 };
@@ -1097,10 +1102,21 @@ TcSplit tc_split(uint32_t tiles, uint32_t n_sb, uint32_t slots, uint32_t sb_ns, 
     return parts > 1 ? TcSplit{left, parts} : TcSplit{0, 1};
 }
 
+// Q6_K: whether 128 x 128 tiles of single CTAs are expected to finish before pairs, whose tiles, shared ones too, each take some 12 us beside their
+// 3.6 a super-block; 6 and 3.2 alone.  us, alone / pairs: 4096 x 512 x 384 26 / 33, 8192 x 1024 x 200 32 / 38, 14336 x 512 x 640 66 / 72; 4096 x 512 x 640
+// 41 / 35, 4096 x 2048 x 500 53 / 44.
+bool tc6_alone(uint32_t tiles, uint32_t m, uint32_t n_sb) {
+    const uint32_t sms = (uint32_t)sm_count(), slots = sms / 2, ones = tiles * ((m + TC_BN - 1) / TC_BN), pairs = (tiles + 1) / 2 * ((m + 2 * TC_BN - 1) / (2 * TC_BN));
+    const TcSplit s = tc_split(pairs, n_sb, slots, TC6_PAIR_SB_NS, 4 * TC_BN);
+    const uint32_t whole = s.left ? pairs / slots : (pairs + slots - 1) / slots, shared = s.left ? (s.left * s.parts + slots - 1) / slots : 0;
+    const uint64_t t_pairs = whole * (12000ull + 3600 * n_sb) + shared * (14000ull + 3600 * ((n_sb + s.parts - 1) / s.parts));
+    return (ones + sms - 1) / sms * (6000ull + 3200 * n_sb) <= t_pairs;
+}
+
 // img_bytes: the activation images.
-template <bool Q6, bool PAIR>
+template <bool Q6, bool PAIR, int TILES>
 int32_t launch_tc_wide(const TcParams &p, uint32_t tiles, size_t img_bytes, cudaStream_t st) {
-    using S = Wide<Q6, PAIR>;
+    using S = Wide<Q6, PAIR, TILES>;
     TcMaps maps{};
     if (PAIR) {
         auto rows = [](CUtensorMap *map, const void *base, size_t bytes, uint32_t box_rows) {
@@ -1117,12 +1133,12 @@ int32_t launch_tc_wide(const TcParams &p, uint32_t tiles, size_t img_bytes, cuda
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_dev != dev) {
-        CERA_CUDA_TRY(cudaFuncSetAttribute(gemm_tcw_kernel<Q6, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
+        CERA_CUDA_TRY(cudaFuncSetAttribute(gemm_tcw_kernel<Q6, PAIR, TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
         configured_dev = dev;
     }
     count_launch();
-    if (PAIR) return check_cuda(launch_pairs(gemm_tcw_kernel<Q6, PAIR>, tiles, dim3(TCW_THREADS), (size_t)S::SMEM, st, p, maps), "gemm (tcgen05, pairs) launch");
-    return check_cuda(launch_k(gemm_tcw_kernel<Q6, PAIR>, dim3(tiles), dim3(TCW_THREADS), (size_t)S::SMEM, st, p, maps), "gemm (tcgen05, wide) launch");
+    if (PAIR) return check_cuda(launch_pairs(gemm_tcw_kernel<Q6, PAIR, TILES>, tiles, dim3(TCW_THREADS), (size_t)S::SMEM, st, p, maps), "gemm (tcgen05, pairs) launch");
+    return check_cuda(launch_k(gemm_tcw_kernel<Q6, PAIR, TILES>, dim3(tiles), dim3(TCW_THREADS), (size_t)S::SMEM, st, p, maps), "gemm (tcgen05, wide) launch");
 }
 
 }  // namespace
@@ -1222,21 +1238,22 @@ int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, s
     const size_t need = img_bytes + min_bytes + xm_bytes + (size_t)n_pad * 8;
     // With weight images: the wide kernel when its 128 x 256 tiles alone fill the device, in pairs unless they would leave a quarter of their tokens
     // empty (one or three token tiles); else the 128 x 128 one.  Whole products, 128 x 128, wide, pairs: 28672 x 4096 x 512 255, 227, 204 us;
-    // 6144 x 2047 228, 222, 200; 4096 x 384 57, 52, 55; 4096 x 512 58, 60, 63.  Q6_K takes pairs at every size it has.
+    // 6144 x 2047 228, 222, 200; 4096 x 384 57, 52, 55; 4096 x 512 58, 60, 63.  Q6_K: tc6_alone.
     static const int tile_pref = [] {
         const char *e = getenv("CERA_CUDA_GEMM_TILE");
         return e ? atoi(e) : 0;
     }();
     uint32_t wide_y = 0;
     for (int i = 0; i < count; ++i) wide_y += (t[i].w.m + 2 * TC_BN - 1) / (2 * TC_BN);
-    const bool q6 = w.type == CERA_TYPE_Q6_K, fills = tiles * wide_y >= 120, pair = q6 || (w.tc && tile_pref == 0 && fills && (tiles % 2 == 0 || tiles >= 5));
-    const bool wide = !pair && w.tc && (tile_pref == 256 || (tile_pref != 128 && fills));
+    const bool q6 = w.type == CERA_TYPE_Q6_K, fills = tiles * wide_y >= 120;
+    const bool pair = q6 ? tile_pref != 128 && !tc6_alone(tiles, w.m, n_sb) : w.tc && tile_pref == 0 && fills && (tiles % 2 == 0 || tiles >= 5);
+    const bool wide = !pair && !q6 && w.tc && (tile_pref == 256 || (tile_pref != 128 && fills));
     const uint32_t rows = pair || wide ? 2 * TC_BN : TC_BN, halves = pair ? 2 : 1, x_tiles = (tiles + halves - 1) / halves;
     uint32_t y = 0;
     for (int i = 0; i < count; ++i) y += (t[i].w.m + rows - 1) / rows;
     // (nanoseconds of a super-block, as measured: Q6_K in pairs, pairs, wide, 128 x 128)
-    const uint32_t sb_ns = q6 ? 4000 : pair ? 2900 : wide ? 3600 : 1650;
-    TcSplit split = w.tc ? tc_split(x_tiles * y, n_sb, (uint32_t)sm_count() / halves, sb_ns, halves * rows) : TcSplit{0, 1};
+    const uint32_t sb_ns = q6 ? TC6_PAIR_SB_NS : pair ? 2900 : wide ? 3600 : 1650;
+    TcSplit split = w.tc && (pair || !q6) ? tc_split(x_tiles * y, n_sb, (uint32_t)sm_count() / halves, sb_ns, halves * rows) : TcSplit{0, 1};
     // partial sums of the tiles that are shared; without room for them the tiles stay whole
     const size_t parts_bytes = (size_t)split.left * split.parts * halves * rows * TC_BM * 4;
     const bool borrowed = lent.p && lent.bytes >= need;
@@ -1295,9 +1312,11 @@ int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, s
     const uint32_t work = p.whole + split.left * split.parts;
     if (rc == CERA_CUDA_OK && pair) {
         const size_t images = img_bytes + min_bytes + xm_bytes;
-        rc = q6 ? launch_tc_wide<true, true>(p, work, images, st) : launch_tc_wide<false, true>(p, work, images, st);
+        rc = q6 ? launch_tc_wide<true, true, 2>(p, work, images, st) : launch_tc_wide<false, true, 2>(p, work, images, st);
     } else if (rc == CERA_CUDA_OK && wide) {
-        rc = launch_tc_wide<false, false>(p, work, 0, st);
+        rc = launch_tc_wide<false, false, 2>(p, work, 0, st);
+    } else if (rc == CERA_CUDA_OK && q6) {
+        rc = launch_tc_wide<true, false, 1>(p, work, 0, st);
     } else if (rc == CERA_CUDA_OK) {
         if (w.tc)
             rc = w.type == CERA_TYPE_Q4_K ? launch_tc_typed<CERA_TYPE_Q4_K, true>(p, work, st) : launch_tc_typed<CERA_TYPE_Q5_K, true>(p, work, st);

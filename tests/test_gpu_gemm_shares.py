@@ -17,9 +17,10 @@ def test_shared_tiles_equal_whole_ones(t, rows, x_tiles, beyond, k):
     check(t, (sms + beyond + x_tiles - 1) // x_tiles * rows - 5, x_tiles * 128 - 3, k)
 
 
-# odd token tiles (a pair's last half is empty; one and three tiles go without pairs), odd row tiles, a row and a token beyond a tile
+# Q6_K on both sides of its line between pairs and single CTAs (short k); odd token tiles (a pair's last half is empty; one and three tiles go without pairs), odd row tiles, a row and a token beyond a tile
 @pytest.mark.parametrize("t", [O.Q4_K, O.Q5_K, O.Q6_K])
-@pytest.mark.parametrize("m,n,k", [(6145, 602, 1024), (6528, 513, 2048), (30800, 100, 512), (30721, 129, 256), (10300, 257, 768), (700, 1000, 2304)])
+@pytest.mark.parametrize("m,n,k", [(6145, 602, 1024), (6528, 513, 2048), (30800, 100, 512), (30721, 129, 256), (10300, 257, 768), (700, 1000, 2304),
+                                   (4093, 500, 512), (1000, 140, 256), (8190, 200, 1024), (4096, 640, 512)])
 def test_pairs_equal_small_products(t, m, n, k):
     check(t, m, n, k)
 
