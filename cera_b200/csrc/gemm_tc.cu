@@ -1223,8 +1223,9 @@ int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, s
     if (off || count < 1 || count > 3 || n <= 32) return CERA_CUDA_OK;
     const WeightView &w = t[0].w;
     if (w.k % 256 || (w.type != CERA_TYPE_Q4_K && w.type != CERA_TYPE_Q5_K && w.type != CERA_TYPE_Q6_K)) return CERA_CUDA_OK;
-    // Q6_K: only over its image, and only with at least two token tiles (a single tile of a long-k matrix leaves each of
-    // the few CTAs a serial walk that the warp-level kernel's split-k clusters beat: 189 against 111 us at 4096 x 14336 x 64)
+    // Q6_K: only over its image, and only with at least two token tiles: one is mostly left to the kernel from quantized bytes (that one / pairs, us, 64 and
+    // 128 columns: 4096 x 14336 72 / 83 and 89 / 85, 14336 x 4096 74 / 87 and 91 / 87, 4096 x 4096 34 / 42 and 39 / 42; pairs would gain below its 48 columns
+    // on large matrices, 33 columns of 4096 x 14336 116 / 83).
     if (w.type == CERA_TYPE_Q6_K && (!w.tc || n <= 128 || count > 1)) return CERA_CUDA_OK;
     for (int i = 1; i < count; ++i)  // several weights: the same k, Q4_K / Q5_K, every one with its image
         if (t[i].w.k != w.k || !t[i].w.tc || !w.tc || (t[i].w.type != CERA_TYPE_Q4_K && t[i].w.type != CERA_TYPE_Q5_K)) return CERA_CUDA_OK;
