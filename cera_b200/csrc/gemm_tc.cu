@@ -1008,7 +1008,7 @@ int32_t launch_tc_typed(const TcParams &p, uint32_t ctas, cudaStream_t st) {
 // integer up to 4096) and that bit (0 or 1); per k-step the kernel issues three MMAs into one accumulator - even part x
 // activations high, even part x activations low, low bit x activations high (low bit x activations low is below 2^-22
 // of the sum) - and the epilogue is out += d * D / g per super-block (Q6_K has no min term): gemm_tcw_kernel, by
-// pairs of CTAs or 128 x 128 alone (tc6_alone), in stages of 32 k (activations 2 x 8 KB out of the 64-k tiles of tc_token_image_kernel, weights 16 KB), six
+// pairs of CTAs or 128 x 128 alone (tc_pairs), in stages of 32 k (activations 2 x 8 KB out of the 64-k tiles of tc_token_image_kernel, weights 16 KB), six
 // of them.
 constexpr int TC6_KS = Wide<true, true, 2>::KS;
 constexpr uint32_t TC6_HALF = TC_OP_BYTES / 2;  // one operand tile of a 32-k stage: 8 KB
@@ -1088,7 +1088,7 @@ __global__ void __launch_bounds__(256) tc_parts_kernel(const TcParams p, uint32_
 // 448 tiles of 128 x 256 on 148 SMs, k = 4096 (gate / up of 512 tokens: three rounds and four tiles): 280 us whole, 212 shared; 32 tiles of 128 x 128
 // (4096 x 64 x 4096, the whole product) 63 us whole, 35 in eight shares each.
 constexpr uint32_t TC_SHARES = 3;  // partial tiles a slot has room for
-constexpr uint32_t TC6_PAIR_SB_NS = 4000;
+constexpr uint32_t TC_SB_NS = 1650, TC_WIDE_SB_NS = 3600, TC_PAIR_SB_NS = 2900, TC6_PAIR_SB_NS = 4000;  // a super-block: 128 x 128, wide, pairs, Q6_K in pairs
 struct TcSplit {
     uint32_t left, parts;
 };
@@ -1102,15 +1102,21 @@ TcSplit tc_split(uint32_t tiles, uint32_t n_sb, uint32_t slots, uint32_t sb_ns, 
     return parts > 1 ? TcSplit{left, parts} : TcSplit{0, 1};
 }
 
-// Q6_K: whether 128 x 128 tiles of single CTAs are expected to finish before pairs, whose tiles, shared ones too, each take some 12 us beside their
-// 3.6 a super-block; 6 and 3.2 alone.  us, alone / pairs: 4096 x 512 x 384 26 / 33, 8192 x 1024 x 200 32 / 38, 14336 x 512 x 640 66 / 72; 4096 x 512 x 640
-// 41 / 35, 4096 x 2048 x 500 53 / 44.
-bool tc6_alone(uint32_t tiles, uint32_t m, uint32_t n_sb) {
-    const uint32_t sms = (uint32_t)sm_count(), slots = sms / 2, ones = tiles * ((m + TC_BN - 1) / TC_BN), pairs = (tiles + 1) / 2 * ((m + 2 * TC_BN - 1) / (2 * TC_BN));
-    const TcSplit s = tc_split(pairs, n_sb, slots, TC6_PAIR_SB_NS, 4 * TC_BN);
-    const uint32_t whole = s.left ? pairs / slots : (pairs + slots - 1) / slots, shared = s.left ? (s.left * s.parts + slots - 1) / slots : 0;
-    const uint64_t t_pairs = whole * (12000ull + 3600 * n_sb) + shared * (14000ull + 3600 * ((n_sb + s.parts - 1) / s.parts));
-    return (ones + sms - 1) / sms * (6000ull + 3200 * n_sb) <= t_pairs;
+// What a grid of tiles is expected to take, ns: rounds of whole tiles, each `tile_ns` and `sb_ns` a super-block, and one of shared tiles with the launch that
+// adds them up.
+uint64_t tc_expected(uint32_t tiles, uint32_t slots, TcSplit s, uint32_t n_sb, uint32_t tile_ns, uint32_t sb_ns) {
+    const uint32_t whole = s.left ? tiles / slots : (tiles + slots - 1) / slots, shared = s.left ? (s.left * s.parts + slots - 1) / slots : 0;
+    return whole * ((uint64_t)tile_ns + sb_ns * n_sb) + shared * ((uint64_t)tile_ns + 2000 + sb_ns * ((n_sb + s.parts - 1) / s.parts));
+}
+// Whether pairs of CTAs (256 x 256) are expected to finish no later than single ones: 128 x 256 or, with Q6_K, 128 x 128.  A pair costs more beside its
+// super-blocks, and an odd last token tile leaves half of one empty.  From products of 1 to 6 super-blocks; us, single CTAs / pairs: Q4_K 14336 x 256 x 500
+// 43 / 47, 14336 x 512 x 500 51 / 51, x 640 54 / 68, 14336 x 1536 x 640 88 / 93; Q6_K 4096 x 512 x 384 26 / 33, 8192 x 1024 x 200 32 / 38,
+// 14336 x 512 x 640 66 / 72, 4096 x 512 x 640 41 / 35, 4096 x 2048 x 500 53 / 44.
+bool tc_pairs(bool q6, uint32_t token_tiles, uint32_t y256, uint32_t y128, uint32_t n_sb) {
+    const uint32_t sms = (uint32_t)sm_count(), slots = sms / 2, pairs = (token_tiles + 1) / 2 * y256, ones = token_tiles * (q6 ? y128 : y256);
+    const uint64_t t_pairs = tc_expected(pairs, slots, tc_split(pairs, n_sb, slots, q6 ? TC6_PAIR_SB_NS : TC_PAIR_SB_NS, 4 * TC_BN), n_sb, 12000, q6 ? 3600 : 2600);
+    return t_pairs < (q6 ? tc_expected(ones, sms, {0, 1}, n_sb, 6000, 3200)
+                         : tc_expected(ones, sms, tc_split(ones, n_sb, sms, TC_WIDE_SB_NS, 2 * TC_BN), n_sb, 10000, 3600));
 }
 
 // img_bytes: the activation images.
@@ -1237,23 +1243,21 @@ int32_t launch_gemm_tc_multi(const GemmTarget *t, int count, const ActView &x, s
     const size_t img_bytes = (size_t)tiles * n_it * (2 * TC_OP_BYTES), min_bytes = (size_t)tiles * n_sb * TC_MINOP_BYTES,
                  xm_bytes = (size_t)tiles * n_mit * (2 * TCW_MINT_BYTES);
     const size_t need = img_bytes + min_bytes + xm_bytes + (size_t)n_pad * 8;
-    // With weight images: the wide kernel when its 128 x 256 tiles alone fill the device, in pairs unless they would leave a quarter of their tokens
-    // empty (one or three token tiles); else the 128 x 128 one.  Whole products, 128 x 128, wide, pairs: 28672 x 4096 x 512 255, 227, 204 us;
-    // 6144 x 2047 228, 222, 200; 4096 x 384 57, 52, 55; 4096 x 512 58, 60, 63.  Q6_K: tc6_alone.
+    // With weight images: the wide kernel when its 128 x 256 tiles alone fill the device, in pairs where they are faster; else the 128 x 128 one.  Whole products, 128 x 128, wide, pairs: 28672 x 4096 x 512 255, 227, 204 us;
+    // 6144 x 2047 228, 222, 200; 4096 x 384 57, 52, 55; 4096 x 512 58, 60, 63.  Q6_K: pairs or 128 x 128.
     static const int tile_pref = [] {
         const char *e = getenv("CERA_CUDA_GEMM_TILE");
         return e ? atoi(e) : 0;
     }();
-    uint32_t wide_y = 0;
-    for (int i = 0; i < count; ++i) wide_y += (t[i].w.m + 2 * TC_BN - 1) / (2 * TC_BN);
+    uint32_t wide_y = 0, y128 = 0;
+    for (int i = 0; i < count; ++i) wide_y += (t[i].w.m + 2 * TC_BN - 1) / (2 * TC_BN), y128 += (t[i].w.m + TC_BN - 1) / TC_BN;
     const bool q6 = w.type == CERA_TYPE_Q6_K, fills = tiles * wide_y >= 120;
-    const bool pair = q6 ? tile_pref != 128 && !tc6_alone(tiles, w.m, n_sb) : w.tc && tile_pref == 0 && fills && (tiles % 2 == 0 || tiles >= 5);
+    const bool pair = (q6 ? tile_pref != 128 : w.tc && tile_pref == 0 && fills) && tc_pairs(q6, tiles, wide_y, y128, n_sb);
     const bool wide = !pair && !q6 && w.tc && (tile_pref == 256 || (tile_pref != 128 && fills));
     const uint32_t rows = pair || wide ? 2 * TC_BN : TC_BN, halves = pair ? 2 : 1, x_tiles = (tiles + halves - 1) / halves;
     uint32_t y = 0;
     for (int i = 0; i < count; ++i) y += (t[i].w.m + rows - 1) / rows;
-    // (nanoseconds of a super-block, as measured: Q6_K in pairs, pairs, wide, 128 x 128)
-    const uint32_t sb_ns = q6 ? TC6_PAIR_SB_NS : pair ? 2900 : wide ? 3600 : 1650;
+    const uint32_t sb_ns = q6 ? TC6_PAIR_SB_NS : pair ? TC_PAIR_SB_NS : wide ? TC_WIDE_SB_NS : TC_SB_NS;
     TcSplit split = w.tc && (pair || !q6) ? tc_split(x_tiles * y, n_sb, (uint32_t)sm_count() / halves, sb_ns, halves * rows) : TcSplit{0, 1};
     // partial sums of the tiles that are shared; without room for them the tiles stay whole
     const size_t parts_bytes = (size_t)split.left * split.parts * halves * rows * TC_BM * 4;
