@@ -25,6 +25,51 @@ def test_pairs_equal_small_products(t, m, n, k):
     check(t, m, n, k)
 
 
+# three token tiles: 128 x 256 tiles of single CTAs, the last round shared
+@pytest.mark.parametrize("t", [O.Q4_K, O.Q5_K])
+def test_shared_tiles_of_single_wide_ctas(t):
+    check(t, 28670, 383, 2048)
+
+
+# one token tile of q, k and v together, every row tile shared along k: a weight's first tiles follow another's last, token-major
+@pytest.mark.parametrize("n", [100, 128])
+def test_shared_tiles_of_several_weights(n):
+    torch = need_gpu()
+    import cera_b200 as cb
+    from cera_b200.model import Role
+    width, kv, vocab = 4096, 1024, 256
+    model = cb.CudaModel(n_layers=1, hidden_size=width, intermediate_size=512, n_heads=32, n_kv_heads=8, head_dim=128, vocab_size=vocab, rope_theta=10000.0,
+                         rms_norm_eps=1e-5, rope_type=0, kv_f16=0, max_seq_len=n)
+    raw = {}
+    for role, rows, cols in ((Role.TOKEN_EMBD, vocab, width), (Role.OUTPUT, vocab, width), (Role.ATTN_Q, width, width), (Role.ATTN_K, kv, width), (Role.ATTN_V, kv, width),
+                             (Role.ATTN_OUTPUT, width, width), (Role.FFN_GATE, 512, width), (Role.FFN_UP, 512, width), (Role.FFN_DOWN, width, 512)):
+        raw[role] = cb.quantize_weights(O.Q4_K, cb.synth_normal(rows * cols, seed=int(role) + 1, sigma=0.02))
+        model.add_tensor(role, 0, O.Q4_K, rows, cols, raw[role])
+    ones = np.ones(width, dtype=np.float32)
+    for role in (Role.OUTPUT_NORM, Role.ATTN_NORM, Role.FFN_NORM):
+        model.add_tensor(role, 0, cb.types.F32, 1, width, ones)
+    torch.cuda.synchronize()
+    model.finalize()
+    tokens = (np.arange(n) * 7 % vocab).astype(np.uint32)
+    model.forward_prefill(tokens, 0)
+    k_got, v_got = (np.asarray(c).reshape(-1).view(np.float32).reshape(n, kv) for c in model.state_snapshot()["layers"][0])
+    model.close()
+    rows = cb.dequantize_rows(cb.QuantWeight(O.Q4_K, vocab, width, raw[Role.TOKEN_EMBD]))
+    weight = torch.ones(width, device="cuda")
+    pairs = lambda a: np.hypot(a[:, ::2].astype(np.float64), a[:, 1::2].astype(np.float64))  # noqa: E731  what the rotation leaves of keys
+    for role, got in ((Role.ATTN_K, pairs(k_got)), (Role.ATTN_V, v_got.astype(np.float64))):
+        w = cb.QuantWeight(O.Q4_K, kv, width, raw[role])
+        size = cb.dequantize_rows(w).double().norm(dim=1).cpu().numpy()
+        for j in (0, 1, 63, n - 1):
+            acts = cb.rmsnorm_q8_0(rows[int(tokens[j])].contiguous(), weight, 1e-5)[1]
+            want = cb.gemm_preq(w, acts)[:, 0].cpu().numpy()[None]
+            norm = float((acts.quants.view(-1, 32).double() * acts.scales.view(-1, 1).double()).norm())
+            bound = (2 * (width // 256 + 1) * 2.0 ** -24 + 2.0 ** -22) * size * norm  # as below
+            if role == Role.ATTN_K:  # two values, turned by a cosine and a sine of 24 bits
+                want, bound = pairs(want), (bound[::2] + bound[1::2]) + 2.0 ** -22 * (size[::2] + size[1::2]) * norm
+            assert (np.abs(got[j] - want[0]) <= bound).all(), (role, j)
+
+
 def check(t, m, n, k):
     torch = need_gpu()
     import cera_b200 as cb

@@ -94,17 +94,30 @@ def test_one_token_equals_the_first_of_two(t, experts, used, hidden, ff, softmax
     moe.close()
 
 
-@pytest.mark.parametrize("t", [O.Q4_K, O.Q5_K, O.Q6_K])
-@pytest.mark.parametrize("k", [256, 1280])
-@pytest.mark.parametrize("warps", [20, 21, 22, 32])  # warps of a CTA, around the line between the two register budgets
-def test_gemv_of_many_rows_equals_its_parts(t, k, warps):
+# rows an SM in eights, and the lone warps of a CTA that shared memory leaves: the line between the two register budgets lies at 21
+@pytest.mark.parametrize("t,k,share,warps", [(O.Q4_K, 512, 18, 18), (O.Q4_K, 512, 25, 25), (O.Q4_K, 1536, 32, 28), (O.Q5_K, 512, 21, 21), (O.Q5_K, 512, 22, 22),
+                                             (O.Q5_K, 1536, 32, 25), (O.Q6_K, 512, 18, 18), (O.Q6_K, 512, 22, 22), (O.Q6_K, 1536, 32, 21)])
+def test_gemv_of_many_rows_equals_its_parts(t, k, share, warps):
     torch = need_gpu()
     import cera_b200 as cb
-    m, part = torch.cuda.get_device_properties(0).multi_processor_count * 8 * warps - 3, 1000
-    raw = cb.quantize_weights(t, cb.synth_normal(m * k, seed=warps, sigma=0.02)).cpu().numpy()
+    assert _lone_warps(t, k, share) == warps
+    m, part = torch.cuda.get_device_properties(0).multi_processor_count * 8 * share - 3, 1000
+    raw = cb.quantize_weights(t, cb.synth_normal(m * k, seed=share, sigma=0.02)).cpu().numpy()
     x = torch.from_numpy(O.synth_normal(k, 5, 1.0)).cuda()
-    got = cb.gemv(cb.QuantWeight(t, m, k, raw), x).cpu().numpy()
+    w = cb.QuantWeight(t, m, k, raw)
+    got = cb.gemv(w, x).cpu().numpy()
+    assert_bits(cb.gemm_preq(w, cb.quantize_q8_0(x))[:, 0].cpu().numpy(), got, f"{O.NAMES[t]} quantized ahead")
     per_row = raw.size // m
     for a in (0, m // 2, m - part):
         rows = np.ascontiguousarray(raw.reshape(-1)[a * per_row:(a + part) * per_row])
         assert_bits(got[a:a + part], cb.gemv(cb.QuantWeight(t, part, k, rows), x).cpu().numpy(), f"{O.NAMES[t]} rows from {a}")
+
+
+def _lone_warps(t, k, share):
+    """The warps that the product in reference order gives a CTA: its share of the row groups, or what 224 KB hold beside the column."""
+    segment = {O.Q4_K: 2304, O.Q5_K: 2816, O.Q6_K: 3456}[t]
+    room = 224 * 1024 - (2112 + k + k // 32 * 8 + k // 16 * 4)
+    most = {s: min(32, room // (s * segment + 2 * 1024 + 2 * 640)) for s in (8, 4, 2)}
+    if share <= most[8] or share <= most[4]:
+        return share
+    return most[4] if 4 * most[4] >= 3 * min(share, 32) else min(share, most[2])
