@@ -3,7 +3,7 @@
 //
 // A CTA owns 128 queries of one head and walks tiles of 64 keys: S = Q K^T (a part against the head's or group's own keys
 // and, with latent attention, the rotated part against the shared rotated key; one accumulator), softmax on the CUDA cores in
-// f32, O += P V with P as a bf16 operand in shared memory and V stored transposed.  One warp loads by TMA, one issues
+// f32, O += P V with P as a bf16 operand in shared memory and V stored transposed.  One thread loads by TMA, one warp issues
 // MMAs, four warps do the softmax (thread = query).  S and P are double-buffered so that the next tile's scores are formed
 // during this tile's softmax.  O stays in TMEM and is rescaled only when a row's maximum has grown by more than 2^8.
 // Scores may be soft-capped.  A sink enters the denominator at the end; a head's gate multiplies the stored output (both

@@ -419,7 +419,8 @@ __global__ void __launch_bounds__(TC_BN) tc_weight_min_kernel(const WeightView w
 // The wide kernel, over resident images.  Alone a CTA does 128 tokens x TILES row tiles (of 128) of the image; in a PAIR (cta_group::2)
 // two CTAs do 256 tokens x 256 rows, each with its own 128 tokens and one of the row tiles, which the tensor cores of both read.
 // What bounds it: shared memory, which a CTA alone reads and writes 192 KB per 64 k (its 16 products of N = 128 take 1212 cycles in a ring without an
-// epilogue and 1370 with it, 1024 being the tensor core's rate), in a pair 112 KB; and then the chip's power, which holds the clock near 1.45 GHz.
+// epilogue and 1370 with it, 1024 being the tensor core's rate), in a pair 112 KB; and then the chip's power: in a loop of the first product
+// below the clock settles at 1.55 GHz (pairs) and 1.60 (alone), of the Q6_K one at 1.52, at 985 W with sw_power_cap.
 // 512 tokens: gate / up 28672 x 4096 212 us alone, 194 in pairs; Q6_K 4096 x 14336 168 us with 128 x 128 tiles, 119 in pairs.
 // TMEM holds nothing but the two double-buffered accumulators (2 x 256 columns), so
 //  * the running output lives in the epilogue threads' registers (thread = token lane x half of the tile's rows), and

@@ -1,4 +1,4 @@
-// tcgen05 / TMEM wrappers (one CTA, cta_group::1) shared by the tensor-core kernels.
+// tcgen05 / TMEM wrappers shared by the tensor-core kernels: one CTA (cta_group::1), and pairs of CTAs (cta_group::2).
 #pragma once
 
 #include "tma.cuh"
