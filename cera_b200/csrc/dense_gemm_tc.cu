@@ -292,7 +292,8 @@ int32_t launch_dense_gemm_tc(const DenseGemm &g, cudaStream_t st, bool *taken) {
     *taken = true;
     const bool unit = g.out_kind == DENSE_GATED_UNIT;
     // A pair of CTAs per tile where a tile has more than 64 columns - of experts, where they fill it on average: 52 columns an expert, width 2048, 60.5 us
-    // alone and 61.4 in pairs, 64 60.7 and 61.3, 96 67.9 and 67.0, 128 70.9 and 70.1 (width 4096 218 and 211), whole prompts even at 128 - unless the last pair of row tiles would leave more than an eighth of the work for rows that are not there.  2048 tokens at
+    // alone and 61.4 in pairs, 64 60.7 and 61.3, 96 67.9 and 67.0, 128 70.9 and 70.1 (width 4096 218 and 211), whole prompts even at 128 - unless the last pair of
+    // row tiles would leave more than an eighth of the work for rows that are not there.  2048 tokens at
     // width 4096, single CTAs and pairs: four layers of experts 4.22 and 4.05 ms, eight dense layers 6.65 and 6.36; 200 tokens through a gated unit 43.2
     // and 41.0 us (at up to 64 columns the weights are read once either way).
     const uint32_t rows = (g.tiles ? g.rows_per_expert : g.w.rows) / (unit ? 2 : 1), whole = (rows + DT_BM - 1) / DT_BM;
