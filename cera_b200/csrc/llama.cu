@@ -59,11 +59,10 @@ struct Layer {
 };
 
 constexpr size_t PREFILL_CHUNK = 512;
-// A prompt that needs only its last logits goes through the layers this many tokens at a time on one GPU.  Wider products have fewer
-// nearly empty last rounds of tiles (the 8B shape's gate and up matrices: 3.03 rounds paid as 4 at 512, 12.1 as 13 at 2048), and everything
-// else fewer launches.  Two layers, ms, chunks of 512 / 1024 / 2048 / 4096: width 1024 and 1000 tokens 1.29 / 0.87 / 0.87 / 0.86; 2047
-// tokens 2.78 / 2.06 / 1.55 / 1.55, width 4096 9.01 / 8.24 / 7.68 / 7.68; 4096 tokens 7.4 / 5.6 / 4.6 / 4.2, width 4096 24.0 / 21.8 / 20.6 /
-// 19.9, for twice the buffers (1.2 GB).
+// A prompt that needs only its last logits goes through the layers this many tokens at a time on one GPU: wider products have fewer rounds of tiles that do
+// not fill the device, everything else fewer launches.  Two layers, 2047 tokens, ms, chunks of 1024 / 2048: width 1024 and a feed-forward of 1024
+// 1.59 / 1.15, of 3584 1.80 / 1.35; width 4096 and 4096 4.70 / 4.36, 14336 6.37 / 6.04.  Chunks of 4096 made prompts of as many tokens a tenth
+// (width 1024) and a thirtieth shorter when the products were by single CTAs, for twice the buffers (1.2 GB).
 constexpr size_t PROMPT_CHUNK = 2048;
 
 struct LlamaModel : cera_cuda_model {
