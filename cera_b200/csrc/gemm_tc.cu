@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
         const uint8_t *sd0 = sub.tc + side + ((size_t)t0 * L.n_sb + tile.sb0) * side_step + (Q6 ? 0 : TC_MINOP_BYTES);  // d[128] of a super-block
         const uint8_t *sd1 = sub.tc + side + ((size_t)t1 * L.n_sb + tile.sb0) * side_step + (Q6 ? 0 : TC_MINOP_BYTES);
         const CUtensorMap *map_w = &maps.w[sub.index];
-        uint32_t it = 0;
+        uint32_t it = 0, slots = 0;  // stages and d slots asked for
         bool ok = true;
         // a stage that is free again; of a pair the even CTA announces what both ask for
         auto stage = [&](uint32_t bytes) {
@@ -578,6 +578,7 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
             if (sb >= 2) ok = tma::mbar_wait_warp(slot_free + (sb & 1), ((sb - 2) >> 1) & 1, abort_flag, &g_tc_status, 8u);
             if (!ok) return false;
             uint8_t *dv = tc_smem + S::DVAL + (sb & 1) * (S::ROWS * 4);
+            slots = sb + 1;
             tma::mbar_expect_tx_if(full_v + (sb & 1), S::ROWS * 4, me);
             tma::bulk_g2s_if(dv, f0, TC_BN * 4, full_v + (sb & 1), me);
             if constexpr (TILES == 2) tma::bulk_g2s_if(dv + TC_BN * 4, f1, TC_BN * 4, full_v + (sb & 1), me);
@@ -625,6 +626,8 @@ __global__ void __launch_bounds__(TCW_THREADS, 1) gemm_tcw_kernel(const TcParams
             uint64_t *last = PAIR ? empty_ab : full_ab;
             for (uint32_t i = it > (uint32_t)S::STAGES ? it - S::STAGES : 0; i < it; ++i)
                 for (uint32_t n = 0; n < tma::SPIN_LIMIT && !tma::mbar_test(last + i % S::STAGES, (i / S::STAGES) & 1); ++n) __nanosleep(40);
+            for (uint32_t i = slots > 2 ? slots - 2 : 0; i < slots; ++i)
+                for (uint32_t n = 0; n < tma::SPIN_LIMIT && !tma::mbar_test(full_v + (i & 1), (i >> 1) & 1); ++n) __nanosleep(40);
         }
     } else {
         // ---------------------------------------------------------------- epilogue: thread = (token lane, R rows of one image tile)

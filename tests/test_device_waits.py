@@ -48,3 +48,10 @@ def test_a_plain_arrival_at_another_cta_hands_over_tmem_only():
             seen += 1
             assert "tc_fence_before();" in text[:call.start()][-250:], name
     assert seen == 2
+
+
+def test_every_barrier_of_a_loaders_copies_is_waited_for():
+    """The wide prompt product has two: the stages' and the factors' (whose copies no stage's barrier counts)."""
+    body = dict(_sources())["gemm_tc.cu"].split("gemm_tcw_kernel(const TcParams")[1].split("__global__")[0]
+    drain = body[body.index("if (PAIR || *abort_flag)"):]
+    assert re.search(r"mbar_test\(last \+", drain) and re.search(r"mbar_test\(full_v \+", drain)
